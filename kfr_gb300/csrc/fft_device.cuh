@@ -382,7 +382,9 @@ __device__ __forceinline__ void dft_pfa(cpx<T>* v)
 template <typename T, int R>
 __device__ __forceinline__ void dft_codelet(cpx<T>* v)
 {
-    if constexpr (R == 2)
+    if constexpr (R == 1)
+        return;
+    else if constexpr (R == 2)
         dft2(v[0], v[1]);
     else if constexpr (R == 4)
         dft4(v[0], v[1], v[2], v[3]);

@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 
 #include "fft_desc.hpp"
+#include "rp.hpp"
 
 namespace kfr_gpu
 {
@@ -164,6 +165,37 @@ struct fourstep_args
     const void* rtw = nullptr;
     int ccs         = 1;
 };
+
+// Runtime-length kernels (rp_kernels.cu): contiguous signals, `spc` per CTA.
+struct rp_c2c_args
+{
+    const void* in;
+    void* out;
+    long long batch;
+    long long istride, ostride;
+    int inverse, spc;
+    const void* tw;
+    rp_desc d; // RP_SIGNALS
+};
+// Columns of row-major d.n x pitch arrays (RP_COLS; in the arrays' own layout; twA: the four-step twiddle of
+// N = d.n pitch points), or the pitch rows of d.n contiguous points of a four-step transform (RP_ROWS; output
+// k of row r to r + pitch k).  Arrays sig_stride apart.
+struct rp_strided_args
+{
+    const void* in;
+    void* out;
+    long long batch, sig_stride, pitch;
+    int conj_in, conj_out;
+    const void* tw;
+    const void* twA; // null: no twiddle
+    const void* twB;
+    int lbits;
+    rp_desc d;
+};
+template <typename T>
+cudaError_t launch_rp_c2c(const rp_c2c_args& a, int threads, int smem, cudaStream_t st);
+template <typename T>
+cudaError_t launch_rp_strided(const rp_strided_args& a, bool cols, int threads, int smem, cudaStream_t st);
 
 template <typename T>
 cudaError_t launch_c2c(const c2c_args& a, const block_cfg& c, cudaStream_t st);

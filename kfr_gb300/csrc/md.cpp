@@ -30,7 +30,10 @@ md_axes<T>::md_axes(const std::vector<long long>& cshape)
         a.inner = product(cshape, i + 1, d);
         a.outer = product(cshape, 0, i);
         a.tile  = 0;
-        if (block_program<T>::feasible(n))
+        a.rp.reset(new rp_program<T>());
+        if (a.rp->build(n, RP_COLS))
+            a.tile = a.rp->tiles[0].S;
+        else if (a.rp.reset(), block_program<T>::feasible(n))
         {
             a.prog.reset(new block_program<T>());
             a.prog->build(int(n), CT_FOURSTEP);
@@ -41,7 +44,7 @@ md_axes<T>::md_axes(const std::vector<long long>& cshape)
             if (t == 0)
                 a.prog.reset();
         }
-        if (!a.prog) // longer than one CTA: transposed 1-D pass
+        if (!a.prog && !a.rp) // longer than one CTA: transposed 1-D pass
             a.eng.reset(new complex_engine<T>(n));
         axes_.push_back(std::move(a));
     }
@@ -62,7 +65,9 @@ int md_axes<T>::launches(long long batch) const
 {
     int n = 0;
     for (const axis& a : axes_)
-        n += a.eng ? 2 + a.eng->launches(batch * a.outer * a.inner) : int((batch * a.outer + 65534) / 65535);
+        n += a.eng          ? 2 + a.eng->launches(batch * a.outer * a.inner)
+             : a.rp ? 1
+                            : int((batch * a.outer + 65534) / 65535);
     return n;
 }
 
@@ -79,6 +84,21 @@ void md_axes<T>::run(void* data, long long batch, bool inverse, void* scratch, c
             check(launch_transpose<T>(tr, data, batch * ax.outer, ax.n, ax.inner, st), "transpose axis");
             ax.eng->execute(tr, tr, batch * ax.outer * ax.inner, ax.n, ax.n, inverse, scr, st);
             check(launch_transpose<T>(data, tr, batch * ax.outer, ax.inner, ax.n, st), "transpose axis back");
+            continue;
+        }
+        if (ax.rp)
+        {
+            rp_strided_args a;
+            a.in         = data;
+            a.out        = data;
+            a.batch      = batch * ax.outer;
+            a.sig_stride = ax.n * ax.inner;
+            a.pitch      = ax.inner;
+            a.conj_in    = inverse;
+            a.conj_out   = inverse;
+            a.twA = a.twB = nullptr;
+            a.lbits      = 0;
+            ax.rp->run(a, st);
             continue;
         }
         const long long sigs = batch * ax.outer;
@@ -125,7 +145,8 @@ std::string md_axes<T>::describe() const
         if (a.eng)
             s << " axis{n=" << a.n << " inner=" << a.inner << " transposed [" << a.eng->describe() << "]}";
         else
-            s << " axis{n=" << a.n << " inner=" << a.inner << " tile=" << a.tile << " " << a.prog->describe() << "}";
+            s << " axis{n=" << a.n << " inner=" << a.inner << " tile=" << a.tile << " "
+              << (a.rp ? a.rp->describe() : a.prog->describe()) << "}";
     }
     return s.str();
 }

@@ -8,6 +8,7 @@
 #include <atomic>
 #include <cmath>
 #include <cstring>
+#include <map>
 #include <sstream>
 
 namespace kfr_gpu
@@ -278,6 +279,7 @@ static bool is_codelet(int r)
 {
     switch (r)
     {
+    case 1: // a copy (the ends of a runtime-length block FFT whose other radices are primes)
     case 2:
     case 3:
     case 4:
@@ -534,6 +536,95 @@ std::string block_program<T>::describe() const
 }
 
 // ------------------------------------------------------------------------------------------------------
+// rp_program
+// ------------------------------------------------------------------------------------------------------
+
+template <typename T>
+bool rp_program<T>::build(long long n, rp_layout lay)
+{
+    layout            = lay;
+    const int budget  = max_smem_bytes() - 1024;
+    const auto rad    = rp_radices(n);
+    if (rad.empty())
+        return false;
+    if (lay == RP_SIGNALS)
+    {
+        desc      = rp_build(rad, lay, 1, elem);
+        sig_elems = rp_smem_elems(desc, lay, 1);
+        shape     = rp_choose(desc, sig_elems, elem, budget);
+        if (!shape.spc)
+            return false;
+    }
+    else
+    {
+        for (int S = rp_tile(rad, lay, elem, budget); S >= 1 && tiles.size() < 3; S /= 2)
+        {
+            tile t;
+            t.d          = rp_build(rad, lay, S, elem);
+            t.S          = S;
+            t.smem       = rp_smem_elems(t.d, lay, S) * elem;
+            if (t.smem > budget) // more padding than rp_tile allows for
+                continue;
+            const int bf = S * t.d.pass[0].nbf;
+            t.threads    = (std::max(rp_threads_needed(t.d, S), std::min(bf, 256)) + 31) / 32 * 32;
+            tiles.push_back(t);
+        }
+        if (tiles.empty())
+            return false;
+    }
+    radices          = rad;
+    const auto table = pass_twiddles<T>(rad, nullptr);
+    tw.upload(table.data(), table.size() * sizeof(std::complex<T>));
+    return true;
+}
+
+template <typename T>
+void rp_program<T>::configure(rp_c2c_args& a, long long batch, int& threads, int& smem) const
+{
+    const rp_shape s = rp_shrink(desc, shape, batch, 152);
+    a.spc            = s.spc;
+    a.tw             = tw.get();
+    a.d              = desc;
+    threads          = s.threads;
+    smem             = s.spc * sig_elems * elem;
+}
+
+template <typename T>
+const typename rp_program<T>::tile& rp_program<T>::pick(long long count, long long batch) const
+{
+    // narrower tiles where the widest would leave SMs without a CTA, or lanes without a column
+    size_t i = 0;
+    while (i + 1 < tiles.size() &&
+           ((count + tiles[i].S - 1) / tiles[i].S * batch < 2 * 152 || tiles[i].S >= 2 * count))
+        i++;
+    return tiles[i];
+}
+
+template <typename T>
+void rp_program<T>::run(rp_strided_args& a, cudaStream_t st) const
+{
+    const tile& t = pick(a.pitch, a.batch);
+    a.d           = t.d;
+    a.tw          = tw.get();
+    check(launch_rp_strided<T>(a, layout == RP_COLS, t.threads, t.smem, st),
+          layout == RP_COLS ? "launch column DFTs" : "launch row DFTs");
+}
+
+template <typename T>
+std::string rp_program<T>::describe() const
+{
+    std::ostringstream s;
+    s << "block_fft radices=";
+    for (size_t i = 0; i < radices.size(); i++)
+        s << (i ? "x" : "") << radices[i];
+    if (layout == RP_SIGNALS)
+        s << " signals/CTA=" << shape.spc << " threads=" << shape.threads;
+    else
+        s << " tile=" << tiles[0].S << " threads=" << tiles[0].threads;
+    return s.str();
+}
+
+// ------------------------------------------------------------------------------------------------------
 // complex_engine
 // ------------------------------------------------------------------------------------------------------
 
@@ -657,8 +748,15 @@ complex_engine<T>::complex_engine(long long n) : n_(n)
     if (direct_ok && c_direct <= c_rader && c_direct <= c_blue)
     {
         k_ = kind::smem;
-        prog_.build(int(n), CT_C2C);
-        plan_pipe();
+        int ts = 0;
+        std::vector<int> ctr;
+        // lengths without a compile-time kernel: the runtime-length block FFT, or the in-place runtime
+        // passes where that has no plan (a prime factor of 17 to 127, too long for its threads)
+        if (ct_lookup<T>(CT_C2C, int(n), ts, ctr) || !rp_.build(n, RP_SIGNALS))
+        {
+            prog_.build(int(n), CT_C2C);
+            plan_pipe();
+        }
         return;
     }
     if (rader_ok && c_rader <= c_blue)
@@ -941,6 +1039,15 @@ bool complex_engine<T>::plan_fourstep(long long n)
     }
     if (best_n1 == 0)
         return false;
+    {
+        int ts = 0;
+        std::vector<int> ctr;
+        const bool pair = sizeof(T) == 4 && ct_lookup<T>(CT_FOURSTEP, int(best_n1), ts, ctr) &&
+                          ct_lookup<T>(CT_FOURSTEP, int(n / best_n1), ts, ctr) &&
+                          has_ct_fsp_f32(int(best_n1), int(n / best_n1));
+        if (!pair && plan_fourstep_rp(n))
+            return true;
+    }
     k_  = kind::fourstep;
     n1_ = best_n1;
     n2_ = n / best_n1;
@@ -978,6 +1085,13 @@ bool complex_engine<T>::plan_fourstep(long long n)
         err_.alloc(sizeof(int)); // the persistent tensor-copy pair kernels report a copy that never lands
         check(cudaMemset(err_.get(), 0, sizeof(int)), "clear error flag");
     }
+    upload_roots(n);
+    return true;
+}
+
+template <typename T>
+void complex_engine<T>::upload_roots(long long n)
+{
     // two-level table for W_N^m, m < N
     int lb = 0;
     while ((1LL << (2 * lb)) < n)
@@ -998,6 +1112,58 @@ bool complex_engine<T>::plan_fourstep(long long n)
     }
     twA_.upload(A.data(), A.size() * sizeof(std::complex<T>));
     twB_.upload(B.data(), B.size() * sizeof(std::complex<T>));
+}
+
+// Four-step split with both passes on the runtime-length block FFT: the cheapest passes per element, where a
+// tile narrower than a 128-byte row costs extra memory transactions.
+template <typename T>
+bool complex_engine<T>::plan_fourstep_rp(long long n)
+{
+    constexpr int elem = int(2 * sizeof(T));
+    const int budget   = max_smem_bytes() - 1024;
+    const auto cost    = [&](long long m, rp_layout lay) -> double
+    {
+        const auto rad = rp_radices(m);
+        if (rad.empty())
+            return -1;
+        const int S = rp_tile(rad, lay, elem, budget);
+        if (!S)
+            return -1;
+        double c = 0;
+        for (int r : rad)
+            c += rp_pass_cost(r);
+        // a row of S elements against the 128 bytes of a cache line
+        const double width = double(S * elem) / 128;
+        return c + (width >= 1 ? 0.0 : 12.0 * (1 / width - 1));
+    };
+    std::map<long long, double> ccost, rcost;
+    const auto cached = [&](std::map<long long, double>& m, long long v, rp_layout lay)
+    {
+        const auto f = m.find(v);
+        return f != m.end() ? f->second : m[v] = cost(v, lay);
+    };
+    double best = -1;
+    for (long long n1 = 8; n1 * 8 <= n && n1 <= (1 << 14); n1++)
+    {
+        if (n % n1 || n / n1 > (1 << 14))
+            continue;
+        const double c = cached(ccost, n1, RP_COLS), r = c < 0 ? -1 : cached(rcost, n / n1, RP_ROWS);
+        if (r < 0)
+            continue;
+        if (best < 0 || c + r < best)
+        {
+            best = c + r;
+            n1_  = n1;
+        }
+    }
+    if (best < 0 || !rp_cols_.build(n1_, RP_COLS) || !rp_rows_.build(n / n1_, RP_ROWS))
+    {
+        n1_ = 0;
+        return false;
+    }
+    n2_ = n / n1_;
+    k_  = kind::fourstep;
+    upload_roots(n);
     return true;
 }
 
@@ -1043,7 +1209,7 @@ int complex_engine<T>::launches(long long batch) const
             return (batch / pipe_spc_ > 0 ? 1 : 0) + (batch % pipe_spc_ ? 1 : 0);
         return 1;
     case kind::bluestein_smem: return 1;
-    case kind::fourstep: return 2 * int((batch + 65534) / 65535);
+    case kind::fourstep: return rp_cols_.ready() ? 2 : 2 * int((batch + 65534) / 65535);
     case kind::bluestein_multi: return 3 + 2 * inner_->launches(batch);
     case kind::rader_smem: return 1;
     case kind::tensor: return n1_ ? 2 * int((batch + 65534) / 65535) : 1;
@@ -1117,6 +1283,20 @@ void complex_engine<T>::execute(void* out, const void* in, long long batch, long
     }
     case kind::smem:
     {
+        if (rp_.ready())
+        {
+            rp_c2c_args a;
+            a.in      = in;
+            a.out     = out;
+            a.batch   = batch;
+            a.istride = istride;
+            a.ostride = ostride;
+            a.inverse = inverse;
+            int threads = 0, smem = 0;
+            rp_.configure(a, batch, threads, smem);
+            check(launch_rp_c2c<T>(a, threads, smem, st), "launch c2c");
+            return;
+        }
         c2c_args a;
         a.in      = in;
         a.out     = out;
@@ -1217,6 +1397,30 @@ void complex_engine<T>::execute(void* out, const void* in, long long batch, long
     {
         if (istride != n_ || ostride != n_)
             throw std::invalid_argument("internal: four-step needs contiguous signals");
+        if (rp_cols_.ready())
+        {
+            // x (n1 x n2) -> scratch (column DFTs times the twiddle, same layout) -> out[k1 + n1 k2]
+            rp_strided_args a;
+            a.batch      = batch;
+            a.sig_stride = n_;
+            a.in         = in;
+            a.out        = scratch;
+            a.pitch      = n2_;
+            a.conj_in    = inverse;
+            a.conj_out   = 0;
+            a.twA        = twA_.get();
+            a.twB        = twB_.get();
+            a.lbits      = lbits_;
+            rp_cols_.run(a, st);
+            a.in       = scratch;
+            a.out      = out;
+            a.pitch    = n1_;
+            a.conj_in  = 0;
+            a.conj_out = inverse;
+            a.twA = a.twB = nullptr;
+            rp_rows_.run(a, st);
+            return;
+        }
         // a pair kernel for this pass, or false when neither of them can run (the generic pass runs instead)
         const auto run_pair = [&](const fourstep_args& fa, bool cols)
         {
@@ -1339,6 +1543,11 @@ std::string complex_engine<T>::describe() const
           << " operands, FP32 accumulation";
         break;
     case kind::smem:
+        if (rp_.ready())
+        {
+            s << "smem n=" << n_ << " " << rp_.describe();
+            break;
+        }
         s << "smem " << prog_.describe();
         if (pipe_spc_)
             s << " pipelined spc=" << pipe_spc_;
@@ -1347,6 +1556,12 @@ std::string complex_engine<T>::describe() const
         break;
     case kind::bluestein_smem: s << "bluestein_smem n=" << n_ << " m=" << m_ << " [" << prog_.describe() << "]"; break;
     case kind::fourstep:
+        if (rp_cols_.ready())
+        {
+            s << "fourstep n=" << n_ << " = " << n1_ << " x " << n2_ << " cols[" << rp_cols_.describe() << "] rows["
+              << rp_rows_.describe() << "]";
+            break;
+        }
         s << "fourstep" << (pair_ ? " (compile-time pair)" : "") << " n=" << n_ << " = " << n1_ << " x " << n2_
           << " cols[" << pcols_.describe() << " tile=" << tile_c_ << "] rows[" << prows_.describe()
           << " tile=" << tile_r_ << "]";
@@ -1822,6 +2037,8 @@ template int tile_for<float>(const block_program<float>&, int);
 template int tile_for<double>(const block_program<double>&, int);
 template struct block_program<float>;
 template struct block_program<double>;
+template struct rp_program<float>;
+template struct rp_program<double>;
 template class complex_engine<float>;
 template class complex_engine<double>;
 template class real_engine<float>;

@@ -131,6 +131,37 @@ int smem_budget();
 template <typename T>
 int tile_for(const block_program<T>& p, int buffers = 1);
 
+// A length on the runtime-length block FFT (rp.hpp): radices, twiddles and layouts for a tile order.
+template <typename T>
+struct rp_program
+{
+    static constexpr int elem = int(2 * sizeof(T));
+    rp_layout layout = RP_SIGNALS;
+    std::vector<int> radices;
+    dbuf tw;
+    rp_desc desc{};
+    int sig_elems = 0; // RP_SIGNALS: shared elements per signal
+    rp_shape shape;
+    // RP_COLS / RP_ROWS: the widest tile and narrower ones for few columns or little work, widest first
+    struct tile
+    {
+        rp_desc d;
+        int S, threads, smem;
+    };
+    std::vector<tile> tiles;
+
+    // False (nothing built) when n has no such plan.
+    bool build(long long n, rp_layout layout);
+    bool ready() const { return !radices.empty(); }
+    // RP_SIGNALS: launch for `batch` signals (threads and dynamic shared memory returned, spc and d set).
+    void configure(rp_c2c_args& a, long long batch, int& threads, int& smem) const;
+    // RP_COLS / RP_ROWS: the tile for `count` columns or rows in `batch` arrays.
+    const tile& pick(long long count, long long batch) const;
+    // One strided launch (a.d, a.tw are set here).
+    void run(rp_strided_args& a, cudaStream_t st) const;
+    std::string describe() const;
+};
+
 template <typename T>
 class complex_engine
 {
@@ -191,6 +222,7 @@ private:
     kind k_ = kind::trivial;
     mutable bool host_io_ = false;
     block_program<T> prog_; // smem: length n; bluestein_smem: length m
+    rp_program<T> rp_;      // smem: lengths without a compile-time kernel
     // Bluestein
     long long m_ = 0;
     dbuf chirp_, bhat_;
@@ -201,6 +233,7 @@ private:
     int tile_c_ = 1, tile_r_ = 1;
     bool pp_c_ = false, pp_r_ = false; // ping-pong column / row passes
     bool pair_ = false;                 // both passes as fully compile-time pair kernels
+    rp_program<T> rp_cols_, rp_rows_;   // both passes on the runtime-length block FFT
     dbuf twA_, twB_;
     int lbits_ = 0;
     // pipelined smem path (compile-time lengths): signals per tile, 0 = not used
@@ -211,6 +244,8 @@ private:
     void init_bluestein(long long n);
     void init_rader(long long n);
     bool plan_fourstep(long long n);
+    bool plan_fourstep_rp(long long n);
+    void upload_roots(long long n);
     void plan_pipe();
     // tensor-core form (n1_, n2_, twA_, twB_, lbits_ as for the four-step when n > 4096)
     int tc_mode_ = 0;

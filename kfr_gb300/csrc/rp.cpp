@@ -1,0 +1,390 @@
+// Planner of the runtime-length block FFT (see rp.hpp).
+#include "rp.hpp"
+
+#include <algorithm>
+#include <cstring>
+#include <set>
+
+namespace kfr_gpu
+{
+
+double rp_pass_cost(int R)
+{
+    // real operations of the codelet per element, plus shared loads and stores, addresses, twiddle and its
+    // powers (11), the barrier (3) and the index arithmetic of a butterfly (25 instructions)
+    double ops;
+    if (R > kRpMaxRadix)
+        return 14 + 8.0 * R; // a dot product of R terms per output
+    switch (R)
+    {
+    case 1: ops = 0; break;
+    case 2: ops = 2; break;
+    case 3: ops = 5.3; break;
+    case 4: ops = 4; break;
+    case 5: ops = 8; break;
+    case 6: ops = 7.3; break;
+    case 7: ops = 9.5; break;
+    case 8: ops = 8; break;
+    case 9: ops = 12.4; break;
+    case 10: ops = 9.2; break;
+    case 11: ops = 13.6; break;
+    case 12: ops = 9.3; break;
+    case 13: ops = 15.7; break;
+    case 14: ops = 11.4; break;
+    case 15: ops = 12.5; break;
+    default: ops = 11; break;
+    }
+    return ops + 14 + 25.0 / R;
+}
+
+namespace
+{
+
+// every multiset of codelet radices <= `top` with product n, descending
+void splits(long long n, int top, std::vector<int>& cur, std::vector<std::vector<int>>& out)
+{
+    if (n == 1)
+    {
+        out.push_back(cur);
+        return;
+    }
+    if (int(cur.size()) >= kRpMaxPasses)
+        return;
+    for (int r = int(std::min<long long>(top, n)); r >= 2; r--)
+        if (n % r == 0)
+        {
+            cur.push_back(r);
+            splits(n / r, r, cur, out);
+            cur.pop_back();
+        }
+}
+
+// The largest radices in the middle (the in-place passes hold whole butterflies in registers, so their radix
+// bounds the threads a tile needs), the smallest last.
+std::vector<int> pass_order(const std::vector<int>& desc)
+{
+    if (desc.size() < 3)
+        return desc;
+    const size_t mid = desc.size() - 2;
+    std::vector<int> o(desc);
+    o[0] = desc[mid];
+    for (size_t i = 0; i < mid; i++)
+        o[i + 1] = desc[i];
+    return o;
+}
+
+uint32_t magic(int d) { return d <= 1 ? 0u : uint32_t((uint64_t(1) << 32) / uint32_t(d) + 1); }
+
+// Wavefronts beyond the minimum of one warp-wide shared access with the given lane addresses (elements of
+// `elem` bytes): 128 bytes are served at a time, so lanes go 128 / elem at a time.
+int conflicts(const int* addr, int lanes, int elem)
+{
+    const int per = 128 / elem;
+    int extra     = 0;
+    for (int b = 0; b < lanes; b += per)
+    {
+        const int e = std::min(lanes, b + per);
+        int count[16] = {}, worst = 1;
+        for (int i = b; i < e; i++)
+        {
+            bool dup = false;
+            for (int h = b; h < i && !dup; h++)
+                dup = addr[h] == addr[i];
+            if (!dup)
+                worst = std::max(worst, ++count[addr[i] % per]);
+        }
+        extra += worst - 1;
+    }
+    return extra;
+}
+
+struct lane_map
+{
+    int g, j;
+};
+lane_map map_lane(int J, const rp_pass& p, int shift)
+{
+    if (p.fast)
+        return { J & ((1 << shift) - 1), J >> shift };
+    return { J / p.nbf, J % p.nbf };
+}
+
+int store_conflicts(const rp_pass& p, int shift, int elem, int first, int total)
+{
+    int a[32], n = 0;
+    for (int J = first; J < std::min(first + 32, total); J++)
+    {
+        const lane_map m = map_lane(J, p, shift);
+        const int q = m.j / p.ns, k = m.j - q * p.ns;
+        a[n++] = k * p.st_e + q * p.st_q + m.g * p.st_g;
+    }
+    return n ? conflicts(a, n, elem) : 0;
+}
+int load_conflicts(const rp_pass& p, int shift, int elem, int first, int total)
+{
+    int a[32], n = 0;
+    for (int J = first; J < std::min(first + 32, total); J++)
+    {
+        const lane_map m = map_lane(J, p, shift);
+        const int q = m.j / p.ns;
+        a[n++] = m.j * p.ld_e + q * p.ld_q + m.g * p.ld_g;
+    }
+    return n ? conflicts(a, n, elem) : 0;
+}
+
+// The layout after pass i (and before pass i + 1): `pad` slots after every ns' elements.
+void set_layout(rp_desc& d, int i, int S, bool fast_layout, int pad)
+{
+    rp_pass& a   = d.pass[i];
+    rp_pass& b   = d.pass[i + 1];
+    const int e  = fast_layout ? S : 1;
+    const int nn = a.ns * a.radix; // ns'
+    const int sg = fast_layout ? 1 : d.n + d.n / nn * pad;
+    a.st_e = e;
+    a.st_q = nn * e + pad;
+    a.st_g = sg;
+    a.st_r = a.ns * e;
+    b.ld_e = e;
+    b.ld_q = pad;
+    b.ld_g = sg;
+    b.ld_r = b.nbf * e + b.nbf / nn * pad;
+}
+
+} // namespace
+
+std::vector<int> rp_radices(long long n, int largest)
+{
+    std::vector<int> r, primes;
+    if (n < 2 || n > (1 << 16))
+        return {};
+    for (int p = 17; p <= largest; p += 2)
+        while (n % p == 0 && p > 13)
+        {
+            primes.push_back(p); // composite p cannot divide: its factors are gone
+            n /= p;
+        }
+    std::vector<int> cur;
+    std::vector<std::vector<int>> all;
+    splits(n, kRpMaxRadix, cur, all);
+    double best = -1;
+    for (const auto& s : all)
+    {
+        const auto o = pass_order(s);
+        double c     = 0;
+        for (size_t i = 0; i < o.size(); i++)
+        {
+            c += rp_pass_cost(o[i]);
+            // more threads than a CTA of 1024 (or its half, for two of them per SM) to hold a middle pass
+            const bool middle = primes.empty() && i > 0 && i + 1 < o.size();
+            const long long t = middle ? (n / o[i] + rp_hold(o[i]) - 1) / rp_hold(o[i]) : 0;
+            c += t > 1024 ? 1000 : t > 512 ? 4 : 0;
+        }
+        if (best < 0 || c < best)
+        {
+            best = c;
+            r    = o;
+        }
+    }
+    if (best < 0)
+        return {};
+    if (!primes.empty())
+    {
+        // a codelet pass at either end, the primes in between
+        while (r.size() < 2)
+            r.push_back(1);
+        r.insert(r.begin() + 1, primes.begin(), primes.end());
+        if (r.size() > size_t(kRpMaxPasses))
+            return {};
+    }
+    return r;
+}
+
+rp_desc rp_build(const std::vector<int>& radices, rp_layout layout, int S, int elem, bool smem_io)
+{
+    rp_desc d;
+    std::memset(&d, 0, sizeof(d));
+    d.npass = int(radices.size());
+    d.n     = 1;
+    for (int r : radices)
+        d.n *= r;
+    while ((1 << d.shift) < S)
+        d.shift++;
+    int ns = 1, off = 0;
+    for (int i = 0; i < d.npass; i++)
+    {
+        rp_pass& p = d.pass[i];
+        p.radix    = radices[i];
+        p.ns       = ns;
+        p.nbf      = d.n / radices[i];
+        p.mq       = magic(ns);
+        p.mg       = magic(p.nbf);
+        p.fast     = layout == RP_COLS || (layout == RP_ROWS && i > 0);
+        p.tw_off   = off;
+        if (ns > 1)
+            off += ns * (radices[i] - 1);
+        p.wr_off = off;
+        if (radices[i] > kRpMaxRadix)
+            off += radices[i];
+        ns *= radices[i];
+    }
+    const bool fl = layout != RP_SIGNALS;
+    for (int i = 0; i + 1 < d.npass; i++)
+    {
+        const int nn  = d.pass[i].ns * d.pass[i].radix;
+        const int tot = fl ? S : 4;
+        int best = 0, best_c = -1;
+        for (int pad : { 0, 1, 2, 3, 4, 6, 8 })
+        {
+            if (pad * 4 > nn * (fl ? S : 1))
+                break;
+            set_layout(d, i, S, fl, pad);
+            const int ta = tot * d.pass[i].nbf, tb = tot * d.pass[i + 1].nbf;
+            int c = 0;
+            for (int w = 0; w < 3; w++)
+            {
+                const int fa = w * (ta / 3) / 32 * 32, fb = w * (tb / 3) / 32 * 32;
+                c += d.pass[i].radix * store_conflicts(d.pass[i], d.shift, elem, fa, ta);
+                c += d.pass[i + 1].radix * load_conflicts(d.pass[i + 1], d.shift, elem, fb, tb);
+            }
+            if (best_c < 0 || c < best_c)
+            {
+                best_c = c;
+                best   = pad;
+            }
+            if (c == 0)
+                break;
+        }
+        set_layout(d, i, S, fl, best);
+    }
+    if (d.npass > 0)
+    {
+        // the natural layout of a single pass, or of the ends of a transform from and to shared memory
+        rp_pass& f = d.pass[0];
+        rp_pass& l = d.pass[d.npass - 1];
+        if (smem_io || d.npass == 1)
+        {
+            const int e = fl ? S : 1, sg = fl ? 1 : d.n;
+            f.ld_e = e;
+            f.ld_q = 0;
+            f.ld_g = sg;
+            f.ld_r = f.nbf * e;
+            l.st_e = e;
+            l.st_q = d.n * e;
+            l.st_g = sg;
+            l.st_r = l.ns * e;
+        }
+    }
+    return d;
+}
+
+int rp_smem_elems(const rp_desc& d, rp_layout layout, int S, bool smem_io)
+{
+    int m = smem_io || d.npass == 1 ? (layout == RP_SIGNALS ? d.n : d.n * S) : 0;
+    for (int i = 0; i + 1 < d.npass; i++)
+    {
+        const rp_pass& p = d.pass[i];
+        const int groups = d.n / (p.ns * p.radix);
+        m                = std::max(m, groups * p.st_q);
+    }
+    return m;
+}
+
+int rp_threads_needed(const rp_desc& d, int nsig, bool smem_io)
+{
+    int t = 1;
+    for (int i = smem_io ? 0 : 1; i < d.npass - (smem_io ? 0 : 1); i++)
+    {
+        const int R = d.pass[i].radix;
+        const int h = R > kRpMaxRadix ? 1 : rp_hold(R);
+        // a prime pass holds 16 outputs per thread
+        t = std::max(t, R > kRpMaxRadix ? (nsig * d.n + 15) / 16 : (nsig * d.pass[i].nbf + h - 1) / h);
+    }
+    return t;
+}
+
+static double efficiency(const rp_desc& d, int spc, int threads)
+{
+    double useful = 0, spent = 0;
+    for (int i = 0; i < d.npass; i++)
+    {
+        const rp_pass& p = d.pass[i];
+        const double w   = rp_pass_cost(p.radix) * p.radix;
+        const int bf     = spc * p.nbf;
+        useful += w * bf;
+        spent += w * double((bf + threads - 1) / threads) * threads;
+    }
+    return useful / spent;
+}
+
+rp_shape rp_choose(const rp_desc& d, int sig_elems, int elem, int smem_budget, bool smem_io)
+{
+    // the most busy threads per SM: how evenly the passes' butterflies fill the threads times how many
+    // threads are resident (64 registers each), small CTAs first so that one CTA's barriers and global
+    // accesses overlap with others' work
+    rp_shape best;
+    double score   = 0;
+    const int maxt = rp_max_threads(elem);
+    int most = 1; // butterflies of a signal's largest pass
+    for (int i = 0; i < d.npass; i++)
+        most = std::max(most, d.pass[i].nbf);
+    for (int threads : { 64, 96, 128, 160, 192, 224, 256, 320, 384, 448, 512, 640, 768, 896, 1024 })
+        for (int spc = std::max(1, threads / (2 * most)), tried = 0; threads <= maxt && tried < 24; spc++, tried++)
+        {
+            if (rp_threads_needed(d, spc, smem_io) > threads)
+                break;
+            const long long smem = (long long)spc * sig_elems * elem;
+            if (smem > smem_budget || (spc > 1 && (long long)spc * d.n > 8LL * threads * 16 / 8))
+                break;
+            const int ctas     = std::min({ int((smem_budget + 1024) / (smem + 2048)), maxt / threads, 24 });
+            const int resident = std::max(1, ctas) * threads;
+            double s           = efficiency(d, spc, threads) * std::min(1.0, resident / (0.94 * maxt));
+            if (ctas < 3)
+                s *= ctas < 2 ? 0.75 : 0.92;
+            if (threads > 256)
+                s *= 0.97;
+            if (s > score * 1.01)
+            {
+                score = s;
+                best  = { spc, threads };
+            }
+        }
+    return best;
+}
+
+rp_shape rp_shrink(const rp_desc& d, const rp_shape& full, long long batch, int sms, bool smem_io)
+{
+    if (batch >= 2LL * sms * full.spc)
+        return full;
+    rp_shape s;
+    s.spc  = int(std::max<long long>(1, std::min<long long>(full.spc, batch / (2LL * sms))));
+    int bf = 1;
+    for (int i = 0; i < d.npass; i++)
+        bf = std::max(bf, s.spc * d.pass[i].nbf);
+    const int need = rp_threads_needed(d, s.spc, smem_io);
+    s.threads      = (std::max(need, std::min(bf, 512)) + 31) / 32 * 32;
+    return s;
+}
+
+int rp_tile(const std::vector<int>& radices, rp_layout layout, int elem, int smem_budget)
+{
+    (void)layout;
+    long long n = 1;
+    for (int r : radices)
+        n *= r;
+    int widest = 1; // butterflies per column the in-place passes hold at once, threads each
+    for (size_t i = 1; i + 1 < radices.size(); i++)
+    {
+        const int R = radices[i];
+        widest      = std::max<long long>(widest, R > kRpMaxRadix ? (n + 15) / 16
+                                                                  : (n / R + rp_hold(R) - 1) / rp_hold(R));
+    }
+    int S = 128 / elem;
+    while (n * 2 * S * elem <= 32 * 1024 && S < 64)
+        S *= 2;
+    for (; S >= 1; S /= 2)
+        if ((long long)S * widest <= rp_max_threads(elem) && n * S * elem / 16 * 17 <= smem_budget)
+            return S;
+    return 0;
+}
+
+} // namespace kfr_gpu

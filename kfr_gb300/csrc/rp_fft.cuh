@@ -1,0 +1,360 @@
+// Runtime-length block FFT over a tile of signals in one shared buffer (plans and layouts: rp.hpp).
+//
+// What bounds it: instruction issue.  A pass spends, per element, one shared load, one shared store, two
+// address steps, the codelet and a twiddle product whose power comes from one table value per butterfly
+// (binary powering), close to the compile-time passes: the butterfly's two addresses are computed once and
+// the rest are constant steps, with no padding arithmetic per element (rp.hpp), no per-signal thread groups
+// (the tile's butterflies are dealt to the threads in one sequence, so any radix keeps all threads busy) and
+// no register array carried across the radix switch.  The first pass reads its inputs through a functor
+// (global memory, with any pre-processing) and the last pass writes through one, so a transform of two passes
+// crosses shared memory once.  Middle passes are in place: each thread holds rp_hold(R) butterflies across
+// one barrier, which halves the shared memory of ping-pong buffers and so doubles the CTAs whose global
+// accesses overlap.  Figures: k_rp_c2c, k_rp_cols (rp_kernels.cu).
+#pragma once
+
+#include "fft_device.cuh"
+#include "rp.hpp"
+
+namespace kfr_gpu
+{
+
+struct rp_lane
+{
+    int g, j, q, k; // signal of the tile, butterfly, j = q ns + k
+};
+
+__device__ __forceinline__ rp_lane rp_map(const rp_pass& p, const int shift, const int J)
+{
+    rp_lane l;
+    if (p.fast)
+    {
+        l.g = J & ((1 << shift) - 1);
+        l.j = J >> shift;
+    }
+    else
+    {
+        l.g = p.mg ? int(__umulhi(uint32_t(J), p.mg)) : J;
+        l.j = J - l.g * p.nbf;
+    }
+    l.q = p.mq ? int(__umulhi(uint32_t(l.j), p.mq)) : l.j;
+    l.k = l.j - l.q * p.ns;
+    return l;
+}
+
+// v[r] *= W^{k r}, r = 4 a + b, as (W^{4 k})^a (W^k)^b from two table values: a table value's rounding error is
+// multiplied by its power, at most 3 here against R - 1 for the powers of one value, and fewer powers stay
+// live.
+template <typename T, int R>
+__device__ __forceinline__ void rp_powers(cpx<T> (&v)[R], const cpx<T> w1, const cpx<T> w4)
+{
+    const cpx<T> w2 = w1 * w1, w3 = w1 * w2;
+    v[1]            = v[1] * w1;
+    v[2]            = v[2] * w2;
+    v[3]            = v[3] * w3;
+    cpx<T> wa       = w4;
+#pragma unroll
+    for (int a = 4; a < R; a += 4)
+    {
+        if (a > 4)
+            wa = a == 8 ? w4 * w4 : wa * w4;
+        v[a] = v[a] * wa;
+        if (a + 1 < R)
+            v[a + 1] = v[a + 1] * (wa * w1);
+        if (a + 2 < R)
+            v[a + 2] = v[a + 2] * (wa * w2);
+        if (a + 3 < R)
+            v[a + 3] = v[a + 3] * (wa * w3);
+    }
+}
+
+template <typename T, int R>
+__device__ __forceinline__ void rp_twiddle(cpx<T> (&v)[R], const rp_pass& p, const cpx<T>* __restrict__ tw, const int k)
+{
+    if constexpr (R == 1)
+        return;
+    if (p.ns == 1)
+        return;
+    if constexpr (sizeof(T) == 4)
+    {
+        const cpx<T>* t = tw + p.tw_off + k;
+        if constexpr (R >= 8)
+            rp_powers<T, R>(v, ldg(t), ldg(t + 3 * p.ns));
+        else
+            twiddle_powers<T, R>(v, ldg(t));
+    }
+    else
+    {
+        // double precision: every power from the table (FP64 products are slow on this part)
+        const cpx<T>* t = tw + p.tw_off + k;
+#pragma unroll
+        for (int r = 1; r < R; r++)
+            v[r] = v[r] * ldg(t + (r - 1) * p.ns);
+    }
+}
+
+// Shared-memory ends of a pass.
+template <typename T>
+struct rp_smem
+{
+    cpx<T>* buf;
+    __device__ __forceinline__ cpx<T>* src(const rp_pass& p, const rp_lane& l) const
+    {
+        return buf + l.j * p.ld_e + l.q * p.ld_q + l.g * p.ld_g;
+    }
+    __device__ __forceinline__ cpx<T>* dst(const rp_pass& p, const rp_lane& l) const
+    {
+        return buf + l.k * p.st_e + l.q * p.st_q + l.g * p.st_g;
+    }
+};
+
+// First pass: inputs ld(g, i), outputs to shared memory.
+template <typename T, int R, class LD>
+__device__ __forceinline__ void rp_first(const rp_pass& p, const int shift, const int total, const rp_smem<T> sm,
+                                         const LD& ld)
+{
+    for (int J = threadIdx.x; J < total; J += blockDim.x)
+    {
+        const rp_lane l = rp_map(p, shift, J);
+        cpx<T> v[R];
+#pragma unroll
+        for (int r = 0; r < R; r++)
+            v[r] = ld(l.g, l.j + r * p.nbf);
+        dft_codelet<T, R>(v);
+        cpx<T>* d = sm.dst(p, l);
+#pragma unroll
+        for (int r = 0; r < R; r++)
+            d[r * p.st_r] = v[codelet_out<R>(r)];
+    }
+}
+
+// Last pass: inputs from shared memory; fin(g, k, step, o) sees the butterfly's outputs o[r] (output k + r step)
+// before st(g, i, x) stores them.
+template <typename T, int R, class ST, class FIN>
+__device__ __forceinline__ void rp_last(const rp_pass& p, const int shift, const int total, const rp_smem<T> sm,
+                                        const cpx<T>* __restrict__ tw, const ST& st, const FIN& fin)
+{
+    for (int J = threadIdx.x; J < total; J += blockDim.x)
+    {
+        const rp_lane l   = rp_map(p, shift, J);
+        const cpx<T>* s = sm.src(p, l);
+        cpx<T> v[R];
+#pragma unroll
+        for (int r = 0; r < R; r++)
+            v[r] = s[r * p.ld_r];
+        rp_twiddle<T, R>(v, p, tw, l.k);
+        dft_codelet<T, R>(v);
+        cpx<T> o[R];
+#pragma unroll
+        for (int r = 0; r < R; r++)
+            o[r] = v[codelet_out<R>(r)];
+        fin(l.g, l.k, p.ns, o);
+#pragma unroll
+        for (int r = 0; r < R; r++)
+            st(l.g, l.k + r * p.ns, o[r]);
+    }
+}
+
+// In-place pass: the thread's butterflies are held in registers across a barrier (rp_threads_needed).
+template <typename T, int R>
+__device__ __forceinline__ void rp_mid(const rp_pass& p, const int shift, const int total, const rp_smem<T> sm,
+                                       const cpx<T>* __restrict__ tw)
+{
+    constexpr int NB = rp_hold(R);
+    cpx<T> v[NB][R];
+#pragma unroll
+    for (int b = 0; b < NB; b++)
+    {
+        const int J = threadIdx.x + b * blockDim.x;
+        if (J < total)
+        {
+            const rp_lane l   = rp_map(p, shift, J);
+            const cpx<T>* s = sm.src(p, l);
+#pragma unroll
+            for (int r = 0; r < R; r++)
+                v[b][r] = s[r * p.ld_r];
+            rp_twiddle<T, R>(v[b], p, tw, l.k);
+            dft_codelet<T, R>(v[b]);
+        }
+        else
+        {
+            // defined on every path: otherwise ptxas takes the values of all radix cases as live around the
+            // pass loop and spills them (1500 bytes; 3600 points 20% slower)
+#pragma unroll
+            for (int r = 0; r < R; r++)
+                v[b][r] = mk<T>(0, 0);
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int b = 0; b < NB; b++)
+    {
+        const int J = threadIdx.x + b * blockDim.x;
+        if (J < total)
+        {
+            const rp_lane l = rp_map(p, shift, J);
+            cpx<T>* d     = sm.dst(p, l);
+#pragma unroll
+            for (int r = 0; r < R; r++)
+                d[r * p.st_r] = v[b][codelet_out<R>(r)];
+        }
+    }
+}
+
+// In-place pass of a prime radix above 13: the inputs are twiddled where they lie, then each thread holds up to
+// 16 outputs o = s nbf total + J, each a dot product of a butterfly's inputs with the roots W_R^{s r}.
+template <typename T>
+__device__ __forceinline__ void rp_prime(const rp_pass& p, const int shift, const int total, const rp_smem<T> sm,
+                                         const cpx<T>* __restrict__ tw)
+{
+    const int R = p.radix;
+    if (p.ns > 1)
+    {
+        for (int J = threadIdx.x; J < total; J += blockDim.x)
+        {
+            const rp_lane l = rp_map(p, shift, J);
+            cpx<T>* s     = sm.src(p, l);
+            const cpx<T>* t = tw + p.tw_off + l.k;
+#pragma unroll 1
+            for (int r = 1; r < R; r++)
+                s[r * p.ld_r] = s[r * p.ld_r] * ldg(t + (r - 1) * p.ns);
+        }
+        __syncthreads();
+    }
+    constexpr int E  = kRpMaxRadix;
+    const cpx<T>* wr = tw + p.wr_off;
+    cpx<T> v[E];
+#pragma unroll
+    for (int e = 0; e < E; e++)
+    {
+        const int o = threadIdx.x + e * blockDim.x;
+        const int q = o / total;
+        if (q < R)
+        {
+            const cpx<T>* s = sm.src(p, rp_map(p, shift, o - q * total));
+            cpx<T> acc      = s[0];
+            int m           = 0;
+#pragma unroll 1
+            for (int r = 1; r < R; r++)
+            {
+                m += q;
+                if (m >= R)
+                    m -= R;
+                acc = acc + s[r * p.ld_r] * ldg(wr + m);
+            }
+            v[e] = acc;
+        }
+        else
+            v[e] = mk<T>(0, 0);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < E; e++)
+    {
+        const int o = threadIdx.x + e * blockDim.x;
+        const int q = o / total;
+        if (q < R)
+            sm.dst(p, rp_map(p, shift, o - q * total))[q * p.st_r] = v[e];
+    }
+}
+
+#define KFR_GPU_RP_CODELETS(X) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16)
+#define KFR_GPU_RP_RADICES(X) X(1) KFR_GPU_RP_CODELETS(X) // the ends of a transform: radix 1 copies
+
+struct rp_no_fin
+{
+    template <class O>
+    __device__ __forceinline__ void operator()(int, int, int, O&) const
+    {
+    }
+};
+
+// The whole transform of `nsig` signals.  D: anything with n, npass, shift and pass[] (a kernel parameter, or a
+// copy in shared memory); every thread of the CTA takes part.  ld(g, i) reads input i of signal g, st(g, i, x)
+// takes output i.  Every input is read before the first output is stored when npass > 1 (or, for one pass,
+// by the thread that stores the signal's outputs), so the two may be the same memory.  Shared memory is free
+// again only after a barrier.
+template <typename T, class D, class LD, class ST, class FIN = rp_no_fin>
+__device__ __forceinline__ void rp_run(const D& d, cpx<T>* buf, const int nsig, const cpx<T>* __restrict__ tw,
+                                       const LD& ld, const ST& st, const FIN& fin = FIN())
+{
+    const rp_smem<T> sm{ buf };
+    const int np = d.npass, sh = d.shift;
+    {
+        const rp_pass& p = d.pass[0];
+        const int total  = nsig * p.nbf;
+        switch (p.radix)
+        {
+#define KFR_GPU_RP_CASE(R)                                                                                 \
+    case R: rp_first<T, R>(p, sh, total, sm, ld); break;
+            KFR_GPU_RP_RADICES(KFR_GPU_RP_CASE)
+#undef KFR_GPU_RP_CASE
+        default: break;
+        }
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int i = 1; i + 1 < np; i++)
+    {
+        const rp_pass& p = d.pass[i];
+        const int total  = nsig * p.nbf;
+        switch (p.radix)
+        {
+#define KFR_GPU_RP_CASE(R)                                                                                 \
+    case R: rp_mid<T, R>(p, sh, total, sm, tw); break;
+            KFR_GPU_RP_CODELETS(KFR_GPU_RP_CASE)
+#undef KFR_GPU_RP_CASE
+        default: rp_prime<T>(p, sh, total, sm, tw); break;
+        }
+        __syncthreads();
+    }
+    if (np == 1)
+    {
+        // one codelet: its outputs lie in natural order
+        const rp_pass& p = d.pass[0];
+        const int n      = p.radix;
+        for (int i = threadIdx.x; i < nsig * n; i += blockDim.x)
+        {
+            const int g = p.fast ? i & ((1 << sh) - 1) : i / n;
+            const int k = p.fast ? i >> sh : i - g * n;
+            cpx<T> o[1] = { buf[k * p.st_r + g * p.st_g] };
+            fin(g, k, 0, o);
+            st(g, k, o[0]);
+        }
+        return;
+    }
+    const rp_pass& p = d.pass[np - 1];
+    const int total  = nsig * p.nbf;
+    switch (p.radix)
+    {
+#define KFR_GPU_RP_CASE(R)                                                                                 \
+    case R: rp_last<T, R>(p, sh, total, sm, tw, st, fin); break;
+        KFR_GPU_RP_RADICES(KFR_GPU_RP_CASE)
+#undef KFR_GPU_RP_CASE
+    default: break;
+    }
+}
+
+// The transform from and to shared memory (natural order at both ends), every pass in place.  Ends with a
+// barrier.
+template <typename T, class D>
+__device__ __forceinline__ void rp_run_smem(const D& d, cpx<T>* buf, const int nsig, const cpx<T>* __restrict__ tw)
+{
+    const rp_smem<T> sm{ buf };
+#pragma unroll 1
+    for (int i = 0; i < d.npass; i++)
+    {
+        const rp_pass& p = d.pass[i];
+        const int total  = nsig * p.nbf;
+        switch (p.radix)
+        {
+#define KFR_GPU_RP_CASE(R)                                                                                 \
+    case R: rp_mid<T, R>(p, d.shift, total, sm, tw); break;
+            KFR_GPU_RP_CODELETS(KFR_GPU_RP_CASE)
+#undef KFR_GPU_RP_CASE
+        default: rp_prime<T>(p, d.shift, total, sm, tw); break;
+        }
+        __syncthreads();
+    }
+}
+
+} // namespace kfr_gpu

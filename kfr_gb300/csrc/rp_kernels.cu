@@ -1,0 +1,165 @@
+// Kernels on the runtime-length block FFT (rp_fft.cuh): contiguous complex signals, columns and rows of the
+// four-step transform, axes of multi-dimensional transforms.
+#include "launch.hpp"
+#include "rp_fft.cuh"
+
+namespace kfr_gpu
+{
+
+// four-step twiddle W_N^m = twA[m >> lbits] twB[m & mask]
+template <typename T>
+__device__ __forceinline__ cpx<T> rp_root(const cpx<T>* __restrict__ A, const cpx<T>* __restrict__ B, long long m,
+                                          int lbits)
+{
+    return ldg(A + (m >> lbits)) * ldg(B + (m & ((1LL << lbits) - 1)));
+}
+
+// ---------------------------------------------------------------------------------------------------
+// Complex DFT of contiguous signals whose length is a product of 2, 3, 5, 7, 11 and 13: one CTA per tile of
+// `spc` signals, the first pass reading and the last pass writing global memory with the lanes along the
+// signal (any 8-byte aligned pointers and strides), the CTAs of an SM overlapping one another's accesses.
+// Bound by instruction issue (about 25 instructions per element and pass).  4096 signals of 3600 points
+// (15 x 16 x 15, one signal per 256-thread CTA): 59 us, 59% of the HBM copy rate, against 207 us for k_c2c's
+// runtime passes; 2000 points (four passes) 40%, 100 points (two) 84%.
+// ---------------------------------------------------------------------------------------------------
+template <typename T>
+__global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T)), 1)
+    k_rp_c2c(const __grid_constant__ rp_c2c_args a)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const long long s0 = (long long)blockIdx.x * a.spc;
+    const int cnt      = int(a.batch - s0 < a.spc ? a.batch - s0 : a.spc);
+    const cpx<T>* in   = reinterpret_cast<const cpx<T>*>(a.in) + s0 * a.istride;
+    cpx<T>* out        = reinterpret_cast<cpx<T>*>(a.out) + s0 * a.ostride;
+    const bool inv     = a.inverse != 0;
+    rp_run<T>(
+        a.d, reinterpret_cast<cpx<T>*>(smem_raw), cnt, reinterpret_cast<const cpx<T>*>(a.tw),
+        [&](int g, int i) { return conj_if(in[g * a.istride + i], inv); },
+        [&](int g, int i, cpx<T> v) { out[g * a.ostride + i] = conj_if(v, inv); });
+}
+
+// ---------------------------------------------------------------------------------------------------
+// n-point DFTs down the columns of row-major n x pitch arrays, in the array's own layout: an axis of a
+// multi-dimensional transform, or (twiddle) the first pass of a four-step transform of N = n pitch points,
+// whose output k of column c is multiplied by W_N^{c k}.  A tile is S columns (128-byte rows where S allows);
+// lanes run along the columns, so global and shared accesses are contiguous with no transposition.
+// Bound by instruction issue and, for tiles of 4 or 8 columns, by the 32- and 64-byte rows.  Eight 1080 x 1920
+// complex arrays, both axes: 188 us against 373 us for k_fs_cols and k_c2c.
+// ---------------------------------------------------------------------------------------------------
+template <typename T>
+__global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T)), 1)
+    k_rp_cols(const __grid_constant__ rp_strided_args a)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int S       = 1 << a.d.shift;
+    const int tiles   = int((a.pitch + S - 1) >> a.d.shift);
+    const long long b = blockIdx.x / tiles;
+    const int c0      = int(blockIdx.x - b * tiles) << a.d.shift;
+    const cpx<T>* in  = reinterpret_cast<const cpx<T>*>(a.in) + b * a.sig_stride + c0;
+    cpx<T>* out       = reinterpret_cast<cpx<T>*>(a.out) + b * a.sig_stride + c0;
+    const cpx<T>* twA = reinterpret_cast<const cpx<T>*>(a.twA);
+    const cpx<T>* twB = reinterpret_cast<const cpx<T>*>(a.twB);
+    const int valid   = int(a.pitch - c0 < S ? a.pitch - c0 : S);
+    const bool cin = a.conj_in != 0, cout = a.conj_out != 0;
+    rp_run<T>(
+        a.d, reinterpret_cast<cpx<T>*>(smem_raw), S, reinterpret_cast<const cpx<T>*>(a.tw),
+        [&](int g, int i) { return g < valid ? conj_if(in[i * a.pitch + g], cin) : mk<T>(0, 0); },
+        [&](int g, int i, cpx<T> v)
+        {
+            if (g < valid)
+                out[i * a.pitch + g] = conj_if(v, cout);
+        },
+        [&](int g, int k, int step, auto& o)
+        {
+            if (!twA || g >= valid)
+                return;
+            constexpr int R     = int(sizeof(o) / sizeof(o[0]));
+            const long long col = c0 + g;
+            if constexpr (sizeof(T) == 4)
+            {
+                // W^{col k} times powers of the butterfly's step W^{col step}
+                if constexpr (R > 1)
+                    twiddle_powers<T, R>(o, rp_root(twA, twB, col * step, a.lbits));
+                const cpx<T> w = rp_root(twA, twB, col * k, a.lbits);
+#pragma unroll
+                for (int r = 0; r < R; r++)
+                    o[r] = o[r] * w;
+            }
+            else
+            {
+#pragma unroll
+                for (int r = 0; r < R; r++)
+                    o[r] = o[r] * rp_root(twA, twB, col * (k + (long long)r * step), a.lbits);
+            }
+        });
+}
+
+// ---------------------------------------------------------------------------------------------------
+// Second pass of a four-step transform of N = n1 n points: n-point DFTs along the n1 contiguous rows, output k
+// of row k1 to X[k1 + n1 k].  A tile is S rows: the first pass reads along the rows, the others run with the
+// lanes across the rows, so the stores cover S consecutive outputs; the transposition is the layout change
+// between the first two passes (RP_ROWS).  One complex<double> signal of 2^20 points, both kernels: 179 us
+// against 206 us for k_fs_cols and k_fs_rows (FP64 pipe, latency: one wave of CTAs).
+// ---------------------------------------------------------------------------------------------------
+template <typename T>
+__global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T)), 1)
+    k_rp_rows(const __grid_constant__ rp_strided_args a)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int S       = 1 << a.d.shift;
+    const int tiles   = int((a.pitch + S - 1) >> a.d.shift);
+    const long long b = blockIdx.x / tiles;
+    const int r0      = int(blockIdx.x - b * tiles) << a.d.shift;
+    const int n       = a.d.n;
+    const cpx<T>* in  = reinterpret_cast<const cpx<T>*>(a.in) + b * a.sig_stride + (long long)r0 * n;
+    cpx<T>* out       = reinterpret_cast<cpx<T>*>(a.out) + b * a.sig_stride + r0;
+    const int valid   = int(a.pitch - r0 < S ? a.pitch - r0 : S);
+    const bool cin = a.conj_in != 0, cout = a.conj_out != 0;
+    rp_run<T>(
+        a.d, reinterpret_cast<cpx<T>*>(smem_raw), S, reinterpret_cast<const cpx<T>*>(a.tw),
+        [&](int g, int i) { return g < valid ? conj_if(in[(long long)g * n + i], cin) : mk<T>(0, 0); },
+        [&](int g, int i, cpx<T> v)
+        {
+            if (g < valid)
+                out[i * a.pitch + g] = conj_if(v, cout);
+        });
+}
+
+// ---------------------------------------------------------------------------------------------------
+
+template <typename A>
+static cudaError_t rp_go(void (*kernel)(const A), const A& a, long long grid, int threads, int smem, cudaStream_t st)
+{
+    if (grid <= 0)
+        return cudaSuccess;
+    if (grid > 0x7fffffffLL)
+        return cudaErrorInvalidConfiguration;
+    if (smem > 48 * 1024)
+    {
+        const cudaError_t e = prepare_launch(reinterpret_cast<const void*>(kernel), threads, smem);
+        if (e != cudaSuccess)
+            return e;
+    }
+    kernel<<<unsigned(grid), threads, smem, st>>>(a);
+    return cudaGetLastError();
+}
+
+template <typename T>
+cudaError_t launch_rp_c2c(const rp_c2c_args& a, int threads, int smem, cudaStream_t st)
+{
+    return rp_go(k_rp_c2c<T>, a, (a.batch + a.spc - 1) / a.spc, threads, smem, st);
+}
+
+template <typename T>
+cudaError_t launch_rp_strided(const rp_strided_args& a, bool cols, int threads, int smem, cudaStream_t st)
+{
+    const long long tiles = (a.pitch + (1 << a.d.shift) - 1) >> a.d.shift;
+    return rp_go(cols ? k_rp_cols<T> : k_rp_rows<T>, a, tiles * a.batch, threads, smem, st);
+}
+
+template cudaError_t launch_rp_c2c<float>(const rp_c2c_args&, int, int, cudaStream_t);
+template cudaError_t launch_rp_c2c<double>(const rp_c2c_args&, int, int, cudaStream_t);
+template cudaError_t launch_rp_strided<float>(const rp_strided_args&, bool, int, int, cudaStream_t);
+template cudaError_t launch_rp_strided<double>(const rp_strided_args&, bool, int, int, cudaStream_t);
+
+} // namespace kfr_gpu
