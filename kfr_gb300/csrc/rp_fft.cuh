@@ -107,10 +107,11 @@ struct rp_smem
     }
 };
 
-// First pass: inputs ld(g, i), outputs to shared memory.
-template <typename T, int R, class LD>
+// First pass: inputs ld(g, i), outputs to shared memory; prep(g, j, step, v) sees a butterfly's inputs v[r]
+// (input j + r step) once all of them are loaded.
+template <typename T, int R, class LD, class PREP>
 __device__ __forceinline__ void rp_first(const rp_pass& p, const int shift, const int total, const rp_smem<T> sm,
-                                         const LD& ld)
+                                         const LD& ld, const PREP& prep)
 {
     for (int J = threadIdx.x; J < total; J += blockDim.x)
     {
@@ -119,6 +120,7 @@ __device__ __forceinline__ void rp_first(const rp_pass& p, const int shift, cons
 #pragma unroll
         for (int r = 0; r < R; r++)
             v[r] = ld(l.g, l.j + r * p.nbf);
+        prep(l.g, l.j, p.nbf, v);
         dft_codelet<T, R>(v);
         cpx<T>* d = sm.dst(p, l);
 #pragma unroll
@@ -257,10 +259,18 @@ __device__ __forceinline__ void rp_prime(const rp_pass& p, const int shift, cons
     }
 }
 
+// Element i of the array at p whose elements are `bytes` apart: one wide multiply-add.
+template <typename C>
+__device__ __forceinline__ C* rp_at(C* p, int i, uint32_t bytes)
+{
+    using B = std::conditional_t<std::is_const_v<C>, const char, char>;
+    return reinterpret_cast<C*>(reinterpret_cast<B*>(p) + (unsigned long long)(uint32_t(i)) * bytes);
+}
+
 #define KFR_GPU_RP_CODELETS(X) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(9) X(10) X(11) X(12) X(13) X(14) X(15) X(16)
 #define KFR_GPU_RP_RADICES(X) X(1) KFR_GPU_RP_CODELETS(X) // the ends of a transform: radix 1 copies
 
-struct rp_no_fin
+struct rp_no_hook
 {
     template <class O>
     __device__ __forceinline__ void operator()(int, int, int, O&) const
@@ -270,12 +280,14 @@ struct rp_no_fin
 
 // The whole transform of `nsig` signals.  D: anything with n, npass, shift and pass[] (a kernel parameter, or a
 // copy in shared memory); every thread of the CTA takes part.  ld(g, i) reads input i of signal g, st(g, i, x)
-// takes output i.  Every input is read before the first output is stored when npass > 1 (or, for one pass,
+// takes output i; work that depends on uniform flags belongs in the hooks (rp_first, rp_last), which run once
+// per butterfly.  Every input is read before the first output is stored when npass > 1 (or, for one pass,
 // by the thread that stores the signal's outputs), so the two may be the same memory.  Shared memory is free
 // again only after a barrier.
-template <typename T, class D, class LD, class ST, class FIN = rp_no_fin>
+template <typename T, class D, class LD, class ST, class FIN = rp_no_hook, class PREP = rp_no_hook>
 __device__ __forceinline__ void rp_run(const D& d, cpx<T>* buf, const int nsig, const cpx<T>* __restrict__ tw,
-                                       const LD& ld, const ST& st, const FIN& fin = FIN())
+                                       const LD& ld, const ST& st, const FIN& fin = FIN(),
+                                       const PREP& prep = PREP())
 {
     const rp_smem<T> sm{ buf };
     const int np = d.npass, sh = d.shift;
@@ -285,7 +297,7 @@ __device__ __forceinline__ void rp_run(const D& d, cpx<T>* buf, const int nsig, 
         switch (p.radix)
         {
 #define KFR_GPU_RP_CASE(R)                                                                                 \
-    case R: rp_first<T, R>(p, sh, total, sm, ld); break;
+    case R: rp_first<T, R>(p, sh, total, sm, ld, prep); break;
             KFR_GPU_RP_RADICES(KFR_GPU_RP_CASE)
 #undef KFR_GPU_RP_CASE
         default: break;

@@ -19,8 +19,8 @@ __device__ __forceinline__ cpx<T> rp_root(const cpx<T>* __restrict__ A, const cp
 // `spc` signals, the first pass reading and the last pass writing global memory with the lanes along the
 // signal (any 8-byte aligned pointers and strides), the CTAs of an SM overlapping one another's accesses.
 // Bound by instruction issue (about 25 instructions per element and pass).  4096 signals of 3600 points
-// (15 x 16 x 15, one signal per 256-thread CTA): 59 us, 59% of the HBM copy rate, against 207 us for k_c2c's
-// runtime passes; 2000 points (four passes) 40%, 100 points (two) 84%.
+// (15 x 16 x 15, one signal per 256-thread CTA): 56 us, 62% of the HBM copy rate, against 207 us for k_c2c's
+// runtime passes; 2000 points (four passes) 41%, 100 points (two) 88%.
 // ---------------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T)), 1)
@@ -34,8 +34,8 @@ __global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T)), 1)
     const bool inv     = a.inverse != 0;
     rp_run<T>(
         a.d, reinterpret_cast<cpx<T>*>(smem_raw), cnt, reinterpret_cast<const cpx<T>*>(a.tw),
-        [&](int g, int i) { return conj_if(in[g * a.istride + i], inv); },
-        [&](int g, int i, cpx<T> v) { out[g * a.ostride + i] = conj_if(v, inv); });
+        [&](int g, int i) { return conj_if(*rp_at(in + g * a.istride, i, sizeof(cpx<T>)), inv); },
+        [&](int g, int i, cpx<T> v) { *rp_at(out + g * a.ostride, i, sizeof(cpx<T>)) = conj_if(v, inv); });
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -44,7 +44,7 @@ __global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T)), 1)
 // whose output k of column c is multiplied by W_N^{c k}.  A tile is S columns (128-byte rows where S allows);
 // lanes run along the columns, so global and shared accesses are contiguous with no transposition.
 // Bound by instruction issue and, for tiles of 4 or 8 columns, by the 32- and 64-byte rows.  Eight 1080 x 1920
-// complex arrays, both axes: 188 us against 373 us for k_fs_cols and k_c2c.
+// complex arrays, both axes: 173 us against 373 us for k_fs_cols and k_c2c.
 // ---------------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T)), 1)
@@ -59,22 +59,20 @@ __global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T)), 1)
     cpx<T>* out       = reinterpret_cast<cpx<T>*>(a.out) + b * a.sig_stride + c0;
     const cpx<T>* twA = reinterpret_cast<const cpx<T>*>(a.twA);
     const cpx<T>* twB = reinterpret_cast<const cpx<T>*>(a.twB);
-    const int valid   = int(a.pitch - c0 < S ? a.pitch - c0 : S);
-    const bool cin = a.conj_in != 0, cout = a.conj_out != 0;
+    // lanes beyond the last column repeat it: they read the same values and store the same results
+    const int last  = int(a.pitch - c0 < S ? a.pitch - c0 : S) - 1;
+    const bool cin  = a.conj_in != 0, cout = a.conj_out != 0;
+    const uint32_t bytes = uint32_t(a.pitch * sizeof(cpx<T>));
     rp_run<T>(
         a.d, reinterpret_cast<cpx<T>*>(smem_raw), S, reinterpret_cast<const cpx<T>*>(a.tw),
-        [&](int g, int i) { return g < valid ? conj_if(in[i * a.pitch + g], cin) : mk<T>(0, 0); },
-        [&](int g, int i, cpx<T> v)
-        {
-            if (g < valid)
-                out[i * a.pitch + g] = conj_if(v, cout);
-        },
+        [&](int g, int i) { return conj_if(*rp_at(in + min(g, last), i, bytes), cin); },
+        [&](int g, int i, cpx<T> v) { *rp_at(out + min(g, last), i, bytes) = conj_if(v, cout); },
         [&](int g, int k, int step, auto& o)
         {
-            if (!twA || g >= valid)
+            if (!twA)
                 return;
             constexpr int R     = int(sizeof(o) / sizeof(o[0]));
-            const long long col = c0 + g;
+            const long long col = c0 + min(g, last);
             if constexpr (sizeof(T) == 4)
             {
                 // W^{col k} times powers of the butterfly's step W^{col step}
@@ -113,16 +111,14 @@ __global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T)), 1)
     const int n       = a.d.n;
     const cpx<T>* in  = reinterpret_cast<const cpx<T>*>(a.in) + b * a.sig_stride + (long long)r0 * n;
     cpx<T>* out       = reinterpret_cast<cpx<T>*>(a.out) + b * a.sig_stride + r0;
-    const int valid   = int(a.pitch - r0 < S ? a.pitch - r0 : S);
-    const bool cin = a.conj_in != 0, cout = a.conj_out != 0;
+    // lanes beyond the last row repeat it
+    const int last  = int(a.pitch - r0 < S ? a.pitch - r0 : S) - 1;
+    const bool cin  = a.conj_in != 0, cout = a.conj_out != 0;
+    const uint32_t bytes = uint32_t(a.pitch * sizeof(cpx<T>));
     rp_run<T>(
         a.d, reinterpret_cast<cpx<T>*>(smem_raw), S, reinterpret_cast<const cpx<T>*>(a.tw),
-        [&](int g, int i) { return g < valid ? conj_if(in[(long long)g * n + i], cin) : mk<T>(0, 0); },
-        [&](int g, int i, cpx<T> v)
-        {
-            if (g < valid)
-                out[i * a.pitch + g] = conj_if(v, cout);
-        });
+        [&](int g, int i) { return conj_if(*rp_at(in + (long long)min(g, last) * n, i, sizeof(cpx<T>)), cin); },
+        [&](int g, int i, cpx<T> v) { *rp_at(out + min(g, last), i, bytes) = conj_if(v, cout); });
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -153,6 +149,8 @@ cudaError_t launch_rp_c2c(const rp_c2c_args& a, int threads, int smem, cudaStrea
 template <typename T>
 cudaError_t launch_rp_strided(const rp_strided_args& a, bool cols, int threads, int smem, cudaStream_t st)
 {
+    if (a.pitch * (long long)(2 * sizeof(T)) > 0xffffffffLL) // the kernels step by 32-bit byte pitches
+        return cudaErrorInvalidValue;
     const long long tiles = (a.pitch + (1 << a.d.shift) - 1) >> a.d.shift;
     return rp_go(cols ? k_rp_cols<T> : k_rp_rows<T>, a, tiles * a.batch, threads, smem, st);
 }

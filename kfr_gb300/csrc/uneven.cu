@@ -2,6 +2,7 @@
 // (uneven.hpp).
 #include "uneven.hpp"
 #include "kernels.cuh"
+#include "rp_fft.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -35,21 +36,31 @@ __device__ __forceinline__ cpx<double> ld_cg(const cpx<double>* p)
     return mk<double>(v.x, v.y);
 }
 
+// The persistent kernel on the runtime-length block FFT (rp_fft.cuh).  Every item is a tile of signals, columns
+// or rows whose element i of signal g lies at base[g] + i stride, so one instance of the passes serves all
+// of them; the first pass reads and the last pass writes global memory, with the chirps, the spectrum product
+// and the four-step twiddle in its functors.  Four 256-thread CTAs per SM (64 registers; two of 512 threads
+// for plans with passes longer than 4096 points), so that one's queue round trip, loads and barriers overlap
+// with the others' arithmetic.  Bound by instruction issue and by the latency of an item's chain (queue, job,
+// loads, barriers).  1024 signals of 64 to 65536 points: 384 us against 746 us for runtime passes of 690
+// instructions per element in one 512-thread CTA per SM; with 16-wide tiles of every length (items of 256
+// elements) 804 us, with per-element tests for the padding and the last column 440 us.
 template <typename T>
-__global__ void __launch_bounds__(kUnevenThreads, 1) k_uneven(const uneven_launch a)
+__global__ void __launch_bounds__(kUnevenThreads, 2) k_uneven(const __grid_constant__ uneven_launch a)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ pass_desc sp[kMaxPasses];
-    __shared__ long long s_off[kUnevenMaxSpc];
+    __shared__ rp_desc D;
+    // input and output 0 of each signal of the tile, and its column / row
+    __shared__ const cpx<T>* s_src[kUnevenMaxSpc];
+    __shared__ cpx<T>* s_dst[kUnevenMaxSpc];
+    __shared__ int s_col[kUnevenMaxSpc];
+    // the last input and the first output index outside a Bluestein transform's signal
+    __shared__ int s_ilim[kUnevenMaxSpc], s_olim[kUnevenMaxSpc];
     __shared__ uneven_job J;
-    __shared__ int s_item, s_count, s_first, s_fft, s_m, s_ts, s_stride, s_npass;
-    __shared__ fast_div s_div;
-    __shared__ const cpx<T>* s_tw;
+    __shared__ uneven_item W;
+    __shared__ int s_item, s_fft;
     cpx<T>* sm = reinterpret_cast<cpx<T>*>(smem_raw);
-    const cpx<T>* gin = reinterpret_cast<const cpx<T>*>(a.in);
-    cpx<T>* gout      = reinterpret_cast<cpx<T>*>(a.out);
-    cpx<T>* gscr      = reinterpret_cast<cpx<T>*>(a.scratch);
-    const bool inv    = a.inverse != 0;
+    const bool inv = a.inverse != 0;
     if (threadIdx.x == 0)
         s_fft = -1;
     for (;;)
@@ -61,23 +72,8 @@ __global__ void __launch_bounds__(kUnevenThreads, 1) k_uneven(const uneven_launc
             s_item       = it;
             if (it < a.nitems)
             {
-                const uneven_item w = a.items[it];
-                J                   = a.jobs[w.job];
-                s_count             = w.count;
-                s_first             = w.first;
-                if (J.fft != s_fft)
-                {
-                    const uneven_fft& F = a.ffts[J.fft];
-                    s_fft    = J.fft;
-                    s_m      = F.m;
-                    s_ts     = F.ts;
-                    s_stride = F.stride;
-                    s_npass  = F.d.npass;
-                    s_div    = F.div_m;
-                    s_tw     = reinterpret_cast<const cpx<T>*>(F.tw);
-                    for (int p = 0; p < F.d.npass; p++)
-                        sp[p] = F.d.pass[p];
-                }
+                W = a.items[it];
+                J = a.jobs[W.job];
                 if (J.wait >= 0)
                 {
                     // every tile of the stage waited for was dequeued before this one and runs on a resident
@@ -96,160 +92,127 @@ __global__ void __launch_bounds__(kUnevenThreads, 1) k_uneven(const uneven_launc
             }
         }
         __syncthreads();
-        const int it = s_item;
-        if (it >= a.nitems)
+        if (s_item >= a.nitems)
             break;
-        const int mode = J.mode, cnt = s_count, m = s_m, stride = s_stride;
-        if (mode <= UM_BLUE1)
+        const int mode = J.mode, cnt = W.count, first = W.first;
+        const int n1 = J.n1, n2 = J.n2;
+        if (J.fft != s_fft)
         {
-            if (int(threadIdx.x) < cnt)
-                s_off[threadIdx.x] = a.offsets[s_first + threadIdx.x];
-            __syncthreads();
-            const int n = J.n;
-            const fast_div dm   = s_div;
-            const cpx<T>* chirp = mode == UM_BLUE1 ? reinterpret_cast<const cpx<T>*>(J.chirp) : nullptr;
-#pragma unroll 4
+            const int* src = reinterpret_cast<const int*>(&a.ffts[J.fft].d);
+            for (int i = threadIdx.x; i < int(sizeof(rp_desc) / sizeof(int)); i += blockDim.x)
+                reinterpret_cast<int*>(&D)[i] = src[i];
+        }
+        if (int(threadIdx.x) < cnt)
+        {
+            const cpx<T>* src = reinterpret_cast<const cpx<T>*>(J.src == 0 ? a.in : J.src == 1 ? a.out : a.scratch) + J.src_off;
+            cpx<T>* dst       = reinterpret_cast<cpx<T>*>(J.dst == 2 ? a.scratch : a.out) + J.dst_off;
+            const int g       = threadIdx.x;
+            // columns and rows beyond the last repeat it: they read the same values and store the same results
+            const int c = mode <= UM_BLUE1 ? 0 : min(first + g, (mode == UM_COL ? n2 : n1) - 1);
+            const long long b = mode <= UM_BLUE1 ? a.offsets[first + g] : c;
+            const int nv      = int(J.nvalid);
+            s_src[g]          = src + (mode == UM_ROW ? (long long)c * n2 : J.pre ? min(c, nv - 1) : b);
+            s_dst[g]          = dst + b;
+            s_col[g]          = c;
+            s_ilim[g]         = J.pre ? max(nv - 1 - c, 0) / n2 : 0x7fffffff;
+            s_olim[g]         = J.post == 2 ? (max(nv - c, 0) + n1 - 1) / n1 : 0x7fffffff;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0)
+            s_fft = J.fft;
+        const cpx<T>* tw    = reinterpret_cast<const cpx<T>*>(a.ffts[J.fft].tw);
+        const cpx<T>* chirp = reinterpret_cast<const cpx<T>*>(J.chirp);
+        const cpx<T>* bhat  = reinterpret_cast<const cpx<T>*>(J.bhat);
+        if (mode == UM_BLUE1)
+        {
+            // one-CTA Bluestein: both transforms from and to shared memory
+            const int m = D.n, n = J.n;
             for (int i = threadIdx.x; i < cnt * m; i += blockDim.x)
             {
-                const int s = int(fdiv(uint32_t(i), dm));
-                const int e = i - s * m;
-                cpx<T> v    = mk<T>(0, 0);
-                if (e < n)
-                {
-                    v = conj_if(gin[s_off[s] + e], inv);
-                    if (chirp)
-                        v = v * ldg(chirp + e);
-                }
-                sm[s * stride + pidx<T>(e)] = v;
+                const int g = i / m, e = i - g * m;
+                sm[i]       = e < n ? conj_if(ld_cg(s_src[g] + e), inv) * ldg(chirp + e) : mk<T>(0, 0);
+            }
+            __syncthreads();
+#pragma unroll 1
+            for (int round = 0;; round++)
+            {
+                rp_run_smem<T>(D, sm, cnt, tw);
+                if (round)
+                    break;
+                for (int i = threadIdx.x; i < cnt * m; i += blockDim.x)
+                    sm[i] = conj(sm[i] * ldg(bhat + i % m));
+                __syncthreads();
+            }
+            for (int i = threadIdx.x; i < cnt * n; i += blockDim.x)
+            {
+                const int g = i / n, e = i - g * n;
+                s_dst[g][e] = conj_if(conj(sm[g * m + e]) * ldg(chirp + e), inv);
             }
         }
         else
         {
-            // a tile of `cnt` (a power of two) columns (COL) or rows (ROW) of a four-step transform
-            const int S = cnt, sh = 31 - __clz(cnt);
-            const int n1 = J.n1, n2 = J.n2, c0 = s_first;
-            const cpx<T>* src = (J.src == 0 ? gin : J.src == 1 ? gout : gscr) + J.src_off;
-            const bool cj     = J.first && inv;
-            if (mode == UM_COL)
-            {
-                const cpx<T>* chirp = J.pre ? reinterpret_cast<const cpx<T>*>(J.chirp) : nullptr;
-                const long long nv  = J.nvalid;
-#pragma unroll 4
-                for (int i = threadIdx.x; i < S * m; i += blockDim.x)
+            const bool cin = J.first && inv, cout = J.last && inv;
+            // bytes between a signal's input / output elements; elements between them
+            const int is = mode == UM_COL ? n2 : 1, os = mode == UM_COL ? n2 : mode == UM_ROW ? n1 : 1;
+            const uint32_t isb = uint32_t(is) * sizeof(cpx<T>), osb = uint32_t(os) * sizeof(cpx<T>);
+            const int nv = int(J.nvalid), pre = J.pre, post = J.post;
+            rp_run<T>(
+                D, sm, cnt, tw,
+                [&](int g, int i)
                 {
-                    const int j1 = i >> sh, c = i & (S - 1), col = c0 + c;
-                    const long long g = (long long)j1 * n2 + col;
-                    cpx<T> v          = mk<T>(0, 0);
-                    if (col < n2 && (!chirp || g < nv))
+                    // the zero padding repeats a column's last value (prep clears it)
+                    return conj_if(ld_cg(rp_at(s_src[g], min(i, s_ilim[g]), isb)), cin);
+                },
+                [&](int g, int i, cpx<T> v)
+                {
+                    if (i < s_olim[g])
+                        *rp_at(s_dst[g], i, osb) = conj_if(v, cout);
+                },
+                [&](int g, int k, int step, auto& o)
+                {
+                    constexpr int R = int(sizeof(o) / sizeof(o[0]));
+                    const int col   = s_col[g];
+                    if (post)
                     {
-                        v = J.src == 2 ? ld_cg(src + g) : src[g];
-                        v = conj_if(v, cj);
-                        if (chirp)
-                            v = v * ldg(chirp + g);
+                        // 1: conj(v bhat), 2: conj(v) chirp, conjugated once more for the inverse
+#pragma unroll
+                        for (int r = 0; r < R; r++)
+                        {
+                            const int e = col + (k + r * step) * os;
+                            if (post == 1)
+                                o[r] = conj(o[r] * ldg(bhat + e));
+                            else if (e < nv)
+                                o[r] = conj(o[r]) * ldg(chirp + e);
+                        }
                     }
-                    sm[c * stride + pidx<T>(j1)] = v;
-                }
-            }
-            else
-            {
-#pragma unroll 4
-                for (int i = threadIdx.x; i < S * m; i += blockDim.x)
+                    if (mode != UM_COL)
+                        return;
+                    // four-step twiddle: W^{col k} times powers of the butterfly's step W^{col step}; col k and
+                    // col step are below the length, at most 8192^2
+                    const cpx<T>* twA = reinterpret_cast<const cpx<T>*>(J.twA);
+                    const cpx<T>* twB = reinterpret_cast<const cpx<T>*>(J.twB);
+                    const int lbits   = J.lbits, mask = (1 << lbits) - 1;
+                    const auto root = [&](int m) { return ldg(twA + (m >> lbits)) * ldg(twB + (m & mask)); };
+                    if constexpr (R > 1)
+                        twiddle_powers<T, R>(o, root(col * step));
+                    const cpx<T> w = root(col * k);
+#pragma unroll
+                    for (int r = 0; r < R; r++)
+                        o[r] = o[r] * w;
+                },
+                [&](int g, int j, int step, auto& v)
                 {
-                    const int n2i = i >> sh, r = i & (S - 1), row = c0 + r;
-                    cpx<T> v      = mk<T>(0, 0);
-                    if (row < n1)
+                    if (!pre)
+                        return;
+                    // Bluestein's chirp, zero beyond the signal
+                    constexpr int R = int(sizeof(v) / sizeof(v[0]));
+#pragma unroll
+                    for (int r = 0; r < R; r++)
                     {
-                        const long long g = (long long)n2i * n1 + row;
-                        v = J.src == 2 ? ld_cg(src + g) : src[g];
-                        v = conj_if(v, cj);
+                        const int e = s_col[g] + (j + r * step) * is;
+                        v[r]        = e < nv ? v[r] * ldg(chirp + e) : mk<T>(0, 0);
                     }
-                    sm[r * stride + pidx<T>(n2i)] = v;
-                }
-            }
-        }
-        // one FFT call site, run twice for a one-CTA Bluestein tile (times the kernel spectrum in between)
-        for (int round = 0;; round++)
-        {
-            __syncthreads();
-            {
-                const group_map gm(s_ts, cnt);
-                block_fft<T, 16>(sm + gm.g * s_stride, sp, s_npass, s_m, s_tw, gm.lt, s_ts);
-            }
-            if (J.mode != UM_BLUE1 || round == 1)
-                break;
-            const int mm = s_m, st = s_stride;
-            const fast_div dm  = s_div;
-            const cpx<T>* bhat = reinterpret_cast<const cpx<T>*>(J.bhat);
-            for (int i = threadIdx.x; i < cnt * mm; i += blockDim.x)
-            {
-                const int s = int(fdiv(uint32_t(i), dm));
-                const int e = i - s * mm;
-                cpx<T>& r   = sm[s * st + pidx<T>(e)];
-                r           = conj(r * ldg(bhat + e));
-            }
-        }
-        if (mode <= UM_BLUE1)
-        {
-            const int n = J.n;
-            const fast_div dm   = s_div;
-            const cpx<T>* chirp = mode == UM_BLUE1 ? reinterpret_cast<const cpx<T>*>(J.chirp) : nullptr;
-#pragma unroll 4
-            for (int i = threadIdx.x; i < cnt * m; i += blockDim.x)
-            {
-                const int s = int(fdiv(uint32_t(i), dm));
-                const int e = i - s * m;
-                if (e < n)
-                {
-                    const cpx<T> r     = sm[s * stride + pidx<T>(e)];
-                    gout[s_off[s] + e] = chirp ? conj_if(conj(r) * ldg(chirp + e), inv) : conj_if(r, inv);
-                }
-            }
-        }
-        else
-        {
-            const int S = cnt, sh = 31 - __clz(cnt);
-            const int n1 = J.n1, n2 = J.n2, c0 = s_first;
-            cpx<T>* dst   = (J.dst == 1 ? gout : gscr) + J.dst_off;
-            const bool cj = J.last && inv;
-            if (mode == UM_COL)
-            {
-                const cpx<T>* twA = reinterpret_cast<const cpx<T>*>(J.twA);
-                const cpx<T>* twB = reinterpret_cast<const cpx<T>*>(J.twB);
-                const fast_div dm = s_div;
-#pragma unroll 4
-                for (int i = threadIdx.x; i < S * m; i += blockDim.x)
-                {
-                    const int c = int(fdiv(uint32_t(i), dm)), k1 = i - c * m, col = c0 + c;
-                    if (col < n2)
-                    {
-                        const cpx<T> v = sm[c * stride + pidx<T>(k1)] *
-                                         twiddle_2level(twA, twB, (long long)col * k1, J.lbits);
-                        dst[(long long)col * n1 + k1] = conj_if(v, cj);
-                    }
-                }
-            }
-            else
-            {
-                const cpx<T>* chirp = reinterpret_cast<const cpx<T>*>(J.chirp);
-                const cpx<T>* bhat  = reinterpret_cast<const cpx<T>*>(J.bhat);
-                const int post      = J.post;
-                const long long nv  = J.nvalid;
-#pragma unroll 4
-                for (int i = threadIdx.x; i < S * m; i += blockDim.x)
-                {
-                    const int k2 = i >> sh, r = i & (S - 1), row = c0 + r;
-                    if (row >= n1)
-                        continue;
-                    const long long k = row + (long long)n1 * k2;
-                    const cpx<T> v    = sm[r * stride + pidx<T>(k2)];
-                    if (post == 0)
-                        dst[k] = conj_if(v, cj);
-                    else if (post == 1)
-                        dst[k] = conj(v * ldg(bhat + k));
-                    else if (k < nv)
-                        dst[k] = conj_if(conj(v) * ldg(chirp + k), inv);
-                }
-            }
+                });
         }
         __syncthreads();
         if (threadIdx.x == 0 && J.done >= 0)
@@ -260,21 +223,18 @@ __global__ void __launch_bounds__(kUnevenThreads, 1) k_uneven(const uneven_launc
     }
 }
 
-cudaError_t launch_uneven_f32(const uneven_launch& a, int smem, int grid, cudaStream_t st)
+cudaError_t launch_uneven_f32(const uneven_launch& a, int threads, int smem, int grid, cudaStream_t st)
 {
-    const cudaError_t e = prepare_launch(reinterpret_cast<const void*>(k_uneven<float>), kUnevenThreads, smem);
+    const cudaError_t e = prepare_launch(reinterpret_cast<const void*>(k_uneven<float>), threads, smem);
     if (e != cudaSuccess)
         return e;
-    k_uneven<float><<<unsigned(grid), kUnevenThreads, smem, st>>>(a);
+    k_uneven<float><<<unsigned(grid), threads, smem, st>>>(a);
     return cudaGetLastError();
 }
 
-int uneven_max_smem()
-{
-    // dynamic shared memory beside the kernel's static pass list, offsets and job
-    return max_smem_bytes() - int(sizeof(pass_desc)) * kMaxPasses - int(sizeof(long long)) * kUnevenMaxSpc -
-           int(sizeof(uneven_job)) - 1024;
-}
+// Dynamic shared memory of one of four 256-thread or two 512-thread CTAs per SM, beside the kernel's static
+// descriptor, offsets and job.
+static int uneven_smem(int threads) { return threads <= 256 ? 48 * 1024 : 104 * 1024; }
 
 // ------------------------------------------------------------------------------------------------------
 // plan
@@ -286,23 +246,48 @@ namespace
 std::mutex g_tune_mu;
 std::map<long long, std::pair<std::vector<int>, int>> g_tune; // length -> fastest radix order and tile
 
-bool fits_one_cta(long long m, const std::vector<int>& order, int& ts)
+// descriptor of a one-CTA transform, or of a tile of S columns / rows; false if it does not fit a CTA
+bool fits(int threads, const std::vector<int>& order, rp_layout layout, int S, bool smem_io, rp_desc& d, int& elems)
 {
-    if (order.empty() || m > 8192)
+    if (order.empty())
         return false;
-    ts = threads_needed(m, order, 16);
-    return ts > 0 && ts <= kUnevenThreads && padded_len_host<float>(int(m)) * 8 <= uneven_max_smem();
+    d     = rp_build(order, layout, S, 8, smem_io);
+    elems = rp_smem_elems(d, layout, S, smem_io);
+    return rp_threads_needed(d, S, smem_io) <= threads && elems * 8 <= uneven_smem(threads);
+}
+
+std::vector<int> radices_of(long long m)
+{
+    return m == 1 ? std::vector<int>{ 1 } : rp_radices(m, kGenericMax);
+}
+
+bool fits_one_cta(int threads, long long m, const std::vector<int>& order, bool smem_io)
+{
+    rp_desc d;
+    int elems = 0;
+    return m <= threads * kRpMaxRadix && fits(threads, order, RP_SIGNALS, 1, smem_io, d, elems);
+}
+
+// most signals of one item: about 16 values per thread, every in-place butterfly held
+int most_signals(int threads, const rp_desc& d, int elems, bool smem_io)
+{
+    int spc = std::max(1, std::min({ threads * kRpMaxRadix / std::max(1, d.n), uneven_smem(threads) / (elems * 8),
+                                     kUnevenMaxSpc }));
+    while (spc > 1 && rp_threads_needed(d, spc, smem_io) > threads)
+        spc--;
+    return spc;
 }
 
 std::vector<std::vector<int>> candidate_orders(long long m)
 {
     std::vector<std::vector<int>> c;
-    const auto a = factor_radices(m);
+    const auto a = radices_of(m);
     if (a.empty())
         return c;
     auto add = [&](std::vector<int> v)
     {
-        if (std::find(c.begin(), c.end(), v) == c.end())
+        // the ends are codelets
+        if (v.front() <= kRpMaxRadix && v.back() <= kRpMaxRadix && std::find(c.begin(), c.end(), v) == c.end())
             c.push_back(v);
     };
     add(a);
@@ -315,75 +300,109 @@ std::vector<std::vector<int>> candidate_orders(long long m)
     return c;
 }
 
-// largest power-of-two tile (<= 16) of columns / rows of an m-point FFT of `ts` threads within one CTA
-int tile_of(int m, int ts)
+// Columns / rows of an m-point FFT per item: the largest power of two of about 16 values per thread that fits
+// (an item costs a queue round trip and a few barriers whatever its size: 16-wide tiles of every length took
+// 804 us for 1024 signals), 0 if none.
+int tile_of(int threads, const std::vector<int>& order, rp_layout layout)
 {
-    int s = 16;
-    while (s > 1 && (s * ts > kUnevenThreads || s * padded_len_host<float>(m) * 8 > uneven_max_smem()))
-        s /= 2;
-    return s;
+    rp_desc d;
+    int elems   = 0;
+    long long m = 1;
+    for (int r : order)
+        m *= r;
+    for (int S = kUnevenMaxSpc; S >= 1; S /= 2)
+        if (S * m <= threads * kRpMaxRadix && fits(threads, order, layout, S, false, d, elems))
+            return S;
+    return 0;
 }
 
-// four-step split n = n1 * n2 with both factors one-CTA lengths, as balanced as possible
-bool split_of(long long n, int& n1, int& n2)
+// four-step split n = n1 * n2 with the cheapest passes (rows of fewer than 16 columns cost extra sectors)
+struct splitter
 {
-    long long best = 0;
-    for (long long a = 2; a * a <= n; a++)
+    int threads;
+    std::map<std::pair<long long, int>, double> memo;
+    double cost(long long m, rp_layout layout)
     {
-        if (n % a)
-            continue;
-        const long long b = n / a;
-        int t1 = 0, t2 = 0;
-        if (fits_one_cta(a, factor_radices(a), t1) && fits_one_cta(b, factor_radices(b), t2))
-            best = a;
+        const auto key = std::make_pair(m, int(layout));
+        auto f         = memo.find(key);
+        if (f != memo.end())
+            return f->second;
+        double c       = -1;
+        const auto rad = radices_of(m);
+        const int S    = rad.empty() ? 0 : tile_of(threads, rad, layout);
+        if (S)
+        {
+            c = 12.0 * (16.0 / std::min(S, 16) - 1);
+            for (int r : rad)
+                c += rp_pass_cost(r);
+        }
+        return memo[key] = c;
     }
-    if (!best)
-        return false;
-    n1 = int(best);
-    n2 = int(n / best);
-    return true;
+    bool split(long long n, int& n1, int& n2)
+    {
+        double best       = -1;
+        const long long t = (long long)threads * kRpMaxRadix;
+        for (long long a = 2; a <= t && a * 2 <= n; a++)
+        {
+            if (n % a || n / a > t)
+                continue;
+            const double c = cost(a, RP_COLS), r = c < 0 ? -1 : cost(n / a, RP_ROWS);
+            // of equal splits the most balanced
+            if (r >= 0 && (best < 0 || c + r < best - 1e-9 ||
+                           (c + r < best + 1e-9 && std::max(a, n / a) < std::max(n1, n2))))
+            {
+                best = c + r;
+                n1   = int(a);
+                n2   = int(n / a);
+            }
+        }
+        return best >= 0;
+    }
+};
+
+// Convolution length of a Bluestein transform: the smallest power of two >= 2n - 1.
+long long bluestein_length(long long n)
+{
+    long long m = 1;
+    while (m < 2 * n - 1)
+        m <<= 1;
+    return m;
 }
 
 } // namespace
 
-int uneven_plan::get_shape(long long m, int, const std::vector<int>* order)
+int uneven_plan::get_shape(long long m, int layout, int S, bool smem_io)
 {
-    std::vector<int> o = order ? *order : factor_radices(m);
-    if (!order)
+    const shape_key key(m, layout, S, smem_io);
+    auto f = shape_of_.find(key);
+    if (f != shape_of_.end())
+        return f->second;
+    std::vector<int> o = radices_of(m);
+    if (layout == RP_SIGNALS && !smem_io)
     {
         std::lock_guard<std::mutex> g(g_tune_mu);
-        auto f = g_tune.find(m);
-        if (f != g_tune.end())
-            o = f->second.first;
+        auto t = g_tune.find(m);
+        rp_desc d;
+        int elems = 0;
+        if (t != g_tune.end() && fits(threads_, t->second.first, RP_SIGNALS, 1, false, d, elems))
+            o = t->second.first;
     }
-    const std::pair<long long, int> key(m, 0);
-    auto f = shape_of_.find(key);
-    if (f != shape_of_.end() && !order)
-        return f->second;
-    std::unique_ptr<shape> s(new shape);
-    if (m == 1)
+    shape s;
+    if (!fits(threads_, o, rp_layout(layout), S, smem_io, s.d, s.elems))
+        throw std::invalid_argument("internal: uneven batch shape exceeds one CTA");
+    // one twiddle table per radix order
+    auto t = tw_of_.find(o);
+    if (t == tw_of_.end())
     {
-        // length 1: no passes (the transform is the identity); a one-element table keeps tw valid
-        std::memset(&s->prog.desc, 0, sizeof(s->prog.desc));
-        s->prog.desc.n = 1;
-        s->prog.n      = 1;
-        s->prog.gstride = padded_len_host<float>(1);
-        const std::complex<float> one(1, 0);
-        s->prog.tw.upload(&one, sizeof(one));
-        s->ts = 1;
+        const auto table = pass_twiddles<float>(o, nullptr);
+        tables_.emplace_back(new dbuf);
+        tables_.back()->upload(table.data(), table.size() * sizeof(table[0]));
+        t = tw_of_.emplace(o, tables_.back()->get()).first;
     }
-    else
-    {
-        int ts = 0;
-        if (!fits_one_cta(m, o, ts))
-            throw std::invalid_argument("internal: uneven batch shape exceeds one CTA");
-        s->prog.build(int(m), CT_NONE, &o, 16);
-        s->ts = s->prog.ts;
-    }
+    s.tw          = t->second;
     const int idx = int(shapes_.size());
-    shapes_.push_back(std::move(s));
-    if (!order)
-        shape_of_[key] = idx;
+    shapes_.push_back(s);
+    shape_of_[key] = idx;
     return idx;
 }
 
@@ -401,6 +420,22 @@ uneven_plan::uneven_plan(const std::vector<long long>& lengths, bool autotune) :
     derr_.alloc(sizeof(int));
     check(cudaMemset(derr_.get(), 0, sizeof(int)), "clear error flag");
 
+    // 256-thread CTAs, four per SM, unless a length needs passes that only 512 threads can hold
+    const auto plannable = [&](splitter& sp, long long n)
+    {
+        const bool smooth = n == 1 || !factor_radices(n).empty();
+        const long long m = smooth ? n : bluestein_length(n);
+        int n1 = 0, n2 = 0;
+        return fits_one_cta(sp.threads, m, radices_of(m), !smooth) || sp.split(m, n1, n2);
+    };
+    splitter splits{ 256, {} };
+    if (!std::all_of(lengths.begin(), lengths.end(), [&](long long n) { return plannable(splits, n); }))
+        splits = splitter{ kUnevenThreads, {} };
+    threads_ = splits.threads;
+    int dev = 0, sms = 152;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+
     // autotuner for the one-CTA lengths present: time candidate radix orders and tiles on a synthetic batch
     // of that length alone, keep the fastest for the process
     if (autotune)
@@ -408,13 +443,12 @@ uneven_plan::uneven_plan(const std::vector<long long>& lengths, bool autotune) :
         std::vector<long long> todo;
         for (long long n : lengths)
         {
-            int ts = 0;
-            if (n > 1 && fits_one_cta(n, factor_radices(n), ts))
+            if (n > 1 && fits_one_cta(threads_, n, radices_of(n), false))
                 todo.push_back(n);
         }
         std::sort(todo.begin(), todo.end());
         todo.erase(std::unique(todo.begin(), todo.end()), todo.end());
-        dbuf tin, tout, tffts, tjobs, titems, toffs, tq;
+        dbuf tin, tout, tffts, tjobs, titems, toffs, tq, ttw;
         const long long tune_elems = 1 << 20;
         tin.alloc(size_t(tune_elems) * 8);
         tout.alloc(size_t(tune_elems) * 8);
@@ -431,16 +465,17 @@ uneven_plan::uneven_plan(const std::vector<long long>& lengths, bool autotune) :
                     continue;
             }
             float best = 1e30f;
-            std::pair<std::vector<int>, int> best_cfg(factor_radices(n), 0);
+            std::pair<std::vector<int>, int> best_cfg(radices_of(n), 0);
             for (const auto& order : candidate_orders(n))
             {
-                int ts = 0;
-                if (!fits_one_cta(n, order, ts))
+                uneven_fft f{};
+                int elems = 0;
+                if (!fits(threads_, order, RP_SIGNALS, 1, false, f.d, elems))
                     continue;
-                block_program<float> p;
-                p.build(int(n), CT_NONE, &order, 16);
-                const int smax = std::max(1, std::min({ kUnevenThreads / p.ts, uneven_max_smem() / (p.gstride * 8),
-                                                        kUnevenMaxSpc }));
+                const auto table = pass_twiddles<float>(order, nullptr);
+                ttw.upload(table.data(), table.size() * sizeof(table[0]));
+                f.tw           = ttw.get();
+                const int smax = most_signals(threads_, f.d, elems, false);
                 for (int spc : { smax, std::max(1, smax / 2) })
                 {
                     const long long nsig = std::max<long long>(spc, std::min<long long>(4096, tune_elems / n));
@@ -450,9 +485,9 @@ uneven_plan::uneven_plan(const std::vector<long long>& lengths, bool autotune) :
                     std::vector<uneven_item> its;
                     for (long long s = 0; s < nsig; s += spc)
                         its.push_back({ 0, int(s), int(std::min<long long>(spc, nsig - s)) });
-                    uneven_fft f{ p.desc, p.tw.get(), int(n), p.ts, p.gstride, make_fast_div(uint32_t(n)) };
                     uneven_job j{};
                     j.mode = UM_DIRECT;
+                    j.dst  = 1;
                     j.fft  = 0;
                     j.n    = int(n);
                     j.wait = -1;
@@ -465,14 +500,14 @@ uneven_plan::uneven_plan(const std::vector<long long>& lengths, bool autotune) :
                                      static_cast<uneven_item*>(titems.get()), static_cast<long long*>(toffs.get()),
                                      int(its.size()), static_cast<int*>(tq.get()), nullptr,
                                      static_cast<int*>(derr_.get()), tin.get(), tout.get(), nullptr, 0 };
-                    const int smem = spc * p.gstride * 8;
-                    const int grid = std::min<int>(int(its.size()), 152);
+                    const int smem = spc * elems * 8;
+                    const int grid = std::min<int>(int(its.size()), 1024 / threads_ * sms);
                     for (int rep = 0; rep < 4; rep++)
                     {
                         check(cudaMemset(tq.get(), 0, sizeof(int)), "clear queue");
                         if (rep == 1)
                             check(cudaEventRecord(e0), "event");
-                        check(launch_uneven_f32(L, smem, grid, nullptr), "tune");
+                        check(launch_uneven_f32(L, threads_, smem, grid, nullptr), "tune");
                     }
                     float ms = 0;
                     check(cudaEventRecord(e1), "event");
@@ -517,23 +552,18 @@ uneven_plan::uneven_plan(const std::vector<long long>& lengths, bool autotune) :
     {
         const long long n = kv.first;
         const auto& sig   = kv.second;
-        const auto rad    = factor_radices(n);
-        int ts            = 0;
-        const bool direct = n == 1 || fits_one_cta(n, rad, ts);
+        const bool smooth = n == 1 || !factor_radices(n).empty();
+        const bool direct = smooth && fits_one_cta(threads_, n, radices_of(n), false);
         long long m       = n;
-        if (!direct && rad.empty())
-        {
-            // Bluestein convolution length: the smallest power of two >= 2n - 1 (the smallest 7-smooth one
-            // is up to 2x shorter, but its radix-3/5/7 passes cost as much in this kernel: measured the same)
-            m = 1;
-            while (m < 2 * n - 1)
-                m <<= 1;
-        }
-        if (direct || (rad.empty() && fits_one_cta(m, factor_radices(m), ts)))
+        if (!smooth)
+            m = bluestein_length(n);
+        if (direct || (!smooth && fits_one_cta(threads_, m, radices_of(m), true)))
         {
             uneven_job j{};
             j.mode  = direct ? UM_DIRECT : UM_BLUE1;
-            j.fft   = get_shape(m, kUnevenThreads);
+            j.dst   = 1;
+            j.first = j.last = 1;
+            j.fft   = get_shape(m, RP_SIGNALS, 1, !direct);
             j.n     = int(n);
             j.wait  = -1;
             j.done  = -1;
@@ -548,9 +578,9 @@ uneven_plan::uneven_plan(const std::vector<long long>& lengths, bool autotune) :
             }
             else
                 n_direct_ += int(sig.size());
-            const shape& sh = *shapes_[j.fft];
-            int spc = std::max(1, std::min({ kUnevenThreads / sh.ts, uneven_max_smem() / (sh.prog.gstride * 8),
-                                             kUnevenMaxSpc }));
+            const shape& sh = shapes_[j.fft];
+            int spc         = most_signals(threads_, sh.d, sh.elems, !direct);
+            if (direct)
             {
                 std::lock_guard<std::mutex> g(g_tune_mu);
                 auto f = g_tune.find(m);
@@ -568,17 +598,17 @@ uneven_plan::uneven_plan(const std::vector<long long>& lengths, bool autotune) :
                 add_item(0, { jid, first + s, c }, double(c) * double(m) * std::log2(double(std::max<long long>(m, 2))) *
                                                        (direct ? 1.0 : 2.0));
             }
-            smem_ = std::max(smem_, spc * sh.prog.gstride * 8);
+            smem_ = std::max(smem_, spc * sh.elems * 8);
             continue;
         }
         // long signals: four-step (smooth lengths) or four-step Bluestein (a large prime factor), per signal
-        const bool blue = rad.empty();
+        const bool blue = !smooth;
         int n1 = 0, n2 = 0;
-        if (!split_of(m, n1, n2))
+        if (!splits.split(m, n1, n2))
             throw std::invalid_argument("uneven batch: length " + std::to_string(n) + " is not supported");
-        const int f1 = get_shape(n1, kUnevenThreads), f2 = get_shape(n2, kUnevenThreads);
-        const int S1 = tile_of(n1, shapes_[f1]->ts), S2 = tile_of(n2, shapes_[f2]->ts);
-        smem_        = std::max({ smem_, S1 * shapes_[f1]->prog.gstride * 8, S2 * shapes_[f2]->prog.gstride * 8 });
+        const int S1 = tile_of(threads_, radices_of(n1), RP_COLS), S2 = tile_of(threads_, radices_of(n2), RP_ROWS);
+        const int f1 = get_shape(n1, RP_COLS, S1, false), f2 = get_shape(n2, RP_ROWS, S2, false);
+        smem_        = std::max({ smem_, shapes_[f1].elems * 8, shapes_[f2].elems * 8 });
         // W_m^k two-level table
         int lb = 0;
         while ((1LL << (2 * lb)) < m)
@@ -690,9 +720,8 @@ uneven_plan::uneven_plan(const std::vector<long long>& lengths, bool autotune) :
     }
     nitems_ = int(items.size());
     std::vector<uneven_fft> ffts;
-    for (auto& sp : shapes_)
-        ffts.push_back({ sp->prog.desc, sp->prog.tw.get(), sp->prog.n, sp->ts, sp->prog.gstride,
-                         make_fast_div(uint32_t(std::max(1, sp->prog.n))) });
+    for (const shape& sp : shapes_)
+        ffts.push_back({ sp.d, sp.tw });
     if (!ffts.empty())
         dffts_.upload(ffts.data(), ffts.size() * sizeof(uneven_fft));
     if (!jobs.empty())
@@ -705,11 +734,8 @@ uneven_plan::uneven_plan(const std::vector<long long>& lengths, bool autotune) :
     dcounters_.alloc(size_t(std::max(1, ncounters_)) * sizeof(int));
     if (scratch_elems)
         scratch_.alloc(size_t(scratch_elems) * 8);
-    int dev = 0, sms = 152;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    grid_ = std::max(1, std::min(nitems_, sms));
     smem_ = std::max(smem_, 1024);
+    grid_ = std::max(1, std::min(nitems_, 1024 / threads_ * sms));
 }
 
 uneven_plan::~uneven_plan()
@@ -732,7 +758,7 @@ void uneven_plan::enqueue(void* out, const void* in, bool inverse, cudaStream_t 
                      static_cast<int*>(dqueue_.get()), static_cast<int*>(dcounters_.get()),
                      static_cast<int*>(derr_.get()), in, out, scratch_.get(), inverse ? 1 : 0, wait_limit(),
                      unreachable_ ? 1 : 0 };
-    check(launch_uneven_f32(L, smem_, grid_, st), "launch uneven batch");
+    check(launch_uneven_f32(L, threads_, smem_, grid_, st), "launch uneven batch");
 }
 
 void uneven_plan::execute(void* out, const void* in, bool inverse, cudaStream_t st)

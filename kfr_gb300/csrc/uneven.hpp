@@ -19,6 +19,7 @@
 #include <map>
 #include <memory>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "plan.hpp"
@@ -26,13 +27,11 @@
 namespace kfr_gpu
 {
 
-// block FFT shape run inside a tile
+// block FFT run inside a tile
 struct uneven_fft
 {
-    fft_desc d;
+    rp_desc d;
     const void* tw;
-    int m, ts, stride;
-    fast_div div_m;
 };
 
 enum uneven_mode
@@ -73,7 +72,8 @@ struct uneven_item
     int count; // signals (DIRECT / BLUE1) or columns / rows (COL / ROW)
 };
 
-// Threads of the persistent kernel (one CTA per SM; block FFTs of up to 8192 points, 16 values per thread).
+// Most threads of the persistent kernel: 256 (block FFTs of up to 4096 points), or 512 (up to 8192) where a plan
+// needs them.
 constexpr int kUnevenThreads = 512;
 // Most signals or columns one work item carries.
 constexpr int kUnevenMaxSpc = 256;
@@ -96,8 +96,7 @@ struct uneven_launch
     int stage_bias;      // added to every stage count waited for: 0, or 1 to make every such wait run out
 };
 
-cudaError_t launch_uneven_f32(const uneven_launch& a, int smem, int grid, cudaStream_t st);
-int uneven_max_smem();
+cudaError_t launch_uneven_f32(const uneven_launch& a, int threads, int smem, int grid, cudaStream_t st);
 
 class uneven_plan
 {
@@ -120,16 +119,19 @@ public:
 private:
     struct shape
     {
-        block_program<float> prog;
-        int ts = 1;
+        rp_desc d;
+        int elems; // shared elements per signal, or per tile of columns / rows
+        const void* tw;
     };
+    using shape_key = std::tuple<long long, int, int, bool>; // length, rp_layout, signals per tile, smem_io
     std::vector<long long> lengths_, offsets_;
     long long total_ = 0;
-    std::vector<std::unique_ptr<shape>> shapes_;
-    std::map<std::pair<long long, int>, int> shape_of_; // (m, threads cap) -> shape
-    std::vector<std::unique_ptr<dbuf>> tables_;         // chirps, spectra and four-step twiddles
+    std::vector<shape> shapes_;
+    std::map<shape_key, int> shape_of_;
+    std::map<std::vector<int>, const void*> tw_of_; // radix order -> twiddles
+    std::vector<std::unique_ptr<dbuf>> tables_;     // twiddles, chirps, spectra and four-step roots
     dbuf dffts_, djobs_, ditems_, doffsets_, dqueue_, dcounters_, derr_, scratch_;
-    int nitems_ = 0, ncounters_ = 0, smem_ = 0, grid_ = 0;
+    int nitems_ = 0, ncounters_ = 0, smem_ = 0, grid_ = 0, threads_ = 256;
     int n_direct_ = 0, n_blue1_ = 0, n_fourstep_ = 0, n_blue_fs_ = 0;
     std::map<long long, std::unique_ptr<complex_engine<float>>> engines_; // plain form only
     dbuf plain_scratch_;
@@ -142,7 +144,7 @@ private:
     unsigned gspins_  = 0; // wait settings the captured graph was built with
     bool gunreach_    = false;
 
-    int get_shape(long long m, int max_ts, const std::vector<int>* order = nullptr);
+    int get_shape(long long m, int layout, int S, bool smem_io);
     void enqueue(void* out, const void* in, bool inverse, cudaStream_t st);
 };
 
