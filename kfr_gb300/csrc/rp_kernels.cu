@@ -76,7 +76,10 @@ __global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T)), 1)
             if constexpr (sizeof(T) == 4)
             {
                 // W^{col k} times powers of the butterfly's step W^{col step}
-                if constexpr (R > 1)
+                if constexpr (R >= 8)
+                    twiddle_powers4<T, R>(o, rp_root(twA, twB, col * step, a.lbits),
+                                          rp_root(twA, twB, 4 * col * step, a.lbits));
+                else if constexpr (R > 1)
                     twiddle_powers<T, R>(o, rp_root(twA, twB, col * step, a.lbits));
                 const cpx<T> w = rp_root(twA, twB, col * k, a.lbits);
 #pragma unroll

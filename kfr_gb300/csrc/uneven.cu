@@ -193,7 +193,9 @@ __global__ void __launch_bounds__(kUnevenThreads, 2) k_uneven(const __grid_const
                     const cpx<T>* twB = reinterpret_cast<const cpx<T>*>(J.twB);
                     const int lbits   = J.lbits, mask = (1 << lbits) - 1;
                     const auto root = [&](int m) { return ldg(twA + (m >> lbits)) * ldg(twB + (m & mask)); };
-                    if constexpr (R > 1)
+                    if constexpr (R >= 8)
+                        twiddle_powers4<T, R>(o, root(col * step), root(4 * col * step));
+                    else if constexpr (R > 1)
                         twiddle_powers<T, R>(o, root(col * step));
                     const cpx<T> w = root(col * k);
 #pragma unroll
