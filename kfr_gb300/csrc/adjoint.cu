@@ -130,6 +130,14 @@ void fir_backward(const T* taps, long long ntaps, long long channels, long long 
 {
     if (ntaps <= 0 || channels <= 0 || n <= 0)
         throw std::invalid_argument("FIR backward needs taps, channels and samples");
+    if (!grad_x && !grad_h)
+        return;
+    if (fir_backward_blocks<T>(taps, ntaps, channels, n, x, grad_y, grad_x, grad_h, st))
+    {
+        check(cudaStreamSynchronize(st), "FIR backward");
+        return;
+    }
+    // taps longer than one CTA's FFT: whole-signal transforms
     if (grad_x)
     {
         // grad_x = reverse(FIR_h(reverse(grad_y))): the same filter run backwards in time

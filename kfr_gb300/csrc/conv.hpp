@@ -16,24 +16,66 @@
 namespace kfr_gpu
 {
 
+// The c-point complex transform of a convolution block.
+struct conv_fft
+{
+    int ct      = 0; // compile-time length (KFR_CT_CONV_F32), 0: the runtime-length block FFT
+    int threads = 0;
+    int elems   = 0; // shared complex elements (even)
+    rp_desc rp{};
+};
+
+// Tables of real FFTs of f samples in the convolution kernels.
+template <typename T>
+struct fir_tables
+{
+    explicit fir_tables(size_t f);
+    void roots64(size_t f); // w64
+    conv_fft fft;
+    dbuf tw, rtw; // pass twiddles; W_f^k, k <= f / 2
+    dbuf w64;     // W_f^j, j < f, in double precision (gradients: the taps' spectrum)
+};
+
 struct conv_args
 {
     const void* in;    // channels x n samples
     void* out;
-    const void* hist;  // channels x (M-1) previous samples
+    const void* hist;  // channels x nhist previous samples
     long long n;       // samples per channel in this call
-    long long m1;      // M - 1
+    long long nhist;   // M - 1
+    long long m1;      // overlap of the blocks: M - 1 rounded up to even
     long long bo;      // valid outputs per block
     int channels;
     const void* hspec; // c+1 complex: FFT_F(taps) / F
     const void* rtw;   // W_F^k, k = 0..c
     const void* tw;
-    fast_div div_c;
-    fft_desc d;        // c = F/2 point complex FFT
+    conv_fft fft;      // c = F/2 point complex FFT
 };
 
 template <typename T>
-cudaError_t launch_conv_os(const conv_args& a, const block_cfg& c, long long nblocks, cudaStream_t st);
+cudaError_t launch_conv_os(const conv_args& a, long long nblocks, cudaStream_t st);
+
+// k_fir_bwd: gradients of `blocks` blocks per channel.
+struct fir_bwd_args
+{
+    const void* x;
+    const void* grad_y;
+    void* grad_x;  // may be null
+    void* partial; // one spectrum of c + 1 values per CTA (null: no taps gradient)
+    long long n, bo, blocks, channels;
+    const void* hspec;
+    const void* rtw;
+    const void* tw;
+    conv_fft fft;
+    int elems; // shared complex elements of one block
+};
+
+// fir_backward (adjoint.hpp) block by block; false (nothing done) when the taps are too long for one CTA's FFT.
+// Enqueued on st.
+template <typename T>
+bool fir_backward_blocks(const T* taps, long long ntaps, long long channels, long long n, const T* x, const T* grad_y,
+                         T* grad_x, T* grad_h, cudaStream_t st);
+
 template <typename T>
 cudaError_t launch_hist_update(const void* hist_old, void* hist_new, const void* in, long long n, long long m1,
                                int channels, cudaStream_t st);
@@ -60,8 +102,8 @@ private:
     size_t m_, f_, c_, bo_;
     int channels_;
     bool long_ = false;
-    block_program<T> prog_;
-    dbuf hspec_, rtw_, hist_[2];
+    std::unique_ptr<fir_tables<T>> tables_;
+    dbuf hspec_, hist_[2];
     dbuf htaps_, lin_, lout_; // long mode: taps, [history, input] and the full convolution of one channel
     int cur_ = 0;
 };

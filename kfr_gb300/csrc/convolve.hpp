@@ -18,6 +18,9 @@ namespace kfr_gpu
 
 // Process-wide plan cache keyed by (precision, kind, size), guarded by a mutex like dft_cache
 // (include/kfr/dft/cache.hpp:54-83).  Plans live until clear() or process exit.
+template <typename T>
+struct fir_tables; // conv.hpp
+
 class plan_cache
 {
 public:
@@ -26,6 +29,9 @@ public:
     std::shared_ptr<complex_engine<T>> complex(long long n);
     template <typename T>
     std::shared_ptr<real_engine<T>> real(long long n);
+    // tables of the FIR gradients' real FFT of n samples
+    template <typename T>
+    std::shared_ptr<fir_tables<T>> fir(long long n);
     void clear();
     size_t size() const;
 
