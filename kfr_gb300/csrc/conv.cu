@@ -40,7 +40,7 @@ struct conv_ct
     const cpx<float>* tw;
     const F fft;
     __device__ __forceinline__ conv_ct(cpx<float>* b, const void* t, const conv_fft& d)
-        : buf(b), tw(reinterpret_cast<const cpx<float>*>(t)), fft(nullptr, fft_desc(), F::ts)
+        : buf(b), tw(reinterpret_cast<const cpx<float>*>(t)), fft()
     {
         (void)d;
     }
@@ -66,7 +66,7 @@ template <typename T>
 struct conv_rp
 {
     using real                       = T;
-    static constexpr int max_threads = rp_max_threads(2 * sizeof(T));
+    static constexpr int max_threads = rp_max_threads(2 * sizeof(T), kRpHold);
     cpx<T>* buf;
     const cpx<T>* tw;
     const rp_desc& d;
@@ -511,7 +511,7 @@ fir_tables<T>::fir_tables(size_t f)
         fft.elems   = (rp_smem_elems(fft.rp, RP_SIGNALS, 1, true) + 1) / 2 * 2;
         fft.threads = (std::max(rp_threads_needed(fft.rp, 1, true), std::min(c, 64)) + 31) / 32 * 32;
     }
-    const auto t = pass_twiddles<T>(rad, nullptr);
+    const auto t = pass_twiddles<T>(rad);
     tw.upload(t.data(), t.size() * sizeof(t[0]));
     std::vector<std::complex<T>> rt(c + 1);
     for (int k = 0; k <= c; k++)

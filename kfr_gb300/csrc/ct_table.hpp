@@ -2,7 +2,7 @@
 //   X(N, TS, radices...)   N = product of the radices, TS = threads per signal
 // chosen so that no thread holds more than 18 complex values in any pass.  The planner uses an entry when
 // the kernel kind and length match (block_program::build then lays the twiddles out in this radix order);
-// every other length runs the runtime-radix kernel.  Lists are per kernel kind to bound compile time:
+// every other length runs the runtime-length block FFT (rp_fft.cuh).  Lists are per kernel kind to bound compile time:
 // they cover the parity and benchmark configurations and the power-of-two lengths up to 16384.
 #pragma once
 

@@ -7,8 +7,8 @@
 //     buf[(j - j mod Ns)*R + j mod Ns + r*Ns] = V[r],
 // so the result comes out in natural order with no digit-reverse pass.  This replaces the reference's
 // in-place stages plus reorder stage (src/dft/dft-impl.hpp:85-150, 368-494) and its radix-4 DIF passes plus
-// bit reversal (src/dft/fft-impl.hpp:846-1001).  Each pass reads all of its butterflies into registers,
-// synchronises, and writes them back, so a signal needs only N (+1/16 padding) slots of shared memory.
+// bit reversal (src/dft/fft-impl.hpp:846-1001).  Lengths in ct_table.hpp run the compile-time passes below,
+// every other length the runtime ones (rp_fft.cuh).
 #pragma once
 
 #include "ct_table.hpp"
@@ -410,10 +410,6 @@ __device__ __forceinline__ void dft_codelet(cpx<T>* v)
         dft_odd<T, R>(v);
 }
 
-// --------------------------------------------------------------------------------------------------
-// Block FFT descriptor (built on the host by the planner).
-// --------------------------------------------------------------------------------------------------
-
 __device__ __forceinline__ uint32_t fdiv(uint32_t x, const fast_div f)
 {
     if (f.d == 1)
@@ -421,13 +417,6 @@ __device__ __forceinline__ uint32_t fdiv(uint32_t x, const fast_div f)
     uint32_t hi = __umulhi(x, f.m);
     return (hi + ((x - hi) >> 1)) >> (f.s - 1);
 }
-
-// --------------------------------------------------------------------------------------------------
-// One pass, split into a load half (gather butterflies, twiddle, DFT_R, all in the thread's register
-// array v) and a store half (scatter to the self-sorted positions), with a barrier in between.  Every
-// radix works on the same array v[EPT] so that the runtime radix switch keeps one register layout;
-// threads lt in [0, ts) of a signal group own butterflies j = lt + b*ts.
-// --------------------------------------------------------------------------------------------------
 
 // v[r] *= W^{k r} from the one table value w1 = W^k by a binary powering tree, w_r = w_{r/2} w_{r - r/2}
 // (at most ceil(log2 r) products deep): one load per butterfly instead of R - 1.  Both factors have index
@@ -484,182 +473,10 @@ __device__ __forceinline__ void ct_twiddle(cpx<T> (&v)[R], const cpx<T>* __restr
         twiddle_powers<T, R>(v, ldg(tw + k));
 }
 
-template <typename T, int R, int EPT>
-__device__ __forceinline__ void pass_load(cpx<T> (&v)[EPT], const cpx<T>* buf, const int n, const pass_desc& p,
-                                          const cpx<T>* __restrict__ tw, const int lt, const int ts)
-{
-    constexpr int NB = EPT / R;
-    const int nbf    = n / R;
-    const int ns     = p.ns;
-#pragma unroll
-    for (int b = 0; b < NB; b++)
-    {
-        const int j = lt + b * ts;
-        if (j < nbf)
-        {
-#pragma unroll
-            for (int r = 0; r < R; r++)
-                v[b * R + r] = buf[pidx<T>(j + r * nbf)];
-            if (ns > 1)
-            {
-                const int k = j - int(fdiv(uint32_t(j), p.div_ns)) * ns;
-                if constexpr (sizeof(T) == 4)
-                {
-                    // W^{k r} from the one table value W^k (the r = 1 entry) by the powering tree
-                    twiddle_powers<T, R>(reinterpret_cast<cpx<T>(&)[R]>(v[b * R]), ldg(tw + p.tw_off + k));
-                }
-                else
-                {
-                    // double precision: table loads (FP64 products are slow on this part)
-                    const cpx<T>* t = tw + p.tw_off + k;
-#pragma unroll
-                    for (int r = 1; r < R; r++)
-                        v[b * R + r] = v[b * R + r] * ldg(t + (r - 1) * ns);
-                }
-            }
-            dft_codelet<T, R>(&v[b * R]);
-        }
-    }
-}
-
-template <typename T, int R, int EPT>
-__device__ __forceinline__ void pass_store(const cpx<T> (&v)[EPT], cpx<T>* buf, const int n, const pass_desc& p,
-                                           const int lt, const int ts)
-{
-    constexpr int NB = EPT / R;
-    const int nbf    = n / R;
-    const int ns     = p.ns;
-#pragma unroll
-    for (int b = 0; b < NB; b++)
-    {
-        const int j = lt + b * ts;
-        if (j < nbf)
-        {
-            const int k = ns > 1 ? j - int(fdiv(uint32_t(j), p.div_ns)) * ns : 0;
-            const int d = (j - k) * R + k;
-#pragma unroll
-            for (int r = 0; r < R; r++)
-                buf[pidx<T>(d + r * ns)] = v[b * R + codelet_out<R>(r)];
-        }
-    }
-}
-
-// Generic radix (any R, used for primes above 13): each thread computes up to EPT outputs
-// o = lt + e*ts, each a length-R dot product of the twiddled inputs (read from shared memory) with the
-// roots W_R^m.
-template <typename T, int EPT>
-__device__ __forceinline__ void pass_load_generic(cpx<T> (&v)[EPT], const cpx<T>* buf, const int n,
-                                                  const pass_desc& p, const cpx<T>* __restrict__ tw, const int lt,
-                                                  const int ts)
-{
-    const int R      = p.radix;
-    const int nbf    = n / R;
-    const int ns     = p.ns;
-    const cpx<T>* wr = tw + p.wr_off;
-#pragma unroll
-    for (int e = 0; e < EPT; e++)
-    {
-        const int oi = lt + e * ts;
-        if (oi < n)
-        {
-            const int q = oi / nbf;
-            const int j = oi - q * nbf;
-            const int k = ns > 1 ? j - int(fdiv(uint32_t(j), p.div_ns)) * ns : 0;
-            cpx<T> acc  = buf[pidx<T>(j)];
-            int widx    = 0;
-#pragma unroll 1
-            for (int r = 1; r < R; r++)
-            {
-                cpx<T> x = buf[pidx<T>(j + r * nbf)];
-                if (ns > 1)
-                    x = x * ldg(tw + p.tw_off + (r - 1) * ns + k);
-                widx += q;
-                if (widx >= R)
-                    widx -= R;
-                acc = acc + x * ldg(wr + widx);
-            }
-            v[e] = acc;
-        }
-    }
-}
-
-template <typename T, int EPT>
-__device__ __forceinline__ void pass_store_generic(const cpx<T> (&v)[EPT], cpx<T>* buf, const int n,
-                                                   const pass_desc& p, const int lt, const int ts)
-{
-    const int R   = p.radix;
-    const int nbf = n / R;
-    const int ns  = p.ns;
-#pragma unroll
-    for (int e = 0; e < EPT; e++)
-    {
-        const int oi = lt + e * ts;
-        if (oi < n)
-        {
-            const int q = oi / nbf;
-            const int j = oi - q * nbf;
-            const int k = ns > 1 ? j - int(fdiv(uint32_t(j), p.div_ns)) * ns : 0;
-            buf[pidx<T>((j - k) * R + k + q * ns)] = v[e];
-        }
-    }
-}
-
-// Runs every pass on the signal at buf.  The pass descriptors live in shared memory (staged by
-// stage_passes) so that the runtime pass loop never indexes the kernel's parameter block.  Must be reached
-// by all threads of the CTA (it synchronises); threads with lt >= ts only take part in the barriers.
-template <typename T, int EPT>
-__device__ __forceinline__ void block_fft(cpx<T>* buf, const pass_desc* sp, const int npass, const int n,
-                                          const cpx<T>* __restrict__ tw, const int lt, const int ts)
-{
-    const int lta = lt < ts ? lt : n; // inactive threads own no butterflies
-    cpx<T> v[EPT];
-#pragma unroll 1
-    for (int pi = 0; pi < npass; pi++)
-    {
-        const pass_desc p = sp[pi];
-        switch (p.radix)
-        {
-#define KFR_GPU_LOAD_CASE(R)                                                                               \
-    case R: pass_load<T, R, EPT>(v, buf, n, p, tw, lta, ts); break;
-            KFR_GPU_LOAD_CASE(2)
-            KFR_GPU_LOAD_CASE(3)
-            KFR_GPU_LOAD_CASE(4)
-            KFR_GPU_LOAD_CASE(5)
-            KFR_GPU_LOAD_CASE(7)
-            KFR_GPU_LOAD_CASE(8)
-            KFR_GPU_LOAD_CASE(9)
-            KFR_GPU_LOAD_CASE(11)
-            KFR_GPU_LOAD_CASE(13)
-            KFR_GPU_LOAD_CASE(16)
-#undef KFR_GPU_LOAD_CASE
-        default: pass_load_generic<T, EPT>(v, buf, n, p, tw, lta, ts); break;
-        }
-        __syncthreads();
-        switch (p.radix)
-        {
-#define KFR_GPU_STORE_CASE(R)                                                                              \
-    case R: pass_store<T, R, EPT>(v, buf, n, p, lta, ts); break;
-            KFR_GPU_STORE_CASE(2)
-            KFR_GPU_STORE_CASE(3)
-            KFR_GPU_STORE_CASE(4)
-            KFR_GPU_STORE_CASE(5)
-            KFR_GPU_STORE_CASE(7)
-            KFR_GPU_STORE_CASE(8)
-            KFR_GPU_STORE_CASE(9)
-            KFR_GPU_STORE_CASE(11)
-            KFR_GPU_STORE_CASE(13)
-            KFR_GPU_STORE_CASE(16)
-#undef KFR_GPU_STORE_CASE
-        default: pass_store_generic<T, EPT>(v, buf, n, p, lta, ts); break;
-        }
-        __syncthreads();
-    }
-}
-
 // --------------------------------------------------------------------------------------------------
 // Compile-time block FFT: the same Stockham passes for a length and radix sequence fixed at compile time,
 // so every index, divisor and twiddle offset folds to a constant and each pass's butterfly loop unrolls.
-// Used for the lengths listed in ct_table.hpp; the twiddle table layout matches block_program::build with
+// Used for the lengths listed in ct_table.hpp; the twiddle table layout is that of pass_twiddles with
 // the same radix order.
 // --------------------------------------------------------------------------------------------------
 
@@ -924,17 +741,6 @@ __device__ __forceinline__ void ct_block_fft_io(const LD& ld, const MID& mid, co
     const int lta     = lt < TS ? lt : N;
     cpx<T> v[EPT];
     io_chain<T, N, TS, EPT, 1, 0, LD, MID, ST, H, Rs...>(v, ld, mid, st, hook, buf, tw, lta);
-}
-
-// Copies the descriptor's passes into shared memory with compile-time parameter offsets.  Ends with a
-// barrier.
-__device__ __forceinline__ void stage_passes(pass_desc* sp, const fft_desc& d)
-{
-#pragma unroll
-    for (int i = 0; i < kMaxPasses; i++)
-        if (int(threadIdx.x) == i)
-            sp[i] = d.pass[i];
-    __syncthreads();
 }
 
 } // namespace kfr_gpu

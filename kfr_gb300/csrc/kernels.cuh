@@ -11,34 +11,46 @@
 #include "ct_table.hpp"
 #include "fft_device.cuh"
 #include "launch.hpp"
+#include "rp_fft.cuh"
 #include "tma.cuh"
 
 namespace kfr_gpu
 {
 
+// thread -> (signal slot, lane within the signal's thread group)
+struct group_map
+{
+    int g, lt;
+    __device__ __forceinline__ group_map(int ts, int spc)
+    {
+        g  = int(threadIdx.x) / ts;
+        lt = g < spc ? int(threadIdx.x) - g * ts : ts;
+        if (g >= spc)
+            g = 0;
+    }
+};
+
 // FFT policies.  A kernel is instantiated with one of them:
-//   rt_fft<T, EPT>          runtime radix sequence (any one-CTA length), pass list staged in shared memory
+//   rt_fft<T, H>            the runtime-length block FFT (rp_fft.cuh), in place on the tile's signals, threads
+//                           holding H values
 //   ct_fft<T, N, TS, Rs...> compile-time length and radices (ct_table.hpp)
-// Both expose n (length), ts (threads per signal), max_threads (launch bound) and run(buf, tw, lt).
-template <typename T, int EPT>
+// Both expose n (length), max_threads (launch bound), the tile's layout (signals gstride() elements apart,
+// element i at pi(i), `slots` elements in all) and run(tile, tw), which every thread of the CTA calls.
+template <typename T, int H>
 struct rt_fft
 {
     static constexpr bool compile_time = false;
-    // the block FFT keeps EPT complex values per thread in registers
-    static constexpr int max_threads = (sizeof(T) == 4 ? 1024 : 512) / (EPT / 16);
-    const pass_desc* sp;
-    int npass, n, ts;
-    __device__ __forceinline__ rt_fft(pass_desc* s, const fft_desc& d, int ts_) : sp(s), npass(d.npass), n(d.n), ts(ts_)
+    static constexpr int max_threads   = rp_max_threads(2 * sizeof(T), H);
+    const rp_desc& d;
+    const int n, spc;
+    __device__ __forceinline__ rt_fft(const rp_desc& d_, int, int spc_) : d(d_), n(d_.n), spc(spc_) {}
+    __device__ __forceinline__ void run(cpx<T>* tile, const cpx<T>* __restrict__ tw) const
     {
-        stage_passes(s, d);
+        rp_run_smem<T, H>(d, tile, spc, tw);
     }
-    __device__ __forceinline__ void run(cpx<T>* buf, const cpx<T>* __restrict__ tw, int lt) const
-    {
-        block_fft<T, EPT>(buf, sp, npass, n, tw, lt, ts);
-    }
-    // shared-memory layout: signals gstride(n) elements apart, element i at pi(i)
-    static __host__ __device__ constexpr int gstride(int len) { return padded_len<T>(len); }
-    static __device__ __forceinline__ int pi(int i) { return pidx<T>(i); }
+    __device__ __forceinline__ int slots() const { return spc * d.elems; }
+    static __host__ __device__ constexpr int gstride(int len) { return len; }
+    static __device__ __forceinline__ int pi(int i) { return i; }
 };
 
 template <typename T, int N, int TS, int... Rs>
@@ -55,10 +67,14 @@ struct ct_fft
         return sizeof(T) == 4 ? ct_group_stride_f32(N, TS) : padded_len<T>(N);
     }
     static __device__ __forceinline__ int pi(int i) { return pidx_s<ps>(i); }
-    __device__ __forceinline__ ct_fft(pass_desc*, const fft_desc&, int) {}
-    __device__ __forceinline__ void run(cpx<T>* buf, const cpx<T>* __restrict__ tw, int lt) const
+    const int ts_, spc;
+    __device__ __forceinline__ ct_fft(const rp_desc&, int t, int s) : ts_(t), spc(s) {}
+    __device__ __forceinline__ ct_fft() : ts_(TS), spc(1) {}
+    __device__ __forceinline__ int slots() const { return spc * gstride(); }
+    __device__ __forceinline__ void run(cpx<T>* tile, const cpx<T>* __restrict__ tw) const
     {
-        ct_block_fft<T, N, TS, Rs...>(buf, tw, lt);
+        const group_map gm(ts_, spc);
+        ct_block_fft<T, N, TS, Rs...>(tile + gm.g * gstride(), tw, gm.lt);
     }
     static constexpr int npass = sizeof...(Rs);
     // radix of the last pass (whose butterfly j produces outputs j + r n / rlast)
@@ -117,19 +133,6 @@ __device__ __forceinline__ void copy_batched(const int total, const LD& ld, cons
     }
 }
 
-// thread -> (signal slot, lane within the signal's thread group)
-struct group_map
-{
-    int g, lt;
-    __device__ __forceinline__ group_map(int ts, int spc)
-    {
-        g  = int(threadIdx.x) / ts;
-        lt = g < spc ? int(threadIdx.x) - g * ts : ts;
-        if (g >= spc)
-            g = 0;
-    }
-};
-
 // ---------------------------------------------------------------------------------------------------
 // Complex DFT, contiguous batch (dft_plan<T>::execute over many signals)
 // ---------------------------------------------------------------------------------------------------
@@ -137,8 +140,7 @@ template <typename T, class F>
 __global__ void __launch_bounds__(F::max_threads, 1) k_c2c(const c2c_args a, const int ts, const int spc)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ pass_desc sp[kMaxPasses];
-    const F fft(sp, a.d, ts);
+    const F fft(a.d, ts, spc);
     cpx<T>* sm        = reinterpret_cast<cpx<T>*>(smem_raw);
     const int n       = fft.n;
     const int stride  = F::gstride(n);
@@ -157,8 +159,7 @@ __global__ void __launch_bounds__(F::max_threads, 1) k_c2c(const c2c_args a, con
             sm[s * stride + F::pi(e)] = conj_if(in[sig * a.istride + e], inv);
     }
     __syncthreads();
-    const group_map gm(ts, spc);
-    fft.run(sm + gm.g * stride, reinterpret_cast<const cpx<T>*>(a.tw), gm.lt);
+    fft.run(sm, reinterpret_cast<const cpx<T>*>(a.tw));
 #pragma unroll 4
     for (int i = threadIdx.x; i < total; i += blockDim.x)
     {
@@ -189,7 +190,7 @@ __global__ void __launch_bounds__(F::max_threads, 1)
     extern __shared__ __align__(128) unsigned char smem_raw[];
     constexpr int N      = F::n;
     constexpr int STRIDE = F::gstride(N);
-    const F fft(nullptr, a.d, F::ts);
+    const F fft;
     const int tile      = spc * N;
     const int slen      = pipe_stage_len(spc, N, STRIDE);
     cpx<T>* const tiles = reinterpret_cast<cpx<T>*>(smem_raw);
@@ -293,7 +294,7 @@ __global__ void __launch_bounds__(F::max_threads, 1)
     constexpr int N          = F::n;
     constexpr int H          = N / 2;
     constexpr uint32_t hbytes = uint32_t(H) * uint32_t(sizeof(cpx<T>));
-    const F fft(nullptr, a.d, F::ts);
+    const F fft;
     static_assert(N % 2 == 0 && hbytes % 16 == 0, "two halves of whole 16-byte units per signal");
     cpx<T>* buf      = reinterpret_cast<cpx<T>*>(smem_raw);
     cpx<T>* spare    = buf + (F::gstride(N) + 1) / 2 * 2; // on a 16-byte boundary
@@ -372,8 +373,7 @@ __global__ void __launch_bounds__(F::max_threads, 1) k_bluestein(const bluestein
                                                                         const int spc)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ pass_desc sp[kMaxPasses];
-    const F fft(sp, a.d, ts);
+    const F fft(a.d, ts, spc);
     cpx<T>* sm        = reinterpret_cast<cpx<T>*>(smem_raw);
     const int m       = fft.n;
     const int n       = a.n;
@@ -396,9 +396,8 @@ __global__ void __launch_bounds__(F::max_threads, 1) k_bluestein(const bluestein
         sm[s * stride + F::pi(e)] = v;
     }
     __syncthreads();
-    const group_map gm(ts, spc);
     const cpx<T>* tw = reinterpret_cast<const cpx<T>*>(a.tw);
-    fft.run(sm + gm.g * stride, tw, gm.lt);
+    fft.run(sm, tw);
 #pragma unroll 4
     for (int i = threadIdx.x; i < spc * m; i += blockDim.x)
     {
@@ -408,7 +407,7 @@ __global__ void __launch_bounds__(F::max_threads, 1) k_bluestein(const bluestein
         r           = conj(r * ldg(bhat + e));
     }
     __syncthreads();
-    fft.run(sm + gm.g * stride, tw, gm.lt);
+    fft.run(sm, tw);
 #pragma unroll 4
     for (int i = threadIdx.x; i < spc * n; i += blockDim.x)
     {
@@ -429,13 +428,12 @@ template <typename T, class F>
 __global__ void __launch_bounds__(F::max_threads, 1) k_rader(const rader_args a, const int ts, const int spc)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ pass_desc sp[kMaxPasses];
-    const F fft(sp, a.d, ts);
+    const F fft(a.d, ts, spc);
     cpx<T>* sm         = reinterpret_cast<cpx<T>*>(smem_raw);
     const int L        = fft.n;
     const int n        = L + 1;
     const int stride   = F::gstride(L);
-    cpx<T>* x0s        = sm + spc * stride; // spc values
+    cpx<T>* x0s        = sm + fft.slots(); // spc values
     cpx<T>* dcs        = x0s + spc;        // spc values
     const long long s0 = (long long)blockIdx.x * spc;
     const cpx<T>* __restrict__ in   = reinterpret_cast<const cpx<T>*>(a.in);
@@ -455,9 +453,8 @@ __global__ void __launch_bounds__(F::max_threads, 1) k_rader(const rader_args a,
             sm[s * stride + F::pi(__ldg(a.pin + e))] = v;
     }
     __syncthreads();
-    const group_map gm(ts, spc);
     const cpx<T>* tw = reinterpret_cast<const cpx<T>*>(a.tw);
-    fft.run(sm + gm.g * stride, tw, gm.lt);
+    fft.run(sm, tw);
 #pragma unroll 4
     for (int i = threadIdx.x; i < spc * L; i += blockDim.x)
     {
@@ -470,7 +467,7 @@ __global__ void __launch_bounds__(F::max_threads, 1) k_rader(const rader_args a,
         r = conj(A * ldg(bhat + q));
     }
     __syncthreads();
-    fft.run(sm + gm.g * stride, tw, gm.lt);
+    fft.run(sm, tw);
 #pragma unroll 4
     for (int i = threadIdx.x; i < spc * n; i += blockDim.x)
     {
@@ -494,8 +491,7 @@ template <typename T, class F>
 __global__ void __launch_bounds__(F::max_threads, 1) k_r2c(const real_args a, const int ts, const int spc)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ pass_desc sp[kMaxPasses];
-    const F fft(sp, a.d, ts);
+    const F fft(a.d, ts, spc);
     cpx<T>* sm        = reinterpret_cast<cpx<T>*>(smem_raw);
     const int c       = fft.n;
     const int stride  = F::gstride(c);
@@ -519,8 +515,7 @@ __global__ void __launch_bounds__(F::max_threads, 1) k_r2c(const real_args a, co
         }
     }
     __syncthreads();
-    const group_map gm(ts, spc);
-    fft.run(sm + gm.g * stride, reinterpret_cast<const cpx<T>*>(a.tw), gm.lt);
+    fft.run(sm, reinterpret_cast<const cpx<T>*>(a.tw));
     const int olen = a.ccs ? c + 1 : c;
 #pragma unroll 4
     for (int i = threadIdx.x; i < spc * olen; i += blockDim.x)
@@ -580,7 +575,7 @@ __global__ void __launch_bounds__(F::max_threads, 1)
     extern __shared__ __align__(128) unsigned char smem_raw[];
     constexpr int C      = F::n;
     constexpr int STRIDE = F::gstride(C);
-    const F fft(nullptr, a.d, F::ts);
+    const F fft;
     const int slen       = r2c_stage_elems<T, F>(spc);
     const int olen       = a.ccs ? C + 1 : C;
     cpx<T>* const tiles  = reinterpret_cast<cpx<T>*>(smem_raw);
@@ -698,8 +693,7 @@ template <typename T, class F>
 __global__ void __launch_bounds__(F::max_threads, 1) k_c2r(const real_args a, const int ts, const int spc)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ pass_desc sp[kMaxPasses];
-    const F fft(sp, a.d, ts);
+    const F fft(a.d, ts, spc);
     cpx<T>* sm        = reinterpret_cast<cpx<T>*>(smem_raw);
     const int c       = fft.n;
     const int stride  = F::gstride(c);
@@ -734,8 +728,7 @@ __global__ void __launch_bounds__(F::max_threads, 1) k_c2r(const real_args a, co
         sm[s * stride + F::pi(k)] = conj(z);
     }
     __syncthreads();
-    const group_map gm(ts, spc);
-    fft.run(sm + gm.g * stride, reinterpret_cast<const cpx<T>*>(a.tw), gm.lt);
+    fft.run(sm, reinterpret_cast<const cpx<T>*>(a.tw));
 #pragma unroll 4
     for (int i = threadIdx.x; i < spc * c; i += blockDim.x)
     {
@@ -775,7 +768,7 @@ __global__ void __launch_bounds__(F::max_threads, 1)
     extern __shared__ __align__(128) unsigned char smem_raw[];
     constexpr int C      = F::n;
     constexpr int STRIDE = F::gstride(C);
-    const F fft(nullptr, a.d, F::ts);
+    const F fft;
     const int slen       = r2c_stage_elems<T, F>(spc);
     const int ilen       = a.ccs ? C + 1 : C;
     cpx<T>* const tiles  = reinterpret_cast<cpx<T>*>(smem_raw);
@@ -887,8 +880,7 @@ template <typename T, class F>
 __global__ void __launch_bounds__(F::max_threads, 1) k_dct2(const dct_args a, const int ts, const int spc)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ pass_desc sp[kMaxPasses];
-    const F fft(sp, a.d, ts);
+    const F fft(a.d, ts, spc);
     cpx<T>* sm        = reinterpret_cast<cpx<T>*>(smem_raw);
     const int n       = fft.n;
     const int stride  = F::gstride(n);
@@ -908,8 +900,7 @@ __global__ void __launch_bounds__(F::max_threads, 1) k_dct2(const dct_args a, co
         sm[s * stride + F::pi(pos)] = mk<T>(in[sig * a.stride + src], T(0));
     }
     __syncthreads();
-    const group_map gm(ts, spc);
-    fft.run(sm + gm.g * stride, reinterpret_cast<const cpx<T>*>(a.tw), gm.lt);
+    fft.run(sm, reinterpret_cast<const cpx<T>*>(a.tw));
 #pragma unroll 4
     for (int i = threadIdx.x; i < spc * n; i += blockDim.x)
     {
@@ -930,8 +921,7 @@ template <typename T, class F>
 __global__ void __launch_bounds__(F::max_threads, 1) k_dct3(const dct_args a, const int ts, const int spc)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ pass_desc sp[kMaxPasses];
-    const F fft(sp, a.d, ts);
+    const F fft(a.d, ts, spc);
     cpx<T>* sm        = reinterpret_cast<cpx<T>*>(smem_raw);
     const int n       = fft.n;
     const int stride  = F::gstride(n);
@@ -955,8 +945,7 @@ __global__ void __launch_bounds__(F::max_threads, 1) k_dct3(const dct_args a, co
         sm[s * stride + F::pi(k)] = v;
     }
     __syncthreads();
-    const group_map gm(ts, spc);
-    fft.run(sm + gm.g * stride, reinterpret_cast<const cpx<T>*>(a.tw), gm.lt);
+    fft.run(sm, reinterpret_cast<const cpx<T>*>(a.tw));
 #pragma unroll 4
     for (int i = threadIdx.x; i < spc * n; i += blockDim.x)
     {
@@ -995,7 +984,7 @@ __global__ void __launch_bounds__(F::max_threads, 1)
     extern __shared__ __align__(128) unsigned char smem_raw[];
     constexpr int N      = F::n;
     constexpr int STRIDE = F::gstride(N);
-    const F fft(nullptr, a.d, F::ts);
+    const F fft;
     const int slen       = dct_stage_elems<T, F>(spc);
     cpx<T>* const tiles  = reinterpret_cast<cpx<T>*>(smem_raw);
     uint64_t* bars       = reinterpret_cast<uint64_t*>(tiles + 3 * slen);
@@ -1111,8 +1100,7 @@ template <typename T, class F>
 __global__ void __launch_bounds__(F::max_threads, 1) k_fs_cols(const fourstep_args a, const int ts)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ pass_desc sp[kMaxPasses];
-    const F fft(sp, a.d, ts);
+    const F fft(a.d, ts, a.tile);
     cpx<T>* sm       = reinterpret_cast<cpx<T>*>(smem_raw);
     const int n1     = fft.n, n2 = a.n2, S = a.tile, sh = a.tile_shift;
     const int stride = F::gstride(n1);
@@ -1142,7 +1130,7 @@ __global__ void __launch_bounds__(F::max_threads, 1) k_fs_cols(const fourstep_ar
     const cpx<T>* twB = reinterpret_cast<const cpx<T>*>(a.twB);
     if constexpr (F::compile_time)
     {
-        if (a.pingpong && !a.same_layout)
+        if (a.pingpong)
         {
             // ping-pong passes with a second buffer after the tile; the last pass applies W_N^{col k1} and
             // stores the column contiguously (stride one across a signal's threads)
@@ -1161,20 +1149,7 @@ __global__ void __launch_bounds__(F::max_threads, 1) k_fs_cols(const fourstep_ar
             return;
         }
     }
-    fft.run(sm + gm.g * stride, reinterpret_cast<const cpx<T>*>(a.tw), gm.lt);
-    if (a.same_layout)
-    {
-        // an axis of a multi-dimensional transform: no twiddle, back to the input's own layout
-#pragma unroll 4
-        for (int i = threadIdx.x; i < total; i += blockDim.x)
-        {
-            const int k1 = i >> sh;
-            const int c  = i & (S - 1);
-            if (c0 + c < n2)
-                y[(long long)k1 * n2 + c0 + c] = conj_if(sm[c * stride + F::pi(k1)], a.conj_out != 0);
-        }
-        return;
-    }
+    fft.run(sm, reinterpret_cast<const cpx<T>*>(a.tw));
 #pragma unroll 4
     for (int i = threadIdx.x; i < total; i += blockDim.x)
     {
@@ -1194,8 +1169,7 @@ template <typename T, class F>
 __global__ void __launch_bounds__(F::max_threads, 1) k_fs_rows(const fourstep_args a, const int ts)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ pass_desc sp[kMaxPasses];
-    const F fft(sp, a.d, ts);
+    const F fft(a.d, ts, a.tile);
     cpx<T>* sm       = reinterpret_cast<cpx<T>*>(smem_raw);
     const int n1     = a.n1, n2 = fft.n, S = a.tile, sh = a.tile_shift;
     const int stride = F::gstride(n2);
@@ -1245,7 +1219,7 @@ __global__ void __launch_bounds__(F::max_threads, 1) k_fs_rows(const fourstep_ar
             return;
         }
     }
-    fft.run(sm + gm.g * stride, reinterpret_cast<const cpx<T>*>(a.tw), gm.lt);
+    fft.run(sm, reinterpret_cast<const cpx<T>*>(a.tw));
 #pragma unroll 4
     for (int i = threadIdx.x; i < total; i += blockDim.x)
     {
@@ -1299,7 +1273,7 @@ __global__ void __launch_bounds__(1024, 1) k_fsp_cols(const fourstep_args a)
     const cpx<T>* twA  = reinterpret_cast<const cpx<T>*>(a.twA);
     const cpx<T>* twB  = reinterpret_cast<const cpx<T>*>(a.twB);
     const auto nothing = []() {};
-    const FA fa(nullptr, a.d, TS);
+    const FA fa;
     fa.run_pp([&](int p) { return sm[gg * GA + FA::pi(p)]; },
               [&](int k1, cpx<T> v)
               {
@@ -1337,7 +1311,7 @@ __global__ void __launch_bounds__(1024, 1) k_fsp_rows(const fourstep_args a)
     cpx<T>* B          = sm + S * GB;
     cpx<T>* stg        = FB::npass % 2 == 0 ? sm : B;
     const auto nothing = []() {};
-    const FB fb(nullptr, a.d, TS);
+    const FB fb;
     fb.run_pp([&](int p) { return sm[gg * GB + FB::pi(p)]; },
               [&](int k2, cpx<T> v) { stg[k2 * S + (gg ^ (k2 & (S - 1)))] = v; }, nothing, nothing, sm + gg * GB,
               B + gg * GB, reinterpret_cast<const cpx<T>*>(a.tw), lt);
@@ -1462,7 +1436,7 @@ __global__ void __launch_bounds__(fspt_threads<FA>(), fspt_min_ctas<FA>())
     const cpx<T>* twA = reinterpret_cast<const cpx<T>*>(a.twA);
     const cpx<T>* twB = reinterpret_cast<const cpx<T>*>(a.twB);
     const cpx<T>* tw  = reinterpret_cast<const cpx<T>*>(a.tw);
-    const FA fa(nullptr, a.d, TS);
+    const FA fa;
     if (threadIdx.x == 0)
     {
         mbar_init(&bars[0], 1);
@@ -1567,7 +1541,7 @@ __global__ void __launch_bounds__(fspt_threads<FB>(), fspt_min_ctas<FB>())
     const int lt = three ? int(threadIdx.x) / S : int(threadIdx.x) - g * TS;
     const cpx<T>* tw = reinterpret_cast<const cpx<T>*>(a.tw);
     const auto nothing = []() {};
-    const FB fb(nullptr, a.d, TS);
+    const FB fb;
     if (threadIdx.x == 0)
     {
         mbar_init(&bars[0], 1);
@@ -1669,7 +1643,7 @@ __global__ void __launch_bounds__(fspt_threads<FB>(), fspt_min_ctas<FB>())
     const bool ccs    = a.ccs != 0;
     const long long olen = ccs ? C + 1 : C;
     const auto nothing = []() {};
-    const FB fb(nullptr, a.d, TS);
+    const FB fb;
     // X[k] from Z[k] = u and Z[c - k] = v, w = W_2c^k
     const auto split = [](cpx<T> u, cpx<T> v, cpx<T> w)
     { return scale(u + conj(v), T(0.5)) + w * scale(mul_mi(u - conj(v)), T(0.5)); };
@@ -1767,7 +1741,7 @@ __global__ void __launch_bounds__(fspt_threads<FB>(), fspt_min_ctas<FB>())
 
 // ---------------------------------------------------------------------------------------------------
 // Launchers.  A block_cfg with ct != 0 selects the compile-time kernel of that length (single precision,
-// launched by the launch_ct_* functions of kernels_ct_*.cu); otherwise cfg.ept picks the runtime kernel.
+// launched by the launch_ct_* functions of kernels_ct_*.cu); otherwise the runtime-length kernel runs.
 // ---------------------------------------------------------------------------------------------------
 
 template <typename K, typename... Args>
@@ -1783,14 +1757,6 @@ static cudaError_t go(K kernel, dim3 grid, const block_cfg& c, cudaStream_t st, 
     return cudaGetLastError();
 }
 
-#define KFR_GPU_RUNTIME_DISPATCH(KERNEL, GRID, ...)                                                        \
-    switch (c.ept)                                                                                         \
-    {                                                                                                      \
-    case 16: return go(KERNEL<T, rt_fft<T, 16>>, GRID, c, st, __VA_ARGS__);                                \
-    case 32: return go(KERNEL<T, rt_fft<T, 32>>, GRID, c, st, __VA_ARGS__);                                \
-    default: return cudaErrorInvalidValue;                                                                 \
-    }
-
 #define KFR_GPU_CT_HOOK(CTFN)                                                                              \
     if (c.ct)                                                                                              \
     {                                                                                                      \
@@ -1804,73 +1770,62 @@ static cudaError_t go(K kernel, dim3 grid, const block_cfg& c, cudaStream_t st, 
 #define KFR_GPU_GRID2 dim3(unsigned(c.grid), unsigned(a.batch))
 
 template <typename T>
-cudaError_t launch_c2c(const c2c_args& a, const block_cfg& c, cudaStream_t st)
-{
-    KFR_GPU_CT_HOOK(launch_ct_c2c_f32)
-    KFR_GPU_RUNTIME_DISPATCH(k_c2c, KFR_GPU_GRID1, a, c.ts, c.spc)
-}
-template <typename T>
 cudaError_t launch_bluestein(const bluestein_args& a, const block_cfg& c, cudaStream_t st)
 {
     KFR_GPU_CT_HOOK(launch_ct_bluestein_f32)
-    KFR_GPU_RUNTIME_DISPATCH(k_bluestein, KFR_GPU_GRID1, a, c.ts, c.spc)
+    return a.d.hold == kRpHold ? go(k_bluestein<T, rt_fft<T, kRpHold>>, KFR_GPU_GRID1, c, st, a, c.ts, c.spc)
+                               : go(k_bluestein<T, rt_fft<T, kRpLongHold>>, KFR_GPU_GRID1, c, st, a, c.ts, c.spc);
 }
 template <typename T>
 cudaError_t launch_rader(const rader_args& a, const block_cfg& c, cudaStream_t st)
 {
     KFR_GPU_CT_HOOK(launch_ct_rader_f32)
-    KFR_GPU_RUNTIME_DISPATCH(k_rader, KFR_GPU_GRID1, a, c.ts, c.spc)
+    return a.d.hold == kRpHold ? go(k_rader<T, rt_fft<T, kRpHold>>, KFR_GPU_GRID1, c, st, a, c.ts, c.spc)
+                               : go(k_rader<T, rt_fft<T, kRpLongHold>>, KFR_GPU_GRID1, c, st, a, c.ts, c.spc);
 }
 template <typename T>
 cudaError_t launch_r2c(const real_args& a, const block_cfg& c, cudaStream_t st)
 {
     KFR_GPU_CT_HOOK(launch_ct_r2c_f32)
-    KFR_GPU_RUNTIME_DISPATCH(k_r2c, KFR_GPU_GRID1, a, c.ts, c.spc)
+    return a.d.hold == kRpHold ? go(k_r2c<T, rt_fft<T, kRpHold>>, KFR_GPU_GRID1, c, st, a, c.ts, c.spc)
+                               : go(k_r2c<T, rt_fft<T, kRpLongHold>>, KFR_GPU_GRID1, c, st, a, c.ts, c.spc);
 }
 template <typename T>
 cudaError_t launch_c2r(const real_args& a, const block_cfg& c, cudaStream_t st)
 {
     KFR_GPU_CT_HOOK(launch_ct_c2r_f32)
-    KFR_GPU_RUNTIME_DISPATCH(k_c2r, KFR_GPU_GRID1, a, c.ts, c.spc)
+    return a.d.hold == kRpHold ? go(k_c2r<T, rt_fft<T, kRpHold>>, KFR_GPU_GRID1, c, st, a, c.ts, c.spc)
+                               : go(k_c2r<T, rt_fft<T, kRpLongHold>>, KFR_GPU_GRID1, c, st, a, c.ts, c.spc);
 }
 template <typename T>
 cudaError_t launch_dct2(const dct_args& a, const block_cfg& c, cudaStream_t st)
 {
     KFR_GPU_CT_HOOK(launch_ct_dct2_f32)
-    KFR_GPU_RUNTIME_DISPATCH(k_dct2, KFR_GPU_GRID1, a, c.ts, c.spc)
+    return a.d.hold == kRpHold ? go(k_dct2<T, rt_fft<T, kRpHold>>, KFR_GPU_GRID1, c, st, a, c.ts, c.spc)
+                               : go(k_dct2<T, rt_fft<T, kRpLongHold>>, KFR_GPU_GRID1, c, st, a, c.ts, c.spc);
 }
 template <typename T>
 cudaError_t launch_dct3(const dct_args& a, const block_cfg& c, cudaStream_t st)
 {
     KFR_GPU_CT_HOOK(launch_ct_dct3_f32)
-    KFR_GPU_RUNTIME_DISPATCH(k_dct3, KFR_GPU_GRID1, a, c.ts, c.spc)
+    return a.d.hold == kRpHold ? go(k_dct3<T, rt_fft<T, kRpHold>>, KFR_GPU_GRID1, c, st, a, c.ts, c.spc)
+                               : go(k_dct3<T, rt_fft<T, kRpLongHold>>, KFR_GPU_GRID1, c, st, a, c.ts, c.spc);
 }
-template <typename T>
-cudaError_t launch_fs_cols(const fourstep_args& a, const block_cfg& c, cudaStream_t st)
-{
-    KFR_GPU_CT_HOOK(launch_ct_fs_cols_f32)
-    KFR_GPU_RUNTIME_DISPATCH(k_fs_cols, KFR_GPU_GRID2, a, c.ts)
-}
-template <typename T>
-cudaError_t launch_fs_rows(const fourstep_args& a, const block_cfg& c, cudaStream_t st)
-{
-    KFR_GPU_CT_HOOK(launch_ct_fs_rows_f32)
-    KFR_GPU_RUNTIME_DISPATCH(k_fs_rows, KFR_GPU_GRID2, a, c.ts)
-}
-
 // Compile-time kernel cases for the launch_ct_* functions: CT_KERNEL and CT_ARGS are defined by the caller.
 #define KFR_GPU_CT_CASE(N, TS, ...)                                                                        \
     case N: return go(CT_KERNEL<float, ct_fft<float, N, TS, __VA_ARGS__>>, CT_GRID, c, st, CT_ARGS);
 
-#define KFR_GPU_INSTANTIATE(T)                                                                             \
-    template cudaError_t launch_c2c<T>(const c2c_args&, const block_cfg&, cudaStream_t);                   \
+// The runtime-length kernels, three files per type so that they compile in parallel.  Against the former passes of
+// a fixed register array per thread: real 3600 x 8000 forward 208 -> 143 us, inverse 191 -> 124 us; DCT-II
+// 1000 x 20000 222 -> 175 us; Bluestein 8009 x 500 111 -> 103 us.
+#define KFR_GPU_INSTANTIATE_CONVOLVED(T)                                                                   \
     template cudaError_t launch_bluestein<T>(const bluestein_args&, const block_cfg&, cudaStream_t);       \
-    template cudaError_t launch_rader<T>(const rader_args&, const block_cfg&, cudaStream_t);               \
+    template cudaError_t launch_rader<T>(const rader_args&, const block_cfg&, cudaStream_t);
+#define KFR_GPU_INSTANTIATE_REAL(T)                                                                        \
     template cudaError_t launch_r2c<T>(const real_args&, const block_cfg&, cudaStream_t);                  \
-    template cudaError_t launch_c2r<T>(const real_args&, const block_cfg&, cudaStream_t);                  \
+    template cudaError_t launch_c2r<T>(const real_args&, const block_cfg&, cudaStream_t);
+#define KFR_GPU_INSTANTIATE_DCT(T)                                                                         \
     template cudaError_t launch_dct2<T>(const dct_args&, const block_cfg&, cudaStream_t);                  \
-    template cudaError_t launch_dct3<T>(const dct_args&, const block_cfg&, cudaStream_t);                  \
-    template cudaError_t launch_fs_cols<T>(const fourstep_args&, const block_cfg&, cudaStream_t);          \
-    template cudaError_t launch_fs_rows<T>(const fourstep_args&, const block_cfg&, cudaStream_t);
+    template cudaError_t launch_dct3<T>(const dct_args&, const block_cfg&, cudaStream_t);
 
 } // namespace kfr_gpu

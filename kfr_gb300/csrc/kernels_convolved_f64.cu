@@ -1,0 +1,7 @@
+// Double-precision Bluestein and Rader kernels.
+#include "kernels.cuh"
+
+namespace kfr_gpu
+{
+KFR_GPU_INSTANTIATE_CONVOLVED(double)
+} // namespace kfr_gpu

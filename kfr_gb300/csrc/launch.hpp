@@ -21,11 +21,9 @@ constexpr unsigned kDefaultWaitSpins = 1u << 22;
 unsigned wait_limit();
 unsigned set_wait_limit(unsigned spins);
 
-// Shape of one shared-memory FFT launch: `spc` signals per CTA, `ts` threads per signal, each thread owning
-// at most `ept` elements per pass.
+// Shape of one shared-memory FFT launch: `spc` signals per CTA, `ts` threads per signal (compile-time lengths).
 struct block_cfg
 {
-    int ept;
     int ts;
     int spc;
     int threads;
@@ -44,7 +42,7 @@ struct c2c_args
     int inverse;
     const void* tw;
     fast_div div_n;
-    fft_desc d;
+    rp_desc d; // runtime lengths
     unsigned wait_spins = kDefaultWaitSpins; // persistent pipelined kernels: see kDefaultWaitSpins
 };
 
@@ -61,7 +59,7 @@ struct bluestein_args
     const void* bhat;  // M values: FFT_M of the conjugate chirp, scaled by 1/M
     const void* tw;
     fast_div div_n, div_m;
-    fft_desc d;
+    rp_desc d; // runtime lengths
 };
 
 // Rader's algorithm for a prime length n whose cyclic convolution length L = n - 1 = d.n fits one CTA:
@@ -80,7 +78,7 @@ struct rader_args
     const void* bhat; // L values: DFT_L(b) / L
     const void* tw;
     fast_div div_n, div_l;
-    fft_desc d;
+    rp_desc d; // runtime lengths
 };
 
 // Rader's algorithm with prime-factor convolution DFTs (rader_pfa.cu): in and out 16-byte aligned, signals
@@ -116,7 +114,7 @@ struct real_args
     const void* rtw; // W_{2c}^k for k = 0..c
     const void* tw;
     fast_div div_n, div_out;
-    fft_desc d;
+    rp_desc d; // runtime lengths
     unsigned wait_spins = kDefaultWaitSpins; // persistent pipelined kernels: see kDefaultWaitSpins
 };
 
@@ -130,7 +128,7 @@ struct dct_args
     const void* dtw;  // (cos(pi k / 2n), sin(pi k / 2n)) for k < n
     const void* tw;
     fast_div div_n;
-    fft_desc d;
+    rp_desc d; // runtime lengths
     unsigned wait_spins = kDefaultWaitSpins; // pipelined kernels: see kDefaultWaitSpins
 };
 
@@ -147,13 +145,12 @@ struct fourstep_args
     int tile;             // columns (cols pass) or k1 rows (rows pass) per CTA
     int conj_in, conj_out;
     const void* tw;
-    fft_desc d;
+    rp_desc d; // runtime lengths
     // two-level table for W_N^m: W_N^m = twA[m >> lbits] * twB[m & ((1 << lbits) - 1)]
     const void* twA;
     const void* twB;
     int lbits;
     int tile_shift;  // log2(tile)
-    int same_layout; // cols pass: store back to x's own layout (multi-dimensional axes) and skip the twiddle
     int pingpong;    // compile-time kernels: ping-pong passes over two buffers per signal (2x shared memory)
     fast_div div_n;  // divides by the FFT length of this pass
     int* err;        // persistent pair kernels: set when a wait for a tile copy runs out (may be null)
@@ -192,13 +189,12 @@ struct rp_strided_args
     int lbits;
     rp_desc d;
 };
-template <typename T>
+// H: a.d.hold.
+template <typename T, int H>
 cudaError_t launch_rp_c2c(const rp_c2c_args& a, int threads, int smem, cudaStream_t st);
-template <typename T>
+template <typename T, int H>
 cudaError_t launch_rp_strided(const rp_strided_args& a, bool cols, int threads, int smem, cudaStream_t st);
 
-template <typename T>
-cudaError_t launch_c2c(const c2c_args& a, const block_cfg& c, cudaStream_t st);
 template <typename T>
 cudaError_t launch_bluestein(const bluestein_args& a, const block_cfg& c, cudaStream_t st);
 template <typename T>
@@ -211,10 +207,6 @@ template <typename T>
 cudaError_t launch_dct2(const dct_args& a, const block_cfg& c, cudaStream_t st);
 template <typename T>
 cudaError_t launch_dct3(const dct_args& a, const block_cfg& c, cudaStream_t st);
-template <typename T>
-cudaError_t launch_fs_cols(const fourstep_args& a, const block_cfg& c, cudaStream_t st);
-template <typename T>
-cudaError_t launch_fs_rows(const fourstep_args& a, const block_cfg& c, cudaStream_t st);
 
 // Grid-stride elementwise kernels for the multi-kernel paths: Bluestein at lengths whose convolution does
 // not fit one CTA, and real-DFT / DCT pre- and post-processing around a multi-kernel complex DFT.  The
@@ -310,8 +302,6 @@ cudaError_t prepare_launch(const void* kernel, int threads, int smem, int* per_s
 // SMs of the current device (0 if the query fails), queried once per device.
 int device_sm_count();
 
-// Largest thread count a block FFT kernel may be launched with (elem_bytes = sizeof(real type)).
-int max_threads_for(int elem_bytes, int ept);
 // Largest dynamic shared memory a kernel may use on this device.
 int max_smem_bytes();
 

@@ -71,4 +71,14 @@ int device_sm_count()
     return it->second;
 }
 
+int max_smem_bytes()
+{
+    int dev = 0, v = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess)
+        return 227 * 1024;
+    if (cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess || v <= 0)
+        return 227 * 1024;
+    return v;
+}
+
 } // namespace kfr_gpu

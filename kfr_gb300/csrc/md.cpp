@@ -33,19 +33,11 @@ md_axes<T>::md_axes(const std::vector<long long>& cshape)
         a.rp.reset(new rp_program<T>());
         if (a.rp->build(n, RP_COLS))
             a.tile = a.rp->tiles[0].S;
-        else if (a.rp.reset(), block_program<T>::feasible(n))
+        else
         {
-            a.prog.reset(new block_program<T>());
-            a.prog->build(int(n), CT_FOURSTEP);
-            int t = tile_for(*a.prog);
-            while (t > 1 && t / 2 >= a.inner)
-                t /= 2;
-            a.tile = t;
-            if (t == 0)
-                a.prog.reset();
+            a.rp.reset();
+            a.eng.reset(new complex_engine<T>(n)); // longer than one CTA: transposed 1-D pass
         }
-        if (!a.prog && !a.rp) // longer than one CTA: transposed 1-D pass
-            a.eng.reset(new complex_engine<T>(n));
         axes_.push_back(std::move(a));
     }
 }
@@ -65,9 +57,7 @@ int md_axes<T>::launches(long long batch) const
 {
     int n = 0;
     for (const axis& a : axes_)
-        n += a.eng          ? 2 + a.eng->launches(batch * a.outer * a.inner)
-             : a.rp ? 1
-                            : int((batch * a.outer + 65534) / 65535);
+        n += a.eng ? 2 + a.eng->launches(batch * a.outer * a.inner) : 1;
     return n;
 }
 
@@ -86,53 +76,17 @@ void md_axes<T>::run(void* data, long long batch, bool inverse, void* scratch, c
             check(launch_transpose<T>(data, tr, batch * ax.outer, ax.inner, ax.n, st), "transpose axis back");
             continue;
         }
-        if (ax.rp)
-        {
-            rp_strided_args a;
-            a.in         = data;
-            a.out        = data;
-            a.batch      = batch * ax.outer;
-            a.sig_stride = ax.n * ax.inner;
-            a.pitch      = ax.inner;
-            a.conj_in    = inverse;
-            a.conj_out   = inverse;
-            a.twA = a.twB = nullptr;
-            a.lbits      = 0;
-            ax.rp->run(a, st);
-            continue;
-        }
-        const long long sigs = batch * ax.outer;
-        for (long long b0 = 0; b0 < sigs; b0 += 65535)
-        {
-            const long long nb = std::min<long long>(65535, sigs - b0);
-            char* base         = static_cast<char*>(data) + b0 * ax.n * ax.inner * 2 * sizeof(T);
-            fourstep_args a;
-            a.err         = nullptr;
-            a.in          = base;
-            a.out         = base;
-            a.batch       = nb;
-            a.sig_stride  = ax.n * ax.inner;
-            a.n1          = int(ax.n);
-            a.n2          = int(ax.inner);
-            a.tile        = ax.tile;
-            int sh        = 0;
-            while ((1 << sh) < ax.tile)
-                sh++;
-            a.tile_shift  = sh;
-            a.same_layout = 1;
-            a.pingpong    = 0;
-            a.conj_in     = inverse;
-            a.conj_out    = inverse;
-            a.tw          = ax.prog->tw.get();
-            a.d           = ax.prog->desc;
-            a.twA         = nullptr;
-            a.twB         = nullptr;
-            a.lbits       = 0;
-            a.div_n       = make_fast_div(uint32_t(ax.n));
-            block_cfg c   = ax.prog->cfg_tile(ax.tile);
-            c.grid        = (ax.inner + ax.tile - 1) / ax.tile;
-            check(launch_fs_cols<T>(a, c, st), "launch multi-dimensional axis pass");
-        }
+        rp_strided_args a;
+        a.in         = data;
+        a.out        = data;
+        a.batch      = batch * ax.outer;
+        a.sig_stride = ax.n * ax.inner;
+        a.pitch      = ax.inner;
+        a.conj_in    = inverse;
+        a.conj_out   = inverse;
+        a.twA = a.twB = nullptr;
+        a.lbits      = 0;
+        ax.rp->run(a, st);
     }
 }
 
@@ -146,7 +100,7 @@ std::string md_axes<T>::describe() const
             s << " axis{n=" << a.n << " inner=" << a.inner << " transposed [" << a.eng->describe() << "]}";
         else
             s << " axis{n=" << a.n << " inner=" << a.inner << " tile=" << a.tile << " "
-              << (a.rp ? a.rp->describe() : a.prog->describe()) << "}";
+              << a.rp->describe() << "}";
     }
     return s.str();
 }

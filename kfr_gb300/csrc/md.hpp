@@ -39,8 +39,7 @@ private:
     {
         long long n, inner, outer;
         int tile;
-        std::unique_ptr<rp_program<T>> rp;      // column pass on the runtime-length block FFT
-        std::unique_ptr<block_program<T>> prog; // column pass of the other axes that fit one CTA
+        std::unique_ptr<rp_program<T>> rp;      // column pass (axes that fit one CTA)
         std::unique_ptr<complex_engine<T>> eng; // transposed 1-D pass (longer axes)
     };
     std::vector<axis> axes_;

@@ -217,109 +217,12 @@ void host_dft(std::vector<std::complex<double>>& a)
     }
 }
 
-std::vector<int> factor_radices(long long n)
+bool is_smooth(long long n)
 {
-    std::vector<int> r;
-    if (n <= 1)
-        return r;
-    int a = 0;
-    while (n % 2 == 0)
-    {
-        n /= 2;
-        a++;
-    }
-    const int q = a / 4, rem = a % 4;
-    if (rem == 1 && q >= 1)
-    {
-        for (int i = 0; i < q - 1; i++)
-            r.push_back(16);
-        r.push_back(8);
-        r.push_back(4);
-    }
-    else
-    {
-        for (int i = 0; i < q; i++)
-            r.push_back(16);
-        if (rem == 1)
-            r.push_back(2);
-        else if (rem == 2)
-            r.push_back(4);
-        else if (rem == 3)
-            r.push_back(8);
-    }
-    while (n % 9 == 0)
-    {
-        r.push_back(9);
-        n /= 9;
-    }
-    for (int p : { 3, 5, 7, 11, 13 })
+    for (long long p = 2; p <= kGenericMax && n > 1; p++)
         while (n % p == 0)
-        {
-            r.push_back(p);
             n /= p;
-        }
-    for (long long p = 17; p * p <= n; p += 2)
-        while (n % p == 0)
-        {
-            if (p > kGenericMax)
-                return {};
-            r.push_back(int(p));
-            n /= p;
-        }
-    if (n > 1)
-    {
-        if (n > kGenericMax)
-            return {};
-        r.push_back(int(n));
-    }
-    return r;
-}
-
-static bool is_codelet(int r)
-{
-    switch (r)
-    {
-    case 1: // a copy (the ends of a runtime-length block FFT whose other radices are primes)
-    case 2:
-    case 3:
-    case 4:
-    case 5:
-    case 7:
-    case 8:
-    case 9:
-    case 11:
-    case 13:
-    case 16: return true;
-    // Good-Thomas composites: only in compile-time radix lists (factor_radices never produces them)
-    case 6:
-    case 10:
-    case 12:
-    case 14:
-    case 15:
-    case 18: return true;
-    default: return false;
-    }
-}
-
-// Threads per signal needed by a radix sequence at `ept` elements per thread (0 = infeasible).
-int threads_needed(long long n, const std::vector<int>& radices, int ept)
-{
-    long long ts = 1;
-    for (int r : radices)
-    {
-        long long need;
-        if (is_codelet(r))
-        {
-            if (ept < r)
-                return 0;
-            const long long per = ept / r;
-            need                = (n / r + per - 1) / per;
-        }
-        else
-            need = (n + ept - 1) / ept;
-        ts = std::max(ts, need);
-    }
-    return int(std::min<long long>(ts, 1 << 20));
+    return n <= 1;
 }
 
 static int ilog2(int x)
@@ -332,8 +235,8 @@ static int ilog2(int x)
 
 int smem_budget()
 {
-    // dynamic shared memory left after the static pass-descriptor array and a small reserve
-    static const int budget = max_smem_bytes() - int(sizeof(pass_desc)) * kMaxPasses - 1024;
+    // dynamic shared memory less a small reserve
+    static const int budget = max_smem_bytes() - 1024;
     return budget;
 }
 
@@ -375,90 +278,64 @@ template bool ct_lookup<double>(int, int, int&, std::vector<int>&);
 // block_program
 // ------------------------------------------------------------------------------------------------------
 
+// Radices of n (prime factors up to kGenericMax) for a one-CTA transform and the values its threads hold; empty if it
+// does not fit.  Threads hold 16 values, 32 where only that fits.
 template <typename T>
-bool block_program<T>::feasible(long long n)
+static std::vector<int> one_cta_radices(long long n, bool smem_io, int& hold)
 {
-    if (n < 2 || n > (1 << 20))
-        return false;
-    const auto rad = factor_radices(n);
-    if (rad.empty() || int(rad.size()) > kMaxPasses)
-        return false;
-    if (static_cast<long long>(padded_len_host<T>(int(n))) * static_cast<long long>(2 * sizeof(T)) > smem_budget())
-        return false;
-    for (int ept : { 16, 32 })
+    for (int h : { kRpHold, kRpLongHold })
     {
-        const int ts = threads_needed(n, rad, ept);
-        if (ts > 0 && ts <= max_threads_for(int(sizeof(T)), ept))
-            return true;
+        const auto rad = rp_radices(n, kGenericMax, h);
+        if (rp_fits(rad, int(2 * sizeof(T)), smem_budget(), smem_io, h))
+        {
+            hold = h;
+            return rad;
+        }
     }
-    return false;
+    return {};
 }
 
 template <typename T>
-void block_program<T>::build(int n_, int kind, const std::vector<int>* order, int ept_only)
+bool block_program<T>::feasible(long long n)
+{
+    int hold = 0;
+    return !one_cta_radices<T>(n, true, hold).empty();
+}
+
+template <typename T>
+void block_program<T>::build(int n_, int kind)
 {
     n  = n_;
     ct = 0;
-    int cts = 0;
-    std::vector<int> ctr;
-    if (!order && kind != CT_NONE && ct_lookup<T>(kind, n, cts, ctr))
+    std::memset(&desc, 0, sizeof(desc));
+    if (ct_lookup<T>(kind, n, ts, radices))
     {
-        radices = ctr;
-        ts      = cts;
-        ept     = 16;
         ct      = n;
+        gstride = ct_group_stride_f32(n, ts);
+        desc.n  = n;
     }
     else
     {
-        radices = order ? *order : factor_radices(n);
-        if (radices.empty() || int(radices.size()) > kMaxPasses)
-            throw std::invalid_argument("internal: length has no one-CTA radix plan");
-        long long prod = 1;
-        for (int r : radices)
-            prod *= r;
-        if (prod != n)
-            throw std::invalid_argument("internal: radix order does not multiply to the length");
-        ept = 0;
-        for (int e : { 16, 32 })
-        {
-            if (ept_only && e != ept_only)
-                continue;
-            const int t = threads_needed(n, radices, e);
-            if (t > 0 && t <= max_threads_for(int(sizeof(T)), e))
-            {
-                ept = e;
-                ts  = t;
-                break;
-            }
-        }
-        if (ept == 0)
+        int hold = 0;
+        radices  = one_cta_radices<T>(n, true, hold);
+        if (radices.empty())
+            throw std::invalid_argument("internal: length exceeds one CTA");
+        desc  = rp_build(radices, RP_SIGNALS, 1, int(2 * sizeof(T)), true, hold);
+        shape = rp_choose(desc, desc.elems, int(2 * sizeof(T)), smem_budget(), true);
+        if (!shape.spc)
             throw std::invalid_argument("internal: length exceeds one CTA");
     }
-    gstride = padded_len_host<T>(n);
-    if (ct && sizeof(T) == 4)
-        gstride = ct_group_stride_f32(n, ts);
-    std::memset(&desc, 0, sizeof(desc));
-    desc.n     = n;
-    desc.npass = int(radices.size());
-    const auto table = pass_twiddles<T>(radices, desc.pass);
+    const auto table = pass_twiddles<T>(radices);
     tw.upload(table.data(), table.size() * sizeof(std::complex<T>));
 }
 
 template <typename T>
-std::vector<std::complex<T>> pass_twiddles(const std::vector<int>& radices, pass_desc* passes)
+std::vector<std::complex<T>> pass_twiddles(const std::vector<int>& radices)
 {
     std::vector<std::complex<T>> table;
     long long ns = 1;
-    for (size_t i = 0; i < radices.size(); i++)
+    for (const int R : radices)
     {
-        const int R = radices[i];
-        if (passes)
-        {
-            passes[i].radix  = R;
-            passes[i].ns     = int(ns);
-            passes[i].div_ns = make_fast_div(uint32_t(ns));
-            passes[i].tw_off = int(table.size());
-        }
         const long long L = ns * R;
         if (ns > 1)
             for (int r = 1; r < R; r++)
@@ -467,9 +344,7 @@ std::vector<std::complex<T>> pass_twiddles(const std::vector<int>& radices, pass
                     const auto w = twiddle(k * r, L);
                     table.emplace_back(T(w.real()), T(w.imag()));
                 }
-        if (passes)
-            passes[i].wr_off = int(table.size());
-        if (!is_codelet(R))
+        if (R > kRpMaxRadix && R != 18) // primes without a codelet
             for (int m = 0; m < R; m++)
             {
                 const auto w = twiddle(m, R);
@@ -482,28 +357,32 @@ std::vector<std::complex<T>> pass_twiddles(const std::vector<int>& radices, pass
     return table;
 }
 
+template std::vector<std::complex<float>> pass_twiddles<float>(const std::vector<int>&);
+template std::vector<std::complex<double>> pass_twiddles<double>(const std::vector<int>&);
+
 template <typename T>
-block_cfg block_program<T>::cfg(long long batch, int spc_cap) const
+block_cfg block_program<T>::cfg(long long batch) const
 {
     block_cfg c;
-    c.ept              = ept;
-    c.ts               = ts;
-    const int per_sig  = gstride * int(2 * sizeof(T));
-    const int max_thr  = ct ? (sizeof(T) == 4 ? 1024 : 512) : max_threads_for(int(sizeof(T)), ept);
-    int spc            = std::max(1, 256 / ts);
-    spc                = std::min(spc, std::max(1, max_thr / ts));
-    spc                = std::min(spc, std::max(1, smem_budget() / per_sig));
+    if (!ct)
+    {
+        const rp_shape s = rp_shrink(desc, shape, batch, 152, true);
+        c.ts             = 0;
+        c.spc            = s.spc;
+        c.threads        = s.threads;
+        c.smem           = s.spc * desc.elems * int(2 * sizeof(T));
+        c.grid           = (batch + s.spc - 1) / s.spc;
+        return c;
+    }
+    const int per_sig = gstride * int(2 * sizeof(T));
+    int spc           = std::max(1, 256 / ts);
+    spc               = std::min(spc, std::max(1, smem_budget() / per_sig));
     // keep at least ~2 CTAs per SM when the batch allows it
     const long long want_ctas = 2LL * 152;
     if (batch < want_ctas * spc)
         spc = int(std::max<long long>(1, std::min<long long>(spc, (batch + want_ctas - 1) / want_ctas)));
-    if (spc_cap > 0)
-        spc = std::min(spc, spc_cap);
-    c.spc     = spc;
-    c.threads = ((spc * ts + 31) / 32) * 32;
-    c.smem    = spc * per_sig;
+    c         = cfg_tile(spc);
     c.grid    = (batch + spc - 1) / spc;
-    c.ct      = ct;
     return c;
 }
 
@@ -511,7 +390,6 @@ template <typename T>
 block_cfg block_program<T>::cfg_tile(int tile) const
 {
     block_cfg c;
-    c.ept     = ept;
     c.ts      = ts;
     c.spc     = tile;
     c.threads = ((tile * ts + 31) / 32) * 32;
@@ -528,10 +406,10 @@ std::string block_program<T>::describe() const
     s << "block_fft n=" << n << " radices=";
     for (size_t i = 0; i < radices.size(); i++)
         s << (i ? "x" : "") << radices[i];
-    s << (ct ? " compile-time" : " ept=") ;
-    if (!ct)
-        s << ept;
-    s << " threads/signal=" << ts;
+    if (ct)
+        s << " compile-time threads/signal=" << ts;
+    else
+        s << " signals/CTA=" << shape.spc << " threads=" << shape.threads;
     return s.str();
 }
 
@@ -540,29 +418,36 @@ std::string block_program<T>::describe() const
 // ------------------------------------------------------------------------------------------------------
 
 template <typename T>
+bool rp_program<T>::feasible(long long n)
+{
+    int hold = 0;
+    return !one_cta_radices<T>(n, false, hold).empty();
+}
+
+template <typename T>
 bool rp_program<T>::build(long long n, rp_layout lay)
 {
-    layout            = lay;
-    const int budget  = max_smem_bytes() - 1024;
-    const auto rad    = rp_radices(n);
+    layout           = lay;
+    const int budget = smem_budget();
+    int hold         = 0;
+    const auto rad   = one_cta_radices<T>(n, false, hold);
     if (rad.empty())
         return false;
     if (lay == RP_SIGNALS)
     {
-        desc      = rp_build(rad, lay, 1, elem);
-        sig_elems = rp_smem_elems(desc, lay, 1);
-        shape     = rp_choose(desc, sig_elems, elem, budget);
+        desc  = rp_build(rad, lay, 1, elem, false, hold);
+        shape = rp_choose(desc, desc.elems, elem, budget);
         if (!shape.spc)
             return false;
     }
     else
     {
-        for (int S = rp_tile(rad, lay, elem, budget); S >= 1 && tiles.size() < 3; S /= 2)
+        for (int S = rp_tile(rad, elem, budget, hold); S >= 1 && tiles.size() < 3; S /= 2)
         {
             tile t;
-            t.d          = rp_build(rad, lay, S, elem);
-            t.S          = S;
-            t.smem       = rp_smem_elems(t.d, lay, S) * elem;
+            t.d    = rp_build(rad, lay, S, elem, false, hold);
+            t.S    = S;
+            t.smem = t.d.elems * elem;
             if (t.smem > budget) // more padding than rp_tile allows for
                 continue;
             const int bf = S * t.d.pass[0].nbf;
@@ -573,7 +458,7 @@ bool rp_program<T>::build(long long n, rp_layout lay)
             return false;
     }
     radices          = rad;
-    const auto table = pass_twiddles<T>(rad, nullptr);
+    const auto table = pass_twiddles<T>(rad);
     tw.upload(table.data(), table.size() * sizeof(std::complex<T>));
     return true;
 }
@@ -586,7 +471,7 @@ void rp_program<T>::configure(rp_c2c_args& a, long long batch, int& threads, int
     a.tw             = tw.get();
     a.d              = desc;
     threads          = s.threads;
-    smem             = s.spc * sig_elems * elem;
+    smem             = s.spc * desc.elems * elem;
 }
 
 template <typename T>
@@ -606,8 +491,21 @@ void rp_program<T>::run(rp_strided_args& a, cudaStream_t st) const
     const tile& t = pick(a.pitch, a.batch);
     a.d           = t.d;
     a.tw          = tw.get();
-    check(launch_rp_strided<T>(a, layout == RP_COLS, t.threads, t.smem, st),
-          layout == RP_COLS ? "launch column DFTs" : "launch row DFTs");
+    // at most 2^31 - 1 tiles per launch
+    const long long total = a.batch, tiles = (a.pitch + t.S - 1) / t.S;
+    const long long most = std::max<long long>(1, 0x7fffffffLL / tiles);
+    const char* in       = static_cast<const char*>(a.in);
+    char* out            = static_cast<char*>(a.out);
+    for (long long b = 0; b < total; b += most)
+    {
+        a.batch = std::min(most, total - b);
+        a.in    = in + b * a.sig_stride * elem;
+        a.out   = out + b * a.sig_stride * elem;
+        check(t.d.hold == kRpHold ? launch_rp_strided<T, kRpHold>(a, layout == RP_COLS, t.threads, t.smem, st)
+                                  : launch_rp_strided<T, kRpLongHold>(a, layout == RP_COLS, t.threads, t.smem, st),
+              layout == RP_COLS ? "launch column DFTs" : "launch row DFTs");
+    }
+    a.batch = total;
 }
 
 template <typename T>
@@ -638,16 +536,15 @@ static bool is_prime(long long n)
     return true;
 }
 
-// Relative cost of a one-CTA FFT of length n: one unit per element per codelet pass, R/4 per element for a
-// generic radix-R pass (a length-R dot product per output).
+// Relative cost of an FFT of length n (instructions), 1e30 if n has no radices.
 static double fft_cost(long long n)
 {
-    const auto rad = factor_radices(n);
+    const auto rad = rp_radices(n, kGenericMax);
     if (rad.empty())
         return 1e30;
     double c = 0;
     for (int r : rad)
-        c += is_codelet(r) ? 1.0 : r / 4.0;
+        c += rp_pass_cost(r);
     return double(n) * c;
 }
 
@@ -739,27 +636,34 @@ complex_engine<T>::complex_engine(long long n) : n_(n)
     long long m = 1;
     while (m < 2 * n - 1)
         m <<= 1;
-    const bool direct_ok    = block_program<T>::feasible(n);
+    const bool direct_ok    = rp_program<T>::feasible(n);
     const bool rader_ok     = is_prime(n) && n > 13 && block_program<T>::feasible(n - 1);
-    const bool bluestein_ok = block_program<T>::feasible(m);
+    const bool bluestein_ok = !direct_ok && !rader_ok ? block_program<T>::feasible(m) : m <= (1 << 14);
     const double c_direct   = direct_ok ? fft_cost(n) : 1e30;
-    const double c_rader    = rader_ok ? 2.0 * fft_cost(n - 1) + 2.0 * n : 1e30;
-    const double c_blue     = bluestein_ok ? 2.0 * fft_cost(m) + 3.0 * n : 1e30;
+    const double c_rader    = rader_ok ? 2.0 * fft_cost(n - 1) + 40.0 * n : 1e30;
+    // (a direct plan with only codelet radices is always the cheapest)
+    const double c_blue = bluestein_ok && c_direct > 200.0 * n && block_program<T>::feasible(m)
+                              ? 2.0 * fft_cost(m) + 60.0 * n
+                              : 1e30;
     if (direct_ok && c_direct <= c_rader && c_direct <= c_blue)
     {
         k_ = kind::smem;
         int ts = 0;
         std::vector<int> ctr;
-        // lengths without a compile-time kernel: the runtime-length block FFT, or the in-place runtime
-        // passes where that has no plan (a prime factor of 17 to 127, too long for its threads)
-        if (ct_lookup<T>(CT_C2C, int(n), ts, ctr) || !rp_.build(n, RP_SIGNALS))
+        // the runtime-length block FFT where there is no compile-time kernel
+        if (!ct_lookup<T>(CT_C2C, int(n), ts, ctr))
+        {
+            if (!rp_.build(n, RP_SIGNALS))
+                throw std::invalid_argument("internal: length exceeds one CTA");
+        }
+        else
         {
             prog_.build(int(n), CT_C2C);
             plan_pipe();
         }
         return;
     }
-    if (rader_ok && c_rader <= c_blue)
+    if (rader_ok && c_rader <= c_blue && c_rader <= c_direct)
     {
         init_rader(n);
         return;
@@ -769,7 +673,7 @@ complex_engine<T>::complex_engine(long long n) : n_(n)
         init_bluestein(n);
         return;
     }
-    if (!factor_radices(n).empty() && plan_fourstep(n))
+    if (is_smooth(n) && plan_fourstep(n))
         return;
     init_bluestein(n);
 }
@@ -980,113 +884,56 @@ void complex_engine<T>::init_bluestein(long long n)
     }
 }
 
-template <typename T>
-int tile_for(const block_program<T>& p, int buffers)
+// Largest power-of-two number of signals (<= 16) of the compile-time length `p` that fit one CTA with `buffers`
+// shared-memory buffers per signal: the column / row tile of the strided passes.
+static int tile_for(const block_program<float>& p, int buffers)
 {
-    const int per_sig = buffers * (p.gstride ? p.gstride : padded_len_host<T>(p.n)) * int(2 * sizeof(T));
-    const int max_thr = p.ct ? (sizeof(T) == 4 ? 1024 : 512) : max_threads_for(int(sizeof(T)), p.ept);
+    const int per_sig = buffers * p.gstride * 8;
     int s             = 16;
-    while (s > 1 && (s * per_sig > smem_budget() || s * p.ts > max_thr))
+    while (s > 1 && (s * per_sig > smem_budget() || s * p.ts > 1024))
         s /= 2;
-    if (s * per_sig > smem_budget() || s * p.ts > max_thr)
-        return 0;
     return s;
 }
 
 template <typename T>
 bool complex_engine<T>::plan_fourstep(long long n)
 {
-    long long best_n1 = 0;
-    int best_score    = -1;
-    double best_bal   = 1e30;
-    for (long long n1 = 2; n1 * 2 <= n && n1 <= (1 << 16); n1++)
+    if constexpr (sizeof(T) == 4)
     {
-        if (n % n1)
-            continue;
-        const long long n2 = n / n1;
-        if (n2 > (1 << 16) || n1 * n2 != n)
-            continue;
-        if (!block_program<T>::feasible(n1) || !block_program<T>::feasible(n2))
-            continue;
-        block_program<T> a, b;
-        a.n = int(n1);
-        b.n = int(n2);
-        // thread shape without uploading tables
-        a.radices = factor_radices(n1);
-        b.radices = factor_radices(n2);
-        for (auto* p : { &a, &b })
-            for (int e : { 16, 32 })
+        int a = 0, b = 0;
+#define KFR_GPU_PAIR_OF(A, B)                                                                              \
+    if (n == (long long)A * B)                                                                             \
+        a = A, b = B;
+        KFR_CT_FSPAIR_F32(KFR_GPU_PAIR_OF)
+#undef KFR_GPU_PAIR_OF
+        if (a)
+        {
+            k_  = kind::fourstep;
+            n1_ = a;
+            n2_ = b;
+            pcols_.build(a, CT_FOURSTEP);
+            prows_.build(b, CT_FOURSTEP);
+            // tiles of the kernels that run where the pair kernels cannot (launch_ct_fsp_f32 then answers
+            // cudaErrorNotSupported): ping-pong passes (two buffers per signal) unless that would shrink a tile
+            // below 8 signals (short row segments coalesce poorly)
+            const auto tiles = [](const block_program<T>& p, int& tile, bool& pp)
             {
-                const int t = threads_needed(p->n, p->radices, e);
-                if (t > 0 && t <= max_threads_for(int(sizeof(T)), e))
-                {
-                    p->ept = e;
-                    p->ts  = t;
-                    break;
-                }
-            }
-        const int sc = tile_for(a), sr = tile_for(b);
-        if (sc == 0 || sr == 0)
-            continue;
-        const int score   = std::min(std::min(sc, sr), 16);
-        const double bal  = std::fabs(std::log(double(n1)) - std::log(double(n2)));
-        if (score > best_score || (score == best_score && bal < best_bal))
-        {
-            best_score = score;
-            best_bal   = bal;
-            best_n1    = n1;
-        }
-    }
-    if (best_n1 == 0)
-        return false;
-    {
-        int ts = 0;
-        std::vector<int> ctr;
-        const bool pair = sizeof(T) == 4 && ct_lookup<T>(CT_FOURSTEP, int(best_n1), ts, ctr) &&
-                          ct_lookup<T>(CT_FOURSTEP, int(n / best_n1), ts, ctr) &&
-                          has_ct_fsp_f32(int(best_n1), int(n / best_n1));
-        if (!pair && plan_fourstep_rp(n))
+                tile         = tile_for(p, 1);
+                const int t2 = tile_for(p, 2);
+                pp           = t2 >= 8 || t2 == tile;
+                if (pp)
+                    tile = t2;
+            };
+            tiles(pcols_, tile_c_, pp_c_);
+            tiles(prows_, tile_r_, pp_r_);
+            pair_ = true;
+            err_.alloc(sizeof(int)); // the persistent tensor-copy pair kernels report a copy that never lands
+            check(cudaMemset(err_.get(), 0, sizeof(int)), "clear error flag");
+            upload_roots(n);
             return true;
-    }
-    k_  = kind::fourstep;
-    n1_ = best_n1;
-    n2_ = n / best_n1;
-    pcols_.build(int(n1_), CT_FOURSTEP);
-    prows_.build(int(n2_), CT_FOURSTEP);
-    tile_c_ = tile_for(pcols_);
-    tile_r_ = tile_for(prows_);
-    // compile-time passes run ping-pong (two buffers per signal) unless that would shrink a tile below 8
-    // signals (short row segments coalesce poorly)
-    pp_c_ = pp_r_ = pair_ = false;
-    // tiles of the generic compile-time passes (run ping-pong unless that would shrink a tile below 8)
-    if (pcols_.ct)
-    {
-        const int t2 = tile_for(pcols_, 2);
-        if (t2 >= 8 || t2 == tile_c_)
-        {
-            tile_c_ = t2;
-            pp_c_   = true;
         }
     }
-    if (prows_.ct)
-    {
-        const int t2 = tile_for(prows_, 2);
-        if (t2 >= 8 || t2 == tile_r_)
-        {
-            tile_r_ = t2;
-            pp_r_   = true;
-        }
-    }
-    // both passes fully compile time (their tiles fixed by the kernels); the generic passes run where the
-    // pair kernels cannot (launch_ct_fsp_f32 then answers cudaErrorNotSupported)
-    if (sizeof(T) == 4 && pcols_.ct && prows_.ct && has_ct_fsp_f32(int(n1_), int(n2_)))
-    {
-        pair_ = true;
-        err_.alloc(sizeof(int)); // the persistent tensor-copy pair kernels report a copy that never lands
-        check(cudaMemset(err_.get(), 0, sizeof(int)), "clear error flag");
-    }
-    upload_roots(n);
-    return true;
+    return plan_fourstep_rp(n);
 }
 
 template <typename T>
@@ -1120,13 +967,13 @@ template <typename T>
 bool complex_engine<T>::plan_fourstep_rp(long long n)
 {
     constexpr int elem = int(2 * sizeof(T));
-    const int budget   = max_smem_bytes() - 1024;
-    const auto cost    = [&](long long m, rp_layout lay) -> double
+    const auto cost    = [&](long long m) -> double
     {
-        const auto rad = rp_radices(m);
+        int hold       = 0;
+        const auto rad = one_cta_radices<T>(m, false, hold);
         if (rad.empty())
             return -1;
-        const int S = rp_tile(rad, lay, elem, budget);
+        const int S = rp_tile(rad, elem, smem_budget(), hold);
         if (!S)
             return -1;
         double c = 0;
@@ -1136,18 +983,19 @@ bool complex_engine<T>::plan_fourstep_rp(long long n)
         const double width = double(S * elem) / 128;
         return c + (width >= 1 ? 0.0 : 12.0 * (1 / width - 1));
     };
-    std::map<long long, double> ccost, rcost;
-    const auto cached = [&](std::map<long long, double>& m, long long v, rp_layout lay)
+    std::map<long long, double> memo;
+    const auto cached = [&](long long v)
     {
-        const auto f = m.find(v);
-        return f != m.end() ? f->second : m[v] = cost(v, lay);
+        const auto f = memo.find(v);
+        return f != memo.end() ? f->second : memo[v] = cost(v);
     };
-    double best = -1;
-    for (long long n1 = 8; n1 * 8 <= n && n1 <= (1 << 14); n1++)
+    double best         = -1;
+    const long long top = smem_budget() / elem; // longest one-CTA length
+    for (long long n1 = 2; n1 * 2 <= n && n1 <= top; n1++)
     {
-        if (n % n1 || n / n1 > (1 << 14))
+        if (n % n1 || n / n1 > top)
             continue;
-        const double c = cached(ccost, n1, RP_COLS), r = c < 0 ? -1 : cached(rcost, n / n1, RP_ROWS);
+        const double c = cached(n1), r = c < 0 ? -1 : cached(n / n1);
         if (r < 0)
             continue;
         if (best < 0 || c + r < best)
@@ -1179,8 +1027,6 @@ bool complex_engine<T>::pair_view_of(pair_view& v) const
     v.twA     = twA_.get();
     v.twB     = twB_.get();
     v.lbits   = lbits_;
-    v.dcols   = pcols_.desc;
-    v.drows   = prows_.desc;
     v.err     = static_cast<int*>(err_.get());
     return true;
 }
@@ -1294,7 +1140,9 @@ void complex_engine<T>::execute(void* out, const void* in, long long batch, long
             a.inverse = inverse;
             int threads = 0, smem = 0;
             rp_.configure(a, batch, threads, smem);
-            check(launch_rp_c2c<T>(a, threads, smem, st), "launch c2c");
+            check(a.d.hold == kRpHold ? launch_rp_c2c<T, kRpHold>(a, threads, smem, st)
+                                      : launch_rp_c2c<T, kRpLongHold>(a, threads, smem, st),
+                  "launch c2c");
             return;
         }
         c2c_args a;
@@ -1331,7 +1179,8 @@ void complex_engine<T>::execute(void* out, const void* in, long long batch, long
             a.in    = static_cast<const char*>(in) + done * n_ * esz;
             a.out   = static_cast<char*>(out) + done * n_ * esz;
             a.batch = batch - done;
-            check(launch_c2c<T>(a, prog_.cfg(batch - done), st), "launch c2c");
+            if constexpr (sizeof(T) == 4) // compile-time lengths
+                check(launch_ct_c2c_f32(a, prog_.cfg(batch - done), st), "launch c2c");
         }
         return;
     }
@@ -1444,7 +1293,6 @@ void complex_engine<T>::execute(void* out, const void* in, long long batch, long
             a.sig_stride = n_;
             a.n1         = int(n1_);
             a.n2         = int(n2_);
-            a.same_layout = 0;
             a.twA        = twA_.get();
             a.twB        = twB_.get();
             a.lbits      = lbits_;
@@ -1465,7 +1313,7 @@ void complex_engine<T>::execute(void* out, const void* in, long long batch, long
                 if (pp_c_)
                     cc.smem *= 2; // ping-pong buffers
                 cc.grid = (n2_ + tile_c_ - 1) / tile_c_;
-                check(launch_fs_cols<T>(a, cc, st), "launch four-step columns");
+                check(launch_ct_fs_cols_f32(a, cc, st), "launch four-step columns");
             }
             // row pass: scratch -> out
             a.in       = scr;
@@ -1484,7 +1332,7 @@ void complex_engine<T>::execute(void* out, const void* in, long long batch, long
                 if (pp_r_)
                     cr.smem *= 2;
                 cr.grid = (n1_ + tile_r_ - 1) / tile_r_;
-                check(launch_fs_rows<T>(a, cr, st), "launch four-step rows");
+                check(launch_ct_fs_rows_f32(a, cr, st), "launch four-step rows");
             }
         }
         return;
@@ -1763,13 +1611,11 @@ void real_engine<T>::forward(void* out, const void* in, long long batch, bool cc
             a.in          = static_cast<const T*>(in) + b0 * n_;
             a.out         = y;
             a.tw          = pv.tw_cols;
-            a.d           = pv.dcols;
             a.div_n       = make_fast_div(uint32_t(pv.n1));
             check(launch_ct_fsp_r2c_f32(a, true, st), "launch r2c four-step columns");
             a.in    = y;
             a.out   = static_cast<std::complex<T>*>(out) + b0 * olen;
             a.tw    = pv.tw_rows;
-            a.d     = pv.drows;
             a.div_n = make_fast_div(uint32_t(pv.n2));
             check(launch_ct_fsp_r2c_f32(a, false, st), "launch r2c four-step rows with the split");
         }
@@ -2033,8 +1879,6 @@ std::string dct_engine<T>::describe() const
     return s.str();
 }
 
-template int tile_for<float>(const block_program<float>&, int);
-template int tile_for<double>(const block_program<double>&, int);
 template struct block_program<float>;
 template struct block_program<double>;
 template struct rp_program<float>;

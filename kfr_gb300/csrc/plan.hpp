@@ -68,8 +68,8 @@ void host_dft(std::vector<std::complex<double>>& a);
 // The same for lengths with small prime factors, over one table of roots (fast for long smooth lengths).
 void host_dft_smooth(std::vector<std::complex<double>>& a);
 
-// Radix sequence for a one-CTA length; empty if a prime factor exceeds kGenericMax.
-std::vector<int> factor_radices(long long n);
+// Whether every prime factor of n is at most kGenericMax.
+bool is_smooth(long long n);
 
 // Kernel kinds with compile-time specialised lengths (ct_table.hpp).
 enum ct_kind
@@ -88,37 +88,35 @@ enum ct_kind
 template <typename T>
 bool ct_lookup(int kind, int n, int& ts, std::vector<int>& radices);
 
-// Descriptor, twiddles and thread shape of a one-CTA FFT of length n.
+// Descriptor, twiddles and thread shape of an in-place one-CTA FFT of length n: a compile-time kernel of `kind`, or
+// the runtime-length block FFT (rp.hpp) from and to shared memory.
 template <typename T>
 struct block_program
 {
     int n   = 0;
-    int ept = 16;
-    int ts  = 1;
+    int ts  = 1; // compile-time lengths: threads per signal
     int ct  = 0; // nonzero: the compile-time kernel of this length is used
-    int gstride = 0; // elements between the shared-memory slots of consecutive signals
-    fft_desc desc{};
+    int gstride = 0; // compile-time lengths: elements between the shared-memory slots of consecutive signals
+    rp_desc desc{};
+    rp_shape shape;
     std::vector<int> radices;
     dbuf tw;
 
     // False if n cannot run in one CTA (size, registers or a large prime factor).
     static bool feasible(long long n);
-    // `kind` selects the compile-time kernel list to look in (CT_NONE: always the runtime kernel).  `order`
-    // forces a runtime radix sequence (product n) and `ept_only` (16 or 32) the register array size.
-    void build(int n, int kind = CT_NONE, const std::vector<int>* order = nullptr, int ept_only = 0);
-    // Launch shape for `batch` signals (`spc_cap` bounds the signals per CTA, 0 = no bound).
-    block_cfg cfg(long long batch, int spc_cap = 0) const;
-    // Launch shape of a four-step tile: exactly `tile` signals per CTA.
+    // `kind` selects the compile-time kernel list to look in.
+    void build(int n, int kind);
+    // Launch shape for `batch` signals.
+    block_cfg cfg(long long batch) const;
+    // Launch shape of exactly `tile` signals per CTA (compile-time lengths).
     block_cfg cfg_tile(int tile) const;
     std::string describe() const;
 };
 
-// Threads per signal a runtime radix sequence needs at `ept` complex values per thread (0 = infeasible).
-int threads_needed(long long n, const std::vector<int>& radices, int ept);
 // twiddle table of a radix order (ns * (R - 1) values W_{ns R}^{k r} per pass with ns > 1, then R roots for a
-// radix without a codelet); fills the passes' offsets when passes is not null
+// radix without a codelet)
 template <typename T>
-std::vector<std::complex<T>> pass_twiddles(const std::vector<int>& radices, pass_desc* passes);
+std::vector<std::complex<T>> pass_twiddles(const std::vector<int>& radices);
 // Bluestein tables for length n and convolution length m: chirp[k] = e^{-i pi k^2 / n} (n values) and
 // bhat = conj(DFT_m(b)) / m of the symmetric chirp sequence b (m values).
 template <typename T>
@@ -126,11 +124,6 @@ void bluestein_tables(long long n, long long m, dbuf& chirp, dbuf& bhat);
 
 // Dynamic shared memory a block FFT kernel may use (device limit less the static pass list and a reserve).
 int smem_budget();
-// Largest power-of-two number of signals (<= 16) of `p` that fit one CTA with `buffers` shared-memory
-// buffers per signal: the column / row tile of the strided passes.  0 if not even one fits.
-template <typename T>
-int tile_for(const block_program<T>& p, int buffers = 1);
-
 // A length on the runtime-length block FFT (rp.hpp): radices, twiddles and layouts for a tile order.
 template <typename T>
 struct rp_program
@@ -140,7 +133,6 @@ struct rp_program
     std::vector<int> radices;
     dbuf tw;
     rp_desc desc{};
-    int sig_elems = 0; // RP_SIGNALS: shared elements per signal
     rp_shape shape;
     // RP_COLS / RP_ROWS: the widest tile and narrower ones for few columns or little work, widest first
     struct tile
@@ -152,6 +144,8 @@ struct rp_program
 
     // False (nothing built) when n has no such plan.
     bool build(long long n, rp_layout layout);
+    // Whether build(n, RP_SIGNALS) would succeed.
+    static bool feasible(long long n);
     bool ready() const { return !radices.empty(); }
     // RP_SIGNALS: launch for `batch` signals (threads and dynamic shared memory returned, spc and d set).
     void configure(rp_c2c_args& a, long long batch, int& threads, int& smem) const;
@@ -208,7 +202,6 @@ public:
         const void* twA;
         const void* twB;
         int lbits;
-        fft_desc dcols, drows;
         int* err;
     };
     bool pair_view_of(pair_view& v) const;

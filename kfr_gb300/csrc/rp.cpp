@@ -40,21 +40,23 @@ double rp_pass_cost(int R)
 namespace
 {
 
-// every multiset of codelet radices <= `top` with product n, descending
-void splits(long long n, int top, std::vector<int>& cur, std::vector<std::vector<int>>& out)
+// Calls go_fn(multiset, cost) for the multisets of codelet radices <= `top` with product n (descending) whose pass
+// costs stay below `bound`, which go_fn may lower.
+template <class G>
+void splits(long long n, int top, double cost, std::vector<int>& cur, const double& bound, const G& go_fn)
 {
     if (n == 1)
     {
-        out.push_back(cur);
+        go_fn(cur, cost);
         return;
     }
     if (int(cur.size()) >= kRpMaxPasses)
         return;
     for (int r = int(std::min<long long>(top, n)); r >= 2; r--)
-        if (n % r == 0)
+        if (n % r == 0 && cost + rp_pass_cost(r) < bound)
         {
             cur.push_back(r);
-            splits(n / r, r, cur, out);
+            splits(n / r, r, cost + rp_pass_cost(r), cur, bound, go_fn);
             cur.pop_back();
         }
 }
@@ -152,40 +154,37 @@ void set_layout(rp_desc& d, int i, int S, bool fast_layout, int pad)
 
 } // namespace
 
-std::vector<int> rp_radices(long long n, int largest)
+std::vector<int> rp_radices(long long n, int largest, int hold)
 {
     std::vector<int> r, primes;
     if (n < 2 || n > (1 << 16))
         return {};
-    for (int p = 17; p <= largest; p += 2)
-        while (n % p == 0 && p > 13)
+    for (int p : { 17, 19, 23, 29, 31, 37, 41, 43, 47, 53, 59, 61, 67, 71, 73, 79, 83, 89, 97, 101, 103, 107, 109, 113, 127 })
+        while (p <= largest && n % p == 0)
         {
-            primes.push_back(p); // composite p cannot divide: its factors are gone
+            primes.push_back(p);
             n /= p;
         }
     std::vector<int> cur;
-    std::vector<std::vector<int>> all;
-    splits(n, kRpMaxRadix, cur, all);
-    double best = -1;
-    for (const auto& s : all)
-    {
-        const auto o = pass_order(s);
-        double c     = 0;
-        for (size_t i = 0; i < o.size(); i++)
-        {
-            c += rp_pass_cost(o[i]);
-            // more threads than a CTA of 1024 (or its half, for two of them per SM) to hold a middle pass
-            const bool middle = primes.empty() && i > 0 && i + 1 < o.size();
-            const long long t = middle ? (n / o[i] + rp_hold(o[i]) - 1) / rp_hold(o[i]) : 0;
-            c += t > 1024 ? 1000 : t > 512 ? 4 : 0;
-        }
-        if (best < 0 || c < best)
-        {
-            best = c;
-            r    = o;
-        }
-    }
-    if (best < 0)
+    double best = 1e30;
+    splits(n, kRpMaxRadix, 0, cur, best,
+           [&](const std::vector<int>& s, double c)
+           {
+               const auto o = pass_order(s);
+               for (size_t i = 1; primes.empty() && i + 1 < o.size(); i++)
+               {
+                   // more threads than the largest CTA (or its half, for two of them per SM) to hold a middle pass
+                   const long long t = (n / o[i] + rp_held(o[i], hold) - 1) / rp_held(o[i], hold);
+                   const int most    = rp_max_threads(8, hold);
+                   c += t > most ? 1000 : t > most / 2 ? 4 : 0;
+               }
+               if (c < best)
+               {
+                   best = c;
+                   r    = o;
+               }
+           });
+    if (best >= 1e30)
         return {};
     if (!primes.empty())
     {
@@ -199,11 +198,12 @@ std::vector<int> rp_radices(long long n, int largest)
     return r;
 }
 
-rp_desc rp_build(const std::vector<int>& radices, rp_layout layout, int S, int elem, bool smem_io)
+rp_desc rp_build(const std::vector<int>& radices, rp_layout layout, int S, int elem, bool smem_io, int hold)
 {
     rp_desc d;
     std::memset(&d, 0, sizeof(d));
     d.npass = int(radices.size());
+    d.hold  = hold;
     d.n     = 1;
     for (int r : radices)
         d.n *= r;
@@ -274,6 +274,7 @@ rp_desc rp_build(const std::vector<int>& radices, rp_layout layout, int S, int e
             l.st_r = l.ns * e;
         }
     }
+    d.elems = rp_smem_elems(d, layout, S, smem_io);
     return d;
 }
 
@@ -295,9 +296,8 @@ int rp_threads_needed(const rp_desc& d, int nsig, bool smem_io)
     for (int i = smem_io ? 0 : 1; i < d.npass - (smem_io ? 0 : 1); i++)
     {
         const int R = d.pass[i].radix;
-        const int h = R > kRpMaxRadix ? 1 : rp_hold(R);
-        // a prime pass holds 16 outputs per thread
-        t = std::max(t, R > kRpMaxRadix ? (nsig * d.n + 15) / 16 : (nsig * d.pass[i].nbf + h - 1) / h);
+        const int h = R > kRpMaxRadix ? d.hold : rp_held(R, d.hold);
+        t = std::max(t, ((R > kRpMaxRadix ? nsig * d.n : nsig * d.pass[i].nbf) + h - 1) / h);
     }
     return t;
 }
@@ -316,6 +316,20 @@ static double efficiency(const rp_desc& d, int spc, int threads)
     return useful / spent;
 }
 
+bool rp_fits(const std::vector<int>& radices, int elem, int smem_budget, bool smem_io, int hold)
+{
+    long long n = 1, widest = 1;
+    for (int r : radices)
+        n *= r;
+    for (size_t i = smem_io ? 0 : 1; i < radices.size() && (smem_io || i + 1 < radices.size()); i++)
+    {
+        const int R = radices[i];
+        const int h = R > kRpMaxRadix ? hold : rp_held(R, hold);
+        widest      = std::max(widest, ((R > kRpMaxRadix ? n : n / R) + h - 1) / h);
+    }
+    return !radices.empty() && widest <= rp_max_threads(elem, hold) && n * elem / 16 * 17 + 64 <= smem_budget;
+}
+
 rp_shape rp_choose(const rp_desc& d, int sig_elems, int elem, int smem_budget, bool smem_io)
 {
     // the most busy threads per SM: how evenly the passes' butterflies fill the threads times how many
@@ -323,7 +337,7 @@ rp_shape rp_choose(const rp_desc& d, int sig_elems, int elem, int smem_budget, b
     // accesses overlap with others' work
     rp_shape best;
     double score   = 0;
-    const int maxt = rp_max_threads(elem);
+    const int maxt = rp_max_threads(elem, d.hold);
     int most = 1; // butterflies of a signal's largest pass
     for (int i = 0; i < d.npass; i++)
         most = std::max(most, d.pass[i].nbf);
@@ -361,13 +375,12 @@ rp_shape rp_shrink(const rp_desc& d, const rp_shape& full, long long batch, int 
     for (int i = 0; i < d.npass; i++)
         bf = std::max(bf, s.spc * d.pass[i].nbf);
     const int need = rp_threads_needed(d, s.spc, smem_io);
-    s.threads      = (std::max(need, std::min(bf, 512)) + 31) / 32 * 32;
+    s.threads      = (std::max(need, std::min(bf, d.hold == kRpHold ? 512 : 256)) + 31) / 32 * 32;
     return s;
 }
 
-int rp_tile(const std::vector<int>& radices, rp_layout layout, int elem, int smem_budget)
+int rp_tile(const std::vector<int>& radices, int elem, int smem_budget, int hold)
 {
-    (void)layout;
     long long n = 1;
     for (int r : radices)
         n *= r;
@@ -375,14 +388,14 @@ int rp_tile(const std::vector<int>& radices, rp_layout layout, int elem, int sme
     for (size_t i = 1; i + 1 < radices.size(); i++)
     {
         const int R = radices[i];
-        widest      = std::max<long long>(widest, R > kRpMaxRadix ? (n + 15) / 16
-                                                                  : (n / R + rp_hold(R) - 1) / rp_hold(R));
+        const int h = R > kRpMaxRadix ? hold : rp_held(R, hold);
+        widest      = std::max<long long>(widest, ((R > kRpMaxRadix ? n : n / R) + h - 1) / h);
     }
     int S = 128 / elem;
     while (n * 2 * S * elem <= 32 * 1024 && S < 64)
         S *= 2;
     for (; S >= 1; S /= 2)
-        if ((long long)S * widest <= rp_max_threads(elem) && n * S * elem / 16 * 17 <= smem_budget)
+        if ((long long)S * widest <= rp_max_threads(elem, hold) && n * S * elem / 16 * 17 <= smem_budget)
             return S;
     return 0;
 }

@@ -19,14 +19,19 @@ namespace kfr_gpu
 constexpr int kRpMaxPasses  = 8;
 constexpr int kRpMaxRadix   = 16;
 
-// Threads of a CTA for complex values of `elem` bytes (64 registers per thread for complex<float>, 128 for
-// complex<double>).
+// Values a thread holds across the barrier of an in-place pass: 16, or 32 in half as many threads for lengths
+// that 16 per thread cannot hold.
+constexpr int kRpHold     = 16;
+constexpr int kRpLongHold = 32;
+
+// Threads of a CTA for complex values of `elem` bytes (64 registers per thread for complex<float> at 16 values
+// held, 128 for complex<double>).
 #if defined(__CUDACC__)
 __host__ __device__
 #endif
-    constexpr int rp_max_threads(int elem)
+    constexpr int rp_max_threads(int elem, int hold)
 {
-    return elem == 8 ? 1024 : 512;
+    return (elem == 8 ? 1024 : 512) * kRpHold / hold;
 }
 
 struct rp_pass
@@ -47,17 +52,19 @@ struct rp_desc
 {
     int n, npass;
     int shift; // fast layouts: log2 of the signals per tile
+    int elems; // shared elements per signal (RP_SIGNALS) or per tile
+    int hold;  // values a thread holds
     rp_pass pass[kRpMaxPasses];
 };
 
 // Butterflies of radix R a thread holds in registers across the barrier of an in-place pass (radices above 16,
-// primes, hold 16 outputs of any butterflies instead: see rp_threads_needed).
+// primes, hold `hold` outputs of any butterflies instead: see rp_threads_needed).
 #if defined(__CUDACC__)
 __host__ __device__
 #endif
-    constexpr int rp_hold(int R)
+    constexpr int rp_held(int R, int hold)
 {
-    return kRpMaxRadix / R;
+    return hold / R;
 }
 
 // Order in which a tile's butterflies and signals are laid out.
@@ -68,21 +75,25 @@ enum rp_layout
     RP_ROWS,    // read as contiguous signals, written with the S signals on consecutive threads
 };
 
-// Radices of n in pass order, empty when n has a prime factor above `largest` (13, or up to 127) or needs too
+// Radices of n in pass order for threads that hold `hold` values, empty when n has a prime factor above `largest` (13, or up to 127) or needs too
 // many passes.  Primes above 13 run as in-place passes of dot products between codelet passes (of radix 1, a
 // copy, where no other factor is left).
-std::vector<int> rp_radices(long long n, int largest = 13);
+std::vector<int> rp_radices(long long n, int largest = 13, int hold = kRpHold);
 
 // Descriptor of the radices over a tile.  elem: bytes of a complex value; S (a power of two): signals per tile
 // of RP_COLS and RP_ROWS.  smem_io: the first pass reads and the last pass writes shared memory too, element
 // i of signal g at g n + i.
-rp_desc rp_build(const std::vector<int>& radices, rp_layout layout, int S, int elem, bool smem_io = false);
+rp_desc rp_build(const std::vector<int>& radices, rp_layout layout, int S, int elem, bool smem_io = false,
+                 int hold = kRpHold);
 
 // Shared-memory elements per signal (RP_SIGNALS) or per tile of S signals (RP_COLS, RP_ROWS).
 int rp_smem_elems(const rp_desc& d, rp_layout layout, int S, bool smem_io = false);
 
 // Threads the in-place passes of `nsig` signals need (every butterfly held by some thread); 1 if there are none.
 int rp_threads_needed(const rp_desc& d, int nsig, bool smem_io = false);
+
+// Whether one signal of the radices fits a CTA of `smem_budget` bytes (an estimate that rp_choose confirms).
+bool rp_fits(const std::vector<int>& radices, int elem, int smem_budget, bool smem_io = false, int hold = kRpHold);
 
 // Launch shape for contiguous signals: signals per CTA and threads.
 struct rp_shape
@@ -96,7 +107,7 @@ rp_shape rp_shrink(const rp_desc& d, const rp_shape& full, long long batch, int 
 // Signals per tile of RP_COLS / RP_ROWS: 128-byte rows (16 complex<float>), wider for short signals so that a
 // tile has work for a few warps, narrower where the threads or, with a sixteenth of padding, `smem_budget`
 // bytes need it (0: none).
-int rp_tile(const std::vector<int>& radices, rp_layout layout, int elem, int smem_budget);
+int rp_tile(const std::vector<int>& radices, int elem, int smem_budget, int hold = kRpHold);
 
 // Relative cost per element of a radix-R pass (instructions, from the codelets' operation counts).
 double rp_pass_cost(int R);

@@ -1,0 +1,7 @@
+// Single-precision kernels on the runtime-length block FFT.
+#include "rp_kernels.cuh"
+
+namespace kfr_gpu
+{
+KFR_GPU_RP_INSTANTIATE(float, kRpHold)
+} // namespace kfr_gpu

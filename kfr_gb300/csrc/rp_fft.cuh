@@ -7,7 +7,7 @@
 // (the tile's butterflies are dealt to the threads in one sequence, so any radix keeps all threads busy) and
 // no register array carried across the radix switch.  The first pass reads its inputs through a functor
 // (global memory, with any pre-processing) and the last pass writes through one, so a transform of two passes
-// crosses shared memory once.  Middle passes are in place: each thread holds rp_hold(R) butterflies across
+// crosses shared memory once.  Middle passes are in place: each thread holds rp_held(R) butterflies across
 // one barrier, which halves the shared memory of ping-pong buffers and so doubles the CTAs whose global
 // accesses overlap.  Figures: k_rp_c2c, k_rp_cols (rp_kernels.cu).
 #pragma once
@@ -131,11 +131,11 @@ __device__ __forceinline__ void rp_last(const rp_pass& p, const int shift, const
 }
 
 // In-place pass: the thread's butterflies are held in registers across a barrier (rp_threads_needed).
-template <typename T, int R>
+template <typename T, int R, int H>
 __device__ __forceinline__ void rp_mid(const rp_pass& p, const int shift, const int total, const rp_smem<T> sm,
                                        const cpx<T>* __restrict__ tw)
 {
-    constexpr int NB = rp_hold(R);
+    constexpr int NB = rp_held(R, H);
     cpx<T> v[NB][R];
 #pragma unroll
     for (int b = 0; b < NB; b++)
@@ -177,8 +177,8 @@ __device__ __forceinline__ void rp_mid(const rp_pass& p, const int shift, const 
 }
 
 // In-place pass of a prime radix above 13: the inputs are twiddled where they lie, then each thread holds up to
-// 16 outputs o = s nbf total + J, each a dot product of a butterfly's inputs with the roots W_R^{s r}.
-template <typename T>
+// H outputs o = s nbf total + J, each a dot product of a butterfly's inputs with the roots W_R^{s r}.
+template <typename T, int H>
 __device__ __forceinline__ void rp_prime(const rp_pass& p, const int shift, const int total, const rp_smem<T> sm,
                                          const cpx<T>* __restrict__ tw)
 {
@@ -196,7 +196,7 @@ __device__ __forceinline__ void rp_prime(const rp_pass& p, const int shift, cons
         }
         __syncthreads();
     }
-    constexpr int E  = kRpMaxRadix;
+    constexpr int E  = H;
     const cpx<T>* wr = tw + p.wr_off;
     cpx<T> v[E];
 #pragma unroll
@@ -233,9 +233,10 @@ __device__ __forceinline__ void rp_prime(const rp_pass& p, const int shift, cons
     }
 }
 
-// Element i of the array at p whose elements are `bytes` apart: one wide multiply-add.
-template <typename C>
-__device__ __forceinline__ C* rp_at(C* p, int i, uint32_t bytes)
+// Element i of the array at p whose elements are `bytes` (32 or 64 bits wide) apart: one or two wide
+// multiply-adds.
+template <typename C, typename N>
+__device__ __forceinline__ C* rp_at(C* p, int i, N bytes)
 {
     using B = std::conditional_t<std::is_const_v<C>, const char, char>;
     return reinterpret_cast<C*>(reinterpret_cast<B*>(p) + (unsigned long long)(uint32_t(i)) * bytes);
@@ -258,7 +259,7 @@ struct rp_no_hook
 // per butterfly.  Every input is read before the first output is stored when npass > 1 (or, for one pass,
 // by the thread that stores the signal's outputs), so the two may be the same memory.  Shared memory is free
 // again only after a barrier.
-template <typename T, class D, class LD, class ST, class FIN = rp_no_hook, class PREP = rp_no_hook>
+template <typename T, int H = kRpHold, class D, class LD, class ST, class FIN = rp_no_hook, class PREP = rp_no_hook>
 __device__ __forceinline__ void rp_run(const D& d, cpx<T>* buf, const int nsig, const cpx<T>* __restrict__ tw,
                                        const LD& ld, const ST& st, const FIN& fin = FIN(),
                                        const PREP& prep = PREP())
@@ -286,10 +287,10 @@ __device__ __forceinline__ void rp_run(const D& d, cpx<T>* buf, const int nsig, 
         switch (p.radix)
         {
 #define KFR_GPU_RP_CASE(R)                                                                                 \
-    case R: rp_mid<T, R>(p, sh, total, sm, tw); break;
+    case R: rp_mid<T, R, H>(p, sh, total, sm, tw); break;
             KFR_GPU_RP_CODELETS(KFR_GPU_RP_CASE)
 #undef KFR_GPU_RP_CASE
-        default: rp_prime<T>(p, sh, total, sm, tw); break;
+        default: rp_prime<T, H>(p, sh, total, sm, tw); break;
         }
         __syncthreads();
     }
@@ -322,7 +323,7 @@ __device__ __forceinline__ void rp_run(const D& d, cpx<T>* buf, const int nsig, 
 
 // The transform from and to shared memory (natural order at both ends), every pass in place.  Ends with a
 // barrier.
-template <typename T, class D>
+template <typename T, int H = kRpHold, class D>
 __device__ __forceinline__ void rp_run_smem(const D& d, cpx<T>* buf, const int nsig, const cpx<T>* __restrict__ tw)
 {
     const rp_smem<T> sm{ buf };
@@ -334,10 +335,10 @@ __device__ __forceinline__ void rp_run_smem(const D& d, cpx<T>* buf, const int n
         switch (p.radix)
         {
 #define KFR_GPU_RP_CASE(R)                                                                                 \
-    case R: rp_mid<T, R>(p, d.shift, total, sm, tw); break;
+    case R: rp_mid<T, R, H>(p, d.shift, total, sm, tw); break;
             KFR_GPU_RP_CODELETS(KFR_GPU_RP_CASE)
 #undef KFR_GPU_RP_CASE
-        default: rp_prime<T>(p, d.shift, total, sm, tw); break;
+        default: rp_prime<T, H>(p, d.shift, total, sm, tw); break;
         }
         __syncthreads();
     }

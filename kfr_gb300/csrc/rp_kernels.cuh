@@ -1,5 +1,8 @@
 // Kernels on the runtime-length block FFT (rp_fft.cuh): contiguous complex signals, columns and rows of the
-// four-step transform, axes of multi-dimensional transforms.
+// four-step transform, axes of multi-dimensional transforms.  H: values a thread holds
+// (rp.hpp).  Instantiated by rp_f32.cu, rp_f64.cu, rp_f32_long.cu and rp_f64_long.cu.
+#pragma once
+
 #include "launch.hpp"
 #include "rp_fft.cuh"
 
@@ -22,8 +25,8 @@ __device__ __forceinline__ cpx<T> rp_root(const cpx<T>* __restrict__ A, const cp
 // (15 x 16 x 15, one signal per 256-thread CTA): 56 us, 62% of the HBM copy rate, against 207 us for k_c2c's
 // runtime passes; 2000 points (four passes) 41%, 100 points (two) 88%.
 // ---------------------------------------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T)), 1)
+template <typename T, int H>
+__global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T), H), 1)
     k_rp_c2c(const __grid_constant__ rp_c2c_args a)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -32,10 +35,10 @@ __global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T)), 1)
     const cpx<T>* in   = reinterpret_cast<const cpx<T>*>(a.in) + s0 * a.istride;
     cpx<T>* out        = reinterpret_cast<cpx<T>*>(a.out) + s0 * a.ostride;
     const bool inv     = a.inverse != 0;
-    rp_run<T>(
+    rp_run<T, H>(
         a.d, reinterpret_cast<cpx<T>*>(smem_raw), cnt, reinterpret_cast<const cpx<T>*>(a.tw),
-        [&](int g, int i) { return conj_if(*rp_at(in + g * a.istride, i, sizeof(cpx<T>)), inv); },
-        [&](int g, int i, cpx<T> v) { *rp_at(out + g * a.ostride, i, sizeof(cpx<T>)) = conj_if(v, inv); });
+        [&](int g, int i) { return conj_if(*rp_at(in + g * a.istride, i, uint32_t(sizeof(cpx<T>))), inv); },
+        [&](int g, int i, cpx<T> v) { *rp_at(out + g * a.ostride, i, uint32_t(sizeof(cpx<T>))) = conj_if(v, inv); });
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -46,8 +49,8 @@ __global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T)), 1)
 // Bound by instruction issue and, for tiles of 4 or 8 columns, by the 32- and 64-byte rows.  Eight 1080 x 1920
 // complex arrays, both axes: 173 us against 373 us for k_fs_cols and k_c2c.
 // ---------------------------------------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T)), 1)
+template <typename T, int H>
+__global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T), H), 1)
     k_rp_cols(const __grid_constant__ rp_strided_args a)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -62,8 +65,8 @@ __global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T)), 1)
     // lanes beyond the last column repeat it: they read the same values and store the same results
     const int last  = int(a.pitch - c0 < S ? a.pitch - c0 : S) - 1;
     const bool cin  = a.conj_in != 0, cout = a.conj_out != 0;
-    const uint32_t bytes = uint32_t(a.pitch * sizeof(cpx<T>));
-    rp_run<T>(
+    const unsigned long long bytes = a.pitch * sizeof(cpx<T>);
+    rp_run<T, H>(
         a.d, reinterpret_cast<cpx<T>*>(smem_raw), S, reinterpret_cast<const cpx<T>*>(a.tw),
         [&](int g, int i) { return conj_if(*rp_at(in + min(g, last), i, bytes), cin); },
         [&](int g, int i, cpx<T> v) { *rp_at(out + min(g, last), i, bytes) = conj_if(v, cout); },
@@ -102,8 +105,8 @@ __global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T)), 1)
 // between the first two passes (RP_ROWS).  One complex<double> signal of 2^20 points, both kernels: 179 us
 // against 206 us for k_fs_cols and k_fs_rows (FP64 pipe, latency: one wave of CTAs).
 // ---------------------------------------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T)), 1)
+template <typename T, int H>
+__global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T), H), 1)
     k_rp_rows(const __grid_constant__ rp_strided_args a)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -117,10 +120,10 @@ __global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T)), 1)
     // lanes beyond the last row repeat it
     const int last  = int(a.pitch - r0 < S ? a.pitch - r0 : S) - 1;
     const bool cin  = a.conj_in != 0, cout = a.conj_out != 0;
-    const uint32_t bytes = uint32_t(a.pitch * sizeof(cpx<T>));
-    rp_run<T>(
+    const unsigned long long bytes = a.pitch * sizeof(cpx<T>);
+    rp_run<T, H>(
         a.d, reinterpret_cast<cpx<T>*>(smem_raw), S, reinterpret_cast<const cpx<T>*>(a.tw),
-        [&](int g, int i) { return conj_if(*rp_at(in + (long long)min(g, last) * n, i, sizeof(cpx<T>)), cin); },
+        [&](int g, int i) { return conj_if(*rp_at(in + (long long)min(g, last) * n, i, uint32_t(sizeof(cpx<T>))), cin); },
         [&](int g, int i, cpx<T> v) { *rp_at(out + min(g, last), i, bytes) = conj_if(v, cout); });
 }
 
@@ -143,24 +146,21 @@ static cudaError_t rp_go(void (*kernel)(const A), const A& a, long long grid, in
     return cudaGetLastError();
 }
 
-template <typename T>
+template <typename T, int H>
 cudaError_t launch_rp_c2c(const rp_c2c_args& a, int threads, int smem, cudaStream_t st)
 {
-    return rp_go(k_rp_c2c<T>, a, (a.batch + a.spc - 1) / a.spc, threads, smem, st);
+    return rp_go(k_rp_c2c<T, H>, a, (a.batch + a.spc - 1) / a.spc, threads, smem, st);
 }
 
-template <typename T>
+template <typename T, int H>
 cudaError_t launch_rp_strided(const rp_strided_args& a, bool cols, int threads, int smem, cudaStream_t st)
 {
-    if (a.pitch * (long long)(2 * sizeof(T)) > 0xffffffffLL) // the kernels step by 32-bit byte pitches
-        return cudaErrorInvalidValue;
     const long long tiles = (a.pitch + (1 << a.d.shift) - 1) >> a.d.shift;
-    return rp_go(cols ? k_rp_cols<T> : k_rp_rows<T>, a, tiles * a.batch, threads, smem, st);
+    return rp_go(cols ? k_rp_cols<T, H> : k_rp_rows<T, H>, a, tiles * a.batch, threads, smem, st);
 }
 
-template cudaError_t launch_rp_c2c<float>(const rp_c2c_args&, int, int, cudaStream_t);
-template cudaError_t launch_rp_c2c<double>(const rp_c2c_args&, int, int, cudaStream_t);
-template cudaError_t launch_rp_strided<float>(const rp_strided_args&, bool, int, int, cudaStream_t);
-template cudaError_t launch_rp_strided<double>(const rp_strided_args&, bool, int, int, cudaStream_t);
+#define KFR_GPU_RP_INSTANTIATE(T, H)                                                                       \
+    template cudaError_t launch_rp_c2c<T, H>(const rp_c2c_args&, int, int, cudaStream_t);                  \
+    template cudaError_t launch_rp_strided<T, H>(const rp_strided_args&, bool, int, int, cudaStream_t);
 
 } // namespace kfr_gpu

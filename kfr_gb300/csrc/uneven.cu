@@ -42,9 +42,8 @@ __device__ __forceinline__ cpx<double> ld_cg(const cpx<double>* p)
 // and the four-step twiddle in its functors.  Four 256-thread CTAs per SM (64 registers; two of 512 threads
 // for plans with passes longer than 4096 points), so that one's queue round trip, loads and barriers overlap
 // with the others' arithmetic.  Bound by instruction issue and by the latency of an item's chain (queue, job,
-// loads, barriers).  1024 signals of 64 to 65536 points: 384 us against 746 us for runtime passes of 690
-// instructions per element in one 512-thread CTA per SM; with 16-wide tiles of every length (items of 256
-// elements) 804 us, with per-element tests for the padding and the last column 440 us.
+// loads, barriers).  1024 signals of 64 to 65536 points: 186 us against 746 us for runtime passes of 690
+// instructions per element in one 512-thread CTA per SM.
 template <typename T>
 __global__ void __launch_bounds__(kUnevenThreads, 2) k_uneven(const __grid_constant__ uneven_launch a)
 {
@@ -303,8 +302,7 @@ std::vector<std::vector<int>> candidate_orders(long long m)
 }
 
 // Columns / rows of an m-point FFT per item: the largest power of two of about 16 values per thread that fits
-// (an item costs a queue round trip and a few barriers whatever its size: 16-wide tiles of every length took
-// 804 us for 1024 signals), 0 if none.
+// (an item costs a queue round trip and a few barriers whatever its size), 0 if none.
 int tile_of(int threads, const std::vector<int>& order, rp_layout layout)
 {
     rp_desc d;
@@ -396,7 +394,7 @@ int uneven_plan::get_shape(long long m, int layout, int S, bool smem_io)
     auto t = tw_of_.find(o);
     if (t == tw_of_.end())
     {
-        const auto table = pass_twiddles<float>(o, nullptr);
+        const auto table = pass_twiddles<float>(o); 
         tables_.emplace_back(new dbuf);
         tables_.back()->upload(table.data(), table.size() * sizeof(table[0]));
         t = tw_of_.emplace(o, tables_.back()->get()).first;
@@ -425,7 +423,7 @@ uneven_plan::uneven_plan(const std::vector<long long>& lengths, bool autotune) :
     // 256-thread CTAs, four per SM, unless a length needs passes that only 512 threads can hold
     const auto plannable = [&](splitter& sp, long long n)
     {
-        const bool smooth = n == 1 || !factor_radices(n).empty();
+        const bool smooth = is_smooth(n);
         const long long m = smooth ? n : bluestein_length(n);
         int n1 = 0, n2 = 0;
         return fits_one_cta(sp.threads, m, radices_of(m), !smooth) || sp.split(m, n1, n2);
@@ -474,7 +472,7 @@ uneven_plan::uneven_plan(const std::vector<long long>& lengths, bool autotune) :
                 int elems = 0;
                 if (!fits(threads_, order, RP_SIGNALS, 1, false, f.d, elems))
                     continue;
-                const auto table = pass_twiddles<float>(order, nullptr);
+                const auto table = pass_twiddles<float>(order);
                 ttw.upload(table.data(), table.size() * sizeof(table[0]));
                 f.tw           = ttw.get();
                 const int smax = most_signals(threads_, f.d, elems, false);
@@ -554,7 +552,7 @@ uneven_plan::uneven_plan(const std::vector<long long>& lengths, bool autotune) :
     {
         const long long n = kv.first;
         const auto& sig   = kv.second;
-        const bool smooth = n == 1 || !factor_radices(n).empty();
+        const bool smooth = is_smooth(n);
         const bool direct = smooth && fits_one_cta(threads_, n, radices_of(n), false);
         long long m       = n;
         if (!smooth)

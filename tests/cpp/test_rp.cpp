@@ -1,6 +1,6 @@
 // Walks the descriptors of rp.hpp on the CPU: every shared-memory address in range and written once per pass,
 // every middle butterfly held by a thread, and the transform of random signals equal to the direct DFT.
-//   test_rp LAYOUT S ELEM SMEM_IO N...      (LAYOUT 0 signals, 1 columns, 2 rows)
+//   test_rp LAYOUT S ELEM SMEM_IO HOLD N...      (LAYOUT 0 signals, 1 columns, 2 rows)
 #include "rp.hpp"
 
 #include <cmath>
@@ -29,12 +29,20 @@ static int mulhi(int a, uint32_t m) { return int((uint64_t(uint32_t(a)) * m) >> 
         }                                                                                                  \
     } while (0);
 
-static bool run(int n, rp_layout layout, int S, int elem, bool io)
+static bool run(int n, rp_layout layout, int S, int elem, bool io, int hold)
 {
-    const auto rad = rp_radices(n, 127);
+    const auto rad = rp_radices(n, 127, hold);
     if (rad.empty())
         return false;
-    const rp_desc d = rp_build(rad, layout, S, elem, io);
+    for (int r : rad)
+        if (r > kRpMaxRadix)
+            for (int q = 2; q < r; q++)
+                if (r % q == 0)
+                {
+                    std::printf("n=%d: composite radix %d without a codelet\n", n, r);
+                    return false;
+                }
+    const rp_desc d = rp_build(rad, layout, S, elem, io, hold);
     const int nsig  = layout == RP_SIGNALS ? (n > 512 ? 2 : 5) : S;
     const int elems = rp_smem_elems(d, layout, S, io) * (layout == RP_SIGNALS ? nsig : 1);
     const int thr   = rp_threads_needed(d, nsig, io);
@@ -58,9 +66,9 @@ static bool run(int n, rp_layout layout, int S, int elem, bool io)
         if (!first && !last)
         {
             if (p.radix > kRpMaxRadix)
-                { CHECK((total * p.radix + 15) / 16 <= thr) }
+                { CHECK((total * p.radix + hold - 1) / hold <= thr) }
             else
-                { CHECK((total + rp_hold(p.radix) - 1) / rp_hold(p.radix) <= thr) }
+                { CHECK((total + rp_held(p.radix, hold) - 1) / rp_held(p.radix, hold) <= thr) }
         }
         else
             { CHECK(p.radix <= kRpMaxRadix) }
@@ -135,7 +143,7 @@ static bool run(int n, rp_layout layout, int S, int elem, bool io)
         for (long long batch : { 1LL, 7LL, 300LL, 5000LL, 1000000LL })
         {
             const rp_shape t = rp_shrink(d, s, batch, 152, io);
-            if (s.spc && !(t.spc >= 1 && t.spc <= s.spc && t.threads % 32 == 0 && t.threads <= rp_max_threads(elem) &&
+            if (s.spc && !(t.spc >= 1 && t.spc <= s.spc && t.threads % 32 == 0 && t.threads <= rp_max_threads(elem, hold) &&
                            rp_threads_needed(d, t.spc, io) <= t.threads && (long long)t.spc * sig * elem <= 220 * 1024))
             {
                 std::printf("n=%d batch %lld: shape %d x %d\n", n, batch, t.spc, t.threads);
@@ -156,9 +164,10 @@ static bool run(int n, rp_layout layout, int S, int elem, bool io)
 int main(int argc, char** argv)
 {
     const auto layout = rp_layout(std::atoi(argv[1]));
-    const int S = std::atoi(argv[2]), elem = std::atoi(argv[3]), io = std::atoi(argv[4]);
-    for (int i = 5; i < argc; i++)
-        if (!run(std::atoi(argv[i]), layout, S, elem, io != 0))
+    const int S = std::atoi(argv[2]), elem = std::atoi(argv[3]), io = std::atoi(argv[4]),
+              hold = std::atoi(argv[5]);
+    for (int i = 6; i < argc; i++)
+        if (!run(std::atoi(argv[i]), layout, S, elem, io != 0, hold))
             return 1;
     std::printf("ok\n");
     return 0;

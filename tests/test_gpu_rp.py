@@ -36,12 +36,16 @@ def check(n, batch, sfx, offset=0):
 # part of a tile and of many tiles; pointers aligned to one element only
 @pytest.mark.parametrize("n,batch,offset", [(2, 1, 1), (13, 1000, 1), (15, 77, 0), (18, 4001, 1), (49, 1, 0), (143, 333, 1),
                                             (200, 1, 1), (360, 3001, 0), (847, 19, 1), (1080, 700, 1), (2401, 3, 0),
-                                            (3600, 611, 1), (5005, 5, 0), (6561, 2, 1), (14336, 3, 1), (15625, 2, 0)])
+                                            (3600, 611, 1), (5005, 5, 0), (6561, 2, 1), (14336, 3, 1), (15625, 2, 0),
+                                            # primes of 17 to 127 as passes; 32 values per thread
+                                            (17, 300, 1), (1088, 70, 1), (17 * 19 * 23, 3, 0), (12827, 2, 1),
+                                            (18000, 3, 1), (25000, 2, 0)])
 def test_signals_f32(n, batch, offset):
     check(n, batch, "f32", offset)
 
 
-@pytest.mark.parametrize("n,batch", [(2, 3), (16, 65), (143, 33), (512, 1), (1000, 700), (2197, 3), (4096, 5), (7200, 2)])
+@pytest.mark.parametrize("n,batch", [(2, 3), (16, 65), (143, 33), (512, 1), (1000, 700), (2197, 3), (4096, 5), (7200, 2),
+                                     (6561, 3), (8000, 2), (17 * 64, 9)])
 def test_signals_f64(n, batch):
     check(n, batch, "f64")
 
@@ -72,3 +76,38 @@ def test_axes(shape, batch, sfx):
     assert rel_rms(yd.cpu().numpy(), np.fft.fftn(x.astype(np.complex128), axes=axes)) <= tol
     plan.execute_batch(yd, xd, batch, inverse=True)
     assert rel_rms(yd.cpu().numpy(), np.fft.ifftn(x.astype(np.complex128), axes=axes) * total) <= tol
+
+
+# the in-place kernels of the real DFT and the DCT: a tail of a tile, one signal, 32 values per thread, primes
+@pytest.mark.parametrize("n,batch", [(2 * 30, 1001), (1000, 301), (2 * 1155, 70), (2 * 6561, 3), (2 * 18000, 2), (2 * 17 * 64, 5)])
+@pytest.mark.parametrize("sfx", ["f32", "f64"])
+def test_real(n, batch, sfx):
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((batch, n)).astype(np.float32 if sfx == "f32" else np.float64)
+    tol = (c32_tolerance if sfx == "f32" else c64_tolerance)(n)
+    plan = k.dft_plan_real(n, dtype=sfx)
+    xd = torch.from_numpy(x).cuda()
+    yd = torch.empty((batch, n // 2 + 1), dtype=torch.complex64 if sfx == "f32" else torch.complex128, device="cuda")
+    plan.execute_batch(yd, xd, batch)
+    assert rel_rms(yd.cpu().numpy(), np.fft.rfft(x.astype(np.float64))) <= tol
+    plan.execute_batch(xd, yd, batch, inverse=True)
+    assert rel_rms(xd.cpu().numpy() / n, x.astype(np.float64)) <= 2 * tol
+
+
+@pytest.mark.parametrize("n,batch", [(30, 1001), (1000, 301), (6561, 3), (18000, 2)])
+def test_dct(n, batch):
+    rng = np.random.default_rng(n)
+    x = rng.uniform(-1, 1, (batch, n)).astype(np.float32)
+    x64 = x.astype(np.float64)
+    j, m = np.arange(n), min(n, 400)
+    ks = np.unique(rng.integers(0, n, m))
+    ref = x64 @ np.cos(np.pi * np.outer(2 * j + 1, ks) / (2 * n))
+    plan = k.dct_plan(n)
+    xd = torch.from_numpy(x).cuda()
+    yd = torch.empty_like(xd)
+    plan.execute_batch(yd, xd, batch)
+    assert rel_rms(yd.cpu().numpy()[:, ks], ref) <= c32_tolerance(n)
+    w = x64.copy()
+    w[:, 0] *= 0.5
+    plan.execute_batch(yd, xd, batch, inverse=True)
+    assert rel_rms(yd.cpu().numpy()[:, ks], w @ np.cos(np.pi * np.outer(j, 2 * ks + 1) / (2 * n))) <= c32_tolerance(n)

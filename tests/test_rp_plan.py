@@ -27,16 +27,18 @@ def walker(tmp_path_factory):
     return exe
 
 
-# layout (0 signals, 1 columns, 2 rows), signals per tile, bytes of a complex value, both ends in shared memory
-@pytest.mark.parametrize("layout,s,elem,io", [(0, 1, 8, 0), (0, 1, 16, 0), (0, 1, 8, 1), (1, 16, 8, 0), (1, 4, 8, 0),
-                                              (1, 8, 16, 0), (1, 1, 8, 0), (2, 16, 8, 0), (2, 8, 16, 0), (2, 2, 8, 0)])
-def test_descriptors(walker, layout, s, elem, io):
+# layout (0 signals, 1 columns, 2 rows), signals per tile, bytes of a complex value, both ends in shared memory,
+# values a thread holds
+@pytest.mark.parametrize("layout,s,elem,io,hold", [
+    (0, 1, 8, 0, 16), (0, 1, 16, 0, 16), (0, 1, 8, 1, 16), (0, 1, 8, 0, 32), (0, 1, 16, 1, 32), (1, 16, 8, 0, 16),
+    (1, 4, 8, 0, 16), (1, 8, 16, 0, 32), (1, 1, 8, 0, 16), (2, 16, 8, 0, 16), (2, 8, 16, 0, 16), (2, 2, 8, 0, 32)])
+def test_descriptors(walker, layout, s, elem, io, hold):
     lengths = LENGTHS if s <= 4 else [n for n in LENGTHS if n <= 1080]
-    r = subprocess.run([walker, str(layout), str(s), str(elem), str(io)] + [str(n) for n in lengths], capture_output=True,
+    r = subprocess.run([walker, str(layout), str(s), str(elem), str(io), str(hold)] + [str(n) for n in lengths], capture_output=True,
                        text=True)
     assert r.returncode == 0 and r.stdout.strip().endswith("ok"), r.stdout
 
 
 def test_lengths_without_a_plan(walker):
     for n in (131, 2 * 137, 2 * 65537):
-        assert subprocess.run([walker, "0", "1", "8", "0", str(n)], capture_output=True).returncode == 1
+        assert subprocess.run([walker, "0", "1", "8", "0", "16", str(n)], capture_output=True).returncode == 1
