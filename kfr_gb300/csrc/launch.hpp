@@ -176,17 +176,19 @@ struct rp_c2c_args
 };
 // Columns of row-major d.n x pitch arrays (RP_COLS; in the arrays' own layout; twA: the four-step twiddle of
 // N = d.n pitch points), or the pitch rows of d.n contiguous points of a four-step transform (RP_ROWS; output
-// k of row r to r + pitch k).  Arrays sig_stride apart.
+// k of row r to r + pitch k).  Arrays in_stride / out_stride apart.
 struct rp_strided_args
 {
     const void* in;
     void* out;
-    long long batch, sig_stride, pitch;
+    long long batch, in_stride, out_stride, pitch;
     int conj_in, conj_out;
     const void* tw;
     const void* twA; // null: no twiddle
     const void* twB;
     int lbits;
+    const void* rtw; // real DFTs of 2N reals: W_2N^k, k <= N (columns: the input is the spectrum, N + 1 bins or N for
+    int ccs;         // Perm, merged as it is read; null otherwise)
     rp_desc d;
 };
 // H: a.d.hold.
@@ -194,6 +196,10 @@ template <typename T, int H>
 cudaError_t launch_rp_c2c(const rp_c2c_args& a, int threads, int smem, cudaStream_t st);
 template <typename T, int H>
 cudaError_t launch_rp_strided(const rp_strided_args& a, bool cols, int threads, int smem, cudaStream_t st);
+// The rows of a real forward DFT's half-length four-step, split into the spectrum (a.rtw, a.ccs; the tile of a.d has
+// at least two rows and its last pass leaves shared memory in natural order).
+template <typename T, int H>
+cudaError_t launch_rp_rows_split(const rp_strided_args& a, int threads, int smem, cudaStream_t st);
 
 template <typename T>
 cudaError_t launch_bluestein(const bluestein_args& a, const block_cfg& c, cudaStream_t st);

@@ -76,16 +76,15 @@ void md_axes<T>::run(void* data, long long batch, bool inverse, void* scratch, c
             check(launch_transpose<T>(data, tr, batch * ax.outer, ax.inner, ax.n, st), "transpose axis back");
             continue;
         }
-        rp_strided_args a;
+        rp_strided_args a{};
         a.in         = data;
         a.out        = data;
         a.batch      = batch * ax.outer;
-        a.sig_stride = ax.n * ax.inner;
+        a.in_stride  = ax.n * ax.inner;
+        a.out_stride = ax.n * ax.inner;
         a.pitch      = ax.inner;
         a.conj_in    = inverse;
         a.conj_out   = inverse;
-        a.twA = a.twB = nullptr;
-        a.lbits      = 0;
         ax.rp->run(a, st);
     }
 }

@@ -475,7 +475,7 @@ void rp_program<T>::configure(rp_c2c_args& a, long long batch, int& threads, int
 }
 
 template <typename T>
-const typename rp_program<T>::tile& rp_program<T>::pick(long long count, long long batch) const
+const typename rp_program<T>::tile& rp_program<T>::pick(const std::vector<tile>& tiles, long long count, long long batch)
 {
     // narrower tiles where the widest would leave SMs without a CTA, or lanes without a column
     size_t i = 0;
@@ -486,9 +486,35 @@ const typename rp_program<T>::tile& rp_program<T>::pick(long long count, long lo
 }
 
 template <typename T>
-void rp_program<T>::run(rp_strided_args& a, cudaStream_t st) const
+void rp_program<T>::build_split()
 {
-    const tile& t = pick(a.pitch, a.batch);
+    const int hold = tiles[0].d.hold;
+    for (int S = std::max(2, 2 * tiles[0].S); S >= 2 && split_tiles.size() < 3; S /= 2)
+    {
+        tile t;
+        t.d    = rp_build(radices, RP_ROWS, S, elem, true, hold);
+        t.S    = S;
+        t.smem = t.d.elems * elem;
+        // every pass but the first is in place
+        int need = 1;
+        for (int i = 1; i < t.d.npass; i++)
+        {
+            const int R = t.d.pass[i].radix, h = R > kRpMaxRadix ? hold : rp_held(R, hold);
+            need        = std::max(need, ((R > kRpMaxRadix ? S * t.d.n : S * t.d.pass[i].nbf) + h - 1) / h);
+        }
+        if (t.smem > smem_budget() || need > rp_max_threads(elem, hold))
+            continue;
+        t.threads = (std::max(need, std::min(S * t.d.pass[0].nbf, 256)) + 31) / 32 * 32;
+        if (t.threads > 512 && S > 16) // wider tiles only while two CTAs share an SM
+            continue;
+        split_tiles.push_back(t);
+    }
+}
+
+template <typename T>
+void rp_program<T>::run(rp_strided_args& a, cudaStream_t st, bool split) const
+{
+    const tile& t = split ? pick(split_tiles, a.pitch, a.batch) : pick(tiles, a.pitch, a.batch);
     a.d           = t.d;
     a.tw          = tw.get();
     // at most 2^31 - 1 tiles per launch
@@ -499,9 +525,14 @@ void rp_program<T>::run(rp_strided_args& a, cudaStream_t st) const
     for (long long b = 0; b < total; b += most)
     {
         a.batch = std::min(most, total - b);
-        a.in    = in + b * a.sig_stride * elem;
-        a.out   = out + b * a.sig_stride * elem;
-        check(t.d.hold == kRpHold ? launch_rp_strided<T, kRpHold>(a, layout == RP_COLS, t.threads, t.smem, st)
+        a.in    = in + b * a.in_stride * elem;
+        a.out   = out + b * a.out_stride * elem;
+        if (split)
+            check(t.d.hold == kRpHold ? launch_rp_rows_split<T, kRpHold>(a, t.threads, t.smem, st)
+                                      : launch_rp_rows_split<T, kRpLongHold>(a, t.threads, t.smem, st),
+                  "launch row DFTs with the real split");
+        else
+            check(t.d.hold == kRpHold ? launch_rp_strided<T, kRpHold>(a, layout == RP_COLS, t.threads, t.smem, st)
                                   : launch_rp_strided<T, kRpLongHold>(a, layout == RP_COLS, t.threads, t.smem, st),
               layout == RP_COLS ? "launch column DFTs" : "launch row DFTs");
     }
@@ -519,6 +550,179 @@ std::string rp_program<T>::describe() const
         s << " signals/CTA=" << shape.spc << " threads=" << shape.threads;
     else
         s << " tile=" << tiles[0].S << " threads=" << tiles[0].threads;
+    return s.str();
+}
+
+// ------------------------------------------------------------------------------------------------------
+// rp_fourstep
+// ------------------------------------------------------------------------------------------------------
+
+template <typename T>
+void upload_roots(long long n, dbuf& twA, dbuf& twB, int& lbits)
+{
+    int lb = 0;
+    while ((1LL << (2 * lb)) < n)
+        lb++;
+    lbits              = lb;
+    const long long nb = 1LL << lb;
+    const long long na = (n + nb - 1) / nb;
+    std::vector<std::complex<T>> A(na), B(nb);
+    for (long long i = 0; i < na; i++)
+    {
+        const auto w = twiddle(i * nb, n);
+        A[i]         = std::complex<T>(T(w.real()), T(w.imag()));
+    }
+    for (long long j = 0; j < nb; j++)
+    {
+        const auto w = twiddle(j, n);
+        B[j]         = std::complex<T>(T(w.real()), T(w.imag()));
+    }
+    twA.upload(A.data(), A.size() * sizeof(std::complex<T>));
+    twB.upload(B.data(), B.size() * sizeof(std::complex<T>));
+}
+
+// The split has the cheapest passes per element, where a tile narrower than a 128-byte row costs extra memory
+// transactions.
+template <typename T>
+bool rp_fourstep<T>::build(long long length)
+{
+    n = length;
+    long long split = 0;
+    constexpr int elem = int(2 * sizeof(T));
+    const auto cost    = [&](long long m) -> double
+    {
+        int hold       = 0;
+        const auto rad = one_cta_radices<T>(m, false, hold);
+        if (rad.empty())
+            return -1;
+        const int S = rp_tile(rad, elem, smem_budget(), hold);
+        if (!S)
+            return -1;
+        double c = 0;
+        for (int r : rad)
+            c += rp_pass_cost(r);
+        // a row of S elements against the 128 bytes of a cache line
+        const double width = double(S * elem) / 128;
+        return c + (width >= 1 ? 0.0 : 12.0 * (1 / width - 1));
+    };
+    std::map<long long, double> memo;
+    const auto cached = [&](long long v)
+    {
+        const auto f = memo.find(v);
+        return f != memo.end() ? f->second : memo[v] = cost(v);
+    };
+    double best         = -1;
+    const long long top = smem_budget() / elem; // longest one-CTA length
+    for (long long a = 2; a * 2 <= n && a <= top; a++)
+    {
+        if (n % a || n / a > top)
+            continue;
+        const double c = cached(a), r = c < 0 ? -1 : cached(n / a);
+        if (r < 0)
+            continue;
+        if (best < 0 || c + r < best)
+        {
+            best = c + r;
+            split = a;
+        }
+    }
+    if (best < 0 || !cols.build(split, RP_COLS) || !rows.build(n / split, RP_ROWS))
+        return false;
+    n1 = split;
+    n2 = n / n1;
+    upload_roots<T>(n, twA, twB, lbits);
+    return true;
+}
+
+template <typename T>
+void rp_fourstep<T>::execute(void* out, const void* in, long long batch, bool inverse, void* scratch,
+                             cudaStream_t st) const
+{
+    // x (n1 x n2) -> scratch (column DFTs times the twiddle, same layout) -> out[k1 + n1 k2]
+    rp_strided_args a{};
+    a.batch      = batch;
+    a.in_stride  = n;
+    a.out_stride = n;
+    a.in         = in;
+    a.out        = scratch;
+    a.pitch      = n2;
+    a.conj_in    = inverse;
+    a.twA        = twA.get();
+    a.twB        = twB.get();
+    a.lbits      = lbits;
+    cols.run(a, st);
+    rp_strided_args b{};
+    b.batch      = batch;
+    b.in_stride  = n;
+    b.out_stride = n;
+    b.in         = scratch;
+    b.out        = out;
+    b.pitch      = n1;
+    b.conj_out   = inverse;
+    rows.run(b, st);
+}
+
+template <typename T>
+void rp_fourstep<T>::execute_real_inverse(void* out, const void* in, long long batch, bool ccs, const void* rtw,
+                                          void* scratch, cudaStream_t st) const
+{
+    rp_strided_args a{};
+    a.batch      = batch;
+    a.in_stride  = ccs ? n + 1 : n;
+    a.out_stride = n;
+    a.in         = in;
+    a.out        = scratch;
+    a.pitch      = n2;
+    a.conj_in    = 1;
+    a.twA        = twA.get();
+    a.twB        = twB.get();
+    a.lbits      = lbits;
+    a.rtw        = rtw;
+    a.ccs        = ccs;
+    cols.run(a, st);
+    rp_strided_args b{};
+    b.batch      = batch;
+    b.in_stride  = n;
+    b.out_stride = n;
+    b.in         = scratch;
+    b.out        = out;
+    b.pitch      = n1;
+    b.conj_out   = 1;
+    rows.run(b, st);
+}
+
+template <typename T>
+void rp_fourstep<T>::execute_real(void* out, const void* in, long long batch, bool ccs, const void* rtw, void* scratch,
+                                  cudaStream_t st) const
+{
+    rp_strided_args a{};
+    a.batch      = batch;
+    a.in_stride  = n;
+    a.out_stride = n;
+    a.in         = in;
+    a.out        = scratch;
+    a.pitch      = n2;
+    a.twA        = twA.get();
+    a.twB        = twB.get();
+    a.lbits      = lbits;
+    cols.run(a, st);
+    rp_strided_args b{};
+    b.batch      = batch;
+    b.in_stride  = n;
+    b.out_stride = ccs ? n + 1 : n;
+    b.in         = scratch;
+    b.out        = out;
+    b.pitch      = n1;
+    b.rtw        = rtw;
+    b.ccs        = ccs;
+    rows.run(b, st, true);
+}
+
+template <typename T>
+std::string rp_fourstep<T>::describe() const
+{
+    std::ostringstream s;
+    s << "n=" << n << " = " << n1 << " x " << n2 << " cols[" << cols.describe() << "] rows[" << rows.describe() << "]";
     return s.str();
 }
 
@@ -929,89 +1133,17 @@ bool complex_engine<T>::plan_fourstep(long long n)
             pair_ = true;
             err_.alloc(sizeof(int)); // the persistent tensor-copy pair kernels report a copy that never lands
             check(cudaMemset(err_.get(), 0, sizeof(int)), "clear error flag");
-            upload_roots(n);
+            upload_roots<T>(n, twA_, twB_, lbits_);
+            // an odd row pitch takes no tensor copies: the complex passes then run the runtime-length four-step
+            // (22050 points, 1521 signals: 448 -> 227 us); the pair stays for the real split (pair_view_of)
+            if (a % 2)
+                rp4_.build(n);
             return true;
         }
     }
-    return plan_fourstep_rp(n);
-}
-
-template <typename T>
-void complex_engine<T>::upload_roots(long long n)
-{
-    // two-level table for W_N^m, m < N
-    int lb = 0;
-    while ((1LL << (2 * lb)) < n)
-        lb++;
-    lbits_             = lb;
-    const long long nb = 1LL << lb;
-    const long long na = (n + nb - 1) / nb;
-    std::vector<std::complex<T>> A(na), B(nb);
-    for (long long i = 0; i < na; i++)
-    {
-        const auto w = twiddle(i * nb, n);
-        A[i]         = std::complex<T>(T(w.real()), T(w.imag()));
-    }
-    for (long long j = 0; j < nb; j++)
-    {
-        const auto w = twiddle(j, n);
-        B[j]         = std::complex<T>(T(w.real()), T(w.imag()));
-    }
-    twA_.upload(A.data(), A.size() * sizeof(std::complex<T>));
-    twB_.upload(B.data(), B.size() * sizeof(std::complex<T>));
-}
-
-// Four-step split with both passes on the runtime-length block FFT: the cheapest passes per element, where a
-// tile narrower than a 128-byte row costs extra memory transactions.
-template <typename T>
-bool complex_engine<T>::plan_fourstep_rp(long long n)
-{
-    constexpr int elem = int(2 * sizeof(T));
-    const auto cost    = [&](long long m) -> double
-    {
-        int hold       = 0;
-        const auto rad = one_cta_radices<T>(m, false, hold);
-        if (rad.empty())
-            return -1;
-        const int S = rp_tile(rad, elem, smem_budget(), hold);
-        if (!S)
-            return -1;
-        double c = 0;
-        for (int r : rad)
-            c += rp_pass_cost(r);
-        // a row of S elements against the 128 bytes of a cache line
-        const double width = double(S * elem) / 128;
-        return c + (width >= 1 ? 0.0 : 12.0 * (1 / width - 1));
-    };
-    std::map<long long, double> memo;
-    const auto cached = [&](long long v)
-    {
-        const auto f = memo.find(v);
-        return f != memo.end() ? f->second : memo[v] = cost(v);
-    };
-    double best         = -1;
-    const long long top = smem_budget() / elem; // longest one-CTA length
-    for (long long n1 = 2; n1 * 2 <= n && n1 <= top; n1++)
-    {
-        if (n % n1 || n / n1 > top)
-            continue;
-        const double c = cached(n1), r = c < 0 ? -1 : cached(n / n1);
-        if (r < 0)
-            continue;
-        if (best < 0 || c + r < best)
-        {
-            best = c + r;
-            n1_  = n1;
-        }
-    }
-    if (best < 0 || !rp_cols_.build(n1_, RP_COLS) || !rp_rows_.build(n / n1_, RP_ROWS))
-    {
-        n1_ = 0;
+    if (!rp4_.build(n))
         return false;
-    }
-    n2_ = n / n1_;
-    k_  = kind::fourstep;
-    upload_roots(n);
+    k_ = kind::fourstep;
     return true;
 }
 
@@ -1055,7 +1187,7 @@ int complex_engine<T>::launches(long long batch) const
             return (batch / pipe_spc_ > 0 ? 1 : 0) + (batch % pipe_spc_ ? 1 : 0);
         return 1;
     case kind::bluestein_smem: return 1;
-    case kind::fourstep: return rp_cols_.ready() ? 2 : 2 * int((batch + 65534) / 65535);
+    case kind::fourstep: return rp4_.ready() ? 2 : 2 * int((batch + 65534) / 65535);
     case kind::bluestein_multi: return 3 + 2 * inner_->launches(batch);
     case kind::rader_smem: return 1;
     case kind::tensor: return n1_ ? 2 * int((batch + 65534) / 65535) : 1;
@@ -1246,28 +1378,9 @@ void complex_engine<T>::execute(void* out, const void* in, long long batch, long
     {
         if (istride != n_ || ostride != n_)
             throw std::invalid_argument("internal: four-step needs contiguous signals");
-        if (rp_cols_.ready())
+        if (rp4_.ready())
         {
-            // x (n1 x n2) -> scratch (column DFTs times the twiddle, same layout) -> out[k1 + n1 k2]
-            rp_strided_args a;
-            a.batch      = batch;
-            a.sig_stride = n_;
-            a.in         = in;
-            a.out        = scratch;
-            a.pitch      = n2_;
-            a.conj_in    = inverse;
-            a.conj_out   = 0;
-            a.twA        = twA_.get();
-            a.twB        = twB_.get();
-            a.lbits      = lbits_;
-            rp_cols_.run(a, st);
-            a.in       = scratch;
-            a.out      = out;
-            a.pitch    = n1_;
-            a.conj_in  = 0;
-            a.conj_out = inverse;
-            a.twA = a.twB = nullptr;
-            rp_rows_.run(a, st);
+            rp4_.execute(out, in, batch, inverse, scratch, st);
             return;
         }
         // a pair kernel for this pass, or false when neither of them can run (the generic pass runs instead)
@@ -1404,15 +1517,16 @@ std::string complex_engine<T>::describe() const
         break;
     case kind::bluestein_smem: s << "bluestein_smem n=" << n_ << " m=" << m_ << " [" << prog_.describe() << "]"; break;
     case kind::fourstep:
-        if (rp_cols_.ready())
+        if (rp4_.ready() && !pair_)
         {
-            s << "fourstep n=" << n_ << " = " << n1_ << " x " << n2_ << " cols[" << rp_cols_.describe() << "] rows["
-              << rp_rows_.describe() << "]";
+            s << "fourstep " << rp4_.describe();
             break;
         }
         s << "fourstep" << (pair_ ? " (compile-time pair)" : "") << " n=" << n_ << " = " << n1_ << " x " << n2_
           << " cols[" << pcols_.describe() << " tile=" << tile_c_ << "] rows[" << prows_.describe()
           << " tile=" << tile_r_ << "]";
+        if (rp4_.ready())
+            s << " complex passes: " << rp4_.describe();
         break;
     case kind::bluestein_multi: s << "bluestein_multi n=" << n_ << " m=" << m_ << " inner{" << inner_->describe() << "}"; break;
     case kind::rader_smem:
@@ -1482,6 +1596,9 @@ real_engine<T>::real_engine(long long n) : n_(n), c_(n / 2), ceng_(n / 2)
         }
         rtw2_.upload(r2.data(), r2.size() * sizeof(std::complex<T>));
     }
+    rp4_ = ceng_.runtime_fourstep();
+    if (rp4_ && !rfsp_)
+        rp4_->rows.build_split();
     // Pipelined forward and inverse kernels (compile-time c, single precision): an even number of signals
     // per tile, the most resident threads per SM with at least two CTAs, then the smallest tile.
     if (fused_ && prog_.ct && sizeof(T) == 4)
@@ -1621,6 +1738,12 @@ void real_engine<T>::forward(void* out, const void* in, long long batch, bool cc
         }
         return;
     }
+    if (rp4_ && !rp4_->rows.split_tiles.empty() && reinterpret_cast<uintptr_t>(in) % (2 * sizeof(T)) == 0)
+    {
+        // the split fused into the row pass
+        rp4_->execute_real(out, in, batch, ccs, rtw_.get(), scratch, st);
+        return;
+    }
     char* Z     = static_cast<char*>(scratch);
     char* inner = align_scratch(Z + batch * (c_ + 1) * 2 * sizeof(T));
     if (reinterpret_cast<uintptr_t>(in) % (2 * sizeof(T)))
@@ -1687,6 +1810,13 @@ void real_engine<T>::inverse(void* out, const void* in, long long batch, bool cc
             a.batch = batch - done;
             check(launch_c2r<T>(a, p.cfg(batch - done), st), "launch c2r");
         }
+        return;
+    }
+    if (rp4_ && reinterpret_cast<uintptr_t>(out) % (2 * sizeof(T)) == 0)
+    {
+        // the merge fused into the column pass: two round trips instead of three (44100 points, 1521 signals: 562 ->
+        // 337 us; 48000 points stay on the tensor-copy pair, 354 us against 365)
+        rp4_->execute_real_inverse(out, in, batch, ccs, rtw_.get(), scratch, st);
         return;
     }
     char* Z     = static_cast<char*>(scratch);
@@ -1883,6 +2013,8 @@ template struct block_program<float>;
 template struct block_program<double>;
 template struct rp_program<float>;
 template struct rp_program<double>;
+template struct rp_fourstep<float>;
+template struct rp_fourstep<double>;
 template class complex_engine<float>;
 template class complex_engine<double>;
 template class real_engine<float>;

@@ -150,11 +150,43 @@ struct rp_program
     // RP_SIGNALS: launch for `batch` signals (threads and dynamic shared memory returned, spc and d set).
     void configure(rp_c2c_args& a, long long batch, int& threads, int& smem) const;
     // RP_COLS / RP_ROWS: the tile for `count` columns or rows in `batch` arrays.
-    const tile& pick(long long count, long long batch) const;
-    // One strided launch (a.d, a.tw are set here).
-    void run(rp_strided_args& a, cudaStream_t st) const;
+    static const tile& pick(const std::vector<tile>& tiles, long long count, long long batch);
+    // RP_ROWS: tiles of at least two rows whose last pass leaves the outputs in shared memory (the real split).
+    std::vector<tile> split_tiles;
+    void build_split();
+    // One strided launch (a.d, a.tw are set here); split: k_rp_rows_split.
+    void run(rp_strided_args& a, cudaStream_t st, bool split = false) const;
     std::string describe() const;
 };
+
+// Four-step transform of n = n1 n2 points on the runtime-length block FFT.
+template <typename T>
+struct rp_fourstep
+{
+    long long n = 0, n1 = 0, n2 = 0;
+    rp_program<T> cols, rows;
+    dbuf twA, twB; // W_n^m = twA[m >> lbits] twB[m & mask]
+    int lbits = 0;
+
+    // False (nothing built) when n has no split into two one-CTA lengths.
+    bool build(long long length);
+    bool ready() const { return n1 != 0; }
+    // `batch` contiguous signals; out may alias in; scratch: batch n elements.
+    void execute(void* out, const void* in, long long batch, bool inverse, void* scratch, cudaStream_t st) const;
+    // The inverse real DFT of 2n reals: the merge of the spectrum (n + 1 bins for CCs, n for Perm, rtw =
+    // W_2n^k, k <= n) is fused into the column pass.  out: the reals, aligned to two of them.
+    void execute_real_inverse(void* out, const void* in, long long batch, bool ccs, const void* rtw, void* scratch,
+                              cudaStream_t st) const;
+    // The forward real DFT of 2n reals (in: the reals, aligned to two of them): the split is fused into the row pass
+    // (rows.build_split()).
+    void execute_real(void* out, const void* in, long long batch, bool ccs, const void* rtw, void* scratch,
+                      cudaStream_t st) const;
+    std::string describe() const;
+};
+
+// Two-level table of W_n^m, m < n: W_n^m = A[m >> lbits] B[m & ((1 << lbits) - 1)].
+template <typename T>
+void upload_roots(long long n, dbuf& A, dbuf& B, int& lbits);
 
 template <typename T>
 class complex_engine
@@ -205,6 +237,8 @@ public:
         int* err;
     };
     bool pair_view_of(pair_view& v) const;
+    // The runtime-length four-step (null unless this engine runs one).
+    rp_fourstep<T>* runtime_fourstep() { return rp4_.ready() ? &rp4_ : nullptr; }
     // While set, in and out of execute() are host memory mapped into the device's address space (zero-copy
     // calls): the kernels that read or write through bulk and tensor copies give way to the plain-load ones.
     // The caller holds the plan's lock around the call.
@@ -226,7 +260,7 @@ private:
     int tile_c_ = 1, tile_r_ = 1;
     bool pp_c_ = false, pp_r_ = false; // ping-pong column / row passes
     bool pair_ = false;                 // both passes as fully compile-time pair kernels
-    rp_program<T> rp_cols_, rp_rows_;   // both passes on the runtime-length block FFT
+    rp_fourstep<T> rp4_;                // both passes on the runtime-length block FFT
     dbuf twA_, twB_;
     int lbits_ = 0;
     // pipelined smem path (compile-time lengths): signals per tile, 0 = not used
@@ -237,8 +271,6 @@ private:
     void init_bluestein(long long n);
     void init_rader(long long n);
     bool plan_fourstep(long long n);
-    bool plan_fourstep_rp(long long n);
-    void upload_roots(long long n);
     void plan_pipe();
     // tensor-core form (n1_, n2_, twA_, twB_, lbits_ as for the four-step when n > 4096)
     int tc_mode_ = 0;
@@ -279,6 +311,8 @@ private:
     // input; launch_ct_fsp_r2c_f32), and its two-level table of W_n^k: W_n^k1 (k1 < n1), W_n^(n1 k2)
     bool rfsp_ = false;
     dbuf rtw2_;
+    // half lengths on the runtime-length four-step: the split fused into its row pass, the merge into its column pass
+    rp_fourstep<T>* rp4_ = nullptr; // the complex engine's
 };
 
 // dct_plan<T>: DCT-II forward, DCT-III (X0 halved) inverse, unscaled.

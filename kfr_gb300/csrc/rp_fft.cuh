@@ -321,6 +321,44 @@ __device__ __forceinline__ void rp_run(const D& d, cpx<T>* buf, const int nsig, 
     }
 }
 
+// The transform from ld(g, i) to shared memory (output k of signal g in the natural layout of d's last pass).  Ends
+// with a barrier.
+template <typename T, int H = kRpHold, class D, class LD>
+__device__ __forceinline__ void rp_run_in(const D& d, cpx<T>* buf, const int nsig, const cpx<T>* __restrict__ tw,
+                                          const LD& ld)
+{
+    const rp_smem<T> sm{ buf };
+    const rp_no_hook none{};
+    {
+        const rp_pass& p = d.pass[0];
+        const int total  = nsig * p.nbf;
+        switch (p.radix)
+        {
+#define KFR_GPU_RP_CASE(R)                                                                                 \
+    case R: rp_first<T, R>(p, d.shift, total, sm, ld, none); break;
+            KFR_GPU_RP_RADICES(KFR_GPU_RP_CASE)
+#undef KFR_GPU_RP_CASE
+        default: break;
+        }
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int i = 1; i < d.npass; i++)
+    {
+        const rp_pass& p = d.pass[i];
+        const int total  = nsig * p.nbf;
+        switch (p.radix)
+        {
+#define KFR_GPU_RP_CASE(R)                                                                                 \
+    case R: rp_mid<T, R, H>(p, d.shift, total, sm, tw); break;
+            KFR_GPU_RP_CODELETS(KFR_GPU_RP_CASE)
+#undef KFR_GPU_RP_CASE
+        default: rp_prime<T, H>(p, d.shift, total, sm, tw); break;
+        }
+        __syncthreads();
+    }
+}
+
 // The transform from and to shared memory (natural order at both ends), every pass in place.  Ends with a
 // barrier.
 template <typename T, int H = kRpHold, class D>

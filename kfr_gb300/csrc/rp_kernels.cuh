@@ -49,7 +49,11 @@ __global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T), H), 1)
 // Bound by instruction issue and, for tiles of 4 or 8 columns, by the 32- and 64-byte rows.  Eight 1080 x 1920
 // complex arrays, both axes: 173 us against 373 us for k_fs_cols and k_c2c.
 // ---------------------------------------------------------------------------------------------------
-template <typename T, int H>
+// MERGE: the input is the spectrum X of 2N reals, read as conj(Z[e]) with
+//   Z[e] = X[e] + conj X[N-e] + i conj(W_2N^e) (X[e] - conj X[N-e])
+// (from_fmt, src/dft/fft-impl.hpp:1852-1896; e = 0 takes the real parts of the first and last bins).  Each bin is
+// read by its own column's tile and by the mirrored one, the second time mostly from L2.
+template <typename T, int H, bool MERGE>
 __global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T), H), 1)
     k_rp_cols(const __grid_constant__ rp_strided_args a)
 {
@@ -58,8 +62,8 @@ __global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T), H), 1)
     const int tiles   = int((a.pitch + S - 1) >> a.d.shift);
     const long long b = blockIdx.x / tiles;
     const int c0      = int(blockIdx.x - b * tiles) << a.d.shift;
-    const cpx<T>* in  = reinterpret_cast<const cpx<T>*>(a.in) + b * a.sig_stride + c0;
-    cpx<T>* out       = reinterpret_cast<cpx<T>*>(a.out) + b * a.sig_stride + c0;
+    const cpx<T>* in  = reinterpret_cast<const cpx<T>*>(a.in) + b * a.in_stride + c0;
+    cpx<T>* out       = reinterpret_cast<cpx<T>*>(a.out) + b * a.out_stride + c0;
     const cpx<T>* twA = reinterpret_cast<const cpx<T>*>(a.twA);
     const cpx<T>* twB = reinterpret_cast<const cpx<T>*>(a.twB);
     // lanes beyond the last column repeat it: they read the same values and store the same results
@@ -68,7 +72,24 @@ __global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T), H), 1)
     const unsigned long long bytes = a.pitch * sizeof(cpx<T>);
     rp_run<T, H>(
         a.d, reinterpret_cast<cpx<T>*>(smem_raw), S, reinterpret_cast<const cpx<T>*>(a.tw),
-        [&](int g, int i) { return conj_if(*rp_at(in + min(g, last), i, bytes), cin); },
+        [&](int g, int i)
+        {
+            if constexpr (MERGE)
+            {
+                const cpx<T>* X   = in - c0;
+                const long long N = a.d.n * a.pitch, e = i * a.pitch + c0 + min(g, last);
+                if (e == 0)
+                {
+                    const T x0 = X[0].x, xn = a.ccs ? X[N].x : X[0].y;
+                    return mk<T>(x0 + xn, xn - x0);
+                }
+                const cpx<T> u = X[e], v = conj(X[N - e]);
+                const cpx<T> w = ldg(reinterpret_cast<const cpx<T>*>(a.rtw) + e);
+                return conj((u + v) + mul_pi(conj(w) * (u - v)));
+            }
+            else
+                return conj_if(*rp_at(in + min(g, last), i, bytes), cin);
+        },
         [&](int g, int i, cpx<T> v) { *rp_at(out + min(g, last), i, bytes) = conj_if(v, cout); },
         [&](int g, int k, int step, auto& o)
         {
@@ -115,8 +136,8 @@ __global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T), H), 1)
     const long long b = blockIdx.x / tiles;
     const int r0      = int(blockIdx.x - b * tiles) << a.d.shift;
     const int n       = a.d.n;
-    const cpx<T>* in  = reinterpret_cast<const cpx<T>*>(a.in) + b * a.sig_stride + (long long)r0 * n;
-    cpx<T>* out       = reinterpret_cast<cpx<T>*>(a.out) + b * a.sig_stride + r0;
+    const cpx<T>* in  = reinterpret_cast<const cpx<T>*>(a.in) + b * a.in_stride + (long long)r0 * n;
+    cpx<T>* out       = reinterpret_cast<cpx<T>*>(a.out) + b * a.out_stride + r0;
     // lanes beyond the last row repeat it
     const int last  = int(a.pitch - r0 < S ? a.pitch - r0 : S) - 1;
     const bool cin  = a.conj_in != 0, cout = a.conj_out != 0;
@@ -125,6 +146,57 @@ __global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T), H), 1)
         a.d, reinterpret_cast<cpx<T>*>(smem_raw), S, reinterpret_cast<const cpx<T>*>(a.tw),
         [&](int g, int i) { return conj_if(*rp_at(in + (long long)min(g, last) * n, i, uint32_t(sizeof(cpx<T>))), cin); },
         [&](int g, int i, cpx<T> v) { *rp_at(out + min(g, last), i, bytes) = conj_if(v, cout); });
+}
+
+// ---------------------------------------------------------------------------------------------------
+// Second pass of a real forward DFT of 2N reals, N = n1 n: the row DFTs of k_rp_rows, whose outputs Z[k1 + n1 k] stay
+// in shared memory, then the split (to_fmt, src/dft/fft-impl.hpp:1799-1841)
+//   X[e] = (Z[e] + conj Z[N-e]) / 2 - i W_2N^e (Z[e] - conj Z[N-e]) / 2
+// into the spectrum (N + 1 bins, or N packed).  N - e lies in row n1 - k1, so a tile is S / 2 mirror pairs of rows
+// (k1, n1 - k1), k1 = 1 .. ; the pair 0 is the rows 0 and n1 / 2, which mirror into themselves.  Two round trips
+// instead of three.
+// ---------------------------------------------------------------------------------------------------
+template <typename T, int H>
+__global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T), H), 1)
+    k_rp_rows_split(const __grid_constant__ rp_strided_args a)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int S = 1 << a.d.shift, half = S >> 1;
+    const int n1 = int(a.pitch), n = a.d.n;
+    const int pairs   = (n1 - 1) / 2 + 1;
+    const int tiles   = (pairs + half - 1) / half;
+    const long long b = blockIdx.x / tiles;
+    const int q0      = int(blockIdx.x - b * tiles) * half;
+    const long long N = (long long)n1 * n;
+    const cpx<T>* in  = reinterpret_cast<const cpx<T>*>(a.in) + b * a.in_stride;
+    cpx<T>* out       = reinterpret_cast<cpx<T>*>(a.out) + b * a.out_stride;
+    const cpx<T>* rtw = reinterpret_cast<const cpx<T>*>(a.rtw);
+    cpx<T>* z         = reinterpret_cast<cpx<T>*>(smem_raw);
+    // pair and row of signal g; lanes beyond the last pair repeat it
+    const auto pair_of = [&](int g) { return min(q0 + (g & (half - 1)), pairs - 1); };
+    const auto row_of  = [&](int g, int q)
+    { return g < half ? q : q ? n1 - q : n1 & 1 ? 0 : n1 / 2; };
+    rp_run_in<T, H>(a.d, z, S, reinterpret_cast<const cpx<T>*>(a.tw),
+                    [&](int g, int i)
+                    { return *rp_at(in + (long long)row_of(g, pair_of(g)) * n, i, uint32_t(sizeof(cpx<T>))); });
+    for (int i = threadIdx.x; i < S * n; i += blockDim.x)
+    {
+        const int g = i & (S - 1), k = i >> a.d.shift;
+        const int q = pair_of(g), row = row_of(g, q);
+        // Z[N - e]: the other row of the pair, or the same row
+        const int mg      = q ? g ^ half : g;
+        const int mirror  = row ? n - 1 - k : k ? n - k : 0;
+        const cpx<T> u    = z[i], v = conj(z[mirror * S + mg]);
+        const long long e = row + (long long)n1 * k;
+        if (e == 0)
+        {
+            out[0] = mk<T>(u.x + u.y, a.ccs ? T(0) : u.x - u.y);
+            if (a.ccs)
+                out[N] = mk<T>(u.x - u.y, T(0));
+        }
+        else
+            out[e] = scale(u + v, T(0.5)) + ldg(rtw + e) * scale(mul_mi(u - v), T(0.5));
+    }
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -156,11 +228,20 @@ template <typename T, int H>
 cudaError_t launch_rp_strided(const rp_strided_args& a, bool cols, int threads, int smem, cudaStream_t st)
 {
     const long long tiles = (a.pitch + (1 << a.d.shift) - 1) >> a.d.shift;
-    return rp_go(cols ? k_rp_cols<T, H> : k_rp_rows<T, H>, a, tiles * a.batch, threads, smem, st);
+    return rp_go(!cols ? k_rp_rows<T, H> : a.rtw ? k_rp_cols<T, H, true> : k_rp_cols<T, H, false>, a, tiles * a.batch,
+                 threads, smem, st);
+}
+
+template <typename T, int H>
+cudaError_t launch_rp_rows_split(const rp_strided_args& a, int threads, int smem, cudaStream_t st)
+{
+    const long long pairs = (a.pitch - 1) / 2 + 1, half = 1LL << (a.d.shift - 1);
+    return rp_go(k_rp_rows_split<T, H>, a, (pairs + half - 1) / half * a.batch, threads, smem, st);
 }
 
 #define KFR_GPU_RP_INSTANTIATE(T, H)                                                                       \
     template cudaError_t launch_rp_c2c<T, H>(const rp_c2c_args&, int, int, cudaStream_t);                  \
-    template cudaError_t launch_rp_strided<T, H>(const rp_strided_args&, bool, int, int, cudaStream_t);
+    template cudaError_t launch_rp_strided<T, H>(const rp_strided_args&, bool, int, int, cudaStream_t);    \
+    template cudaError_t launch_rp_rows_split<T, H>(const rp_strided_args&, int, int, cudaStream_t);
 
 } // namespace kfr_gpu

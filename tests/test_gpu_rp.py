@@ -79,7 +79,9 @@ def test_axes(shape, batch, sfx):
 
 
 # the in-place kernels of the real DFT and the DCT: a tail of a tile, one signal, 32 values per thread, primes
-@pytest.mark.parametrize("n,batch", [(2 * 30, 1001), (1000, 301), (2 * 1155, 70), (2 * 6561, 3), (2 * 18000, 2), (2 * 17 * 64, 5)])
+@pytest.mark.parametrize("n,batch", [(2 * 30, 1001), (1000, 301), (2 * 1155, 70), (2 * 6561, 3), (2 * 18000, 2), (2 * 17 * 64, 5),
+                                     # four-step half lengths: the merge in the column pass
+                                     (44100, 3), (100000, 3), (131072, 2)])
 @pytest.mark.parametrize("sfx", ["f32", "f64"])
 def test_real(n, batch, sfx):
     rng = np.random.default_rng(n)
