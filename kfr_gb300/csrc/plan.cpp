@@ -75,6 +75,63 @@ void dbuf::upload(const void* host, size_t bytes)
 }
 
 // ------------------------------------------------------------------------------------------------------
+// error_flag
+// ------------------------------------------------------------------------------------------------------
+
+namespace
+{
+// Words handed out from page-locked pages (one allocation per 1024 plans); returned words are used again.
+struct flag_pool
+{
+    std::mutex mu;
+    std::vector<std::pair<volatile int*, int*>> free;
+};
+flag_pool& flags()
+{
+    static flag_pool* p = new flag_pool; // outlives every plan
+    return *p;
+}
+} // namespace
+
+void error_flag::alloc()
+{
+    if (dev_)
+        return;
+    flag_pool& p = flags();
+    std::lock_guard<std::mutex> lock(p.mu);
+    if (p.free.empty())
+    {
+        constexpr int words = 1024;
+        void *host = nullptr, *dev = nullptr;
+        check(cudaHostAlloc(&host, words * sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped), "allocate error flags");
+        check(cudaHostGetDevicePointer(&dev, host, 0), "map error flags");
+        for (int i = words - 1; i >= 0; i--)
+            p.free.emplace_back(static_cast<int*>(host) + i, static_cast<int*>(dev) + i);
+    }
+    host_ = p.free.back().first;
+    dev_  = p.free.back().second;
+    p.free.pop_back();
+    *host_ = 0;
+}
+
+error_flag::~error_flag()
+{
+    if (!dev_)
+        return;
+    flag_pool& p = flags();
+    std::lock_guard<std::mutex> lock(p.mu);
+    p.free.emplace_back(host_, dev_);
+}
+
+bool error_flag::take() const
+{
+    if (!host_ || !*host_)
+        return false;
+    *host_ = 0;
+    return true;
+}
+
+// ------------------------------------------------------------------------------------------------------
 // Twiddles and factorisation
 // ------------------------------------------------------------------------------------------------------
 
@@ -913,8 +970,7 @@ void complex_engine<T>::init_rader(long long n)
     qof_.upload(qof.data(), qof.size() * sizeof(int));
     if (sizeof(T) == 4)
     {
-        err_.alloc(sizeof(int));
-        check(cudaMemset(err_.get(), 0, sizeof(int)), "clear error flag");
+        err_.alloc();
     }
     bhat_.upload(bh.data(), bh.size() * sizeof(std::complex<T>));
     prog_.build(int(L), CT_RADER);
@@ -1003,28 +1059,19 @@ void complex_engine<T>::plan_pipe()
         if (n >= 8192 && ((prog_.gstride + 1) / 2 * 2 + n / 2) * esz + 16 <= smem_budget())
         {
             reg_ = true;
-            err_.alloc(sizeof(int));
-            check(cudaMemset(err_.get(), 0, sizeof(int)), "clear error flag");
+            err_.alloc();
         }
         return;
     }
     pipe_spc_ = best;
-    err_.alloc(sizeof(int));
-    check(cudaMemset(err_.get(), 0, sizeof(int)), "clear error flag");
+    err_.alloc();
 }
 
 template <typename T>
 void complex_engine<T>::check_device_error() const
 {
-    if (!err_.get())
-        return;
-    int v = 0;
-    check(cudaMemcpy(&v, err_.get(), sizeof(int), cudaMemcpyDeviceToHost), "read error flag");
-    if (v)
-    {
-        cudaMemset(err_.get(), 0, sizeof(int));
+    if (err_.take())
         throw cuda_error("a DFT kernel gave up waiting for its input copy (device error flag set)");
-    }
 }
 
 template <typename T>
@@ -1131,8 +1178,7 @@ bool complex_engine<T>::plan_fourstep(long long n)
             tiles(pcols_, tile_c_, pp_c_);
             tiles(prows_, tile_r_, pp_r_);
             pair_ = true;
-            err_.alloc(sizeof(int)); // the persistent tensor-copy pair kernels report a copy that never lands
-            check(cudaMemset(err_.get(), 0, sizeof(int)), "clear error flag");
+            err_.alloc(); // the persistent tensor-copy pair kernels report a copy that never lands
             upload_roots<T>(n, twA_, twB_, lbits_);
             // an odd row pitch takes no tensor copies: the complex passes then run the runtime-length four-step
             // (22050 points, 1521 signals: 448 -> 227 us); the pair stays for the real split (pair_view_of)
@@ -1159,7 +1205,7 @@ bool complex_engine<T>::pair_view_of(pair_view& v) const
     v.twA     = twA_.get();
     v.twB     = twB_.get();
     v.lbits   = lbits_;
-    v.err     = static_cast<int*>(err_.get());
+    v.err     = err_.get();
     return true;
 }
 
@@ -1292,7 +1338,7 @@ void complex_engine<T>::execute(void* out, const void* in, long long batch, long
         {
             block_cfg rc = prog_.cfg_tile(1);
             rc.smem      = ((prog_.gstride + 1) / 2 * 2 + int(n_ / 2)) * int(esz) + 16;
-            check(launch_ct_c2c_reg_f32(a, rc, batch, static_cast<int*>(err_.get()), st), "launch c2c (one per CTA)");
+            check(launch_ct_c2c_reg_f32(a, rc, batch, err_.get(), st), "launch c2c (one per CTA)");
             done = batch;
         }
         if (pipe_spc_ && !host_io_ && istride == n_ && ostride == n_ && (reinterpret_cast<uintptr_t>(in) % 16) == 0)
@@ -1302,7 +1348,7 @@ void complex_engine<T>::execute(void* out, const void* in, long long batch, long
             {
                 block_cfg pc = prog_.cfg_tile(pipe_spc_);
                 pc.smem = 3 * pipe_stage_len(pipe_spc_, int(n_), prog_.gstride) * int(esz) + 64;
-                check(launch_ct_c2c_pipe_f32(a, pc, ntiles, static_cast<int*>(err_.get()), st), "launch c2c (pipelined)");
+                check(launch_ct_c2c_pipe_f32(a, pc, ntiles, err_.get(), st), "launch c2c (pipelined)");
                 done = ntiles * pipe_spc_;
             }
         }
@@ -1349,7 +1395,7 @@ void complex_engine<T>::execute(void* out, const void* in, long long batch, long
             p.tin     = static_cast<const int*>(tin_.get());
             p.tout    = static_cast<const int*>(tout_.get());
             p.bphys   = bphys_.get();
-            p.err     = static_cast<int*>(err_.get());
+            p.err     = err_.get();
             check(launch_rader_pfa_f32(p, n_, st), "launch rader (prime factor)");
             return;
         }
@@ -1401,7 +1447,7 @@ void complex_engine<T>::execute(void* out, const void* in, long long batch, long
             fourstep_args a;
             // the tensor-copy pair kernels run only with an error flag: host-mapped buffers take the plain-load
             // pair kernels
-            a.err        = pair_ && !host_io_ ? static_cast<int*>(err_.get()) : nullptr;
+            a.err        = pair_ && !host_io_ ? err_.get() : nullptr;
             a.batch      = nb;
             a.sig_stride = n_;
             a.n1         = int(n1_);
@@ -1552,15 +1598,8 @@ template <typename T>
 void real_engine<T>::check_device_error() const
 {
     ceng_.check_device_error();
-    if (!err_.get())
-        return;
-    int v = 0;
-    check(cudaMemcpy(&v, err_.get(), sizeof(int), cudaMemcpyDeviceToHost), "read error flag");
-    if (v)
-    {
-        cudaMemset(err_.get(), 0, sizeof(int));
+    if (err_.take())
         throw cuda_error("a real DFT kernel gave up waiting for its input copy (device error flag set)");
-    }
 }
 
 template <typename T>
@@ -1623,8 +1662,7 @@ real_engine<T>::real_engine(long long n) : n_(n), c_(n / 2), ceng_(n / 2)
         if (best)
         {
             pipe_spc_ = best;
-            err_.alloc(sizeof(int));
-            check(cudaMemset(err_.get(), 0, sizeof(int)), "clear error flag");
+            err_.alloc();
         }
     }
 }
@@ -1693,7 +1731,7 @@ void real_engine<T>::forward(void* out, const void* in, long long batch, bool cc
                 block_cfg pc = p.cfg_tile(pipe_spc_);
                 pc.smem = 3 * ((std::max(pipe_spc_ * int(c_ + 1), pipe_spc_ * p.gstride) + 15) / 16 * 16) *
                               int(2 * sizeof(T)) + 64;
-                check(launch_ct_r2c_pipe_f32(a, pc, ntiles, static_cast<int*>(err_.get()), st), "launch r2c (pipelined)");
+                check(launch_ct_r2c_pipe_f32(a, pc, ntiles, err_.get(), st), "launch r2c (pipelined)");
                 done = ntiles * pipe_spc_;
             }
         }
@@ -1799,7 +1837,7 @@ void real_engine<T>::inverse(void* out, const void* in, long long batch, bool cc
                 block_cfg pc = p.cfg_tile(pipe_spc_);
                 pc.smem = 3 * ((std::max(pipe_spc_ * int(c_ + 1), pipe_spc_ * p.gstride) + 15) / 16 * 16) *
                               int(2 * sizeof(T)) + 64;
-                check(launch_ct_c2r_pipe_f32(a, pc, ntiles, static_cast<int*>(err_.get()), st), "launch c2r (pipelined)");
+                check(launch_ct_c2r_pipe_f32(a, pc, ntiles, err_.get(), st), "launch c2r (pipelined)");
                 done = ntiles * pipe_spc_;
             }
         }
@@ -1899,8 +1937,7 @@ dct_engine<T>::dct_engine(long long n) : n_(n), ceng_(n)
         if (best)
         {
             pipe_spc_ = best;
-            err_.alloc(sizeof(int));
-            check(cudaMemset(err_.get(), 0, sizeof(int)), "clear error flag");
+            err_.alloc();
         }
     }
 }
@@ -1909,15 +1946,8 @@ template <typename T>
 void dct_engine<T>::check_device_error() const
 {
     ceng_.check_device_error();
-    if (!err_.get())
-        return;
-    int v = 0;
-    check(cudaMemcpy(&v, err_.get(), sizeof(int), cudaMemcpyDeviceToHost), "read error flag");
-    if (v)
-    {
-        cudaMemset(err_.get(), 0, sizeof(int));
+    if (err_.take())
         throw cuda_error("a DCT kernel gave up waiting for its input copy (device error flag set)");
-    }
 }
 
 template <typename T>
@@ -1963,7 +1993,7 @@ void dct_engine<T>::execute(void* out, const void* in, long long batch, bool inv
                 block_cfg pc = p.cfg_tile(pipe_spc_);
                 pc.smem = 3 * ((std::max(pipe_spc_ * int(n_) / 2, pipe_spc_ * p.gstride) + 15) / 16 * 16) *
                               int(2 * sizeof(T)) + 64;
-                check(launch_ct_dct_pipe_f32(a, pc, ntiles, static_cast<int*>(err_.get()), inverse, st),
+                check(launch_ct_dct_pipe_f32(a, pc, ntiles, err_.get(), inverse, st),
                       "launch dct (pipelined)");
                 done = ntiles * pipe_spc_;
             }

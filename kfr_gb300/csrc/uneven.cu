@@ -417,8 +417,7 @@ uneven_plan::uneven_plan(const std::vector<long long>& lengths, bool autotune) :
         total_ += lengths[i];
     }
     check(cudaStreamCreateWithFlags(&cap_, cudaStreamNonBlocking), "create stream");
-    derr_.alloc(sizeof(int));
-    check(cudaMemset(derr_.get(), 0, sizeof(int)), "clear error flag");
+    err_.alloc();
 
     // 256-thread CTAs, four per SM, unless a length needs passes that only 512 threads can hold
     const auto plannable = [&](splitter& sp, long long n)
@@ -499,7 +498,7 @@ uneven_plan::uneven_plan(const std::vector<long long>& lengths, bool autotune) :
                     uneven_launch L{ static_cast<uneven_fft*>(tffts.get()), static_cast<uneven_job*>(tjobs.get()),
                                      static_cast<uneven_item*>(titems.get()), static_cast<long long*>(toffs.get()),
                                      int(its.size()), static_cast<int*>(tq.get()), nullptr,
-                                     static_cast<int*>(derr_.get()), tin.get(), tout.get(), nullptr, 0 };
+                                     err_.get(), tin.get(), tout.get(), nullptr, 0 };
                     const int smem = spc * elems * 8;
                     const int grid = std::min<int>(int(its.size()), 1024 / threads_ * sms);
                     for (int rep = 0; rep < 4; rep++)
@@ -756,7 +755,7 @@ void uneven_plan::enqueue(void* out, const void* in, bool inverse, cudaStream_t 
     uneven_launch L{ static_cast<uneven_fft*>(dffts_.get()), static_cast<uneven_job*>(djobs_.get()),
                      static_cast<uneven_item*>(ditems_.get()), static_cast<long long*>(doffsets_.get()), nitems_,
                      static_cast<int*>(dqueue_.get()), static_cast<int*>(dcounters_.get()),
-                     static_cast<int*>(derr_.get()), in, out, scratch_.get(), inverse ? 1 : 0, wait_limit(),
+                     err_.get(), in, out, scratch_.get(), inverse ? 1 : 0, wait_limit(),
                      unreachable_ ? 1 : 0 };
     check(launch_uneven_f32(L, threads_, smem_, grid_, st), "launch uneven batch");
 }
@@ -802,13 +801,8 @@ void uneven_plan::execute(void* out, const void* in, bool inverse, cudaStream_t 
 
 void uneven_plan::check_device_error() const
 {
-    int v = 0;
-    check(cudaMemcpy(&v, derr_.get(), sizeof(int), cudaMemcpyDeviceToHost), "read error flag");
-    if (v)
-    {
-        cudaMemset(derr_.get(), 0, sizeof(int));
+    if (err_.take())
         throw cuda_error("an uneven-batch tile gave up waiting for the stage it depends on (device error flag)");
-    }
 }
 
 void uneven_plan::execute_per_signal(void* out, const void* in, bool inverse, cudaStream_t st)

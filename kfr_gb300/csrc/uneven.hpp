@@ -124,13 +124,14 @@ private:
         const void* tw;
     };
     using shape_key = std::tuple<long long, int, int, bool>; // length, rp_layout, signals per tile, smem_io
+    error_flag err_; // first: destroyed after the device buffers
     std::vector<long long> lengths_, offsets_;
     long long total_ = 0;
     std::vector<shape> shapes_;
     std::map<shape_key, int> shape_of_;
     std::map<std::vector<int>, const void*> tw_of_; // radix order -> twiddles
     std::vector<std::unique_ptr<dbuf>> tables_;     // twiddles, chirps, spectra and four-step roots
-    dbuf dffts_, djobs_, ditems_, doffsets_, dqueue_, dcounters_, derr_, scratch_;
+    dbuf dffts_, djobs_, ditems_, doffsets_, dqueue_, dcounters_, scratch_;
     int nitems_ = 0, ncounters_ = 0, smem_ = 0, grid_ = 0, threads_ = 256;
     int n_direct_ = 0, n_blue1_ = 0, n_fourstep_ = 0, n_blue_fs_ = 0;
     std::map<long long, std::unique_ptr<complex_engine<float>>> engines_; // plain form only
