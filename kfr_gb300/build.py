@@ -30,7 +30,7 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 CU_SOURCES = [
     "kernels_convolved_f32.cu", "kernels_convolved_f64.cu", "kernels_real_f32.cu", "kernels_real_f64.cu",
     "kernels_dct_f32.cu", "kernels_dct_f64.cu", "rp_f32.cu", "rp_f64.cu", "rp_f32_long.cu", "rp_f64_long.cu",
-    "kernels_ct_a.cu", "kernels_ct_b.cu", "kernels_ct_c.cu", "elementwise.cu",
+    "kernels_ct_a.cu", "kernels_ct_b.cu", "kernels_ct_c.cu", "fourstep_ct.cu", "elementwise.cu",
     "conv.cu", "convolve.cu", "adjoint.cu", "uneven.cu", "tensor.cu", "static_scratch.cu", "rader_pfa.cu",
 ]
 CPP_SOURCES = ["plan.cpp", "rp.cpp", "workspace.cpp", "md.cpp", "capi.cpp", "launch_cache.cpp"]

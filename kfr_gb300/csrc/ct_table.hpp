@@ -37,18 +37,14 @@
     X(126, 9, 14, 9)                                                                                         \
     X(8190, 1024, 13, 9, 14, 5)
 
-// four-step pass lengths (columns and rows): the factors of 30720 = 160 x 192, of the power-of-two lengths
-// 2^16 .. 2^24 and of the real-DFT half lengths 22050 = 147 x 150 and 24000 = 150 x 160 (N = 44100, 48000)
+// four-step pass lengths (columns and rows): the factors of 30720 = 160 x 192, 2^16 = 256 x 256 and of the real-DFT
+// half lengths 22050 = 147 x 150 and 24000 = 150 x 160 (N = 44100, 48000)
 #define KFR_CT_FOURSTEP_F32(X)                                                                              \
     X(147, 21, 7, 7, 3)                                                                                      \
     X(150, 15, 10, 15)                                                                                       \
     X(160, 16, 16, 10)                                                                                       \
     X(192, 16, 16, 12)                                                                                       \
-    X(256, 16, 16, 16)                                                                                       \
-    X(512, 64, 8, 8, 8)                                                                                      \
-    X(1024, 64, 16, 16, 4)                                                                                   \
-    X(2048, 128, 16, 16, 8)                                                                                  \
-    X(4096, 256, 16, 16, 16)
+    X(256, 16, 16, 16)
 
 // half lengths c = N/2 of the fused real DFT (dft_plan_real<float>): N = 1920, 2048, 4096, 8192
 #define KFR_CT_REAL_F32(X)                                                                                  \
@@ -74,12 +70,18 @@
 #define KFR_CT_FSPAIR_F32(X)                                                                                \
     X(160, 192)                                                                                              \
     X(256, 256)                                                                                              \
-    X(512, 512)                                                                                              \
-    X(1024, 1024)                                                                                            \
     X(147, 150)                                                                                              \
-    X(150, 160)                                                                                              \
-    X(2048, 2048)                                                                                            \
-    X(4096, 4096)
+    X(150, 160)
+
+// square four-step splits N = n^2 whose passes run on the block FFT of rp_fft.cuh with compile-time indices, tiles of S
+// signals: X(n, S, radices...).  1 GiB batches: 512 (2^18) 811 -> 702 us, 1024 (2^20) 906 -> 803, 2048 (2^22) 1194 ->
+// 944, 4096 (2^24) 1448 -> 1164 against tensor-copy passes of one CTA per SM (three shared buffers; here one, and two
+// or four CTAs).  S and the radices are the fastest of sweeps over S = 2 .. 16 and all orders of radices 4, 8 and 16.
+#define KFR_CT_SQUARE_F32(X)                                                                                \
+    X(512, 8, 16, 8, 4)                                                                                     \
+    X(1024, 8, 16, 8, 8)                                                                                    \
+    X(2048, 4, 16, 8, 16)                                                                                   \
+    X(4096, 4, 16, 16, 16)
 
 // Shared-memory layout of a compile-time length (single precision): X(N, TS, pad shift, extra group stride).
 // Element i of a signal sits at i + (i >> shift) (shift 0: unpadded), signals of a CTA lie `stride` elements

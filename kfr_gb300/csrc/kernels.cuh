@@ -1086,9 +1086,6 @@ __global__ void __launch_bounds__(F::max_threads, 1)
         bulk_wait_all();
 }
 
-// ---------------------------------------------------------------------------------------------------
-// Four-step passes for lengths beyond one CTA (N = n1 * n2).  grid = (tiles, batch).
-// ---------------------------------------------------------------------------------------------------
 template <typename T>
 __device__ __forceinline__ cpx<T> twiddle_2level(const cpx<T>* __restrict__ A, const cpx<T>* __restrict__ B,
                                                  long long m, int lbits)
@@ -1096,143 +1093,9 @@ __device__ __forceinline__ cpx<T> twiddle_2level(const cpx<T>* __restrict__ A, c
     return ldg(A + (m >> lbits)) * ldg(B + (m & ((1LL << lbits) - 1)));
 }
 
-template <typename T, class F>
-__global__ void __launch_bounds__(F::max_threads, 1) k_fs_cols(const fourstep_args a, const int ts)
-{
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const F fft(a.d, ts, a.tile);
-    cpx<T>* sm       = reinterpret_cast<cpx<T>*>(smem_raw);
-    const int n1     = fft.n, n2 = a.n2, S = a.tile, sh = a.tile_shift;
-    const int stride = F::gstride(n1);
-    const int c0     = blockIdx.x * S;
-    const long long sig = blockIdx.y;
-    const cpx<T>* __restrict__ x = reinterpret_cast<const cpx<T>*>(a.in) + sig * a.sig_stride;
-    cpx<T>* __restrict__ y       = reinterpret_cast<cpx<T>*>(a.out) + sig * a.sig_stride;
-    const bool cin  = a.conj_in != 0;
-    const int total = S * n1;
-    copy_batched<8>(
-        total,
-        [&](int i)
-        {
-            const int n1i = i >> sh; // S is a power of two
-            const int c   = i & (S - 1);
-            return c0 + c < n2 ? x[(long long)n1i * n2 + c0 + c] : mk<T>(0, 0);
-        },
-        [&](int i, cpx<T> v)
-        {
-            const int n1i = i >> sh;
-            const int c   = i & (S - 1);
-            sm[c * stride + F::pi(n1i)] = conj_if(v, cin);
-        });
-    __syncthreads();
-    const group_map gm(ts, S);
-    const cpx<T>* twA = reinterpret_cast<const cpx<T>*>(a.twA);
-    const cpx<T>* twB = reinterpret_cast<const cpx<T>*>(a.twB);
-    if constexpr (F::compile_time)
-    {
-        if (a.pingpong)
-        {
-            // ping-pong passes with a second buffer after the tile; the last pass applies W_N^{col k1} and
-            // stores the column contiguously (stride one across a signal's threads)
-            const int col      = c0 + gm.g;
-            const bool cout    = a.conj_out != 0;
-            const auto nothing = []() {};
-            fft.run_pp([&](int p) { return sm[gm.g * stride + F::pi(p)]; },
-                       [&](int k1, cpx<T> v)
-                       {
-                           if (col < n2)
-                               y[(long long)col * n1 + k1] =
-                                   conj_if(v * twiddle_2level(twA, twB, (long long)col * k1, a.lbits), cout);
-                       },
-                       nothing, nothing, sm + gm.g * stride, sm + (S + gm.g) * stride,
-                       reinterpret_cast<const cpx<T>*>(a.tw), gm.lt);
-            return;
-        }
-    }
-    fft.run(sm, reinterpret_cast<const cpx<T>*>(a.tw));
-#pragma unroll 4
-    for (int i = threadIdx.x; i < total; i += blockDim.x)
-    {
-        const int c  = int(div_by(uint32_t(i), a.div_n));
-        const int k1 = i - c * n1;
-        const int col = c0 + c;
-        if (col < n2)
-        {
-            cpx<T> v = sm[c * stride + F::pi(k1)];
-            v        = v * twiddle_2level(twA, twB, (long long)col * k1, a.lbits);
-            y[(long long)col * n1 + k1] = conj_if(v, a.conj_out != 0);
-        }
-    }
-}
-
-template <typename T, class F>
-__global__ void __launch_bounds__(F::max_threads, 1) k_fs_rows(const fourstep_args a, const int ts)
-{
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const F fft(a.d, ts, a.tile);
-    cpx<T>* sm       = reinterpret_cast<cpx<T>*>(smem_raw);
-    const int n1     = a.n1, n2 = fft.n, S = a.tile, sh = a.tile_shift;
-    const int stride = F::gstride(n2);
-    const int r0     = blockIdx.x * S;
-    const long long sig = blockIdx.y;
-    const cpx<T>* __restrict__ y = reinterpret_cast<const cpx<T>*>(a.in) + sig * a.sig_stride;
-    cpx<T>* __restrict__ X       = reinterpret_cast<cpx<T>*>(a.out) + sig * a.sig_stride;
-    const int total = S * n2;
-    const bool cin  = a.conj_in != 0;
-    copy_batched<8>(
-        total,
-        [&](int i)
-        {
-            const int n2i = i >> sh;
-            const int r   = i & (S - 1);
-            return r0 + r < n1 ? y[(long long)n2i * n1 + r0 + r] : mk<T>(0, 0);
-        },
-        [&](int i, cpx<T> v)
-        {
-            const int n2i = i >> sh;
-            const int r   = i & (S - 1);
-            sm[r * stride + F::pi(n2i)] = conj_if(v, cin);
-        });
-    __syncthreads();
-    const group_map gm(ts, S);
-    const bool cout = a.conj_out != 0;
-    if constexpr (F::compile_time)
-    {
-        if (a.pingpong)
-        {
-            // ping-pong passes with a second buffer after the tile; the last pass stages its output as
-            // [k2][row] (rows XOR-swizzled by k2) in the buffer it does not read, for row-contiguous stores
-            cpx<T>* B          = sm + S * stride;
-            cpx<T>* stg        = F::npass % 2 == 0 ? sm : B;
-            const auto nothing = []() {};
-            fft.run_pp([&](int p) { return sm[gm.g * stride + F::pi(p)]; },
-                       [&](int k2, cpx<T> v) { stg[k2 * S + (gm.g ^ (k2 & (S - 1)))] = v; }, nothing, nothing,
-                       sm + gm.g * stride, B + gm.g * stride, reinterpret_cast<const cpx<T>*>(a.tw), gm.lt);
-#pragma unroll 4
-            for (int i = threadIdx.x; i < total; i += blockDim.x)
-            {
-                const int k2 = i >> sh;
-                const int r  = i & (S - 1);
-                if (r0 + r < n1)
-                    X[(long long)(r0 + r) + (long long)n1 * k2] = conj_if(stg[k2 * S + (r ^ (k2 & (S - 1)))], cout);
-            }
-            return;
-        }
-    }
-    fft.run(sm, reinterpret_cast<const cpx<T>*>(a.tw));
-#pragma unroll 4
-    for (int i = threadIdx.x; i < total; i += blockDim.x)
-    {
-        const int k2 = i >> sh;
-        const int r  = i & (S - 1);
-        if (r0 + r < n1)
-            X[(long long)(r0 + r) + (long long)n1 * k2] = conj_if(sm[r * stride + F::pi(k2)], cout);
-    }
-}
-
 // ---------------------------------------------------------------------------------------------------
 // Four-step passes with both lengths, the tile and the twiddle split known at compile time (KFR_CT_FSPAIR):
-// the same work as the ping-pong branches of k_fs_cols / k_fs_rows with every index folded to constants.
+// ping-pong passes on plain loads and stores, every index folded to constants.
 // ---------------------------------------------------------------------------------------------------
 template <int N>
 __host__ __device__ constexpr int lbits_for()
@@ -1326,16 +1189,14 @@ __global__ void __launch_bounds__(1024, 1) k_fsp_rows(const fourstep_args a)
 
 // ---------------------------------------------------------------------------------------------------
 // Four-step pair kernels, persistent, with 2-D tensor copies (TMA).  Same transforms as k_fsp_cols /
-// k_fsp_rows for lengths of two or three passes: a tile is S columns (rows) of the signal, S = 16, 8, 4 or 2
+// k_fsp_rows for columns of two or three passes and rows of two: a tile is S columns (rows) of the signal, S = 16, 8, 4 or 2
 // contiguous 8-byte elements (128 to 16 bytes) per row, loaded as one box per 256 rows with the matching
 // swizzle (128, 64, 32 bytes; none for 16) and double buffered: the next tile streams in while the CTA
 // transforms the current one.  Waits are bounded; one that runs out sets *err and the CTA returns.
 //   column pass: the four-step twiddle per butterfly of the last pass; two passes: the tile's S output
 //     columns (contiguous in the intermediate) are written over the box and stored by one bulk copy; three
 //     passes (the box is the ping-pong A buffer): stored straight from the last pass;
-//   row pass: two passes: the output is written back into the swizzled box and stored by tensor copies;
-//     three passes: threads are ordered row-fastest, so the last pass stores S consecutive outputs per
-//     column index straight to global memory.
+//   row pass (two passes): the output is written back into the swizzled box and stored by tensor copies.
 //   in map (columns): x viewed as (2 N2 floats) x (N1 * batch) rows, box (2 S floats, min(N1, 256))
 //   in / out maps (rows): y and X viewed as (2 N1 floats) x (N2 * batch) rows, box (2 S floats, min(N2, 256))
 // ---------------------------------------------------------------------------------------------------
@@ -1524,21 +1385,18 @@ __global__ void __launch_bounds__(fspt_threads<FB>(), fspt_min_ctas<FB>())
     k_fspt_rows(const fourstep_args a, const __grid_constant__ tensor_map tm_in,
                 const __grid_constant__ tensor_map tm_out, const long long ntiles, int* err)
 {
-    static_assert(fspt_ok<FB>(), "two or three passes on tiles of 16 to 2 rows");
+    static_assert(fspt_ok<FB>(), "two passes on tiles of 16 to 2 rows");
     constexpr int N2 = FB::n, GB = FB::gstride(), TS = FB::ts, S = fspt_tile<FB>();
     constexpr int NTR = (N1 + S - 1) / S;
     constexpr int SE  = fspt_stage_elems<FB>(S);
     constexpr int BR  = N2 < 256 ? N2 : 256;
-    constexpr bool three = FB::npass == 3;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cpx<T>* st0    = reinterpret_cast<cpx<T>*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     cpx<T>* B      = st0 + 2 * SE;
     uint64_t* bars = reinterpret_cast<uint64_t*>(B + S * GB);
     const bool cin = a.conj_in != 0, cout = a.conj_out != 0;
-    // two passes: the S threads' groups are contiguous (each row's TS threads together); three passes: rows
-    // fastest, so that a warp's last-pass stores cover S consecutive outputs
-    const int g  = three ? int(threadIdx.x) % S : int(threadIdx.x) / TS;
-    const int lt = three ? int(threadIdx.x) / S : int(threadIdx.x) - g * TS;
+    const int g  = int(threadIdx.x) / TS;
+    const int lt = int(threadIdx.x) - g * TS;
     const cpx<T>* tw = reinterpret_cast<const cpx<T>*>(a.tw);
     const auto nothing = []() {};
     const FB fb;
@@ -1579,33 +1437,17 @@ __global__ void __launch_bounds__(fspt_threads<FB>(), fspt_min_ctas<FB>())
             fspt_load<S, N2>(st0 + (s ^ 1) * SE, &tm_in, int(tn % NTR) * 2 * S, int(tn / NTR) * N2, &bars[s ^ 1]);
         }
         const auto ld = [&](int p) { return conj_if(stage[swz_8b<S>(p, g)], cin); };
-        if constexpr (three)
+        // pass 1 reads the box, pass 2 writes the transformed rows back into it (same swizzled layout)
+        fb.run_pp(ld, [&](int k2, cpx<T> v) { stage[swz_8b<S>(k2, g)] = conj_if(v, cout); }, nothing, nothing,
+                  stage, B + g * GB, tw, lt);
+        fence_proxy_async_smem();
+        __syncthreads();
+        if (threadIdx.x == 0)
         {
-            const long long b = t / NTR;
-            const int r       = int(t % NTR) * S + g;
-            cpx<T>* X         = reinterpret_cast<cpx<T>*>(a.out) + b * (long long)N1 * N2;
-            fb.run_pp(ld,
-                      [&](int k2, cpx<T> v)
-                      {
-                          if (N1 % S == 0 || r < N1)
-                              X[r + (long long)N1 * k2] = conj_if(v, cout);
-                      },
-                      nothing, nothing, stage + g * GB, B + g * GB, tw, lt);
-        }
-        else
-        {
-            // pass 1 reads the box, pass 2 writes the transformed rows back into it (same swizzled layout)
-            fb.run_pp(ld, [&](int k2, cpx<T> v) { stage[swz_8b<S>(k2, g)] = conj_if(v, cout); }, nothing, nothing,
-                      stage, B + g * GB, tw, lt);
-            fence_proxy_async_smem();
-            __syncthreads();
-            if (threadIdx.x == 0)
-            {
 #pragma unroll 1
-                for (int bx = 0; bx < N2 / BR; bx++)
-                    tensor_s2g_2d(&tm_out, int(t % NTR) * 2 * S, int(t / NTR) * N2 + bx * BR, stage + bx * BR * S);
-                bulk_commit();
-            }
+            for (int bx = 0; bx < N2 / BR; bx++)
+                tensor_s2g_2d(&tm_out, int(t % NTR) * 2 * S, int(t / NTR) * N2 + bx * BR, stage + bx * BR * S);
+            bulk_commit();
         }
     }
     if (threadIdx.x == 0)

@@ -9,36 +9,6 @@
 namespace kfr_gpu
 {
 
-cudaError_t launch_ct_fs_cols_f32(const fourstep_args& a, const block_cfg& c, cudaStream_t st)
-{
-#define CT_KERNEL k_fs_cols
-#define CT_GRID KFR_GPU_GRID2
-#define CT_ARGS a, c.ts
-    switch (c.ct)
-    {
-        KFR_CT_FOURSTEP_F32(KFR_GPU_CT_CASE)
-    default: return cudaErrorInvalidValue;
-    }
-#undef CT_KERNEL
-#undef CT_GRID
-#undef CT_ARGS
-}
-
-cudaError_t launch_ct_fs_rows_f32(const fourstep_args& a, const block_cfg& c, cudaStream_t st)
-{
-#define CT_KERNEL k_fs_rows
-#define CT_GRID KFR_GPU_GRID2
-#define CT_ARGS a, c.ts
-    switch (c.ct)
-    {
-        KFR_CT_FOURSTEP_F32(KFR_GPU_CT_CASE)
-    default: return cudaErrorInvalidValue;
-    }
-#undef CT_KERNEL
-#undef CT_GRID
-#undef CT_ARGS
-}
-
 template <int N>
 struct fs_len;
 #define KFR_GPU_FS_LEN(N, TS, ...)                                                                         \
@@ -171,16 +141,13 @@ template <class FB, int N1>
 static cudaError_t try_fspt_rows(const fourstep_args& a, cudaStream_t st, bool& done)
 {
     done = false;
-    if constexpr (fspt_ok<FB>())
+    if constexpr (fspt_ok<FB>() && FB::npass == 2)
     {
         constexpr int N2 = FB::n, S = fspt_tile<FB>(), BR = N2 < 256 ? N2 : 256;
-        // the three-pass kernel stores from its last pass: no output map (the input map fills the slot)
         tensor_map mi, mo;
         if (!a.err || a.sig_stride != (long long)N1 * N2 || !map_rows(mi, a.in, N1, N2 * a.batch, BR, S))
             return cudaSuccess;
-        if (FB::npass == 3)
-            mo = mi;
-        else if (!map_rows(mo, a.out, N1, N2 * a.batch, BR, S))
+        if (!map_rows(mo, a.out, N1, N2 * a.batch, BR, S))
             return cudaSuccess;
         done = true;
         const long long ntiles = a.batch * ((N1 + S - 1) / S);
@@ -190,25 +157,17 @@ static cudaError_t try_fspt_rows(const fourstep_args& a, cudaStream_t st, bool& 
     return cudaSuccess;
 }
 
-// The per-tile pair kernels where their tiles (at least 8 signals) fit; cudaErrorNotSupported otherwise (the
-// caller then runs the generic four-step kernels).
+// The per-tile pair kernels (plain loads and stores).
 template <class FA, class FB, int A, int B>
 static cudaError_t go_fsp_pair(const fourstep_args& a, bool cols, cudaStream_t st)
 {
     constexpr int SA = fsp_tile(A, FA::ts, kFspSmem), SB = fsp_tile(B, FB::ts, kFspSmem);
+    static_assert(SA >= 8 && SB >= 8, "tiles of at least 8 signals");
     if (cols)
-    {
-        if constexpr (SA >= 8)
-            return go_fsp(k_fsp_cols<float, FA, B>, dim3((B + SA - 1) / SA, unsigned(a.batch)),
-                          (SA * FA::ts + 31) / 32 * 32, 2 * SA * FA::gstride() * 8, st, a);
-        else
-            return cudaErrorNotSupported;
-    }
-    if constexpr (SB >= 8)
-        return go_fsp(k_fsp_rows<float, FB, A>, dim3((A + SB - 1) / SB, unsigned(a.batch)),
-                      (SB * FB::ts + 31) / 32 * 32, 2 * SB * FB::gstride() * 8, st, a);
-    else
-        return cudaErrorNotSupported;
+        return go_fsp(k_fsp_cols<float, FA, B>, dim3((B + SA - 1) / SA, unsigned(a.batch)),
+                      (SA * FA::ts + 31) / 32 * 32, 2 * SA * FA::gstride() * 8, st, a);
+    return go_fsp(k_fsp_rows<float, FB, A>, dim3((A + SB - 1) / SB, unsigned(a.batch)), (SB * FB::ts + 31) / 32 * 32,
+                  2 * SB * FB::gstride() * 8, st, a);
 }
 
 bool has_ct_fsp_r2c_f32(int n1, int n2)

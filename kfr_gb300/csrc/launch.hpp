@@ -142,7 +142,6 @@ struct fourstep_args
     long long batch;
     long long sig_stride; // complex elements between consecutive signals
     int n1, n2;
-    int tile;             // columns (cols pass) or k1 rows (rows pass) per CTA
     int conj_in, conj_out;
     const void* tw;
     rp_desc d; // runtime lengths
@@ -150,8 +149,6 @@ struct fourstep_args
     const void* twA;
     const void* twB;
     int lbits;
-    int tile_shift;  // log2(tile)
-    int pingpong;    // compile-time kernels: ping-pong passes over two buffers per signal (2x shared memory)
     fast_div div_n;  // divides by the FFT length of this pass
     int* err;        // persistent pair kernels: set when a wait for a tile copy runs out (may be null)
     unsigned wait_spins = kDefaultWaitSpins;
@@ -196,6 +193,10 @@ template <typename T, int H>
 cudaError_t launch_rp_c2c(const rp_c2c_args& a, int threads, int smem, cudaStream_t st);
 template <typename T, int H>
 cudaError_t launch_rp_strided(const rp_strided_args& a, bool cols, int threads, int smem, cudaStream_t st);
+// Square splits with compile-time indices (fourstep_ct.cu): whether N = n^2 has one and the radices of its passes, and
+// a pass (a.pitch = n; the columns with the twiddle, or the rows; a.d unused).
+bool ct_square_f32(long long n, std::vector<int>& radices);
+cudaError_t launch_ct_square_f32(const rp_strided_args& a, bool cols, cudaStream_t st);
 // The rows of a real forward DFT's half-length four-step, split into the spectrum (a.rtw, a.ccs; the tile of a.d has
 // at least two rows and its last pass leaves shared memory in natural order).
 template <typename T, int H>
@@ -286,7 +287,6 @@ cudaError_t launch_ct_r2c_f32(const real_args& a, const block_cfg& c, cudaStream
 cudaError_t launch_ct_c2r_f32(const real_args& a, const block_cfg& c, cudaStream_t st);
 cudaError_t launch_ct_dct2_f32(const dct_args& a, const block_cfg& c, cudaStream_t st);
 cudaError_t launch_ct_dct3_f32(const dct_args& a, const block_cfg& c, cudaStream_t st);
-cudaError_t launch_ct_fs_cols_f32(const fourstep_args& a, const block_cfg& c, cudaStream_t st);
 // Compile-time pair kernels (KFR_CT_FSPAIR_F32): the column pass (cols = true) or the row pass of the split
 // a.n1 x a.n2 over a.batch signals (contiguous, a.batch <= 65535).  False / cudaErrorInvalidValue if the pair
 // has no kernel.
@@ -298,7 +298,6 @@ cudaError_t launch_ct_fsp_f32(const fourstep_args& a, bool cols, cudaStream_t st
 // the spectrum).  The caller checks the alignment first: a.in and the scratch 16-byte aligned.
 bool has_ct_fsp_r2c_f32(int n1, int n2);
 cudaError_t launch_ct_fsp_r2c_f32(const fourstep_args& a, bool cols, cudaStream_t st);
-cudaError_t launch_ct_fs_rows_f32(const fourstep_args& a, const block_cfg& c, cudaStream_t st);
 
 // Launch bookkeeping done once per process instead of on every launch (launch_cache.cpp): the kernel's
 // dynamic shared-memory limit is raised to at least `smem` the first time it is needed, and *per_sm (if

@@ -282,14 +282,6 @@ bool is_smooth(long long n)
     return n <= 1;
 }
 
-static int ilog2(int x)
-{
-    int s = 0;
-    while ((1 << s) < x)
-        s++;
-    return s;
-}
-
 int smem_budget()
 {
     // dynamic shared memory less a small reserve
@@ -1135,17 +1127,6 @@ void complex_engine<T>::init_bluestein(long long n)
     }
 }
 
-// Largest power-of-two number of signals (<= 16) of the compile-time length `p` that fit one CTA with `buffers`
-// shared-memory buffers per signal: the column / row tile of the strided passes.
-static int tile_for(const block_program<float>& p, int buffers)
-{
-    const int per_sig = buffers * p.gstride * 8;
-    int s             = 16;
-    while (s > 1 && (s * per_sig > smem_budget() || s * p.ts > 1024))
-        s /= 2;
-    return s;
-}
-
 template <typename T>
 bool complex_engine<T>::plan_fourstep(long long n)
 {
@@ -1164,19 +1145,6 @@ bool complex_engine<T>::plan_fourstep(long long n)
             n2_ = b;
             pcols_.build(a, CT_FOURSTEP);
             prows_.build(b, CT_FOURSTEP);
-            // tiles of the kernels that run where the pair kernels cannot (launch_ct_fsp_f32 then answers
-            // cudaErrorNotSupported): ping-pong passes (two buffers per signal) unless that would shrink a tile
-            // below 8 signals (short row segments coalesce poorly)
-            const auto tiles = [](const block_program<T>& p, int& tile, bool& pp)
-            {
-                tile         = tile_for(p, 1);
-                const int t2 = tile_for(p, 2);
-                pp           = t2 >= 8 || t2 == tile;
-                if (pp)
-                    tile = t2;
-            };
-            tiles(pcols_, tile_c_, pp_c_);
-            tiles(prows_, tile_r_, pp_r_);
             pair_ = true;
             err_.alloc(); // the persistent tensor-copy pair kernels report a copy that never lands
             upload_roots<T>(n, twA_, twB_, lbits_);
@@ -1184,6 +1152,19 @@ bool complex_engine<T>::plan_fourstep(long long n)
             // (22050 points, 1521 signals: 448 -> 227 us); the pair stays for the real split (pair_view_of)
             if (a % 2)
                 rp4_.build(n);
+            return true;
+        }
+    }
+    if constexpr (sizeof(T) == 4)
+    {
+        const long long r = std::llround(std::sqrt(double(n)));
+        if (r * r == n && ct_square_f32(r, square_radices_))
+        {
+            k_  = kind::fourstep;
+            n1_ = n2_ = r;
+            const auto t = pass_twiddles<T>(square_radices_);
+            square_tw_.upload(t.data(), t.size() * sizeof(t[0]));
+            upload_roots<T>(n, twA_, twB_, lbits_);
             return true;
         }
     }
@@ -1233,7 +1214,7 @@ int complex_engine<T>::launches(long long batch) const
             return (batch / pipe_spc_ > 0 ? 1 : 0) + (batch % pipe_spc_ ? 1 : 0);
         return 1;
     case kind::bluestein_smem: return 1;
-    case kind::fourstep: return rp4_.ready() ? 2 : 2 * int((batch + 65534) / 65535);
+    case kind::fourstep: return rp4_.ready() || square_tw_.get() ? 2 : 2 * int((batch + 65534) / 65535);
     case kind::bluestein_multi: return 3 + 2 * inner_->launches(batch);
     case kind::rader_smem: return 1;
     case kind::tensor: return n1_ ? 2 * int((batch + 65534) / 65535) : 1;
@@ -1429,25 +1410,41 @@ void complex_engine<T>::execute(void* out, const void* in, long long batch, long
             rp4_.execute(out, in, batch, inverse, scratch, st);
             return;
         }
-        // a pair kernel for this pass, or false when neither of them can run (the generic pass runs instead)
-        const auto run_pair = [&](const fourstep_args& fa, bool cols)
+        if (square_tw_.get())
         {
-            const cudaError_t e = launch_ct_fsp_f32(fa, cols, st);
-            if (e == cudaErrorNotSupported)
-                return false;
-            check(e, cols ? "launch four-step columns" : "launch four-step rows");
-            return true;
-        };
+            if constexpr (sizeof(T) == 4)
+            {
+                rp_strided_args a{};
+                a.batch      = batch;
+                a.in_stride  = n_;
+                a.out_stride = n_;
+                a.pitch      = n1_;
+                a.in         = in;
+                a.out        = scratch;
+                a.conj_in    = inverse;
+                a.tw         = square_tw_.get();
+                a.twA        = twA_.get();
+                a.twB        = twB_.get();
+                a.lbits      = lbits_;
+                check(launch_ct_square_f32(a, true, st), "launch four-step columns");
+                a.in       = scratch;
+                a.out      = out;
+                a.conj_in  = 0;
+                a.conj_out = inverse;
+                check(launch_ct_square_f32(a, false, st), "launch four-step rows");
+            }
+            return;
+        }
         for (long long b0 = 0; b0 < batch; b0 += 65535)
         {
             const long long nb  = std::min<long long>(65535, batch - b0);
             const char* inb     = static_cast<const char*>(in) + b0 * n_ * esz;
             char* outb          = static_cast<char*>(out) + b0 * n_ * esz;
             char* scr           = static_cast<char*>(scratch) + b0 * n_ * esz;
-            fourstep_args a;
+            fourstep_args a{};
             // the tensor-copy pair kernels run only with an error flag: host-mapped buffers take the plain-load
             // pair kernels
-            a.err        = pair_ && !host_io_ ? err_.get() : nullptr;
+            a.err        = !host_io_ ? err_.get() : nullptr;
             a.batch      = nb;
             a.sig_stride = n_;
             a.n1         = int(n1_);
@@ -1458,41 +1455,17 @@ void complex_engine<T>::execute(void* out, const void* in, long long batch, long
             // column pass: x -> scratch
             a.in       = inb;
             a.out      = scr;
-            a.tile       = tile_c_;
-            a.tile_shift = ilog2(tile_c_);
-            a.conj_in    = inverse;
+            a.conj_in  = inverse;
             a.conj_out = 0;
             a.tw       = pcols_.tw.get();
-            a.d        = pcols_.desc;
-            a.div_n    = make_fast_div(uint32_t(n1_));
-            a.pingpong   = pp_c_;
-            if (!pair_ || !run_pair(a, true))
-            {
-                block_cfg cc = pcols_.cfg_tile(tile_c_);
-                if (pp_c_)
-                    cc.smem *= 2; // ping-pong buffers
-                cc.grid = (n2_ + tile_c_ - 1) / tile_c_;
-                check(launch_ct_fs_cols_f32(a, cc, st), "launch four-step columns");
-            }
+            check(launch_ct_fsp_f32(a, true, st), "launch four-step columns");
             // row pass: scratch -> out
             a.in       = scr;
             a.out      = outb;
-            a.tile       = tile_r_;
-            a.tile_shift = ilog2(tile_r_);
-            a.conj_in    = 0;
+            a.conj_in  = 0;
             a.conj_out = inverse;
             a.tw       = prows_.tw.get();
-            a.d        = prows_.desc;
-            a.div_n    = make_fast_div(uint32_t(n2_));
-            a.pingpong   = pp_r_;
-            if (!pair_ || !run_pair(a, false))
-            {
-                block_cfg cr = prows_.cfg_tile(tile_r_);
-                if (pp_r_)
-                    cr.smem *= 2;
-                cr.grid = (n1_ + tile_r_ - 1) / tile_r_;
-                check(launch_ct_fs_rows_f32(a, cr, st), "launch four-step rows");
-            }
+            check(launch_ct_fsp_f32(a, false, st), "launch four-step rows");
         }
         return;
     }
@@ -1568,9 +1541,15 @@ std::string complex_engine<T>::describe() const
             s << "fourstep " << rp4_.describe();
             break;
         }
-        s << "fourstep" << (pair_ ? " (compile-time pair)" : "") << " n=" << n_ << " = " << n1_ << " x " << n2_
-          << " cols[" << pcols_.describe() << " tile=" << tile_c_ << "] rows[" << prows_.describe()
-          << " tile=" << tile_r_ << "]";
+        if (square_tw_.get())
+        {
+            s << "fourstep (compile-time pair) n=" << n_ << " = " << n1_ << " x " << n2_ << " radices=";
+            for (size_t i = 0; i < square_radices_.size(); i++)
+                s << (i ? "x" : "") << square_radices_[i];
+            break;
+        }
+        s << "fourstep (compile-time pair) n=" << n_ << " = " << n1_ << " x " << n2_ << " cols[" << pcols_.describe()
+          << "] rows[" << prows_.describe() << "]";
         if (rp4_.ready())
             s << " complex passes: " << rp4_.describe();
         break;

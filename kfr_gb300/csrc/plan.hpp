@@ -277,9 +277,9 @@ private:
     // four-step
     long long n1_ = 0, n2_ = 0;
     block_program<T> pcols_, prows_;
-    int tile_c_ = 1, tile_r_ = 1;
-    bool pp_c_ = false, pp_r_ = false; // ping-pong column / row passes
     bool pair_ = false;                 // both passes as fully compile-time pair kernels
+    std::vector<int> square_radices_;   // both passes of n1_ = n2_ points with compile-time indices
+    dbuf square_tw_;
     rp_fourstep<T> rp4_;                // both passes on the runtime-length block FFT
     dbuf twA_, twB_;
     int lbits_ = 0;

@@ -23,9 +23,19 @@ struct rp_lane
     int g, j, q, k; // signal of the tile, butterfly, j = q ns + k
 };
 
+// CT: the pass and shift are compile-time constants (plain divisions fold).
+template <bool CT = false>
 __device__ __forceinline__ rp_lane rp_map(const rp_pass& p, const int shift, const int J)
 {
     rp_lane l;
+    if constexpr (CT)
+    {
+        l.g = p.fast ? J & ((1 << shift) - 1) : int(uint32_t(J) / uint32_t(p.nbf));
+        l.j = p.fast ? J >> shift : int(uint32_t(J) % uint32_t(p.nbf));
+        l.q = int(uint32_t(l.j) / uint32_t(p.ns));
+        l.k = int(uint32_t(l.j) % uint32_t(p.ns));
+        return l;
+    }
     if (p.fast)
     {
         l.g = J & ((1 << shift) - 1);
@@ -83,13 +93,13 @@ struct rp_smem
 
 // First pass: inputs ld(g, i), outputs to shared memory; prep(g, j, step, v) sees a butterfly's inputs v[r]
 // (input j + r step) once all of them are loaded.
-template <typename T, int R, class LD, class PREP>
+template <typename T, int R, bool CT = false, class LD, class PREP>
 __device__ __forceinline__ void rp_first(const rp_pass& p, const int shift, const int total, const rp_smem<T> sm,
                                          const LD& ld, const PREP& prep)
 {
     for (int J = threadIdx.x; J < total; J += blockDim.x)
     {
-        const rp_lane l = rp_map(p, shift, J);
+        const rp_lane l = rp_map<CT>(p, shift, J);
         cpx<T> v[R];
 #pragma unroll
         for (int r = 0; r < R; r++)
@@ -105,13 +115,13 @@ __device__ __forceinline__ void rp_first(const rp_pass& p, const int shift, cons
 
 // Last pass: inputs from shared memory; fin(g, k, step, o) sees the butterfly's outputs o[r] (output k + r step)
 // before st(g, i, x) stores them.
-template <typename T, int R, class ST, class FIN>
+template <typename T, int R, bool CT = false, class ST, class FIN>
 __device__ __forceinline__ void rp_last(const rp_pass& p, const int shift, const int total, const rp_smem<T> sm,
                                         const cpx<T>* __restrict__ tw, const ST& st, const FIN& fin)
 {
     for (int J = threadIdx.x; J < total; J += blockDim.x)
     {
-        const rp_lane l   = rp_map(p, shift, J);
+        const rp_lane l   = rp_map<CT>(p, shift, J);
         const cpx<T>* s = sm.src(p, l);
         cpx<T> v[R];
 #pragma unroll
@@ -131,7 +141,7 @@ __device__ __forceinline__ void rp_last(const rp_pass& p, const int shift, const
 }
 
 // In-place pass: the thread's butterflies are held in registers across a barrier (rp_threads_needed).
-template <typename T, int R, int H>
+template <typename T, int R, int H, bool CT = false>
 __device__ __forceinline__ void rp_mid(const rp_pass& p, const int shift, const int total, const rp_smem<T> sm,
                                        const cpx<T>* __restrict__ tw)
 {
@@ -143,7 +153,7 @@ __device__ __forceinline__ void rp_mid(const rp_pass& p, const int shift, const 
         const int J = threadIdx.x + b * blockDim.x;
         if (J < total)
         {
-            const rp_lane l   = rp_map(p, shift, J);
+            const rp_lane l   = rp_map<CT>(p, shift, J);
             const cpx<T>* s = sm.src(p, l);
 #pragma unroll
             for (int r = 0; r < R; r++)
@@ -167,7 +177,7 @@ __device__ __forceinline__ void rp_mid(const rp_pass& p, const int shift, const 
         const int J = threadIdx.x + b * blockDim.x;
         if (J < total)
         {
-            const rp_lane l = rp_map(p, shift, J);
+            const rp_lane l = rp_map<CT>(p, shift, J);
             cpx<T>* d     = sm.dst(p, l);
 #pragma unroll
             for (int r = 0; r < R; r++)
@@ -319,6 +329,88 @@ __device__ __forceinline__ void rp_run(const D& d, cpx<T>* buf, const int nsig, 
 #undef KFR_GPU_RP_CASE
     default: break;
     }
+}
+
+// Compile-time descriptor of the radices Rs over a tile of S signals of RP_COLS or RP_ROWS (as rp_build, with `pad`
+// spare slots after each group of the first pass and none after the others, whose stores are contiguous).
+template <rp_layout L, int S, int PAD, int... Rs>
+struct rp_ct
+{
+    static constexpr int npass = sizeof...(Rs);
+    static constexpr rp_desc make()
+    {
+        constexpr int rad[] = { Rs... };
+        rp_desc d{};
+        d.npass = npass;
+        d.n     = (Rs * ...);
+        d.hold  = kRpHold;
+        while ((1 << d.shift) < S)
+            d.shift++;
+        int ns = 1, off = 0;
+        for (int i = 0; i < npass; i++)
+        {
+            rp_pass& p = d.pass[i];
+            p.radix    = rad[i];
+            p.ns       = ns;
+            p.nbf      = d.n / rad[i];
+            p.fast     = L == RP_COLS || i > 0;
+            p.tw_off   = off;
+            if (ns > 1)
+                off += ns * (rad[i] - 1);
+            ns *= rad[i];
+        }
+        for (int i = 0; i + 1 < npass; i++)
+        {
+            rp_pass &a = d.pass[i], &b = d.pass[i + 1];
+            const int nn = a.ns * a.radix, pad = i == 0 ? PAD : 0;
+            a.st_e  = S;
+            a.st_q  = nn * S + pad;
+            a.st_g  = 1;
+            a.st_r  = a.ns * S;
+            b.ld_e  = S;
+            b.ld_q  = pad;
+            b.ld_g  = 1;
+            b.ld_r  = b.nbf * S + b.nbf / nn * pad;
+            d.elems = d.elems > d.n / nn * a.st_q ? d.elems : d.n / nn * a.st_q;
+        }
+        return d;
+    }
+    static constexpr rp_desc d = make();
+    static constexpr int threads()
+    {
+        int t = 128;
+        for (int i = 1; i + 1 < npass; i++)
+        {
+            const int h = rp_held(d.pass[i].radix, kRpHold), need = (S * d.pass[i].nbf + h - 1) / h;
+            t = t > need ? t : need;
+        }
+        return (t + 31) / 32 * 32;
+    }
+};
+
+// rp_run with every index a constant.
+template <typename T, class C, int I = 1, class LD, class ST, class FIN = rp_no_hook>
+__device__ __forceinline__ void rp_run_ct(cpx<T>* buf, const cpx<T>* __restrict__ tw, const LD& ld, const ST& st,
+                                          const FIN& fin = FIN())
+{
+    constexpr rp_desc D = C::d;
+    constexpr int S     = 1 << D.shift;
+    const rp_smem<T> sm{ buf };
+    if constexpr (I == 1)
+    {
+        constexpr rp_pass p = D.pass[0];
+        rp_first<T, p.radix, true>(p, D.shift, S * p.nbf, sm, ld, rp_no_hook{});
+        __syncthreads();
+    }
+    constexpr rp_pass p = D.pass[I];
+    if constexpr (I + 1 < D.npass)
+    {
+        rp_mid<T, p.radix, kRpHold, true>(p, D.shift, S * p.nbf, sm, tw);
+        __syncthreads();
+        rp_run_ct<T, C, I + 1>(buf, tw, ld, st, fin);
+    }
+    else
+        rp_last<T, p.radix, true>(p, D.shift, S * p.nbf, sm, tw, st, fin);
 }
 
 // The transform from ld(g, i) to shared memory (output k of signal g in the natural layout of d's last pass).  Ends

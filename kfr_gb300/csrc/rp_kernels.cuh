@@ -201,6 +201,57 @@ __global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T), H), 1)
 
 // ---------------------------------------------------------------------------------------------------
 
+// The four-step passes of k_rp_cols / k_rp_rows for power-of-two lengths known at compile time (C: rp_ct of the pass,
+// P: the other length).
+template <typename T, class C, int P>
+__global__ void __launch_bounds__(C::threads(), 1024 / C::threads()) k_ct_cols(const __grid_constant__ rp_strided_args a)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    constexpr int S = 1 << C::d.shift, tiles = P / S;
+    const long long b = blockIdx.x / tiles;
+    const int c0      = int(blockIdx.x % tiles) * S;
+    const cpx<T>* in  = reinterpret_cast<const cpx<T>*>(a.in) + b * a.in_stride + c0;
+    cpx<T>* out       = reinterpret_cast<cpx<T>*>(a.out) + b * a.out_stride + c0;
+    const cpx<T>* twA = reinterpret_cast<const cpx<T>*>(a.twA);
+    const cpx<T>* twB = reinterpret_cast<const cpx<T>*>(a.twB);
+    const bool cin = a.conj_in != 0;
+    rp_run_ct<T, C>(
+        reinterpret_cast<cpx<T>*>(smem_raw), reinterpret_cast<const cpx<T>*>(a.tw),
+        [&](int g, int i) { return conj_if(in[i * P + g], cin); },
+        [&](int g, int i, cpx<T> v) { out[i * P + g] = v; },
+        [&](int g, int k, int step, auto& o)
+        {
+            // W^{col k} times powers of the butterfly's step W^{col step}
+            constexpr int R = int(sizeof(o) / sizeof(o[0]));
+            const int col   = c0 + g, mask = (1 << a.lbits) - 1;
+            const auto root = [&](int m) { return ldg(twA + (m >> a.lbits)) * ldg(twB + (m & mask)); };
+            if constexpr (R >= 8)
+                twiddle_powers4<T, R>(o, root(col * step), root(4 * col * step));
+            else
+                twiddle_powers<T, R>(o, root(col * step));
+            const cpx<T> w = root(col * k);
+#pragma unroll
+            for (int r = 0; r < R; r++)
+                o[r] = o[r] * w;
+        });
+}
+
+template <typename T, class C, int P>
+__global__ void __launch_bounds__(C::threads(), 1024 / C::threads()) k_ct_rows(const __grid_constant__ rp_strided_args a)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    constexpr int S = 1 << C::d.shift, tiles = P / S;
+    const long long b = blockIdx.x / tiles;
+    const int r0      = int(blockIdx.x % tiles) * S;
+    const cpx<T>* in  = reinterpret_cast<const cpx<T>*>(a.in) + b * a.in_stride + (long long)r0 * C::d.n;
+    cpx<T>* out       = reinterpret_cast<cpx<T>*>(a.out) + b * a.out_stride + r0;
+    const bool cout = a.conj_out != 0;
+    rp_run_ct<T, C>(
+        reinterpret_cast<cpx<T>*>(smem_raw), reinterpret_cast<const cpx<T>*>(a.tw),
+        [&](int g, int i) { return in[g * C::d.n + i]; },
+        [&](int g, int i, cpx<T> v) { out[i * P + g] = conj_if(v, cout); });
+}
+
 template <typename A>
 static cudaError_t rp_go(void (*kernel)(const A), const A& a, long long grid, int threads, int smem, cudaStream_t st)
 {
