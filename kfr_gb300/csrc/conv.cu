@@ -1,5 +1,6 @@
 // FFT convolution filter kernels and host class (see conv.hpp).
 #include "conv.hpp"
+#include "conv16.cuh"
 #include "convolve.hpp"
 #include "kernels.cuh"
 #include "rp_fft.cuh"
@@ -26,42 +27,10 @@ __device__ __forceinline__ cpx<T> rmerge(cpx<T> yk, cpx<T> ykk, cpx<T> w)
     return (yk + ynk) + mul_pi(conj(w) * (yk - ynk));
 }
 
-// Block FFT of one signal per CTA between global memory and one shared buffer, for the convolution kernels:
+// Block FFT of one signal per CTA between global memory and one shared buffer, for convolution blocks of any length
+// (the runtime-length block FFT, in place):
 //   to_smem(ld):   c-point DFT of ld(i), i < c, left at buf[pos(k)]; ends with a barrier;
 //   from_smem(st): c-point DFT of buf[pos(i)], output k to st(k, x).
-// Compile-time lengths keep the signal in registers between the passes, read ld in the first pass and write st
-// in the last.
-template <class F>
-struct conv_ct
-{
-    using real                       = float;
-    static constexpr int max_threads = F::ts;
-    cpx<float>* buf;
-    const cpx<float>* tw;
-    const F fft;
-    __device__ __forceinline__ conv_ct(cpx<float>* b, const void* t, const conv_fft& d)
-        : buf(b), tw(reinterpret_cast<const cpx<float>*>(t)), fft()
-    {
-        (void)d;
-    }
-    __device__ __forceinline__ int n() const { return F::n; }
-    static __device__ __forceinline__ int pos(int i) { return F::pi(i); }
-    template <class LD>
-    __device__ __forceinline__ void to_smem(const LD& ld) const
-    {
-        cpx<float>* b = buf;
-        fft.run_io(ld, []() { __syncthreads(); }, [b](int k, cpx<float> x) { b[F::pi(k)] = x; }, []() {}, b, tw,
-                   int(threadIdx.x));
-        __syncthreads();
-    }
-    template <class ST>
-    __device__ __forceinline__ void from_smem(const ST& st) const
-    {
-        cpx<float>* b = buf;
-        fft.run_io([b](int i) { return b[F::pi(i)]; }, []() { __syncthreads(); }, st, []() {}, b, tw, int(threadIdx.x));
-    }
-};
-// Every other length: the runtime-length block FFT, in place.
 template <typename T>
 struct conv_rp
 {
@@ -121,10 +90,9 @@ __device__ __forceinline__ bool pair_aligned(const void* p)
 }
 
 // One overlap-save block per CTA: blockIdx.x = output block, blockIdx.y = channel.  The overlap a.m1 is even (a
-// zero tap is added to an even tap count), so blocks start at even samples and move as pairs.  Bound by
-// instruction issue (two c-point FFTs, the split, product and merge per block).
+// zero tap is added to an even tap count), so blocks start at even samples and move as pairs.
 template <class P>
-__global__ void __launch_bounds__(P::max_threads, P::max_threads > 256 ? 1 : 1024 / P::max_threads)
+__global__ void __launch_bounds__(P::max_threads, 1)
     k_conv_os(const __grid_constant__ conv_args a)
 {
     using T = typename P::real;
@@ -203,10 +171,10 @@ __global__ void __launch_bounds__(P::max_threads, P::max_threads > 256 ? 1 : 102
 // its own sum in shared memory (every bin owned by one thread); k_fir_reduce adds them in a fixed order and
 // k_fir_taps transforms the sum back.  Bound by instruction issue (three c-point FFTs per block).  64 channels
 // of 2^20 samples, 1023 taps, forward and both gradients: 6397 -> 869 us against reversed copies through the
-// filter and real DFTs of 2^21 points per channel (the filter alone 375 us of either).
+// filter and real DFTs of 2^21 points per channel; 642 us with the paired blocks below.
 // ---------------------------------------------------------------------------------------------------
 template <class P>
-__global__ void __launch_bounds__(P::max_threads, P::max_threads > 256 ? 1 : 512 / P::max_threads)
+__global__ void __launch_bounds__(P::max_threads, 1)
     k_fir_bwd(const __grid_constant__ fir_bwd_args a)
 {
     using T = typename P::real;
@@ -352,7 +320,7 @@ __global__ void __launch_bounds__(P::max_threads, 1) k_fir_taps(const __grid_con
 
 // Spectrum of the taps, H[k] = sum_m h[m] W_F^{m k} / F for k <= c, in double precision on the device, as sums
 // over m = m1 Q + m0: first the inner sums S[m0][k mod F/Q] = sum_{m1} h[m1 Q + m0] W_F^{Q m1 k}, then
-// H[k] = sum_{m0} W_F^{m0 k} S[m0][k mod F/Q].  w: W_F^j, j < F.  (FP64 FFTs of one CTA would take tens of
+// H[k] = sum_{m0} W_F^{m0 k} S[m0][k mod F/Q].  w: W_F^j, j < F; placed: stored for k_fir16_bwd.  (FP64 FFTs of one CTA would take tens of
 // microseconds on this part; these sums spread over all SMs.)
 template <typename T>
 __global__ void __launch_bounds__(128) k_fir_spec_inner(double2* S, const T* __restrict__ h, const double2* __restrict__ w,
@@ -378,7 +346,8 @@ __global__ void __launch_bounds__(128) k_fir_spec_inner(double2* S, const T* __r
 }
 template <typename T>
 __global__ void __launch_bounds__(64) k_fir_spec_outer(cpx<T>* H, const double2* __restrict__ S,
-                                                      const double2* __restrict__ w, int taps, int F, int Q)
+                                                      const double2* __restrict__ w, int taps, int F, int Q,
+                                                      bool placed)
 {
     const int P = F / Q, k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k > F / 2)
@@ -395,7 +364,199 @@ __global__ void __launch_bounds__(64) k_fir_spec_outer(cpx<T>* H, const double2*
         if (at >= F)
             at -= F;
     }
-    H[k] = mk<T>(T(re / F), T(im / F));
+    const cpx<T> h = mk<T>(T(re / F), T(im / F));
+    if (!placed)
+        H[k] = h;
+    else
+    {
+        // all F bins in fft16_place order
+        H[fft16_place(k)]           = h;
+        H[fft16_place((F - k) % F)] = conj(h);
+    }
+}
+
+// ---------------------------------------------------------------------------------------------------
+// Single precision, up to kConv16Overlap samples of overlap: two output blocks of a channel as the real and the
+// imaginary part of one 4096-point transform (conv16.cuh).  The taps are real, so the product with their spectrum
+// filters both, with no split or merge, and it happens in registers between the last forward and the first inverse
+// pass.  Bound by instruction issue (about 115 instructions per complex value) and the latency of the first loads.  64
+// channels of 2^20 samples, 1023 taps: 277 -> 241 us against one block of 8192 samples through a 4096-point transform
+// with split and merge; the gradients 566 -> 367 us.
+// ---------------------------------------------------------------------------------------------------
+__device__ __forceinline__ float conv_sample(const float* in, const float* hist, long long i, long long n, long long nhist)
+{
+    if (i >= 0)
+        return i < n ? in[i] : 0.0f;
+    return i + nhist >= 0 ? hist[i + nhist] : 0.0f; // the latest sample before the call at hist[nhist - 1]
+}
+
+__global__ void __launch_bounds__(fft16::threads, 3) k_conv16(const __grid_constant__ conv_args a)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const fft16 f(smem_raw, a.tw);
+    const float* in   = reinterpret_cast<const float*>(a.in) + (long long)blockIdx.y * a.n;
+    const float* hist = reinterpret_cast<const float*>(a.hist) + (long long)blockIdx.y * a.nhist;
+    float* out        = reinterpret_cast<float*>(a.out) + (long long)blockIdx.y * a.n;
+    const int m1 = int(a.m1), bo = int(a.bo);
+    const long long first = 2LL * blockIdx.x * bo; // first output of the first block
+    const long long start = first - m1;
+    cpx<float> v[16];
+    if (start >= 0 && start + bo + fft16::N <= a.n)
+    {
+        const float* x = in + start + f.t;
+#pragma unroll
+        for (int r = 0; r < 16; r++)
+            v[r] = mk<float>(x[256 * r], x[bo + 256 * r]);
+    }
+    else
+    {
+#pragma unroll
+        for (int r = 0; r < 16; r++)
+        {
+            const long long i = start + f.t + 256 * r;
+            v[r] = mk<float>(conv_sample(in, hist, i, a.n, a.nhist), conv_sample(in, hist, i + bo, a.n, a.nhist));
+        }
+    }
+    f.forward_a(v);
+    __syncthreads();
+    f.forward_b();
+    __syncthreads();
+    f.forward_c(v);
+    const cpx<float>* H = reinterpret_cast<const cpx<float>*>(a.hspec) + f.t;
+#pragma unroll
+    for (int u = 0; u < 16; u++)
+        v[u] = conj(v[u] * ldg(H + 256 * u));
+    f.inverse_c(v);
+    __syncthreads();
+    f.inverse_b();
+    __syncthreads();
+    f.inverse_a(v);
+    // outputs p >= m1 of the block are samples first + p - m1; the others wrapped around
+    const long long left = a.n - first;
+#pragma unroll
+    for (int r = 0; r < 16; r++)
+    {
+        const int p = f.t + 256 * r - m1;
+        if (p < 0)
+            continue;
+        if (p < left)
+            out[first + p] = v[r].x;
+        if (p + bo < left)
+            out[first + bo + p] = -v[r].y;
+    }
+}
+
+// Gradients (see k_fir_bwd) of two blocks of a channel at a time.  With z_g = g_A + i g_B and z_x = x_A + i x_B the sum
+// of Z_g conj(Z_x) over all pairs transforms back to the taps gradient in its real part.  x goes first and its 16 bins
+// per thread wait in registers while g takes the buffer; the next pair's samples of x are loaded during the inverse.
+__global__ void __launch_bounds__(fft16::threads, 2) k_fir16_bwd(const __grid_constant__ fir_bwd_args a)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const fft16 f(smem_raw, a.tw);
+    cpx<float>* acc     = reinterpret_cast<cpx<float>*>(smem_raw) + fft16::elems + f.t; // bin u at 256 u
+    const cpx<float>* H = reinterpret_cast<const cpx<float>*>(a.hspec) + f.t;
+    const bool want_x = a.grad_x != nullptr, want_h = a.partial != nullptr;
+    const int bo = int(a.bo);
+    const long long pairs = (a.blocks + 1) / 2, total = pairs * a.channels;
+    if (want_h)
+#pragma unroll
+        for (int u = 0; u < 16; u++)
+            acc[256 * u] = mk<float>(0, 0);
+    const auto load = [&](cpx<float>(&v)[16], const void* base, long long b, int count)
+    {
+        // samples [t0, t0 + count) and [t0 + bo, t0 + bo + count) of the pair b's channel, zero beyond them
+        const long long ch = b / pairs, t0 = 2 * (b - ch * pairs) * bo;
+        const float* x  = reinterpret_cast<const float*>(base) + ch * a.n + t0 + f.t;
+        const long long left = a.n - t0 - f.t;
+#pragma unroll
+        for (int r = 0; r < 16; r++)
+        {
+            const int i   = 256 * r;
+            const bool in = i + f.t < count;
+            v[r]          = mk<float>(in && i < left ? x[i] : 0.0f, in && i + bo < left ? x[i + bo] : 0.0f);
+        }
+    };
+    cpx<float> px[16];
+    if (want_h && blockIdx.x < total)
+        load(px, a.x, blockIdx.x, bo);
+    for (long long b = blockIdx.x; b < total; b += gridDim.x)
+    {
+        cpx<float> v[16];
+        load(v, a.grad_y, b, fft16::N);
+        if (want_h)
+        {
+            f.forward_a(px);
+            __syncthreads();
+            f.forward_b();
+            __syncthreads();
+            f.forward_c(px);
+            __syncthreads();
+        }
+        f.forward_a(v);
+        __syncthreads();
+        f.forward_b();
+        __syncthreads();
+        f.forward_c(v);
+        if (want_h)
+#pragma unroll
+            for (int u = 0; u < 16; u++)
+                acc[256 * u] = acc[256 * u] + v[u] * conj(px[u]);
+        if (want_h && b + gridDim.x < total)
+            load(px, a.x, b + gridDim.x, bo);
+        if (want_x)
+        {
+#pragma unroll
+            for (int u = 0; u < 16; u++)
+                v[u] = conj(v[u] * conj(ldg(H + 256 * u)));
+            f.inverse_c(v);
+            __syncthreads();
+            f.inverse_b();
+            __syncthreads();
+            f.inverse_a(v);
+            const long long ch = b / pairs, t0 = 2 * (b - ch * pairs) * bo, left = a.n - t0;
+            float* gx = reinterpret_cast<float*>(a.grad_x) + ch * a.n + t0;
+#pragma unroll
+            for (int r = 0; r < 16; r++)
+            {
+                const int p = f.t + 256 * r;
+                if (p >= bo)
+                    continue;
+                if (p < left)
+                    gx[p] = v[r].x;
+                if (p + bo < left)
+                    gx[p + bo] = -v[r].y;
+            }
+        }
+        __syncthreads();
+    }
+    if (want_h)
+    {
+        cpx<float>* p = reinterpret_cast<cpx<float>*>(a.partial) + (long long)blockIdx.x * fft16::N + f.t;
+#pragma unroll
+        for (int u = 0; u < 16; u++)
+            p[256 * u] = acc[256 * u];
+    }
+}
+
+// grad_h[m] = Re IDFT(spectrum)[m] / F, m < taps, the spectrum in fft16_place order (one CTA).
+__global__ void __launch_bounds__(fft16::threads, 1) k_fir16_taps(const __grid_constant__ fir_bwd_args a, float* grad_h,
+                                                                 const cpx<float>* spectrum, const int taps)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const fft16 f(smem_raw, a.tw);
+    cpx<float> v[16];
+#pragma unroll
+    for (int u = 0; u < 16; u++)
+        v[u] = conj(spectrum[f.t + 256 * u]);
+    f.inverse_c(v);
+    __syncthreads();
+    f.inverse_b();
+    __syncthreads();
+    f.inverse_a(v);
+#pragma unroll
+    for (int r = 0; r < 16; r++)
+        if (f.t + 256 * r < taps)
+            grad_h[f.t + 256 * r] = v[r].x * (1.0f / fft16::N);
 }
 
 // new_hist[i] = i + n < m1 ? old_hist[i + n] : in[i + n - m1]
@@ -410,29 +571,6 @@ __global__ void k_hist_update(const T* __restrict__ hold, T* __restrict__ hnew, 
         const long long s  = e + n;
         hnew[i]            = s < m1 ? hold[ch * m1 + s] : in[ch * n + (s - m1)];
     }
-}
-
-// Runs go(policy type) for the transform f: a compile-time length or the runtime-length block FFT.
-template <typename P>
-struct type_of
-{
-    using type = P;
-};
-template <typename T, class G>
-static cudaError_t with_conv_fft(const conv_fft& f, const G& go_fn)
-{
-    if constexpr (std::is_same<T, float>::value)
-    {
-        switch (f.ct)
-        {
-#define KFR_GPU_CONV_CASE(N, TS, ...)                                                                      \
-    case N: return go_fn(type_of<conv_ct<ct_fft<float, N, TS, __VA_ARGS__>>>());
-            KFR_CT_CONV_F32(KFR_GPU_CONV_CASE)
-#undef KFR_GPU_CONV_CASE
-        default: break;
-        }
-    }
-    return go_fn(type_of<conv_rp<T>>());
 }
 
 template <typename K, typename... Args>
@@ -451,13 +589,12 @@ static cudaError_t conv_go(K kernel, dim3 grid, int threads, size_t smem, cudaSt
 template <typename T>
 cudaError_t launch_conv_os(const conv_args& a, long long nblocks, cudaStream_t st)
 {
-    return with_conv_fft<T>(a.fft,
-                            [&](auto p)
-                            {
-                                using P = typename decltype(p)::type;
-                                return conv_go(k_conv_os<P>, dim3(unsigned(nblocks), unsigned(a.channels)), a.fft.threads,
-                                               size_t(a.fft.elems) * 2 * sizeof(T), st, a);
-                            });
+    if constexpr (std::is_same<T, float>::value)
+        if (a.fft.paired)
+            return conv_go(k_conv16, dim3(unsigned((nblocks + 1) / 2), unsigned(a.channels)), fft16::threads,
+                           fft16::elems * sizeof(cpx<float>), st, a);
+    return conv_go(k_conv_os<conv_rp<T>>, dim3(unsigned(nblocks), unsigned(a.channels)), a.fft.threads,
+                   size_t(a.fft.elems) * 2 * sizeof(T), st, a);
 }
 
 template <typename T>
@@ -493,24 +630,20 @@ static size_t conv_fft_max()
 }
 
 template <typename T>
-fir_tables<T>::fir_tables(size_t f)
+fir_tables<T>::fir_tables(size_t f, bool paired)
 {
-    const int c = int(f / 2);
-    int ts      = 0;
-    std::vector<int> rad;
-    if (ct_lookup<T>(CT_CONV, c, ts, rad))
+    if (paired)
     {
-        fft.ct      = c;
-        fft.threads = ts;
-        fft.elems   = (ct_group_stride_f32(c, ts) + 1) / 2 * 2;
+        fft.paired   = true;
+        const auto t = pass_twiddles<T>({ 16, 16, 16 });
+        tw.upload(t.data(), t.size() * sizeof(t[0]));
+        return;
     }
-    else
-    {
-        rad         = rp_radices(c);
-        fft.rp      = rp_build(rad, RP_SIGNALS, 1, int(2 * sizeof(T)), true);
-        fft.elems   = (rp_smem_elems(fft.rp, RP_SIGNALS, 1, true) + 1) / 2 * 2;
-        fft.threads = (std::max(rp_threads_needed(fft.rp, 1, true), std::min(c, 64)) + 31) / 32 * 32;
-    }
+    const int c    = int(f / 2);
+    const auto rad = rp_radices(c);
+    fft.rp         = rp_build(rad, RP_SIGNALS, 1, int(2 * sizeof(T)), true);
+    fft.elems      = (fft.rp.elems + 1) / 2 * 2;
+    fft.threads    = (std::max(rp_threads_needed(fft.rp, 1, true), std::min(c, 64)) + 31) / 32 * 32;
     const auto t = pass_twiddles<T>(rad);
     tw.upload(t.data(), t.size() * sizeof(t[0]));
     std::vector<std::complex<T>> rt(c + 1);
@@ -534,11 +667,21 @@ void fir_tables<T>::roots64(size_t f)
 template struct fir_tables<float>;
 template struct fir_tables<double>;
 
+// Whether blocks with an overlap of m1 samples run in pairs through 4096-point transforms: up to half of a block re-reads
+// the overlap, where the self-sorting transforms of 16384 samples (next_pow2(8 m1)) begin to need fewer instructions.
+template <typename T>
+static bool conv_paired(size_t m1)
+{
+    return sizeof(T) == 4 && m1 <= fft16::N / 2;
+}
+
 // FFT length for an overlap of m1 samples: at least 8 times it (at most 1/8 of each block re-reads the overlap;
 // measured 0.390 -> 0.374 ms against 4x for 64 channels of 2^20 samples and 1023 taps) and twice the block.
 template <typename T>
 static size_t conv_fft_size(size_t m1, size_t block)
 {
+    if (conv_paired<T>(m1))
+        return fft16::N;
     return std::min(std::max({ next_pow2(8 * m1), 2 * next_pow2(block ? block : 1024), size_t(64) }), conv_fft_max<T>());
 }
 
@@ -565,7 +708,7 @@ conv_filter<T>::conv_filter(const T* taps, size_t ntaps, size_t block_size, int 
     const size_t hb = std::max<size_t>(1, m1 * size_t(channels)) * sizeof(T);
     hist_[0].alloc(hb);
     hist_[1].alloc(hb);
-    if (m1 >= f / 2)
+    if (m1 >= f / 2 && !conv_paired<T>(m1))
     {
         // long mode: the taps stay on the device for whole-call convolutions
         long_ = true;
@@ -576,16 +719,18 @@ conv_filter<T>::conv_filter(const T* taps, size_t ntaps, size_t block_size, int 
     }
     f_  = f;
     c_  = f / 2;
-    bo_ = f - (m1 + 1) / 2 * 2; // blocks start at even samples
-    tables_.reset(new fir_tables<T>(f));
+    const bool paired = conv_paired<T>(m1);
+    bo_ = paired ? f - m1 : f - (m1 + 1) / 2 * 2; // unpaired blocks start at even samples
+    tables_.reset(new fir_tables<T>(f, paired));
     // taps spectrum FFT_F(h padded) / F, bins 0..c (set_data, src/dft/convolution-impl.cpp:53-71)
     std::vector<std::complex<double>> a(f, { 0.0, 0.0 });
     for (size_t i = 0; i < ntaps; i++)
         a[i] = double(h[i]);
     host_fft_pow2(a);
-    std::vector<std::complex<T>> hs(c_ + 1);
-    for (size_t k = 0; k <= c_; k++)
-        hs[k] = std::complex<T>(T(a[k].real() / double(f)), T(a[k].imag() / double(f)));
+    // (paired blocks: every bin, in fft16_place order)
+    std::vector<std::complex<T>> hs(paired ? f : c_ + 1);
+    for (size_t k = 0; k < hs.size(); k++)
+        hs[paired ? fft16_place(int(k)) : int(k)] = std::complex<T>(T(a[k].real() / double(f)), T(a[k].imag() / double(f)));
     hspec_.upload(hs.data(), hs.size() * sizeof(std::complex<T>));
     reset();
 }
@@ -647,7 +792,7 @@ void conv_filter<T>::process(T* out, const T* in, size_t n, cudaStream_t st)
     a.hist     = hist_[cur_].get();
     a.n        = (long long)n;
     a.nhist    = m1;
-    a.m1       = (m1 + 1) / 2 * 2;
+    a.m1       = tables_->fft.paired ? m1 : (m1 + 1) / 2 * 2;
     a.bo       = (long long)bo_;
     a.channels = channels_;
     a.hspec    = hspec_.get();
@@ -673,47 +818,44 @@ bool fir_backward_blocks(const T* taps, long long ntaps, long long channels, lon
                          T* grad_x, T* grad_h, cudaStream_t st)
 {
     const size_t m1 = size_t(ntaps - 1);
+    const bool paired = conv_paired<T>(m1);
     // the gradient kernel holds two spectra and a sum: half the one-CTA length
     const size_t f = std::min(conv_fft_size<T>(m1, 1024), conv_fft_max<T>() / 2);
-    if (m1 >= f / 2)
+    if (m1 >= f / 2 && !paired)
         return false;
-    const auto tab = plan_cache::instance().fir<T>((long long)f);
+    const auto tab = plan_cache::instance().fir<T>((long long)f, paired);
     const int c    = int(f / 2);
+    const int bins = paired ? int(f) : c + 1; // bins of a spectrum
     fir_bwd_args a;
     a.x        = x;
     a.grad_y   = grad_y;
     a.grad_x   = grad_x;
     a.n        = n;
-    a.bo       = (long long)(f - (m1 + 1) / 2 * 2);
+    a.bo       = (long long)(f - (paired ? m1 : (m1 + 1) / 2 * 2));
     a.blocks   = (n + a.bo - 1) / a.bo;
     a.channels = channels;
     a.rtw      = tab->rtw.get();
     a.tw       = tab->tw.get();
     a.fft      = tab->fft;
     a.elems    = tab->fft.elems;
-    const size_t smem     = (2 * size_t(a.elems) + c + 1) * 2 * sizeof(T);
-    const long long total = a.blocks * channels;
+    const int threads     = paired ? fft16::threads : a.fft.threads;
+    const size_t smem     = paired ? (size_t(fft16::elems) + fft16::N) * 2 * sizeof(T) : (2 * size_t(a.elems) + c + 1) * 2 * sizeof(T);
+    const long long total = (paired ? (a.blocks + 1) / 2 : a.blocks) * channels;
     // the taps' inner sums of about the square root of F rows
     int Q = 1;
     while (Q * Q < int(f))
         Q <<= 1;
-    int grid            = 0;
-    const cudaError_t e = with_conv_fft<T>(a.fft,
-                                           [&](auto p)
-                                           {
-                                               using P    = typename decltype(p)::type;
-                                               int per_sm = 0;
-                                               const cudaError_t r =
-                                                   prepare_launch(reinterpret_cast<const void*>(k_fir_bwd<P>),
-                                                                  a.fft.threads, int(smem), &per_sm);
-                                               grid = int(std::min<long long>(total, (long long)per_sm * device_sm_count()));
-                                               return r;
-                                           });
-    check(e, "prepare FIR backward");
+    const void* kernel = reinterpret_cast<const void*>(k_fir_bwd<conv_rp<T>>);
+    if constexpr (std::is_same<T, float>::value)
+        if (paired)
+            kernel = reinterpret_cast<const void*>(k_fir16_bwd);
+    int per_sm = 0;
+    check(prepare_launch(kernel, threads, int(smem), &per_sm), "prepare FIR backward");
+    const int grid = int(std::min<long long>(total, (long long)per_sm * device_sm_count()));
     const size_t cpx_b  = 2 * sizeof(T);
-    const size_t hs_b   = (size_t(c + 1) * cpx_b + 255) / 256 * 256;
+    const size_t hs_b   = (size_t(bins) * cpx_b + 255) / 256 * 256;
     const size_t in_b   = f * sizeof(double2);
-    const size_t part_b = grad_h ? size_t(grid) * (c + 1) * cpx_b : 0;
+    const size_t part_b = grad_h ? size_t(grid) * bins * cpx_b : 0;
     // the blocks read gradients that other blocks overwrite when grad_x shares memory with an input
     const auto overlaps = [&](const void* p)
     {
@@ -738,24 +880,40 @@ bool fir_backward_blocks(const T* taps, long long ntaps, long long channels, lon
                                                                      int(ntaps), int(f), Q);
         k_fir_spec_outer<T><<<unsigned((c + 64) / 64), 64, 0, st>>>(reinterpret_cast<cpx<T>*>(H),
                                                                     reinterpret_cast<const double2*>(inner), w, int(ntaps),
-                                                                    int(f), Q);
+                                                                    int(f), Q, paired);
         check(cudaGetLastError(), "taps spectrum");
     }
-    check(with_conv_fft<T>(a.fft,
-                           [&](auto p)
-                           {
-                               using P = typename decltype(p)::type;
-                               cudaError_t r = conv_go(k_fir_bwd<P>, dim3(unsigned(grid)), a.fft.threads, smem, st, a);
-                               if (r == cudaSuccess && grad_h)
-                               {
-                                   k_fir_reduce<T><<<unsigned((c + 32) / 32), 256, 0, st>>>(
-                                       reinterpret_cast<cpx<T>*>(sum), reinterpret_cast<const cpx<T>*>(parts), grid, c + 1);
-                                   r = conv_go(k_fir_taps<P>, dim3(1), a.fft.threads, size_t(a.elems) * cpx_b, st, a,
-                                               static_cast<void*>(grad_h), static_cast<const void*>(sum), int(ntaps));
-                               }
-                               return r;
-                           }),
-          "launch FIR backward");
+    const auto reduce = [&]()
+    {
+        k_fir_reduce<T><<<unsigned((bins + 31) / 32), 256, 0, st>>>(reinterpret_cast<cpx<T>*>(sum),
+                                                                    reinterpret_cast<const cpx<T>*>(parts), grid, bins);
+        check(cudaGetLastError(), "launch FIR backward (sum)");
+    };
+    if (paired)
+    {
+        if constexpr (std::is_same<T, float>::value)
+        {
+            check(conv_go(k_fir16_bwd, dim3(unsigned(grid)), threads, smem, st, a), "launch FIR backward");
+            if (grad_h)
+            {
+                reduce();
+                check(conv_go(k_fir16_taps, dim3(1), threads, size_t(fft16::elems) * cpx_b, st, a, grad_h,
+                              reinterpret_cast<const cpx<float>*>(sum), int(ntaps)),
+                      "launch FIR backward (taps)");
+            }
+        }
+    }
+    else
+    {
+        check(conv_go(k_fir_bwd<conv_rp<T>>, dim3(unsigned(grid)), threads, smem, st, a), "launch FIR backward");
+        if (grad_h)
+        {
+            reduce();
+            check(conv_go(k_fir_taps<conv_rp<T>>, dim3(1), threads, size_t(a.elems) * cpx_b, st, a,
+                          static_cast<void*>(grad_h), static_cast<const void*>(sum), int(ntaps)),
+                  "launch FIR backward (taps)");
+        }
+    }
     if (staged)
         check(cudaMemcpyAsync(grad_x, a.grad_x, size_t(channels * n) * sizeof(T), cudaMemcpyDeviceToDevice, st),
               "copy signal gradient");

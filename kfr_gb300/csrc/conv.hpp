@@ -16,10 +16,11 @@
 namespace kfr_gpu
 {
 
-// The c-point complex transform of a convolution block.
+// The transform of a convolution block: c complex points for F = 2c samples, or pairs of blocks of F = 4096 samples
+// through one complex transform (conv16.cuh; spectra then hold all F bins in fft16_place order).
 struct conv_fft
 {
-    int ct      = 0; // compile-time length (KFR_CT_CONV_F32), 0: the runtime-length block FFT
+    bool paired = false;
     int threads = 0;
     int elems   = 0; // shared complex elements (even)
     rp_desc rp{};
@@ -29,10 +30,10 @@ struct conv_fft
 template <typename T>
 struct fir_tables
 {
-    explicit fir_tables(size_t f);
+    fir_tables(size_t f, bool paired);
     void roots64(size_t f); // w64
     conv_fft fft;
-    dbuf tw, rtw; // pass twiddles; W_f^k, k <= f / 2
+    dbuf tw, rtw; // pass twiddles; W_f^k, k <= f / 2 (unpaired)
     dbuf w64;     // W_f^j, j < f, in double precision (gradients: the taps' spectrum)
 };
 
@@ -43,7 +44,7 @@ struct conv_args
     const void* hist;  // channels x nhist previous samples
     long long n;       // samples per channel in this call
     long long nhist;   // M - 1
-    long long m1;      // overlap of the blocks: M - 1 rounded up to even
+    long long m1;      // overlap of the blocks: M - 1, rounded up to even for unpaired blocks
     long long bo;      // valid outputs per block
     int channels;
     const void* hspec; // c+1 complex: FFT_F(taps) / F

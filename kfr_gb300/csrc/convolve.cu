@@ -60,14 +60,14 @@ std::shared_ptr<real_engine<T>> plan_cache::real(long long n)
 }
 
 template <typename T>
-std::shared_ptr<fir_tables<T>> plan_cache::fir(long long n)
+std::shared_ptr<fir_tables<T>> plan_cache::fir(long long n, bool paired)
 {
     std::lock_guard<std::mutex> lock(mu_);
-    const int kd = 4 + (sizeof(T) == 8 ? 1 : 0);
+    const int kd = 4 + (sizeof(T) == 8 ? 1 : 0) + (paired ? 2 : 0);
     for (auto& e : entries_)
         if (e->kind == kd && e->n == n)
             return std::static_pointer_cast<fir_tables<T>>(e->plan);
-    auto p = std::make_shared<fir_tables<T>>(size_t(n));
+    auto p = std::make_shared<fir_tables<T>>(size_t(n), paired);
     p->roots64(size_t(n));
     entries_.push_back(std::make_shared<entry>(entry{ kd, n, p }));
     return p;
@@ -90,8 +90,8 @@ template std::shared_ptr<complex_engine<float>> plan_cache::complex<float>(long 
 template std::shared_ptr<complex_engine<double>> plan_cache::complex<double>(long long);
 template std::shared_ptr<real_engine<float>> plan_cache::real<float>(long long);
 template std::shared_ptr<real_engine<double>> plan_cache::real<double>(long long);
-template std::shared_ptr<fir_tables<float>> plan_cache::fir<float>(long long);
-template std::shared_ptr<fir_tables<double>> plan_cache::fir<double>(long long);
+template std::shared_ptr<fir_tables<float>> plan_cache::fir<float>(long long, bool);
+template std::shared_ptr<fir_tables<double>> plan_cache::fir<double>(long long, bool);
 
 // ------------------------------------------------------------------------------------------------------
 // kernels

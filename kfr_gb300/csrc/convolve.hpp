@@ -29,9 +29,9 @@ public:
     std::shared_ptr<complex_engine<T>> complex(long long n);
     template <typename T>
     std::shared_ptr<real_engine<T>> real(long long n);
-    // tables of the FIR gradients' real FFT of n samples
+    // tables of the FIR gradients' blocks of n samples
     template <typename T>
-    std::shared_ptr<fir_tables<T>> fir(long long n);
+    std::shared_ptr<fir_tables<T>> fir(long long n, bool paired);
     void clear();
     size_t size() const;
 

@@ -313,7 +313,6 @@ bool ct_lookup(int kind, int n, int& ts, std::vector<int>& radices)
     case CT_FOURSTEP: KFR_CT_FOURSTEP_F32(KFR_CT_HOST) break;
     case CT_REAL: KFR_CT_REAL_F32(KFR_CT_HOST) break;
     case CT_DCT: KFR_CT_DCT_F32(KFR_CT_HOST) break;
-    case CT_CONV: KFR_CT_CONV_F32(KFR_CT_HOST) break;
     default: break;
     }
 #undef KFR_CT_HOST

@@ -99,8 +99,7 @@ enum ct_kind
     CT_RADER,
     CT_FOURSTEP,
     CT_REAL,
-    CT_DCT,
-    CT_CONV
+    CT_DCT
 };
 
 // True (with the thread count and radix order) if `kind` has a compile-time kernel of length n for T.

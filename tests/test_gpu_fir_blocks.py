@@ -12,6 +12,8 @@ pytestmark = pytest.mark.gpu
 
 
 def fft_size(m, sfx):
+    if sfx == "f32" and m <= 2049:
+        return 4096  # paired blocks
     f = 2048
     while f < 8 * (m - 1):
         f *= 2
@@ -25,7 +27,7 @@ def fir(h, x):
 # one tap, odd and even tap counts, signals shorter than the taps, of exactly one block, of one sample more, odd
 # lengths (the second channel is then aligned to one sample only), every FFT length of the kernels
 CASES = [(1, 1, 1), (2, 5000, 2), (16, 2033, 3), (1023, 7169, 2), (1024, 3, 1), (1023, 14340, 2), (255, 1794, 1),
-         (256, 1793, 3), (700, 40001, 2), (2000, 20011, 2), (4000, 70000, 1)]
+         (256, 1793, 3), (700, 40001, 2), (2000, 20011, 2), (4000, 70000, 1), (2049, 6145, 2), (2050, 6145, 1)]
 
 
 @pytest.mark.parametrize("sfx", ["f32", "f64"])
