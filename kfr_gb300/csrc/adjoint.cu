@@ -17,6 +17,7 @@ static unsigned grid_for(long long n)
 template <typename T>
 __global__ void k_spectrum_weight(cpx<T>* out, const cpx<T>* in, long long batch, long long bins, int ccs, T w)
 {
+    stream_order();
     const long long total = batch * bins;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x)
     {
@@ -29,6 +30,7 @@ __global__ void k_spectrum_weight(cpx<T>* out, const cpx<T>* in, long long batch
 template <typename T>
 __global__ void k_scale_first(T* out, const T* in, long long batch, long long n, T f)
 {
+    stream_order();
     const long long total = batch * n;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x)
         out[i] = (i % n == 0) ? in[i] * f : in[i];
@@ -37,6 +39,7 @@ __global__ void k_scale_first(T* out, const T* in, long long batch, long long n,
 template <typename T>
 __global__ void k_reverse(T* out, const T* in, long long channels, long long n)
 {
+    stream_order();
     const long long total = channels * n;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x)
     {
@@ -48,6 +51,7 @@ __global__ void k_reverse(T* out, const T* in, long long channels, long long n)
 template <typename T>
 __global__ void k_pad_real(T* out, const T* in, long long channels, long long n, long long size)
 {
+    stream_order();
     const long long total = channels * size;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x)
     {
@@ -59,6 +63,7 @@ __global__ void k_pad_real(T* out, const T* in, long long channels, long long n,
 template <typename T>
 __global__ void k_scale(T* out, const T* in, long long n, T f)
 {
+    stream_order();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         out[i] = in[i] * f;
 }
@@ -66,6 +71,7 @@ __global__ void k_scale(T* out, const T* in, long long n, T f)
 template <typename T>
 __global__ void k_cmac_conj(cpx<T>* acc, const cpx<T>* a, const cpx<T>* b, long long channels, long long bins, int first)
 {
+    stream_order();
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < bins; k += (long long)gridDim.x * blockDim.x)
     {
         cpx<T> s = first ? mk<T>(0, 0) : acc[k];
@@ -81,9 +87,8 @@ cudaError_t launch_spectrum_weight(void* out, const void* in, long long batch, l
 {
     if (batch * bins <= 0)
         return cudaSuccess;
-    k_spectrum_weight<T><<<grid_for(batch * bins), 256, 0, st>>>(static_cast<cpx<T>*>(out),
-                                                                  static_cast<const cpx<T>*>(in), batch, bins, ccs, interior);
-    return cudaGetLastError();
+    return launch_kernel(k_spectrum_weight<T>, dim3(grid_for(batch * bins)), 256, 0, st, static_cast<cpx<T>*>(out),
+                         static_cast<const cpx<T>*>(in), batch, bins, ccs, interior);
 }
 
 template <typename T>
@@ -91,8 +96,7 @@ cudaError_t launch_scale_first(T* out, const T* in, long long batch, long long n
 {
     if (batch * n <= 0)
         return cudaSuccess;
-    k_scale_first<T><<<grid_for(batch * n), 256, 0, st>>>(out, in, batch, n, f);
-    return cudaGetLastError();
+    return launch_kernel(k_scale_first<T>, dim3(grid_for(batch * n)), 256, 0, st, out, in, batch, n, f);
 }
 
 template <typename T>
@@ -100,8 +104,7 @@ cudaError_t launch_reverse(T* out, const T* in, long long channels, long long n,
 {
     if (channels * n <= 0)
         return cudaSuccess;
-    k_reverse<T><<<grid_for(channels * n), 256, 0, st>>>(out, in, channels, n);
-    return cudaGetLastError();
+    return launch_kernel(k_reverse<T>, dim3(grid_for(channels * n)), 256, 0, st, out, in, channels, n);
 }
 
 template <typename T>
@@ -109,8 +112,7 @@ cudaError_t launch_pad(T* out, const T* in, long long channels, long long n, lon
 {
     if (channels * size <= 0)
         return cudaSuccess;
-    k_pad_real<T><<<grid_for(channels * size), 256, 0, st>>>(out, in, channels, n, size);
-    return cudaGetLastError();
+    return launch_kernel(k_pad_real<T>, dim3(grid_for(channels * size)), 256, 0, st, out, in, channels, n, size);
 }
 
 template <typename T>
@@ -119,9 +121,8 @@ cudaError_t launch_cmac_conj(void* acc, const void* a, const void* b, long long 
 {
     if (bins <= 0)
         return cudaSuccess;
-    k_cmac_conj<T><<<grid_for(bins), 256, 0, st>>>(static_cast<cpx<T>*>(acc), static_cast<const cpx<T>*>(a),
-                                                    static_cast<const cpx<T>*>(b), channels, bins, first);
-    return cudaGetLastError();
+    return launch_kernel(k_cmac_conj<T>, dim3(grid_for(bins)), 256, 0, st, static_cast<cpx<T>*>(acc),
+                         static_cast<const cpx<T>*>(a), static_cast<const cpx<T>*>(b), channels, bins, first);
 }
 
 template <typename T>
@@ -181,7 +182,8 @@ void fir_backward(const T* taps, long long ntaps, long long channels, long long 
         }
         eng->inverse(r.get(), acc.get(), 1, true, scr.get(), st);
         // grad_h = r[0 .. M-1] / P
-        k_scale<T><<<grid_for(ntaps), 256, 0, st>>>(grad_h, static_cast<const T*>(r.get()), ntaps, T(1) / T(P));
+        launch_kernel(k_scale<T>, dim3(grid_for(ntaps)), 256, 0, st, grad_h, static_cast<const T*>(r.get()), ntaps,
+                      T(1) / T(P));
         check(cudaGetLastError(), "scale taps gradient");
         check(cudaStreamSynchronize(st), "FIR backward (taps)");
     }

@@ -95,6 +95,7 @@ template <class P>
 __global__ void __launch_bounds__(P::max_threads, 1)
     k_conv_os(const __grid_constant__ conv_args a)
 {
+    stream_order();
     using T = typename P::real;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const P fft(reinterpret_cast<cpx<T>*>(smem_raw), a.tw, a.fft);
@@ -177,6 +178,7 @@ template <class P>
 __global__ void __launch_bounds__(P::max_threads, 1)
     k_fir_bwd(const __grid_constant__ fir_bwd_args a)
 {
+    stream_order();
     using T = typename P::real;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const P fg(reinterpret_cast<cpx<T>*>(smem_raw), a.tw, a.fft);
@@ -281,6 +283,7 @@ __global__ void __launch_bounds__(P::max_threads, 1)
 template <typename T>
 __global__ void __launch_bounds__(256) k_fir_reduce(cpx<T>* sum, const cpx<T>* partial, int parts, int bins)
 {
+    stream_order();
     __shared__ cpx<T> s[8][32];
     const int k = blockIdx.x * 32 + int(threadIdx.x & 31), row = threadIdx.x >> 5;
     cpx<T> v = mk<T>(0, 0);
@@ -302,6 +305,7 @@ template <class P>
 __global__ void __launch_bounds__(P::max_threads, 1) k_fir_taps(const __grid_constant__ fir_bwd_args a, void* grad_h,
                                                                const void* spectrum, const int taps)
 {
+    stream_order();
     using T = typename P::real;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const P fft(reinterpret_cast<cpx<T>*>(smem_raw), a.tw, a.fft);
@@ -323,9 +327,10 @@ __global__ void __launch_bounds__(P::max_threads, 1) k_fir_taps(const __grid_con
 // H[k] = sum_{m0} W_F^{m0 k} S[m0][k mod F/Q].  w: W_F^j, j < F; placed: stored for k_fir16_bwd.  (FP64 FFTs of one CTA would take tens of
 // microseconds on this part; these sums spread over all SMs.)
 template <typename T>
-__global__ void __launch_bounds__(128) k_fir_spec_inner(double2* S, const T* __restrict__ h, const double2* __restrict__ w,
+__global__ void __launch_bounds__(128) k_fir_spec_inner(double2* S, const T* h, const double2* __restrict__ w,
                                                        int taps, int F, int Q)
 {
+    stream_order();
     const int P = F / Q, i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= Q * P)
         return;
@@ -345,10 +350,11 @@ __global__ void __launch_bounds__(128) k_fir_spec_inner(double2* S, const T* __r
     S[i] = make_double2(re, im);
 }
 template <typename T>
-__global__ void __launch_bounds__(64) k_fir_spec_outer(cpx<T>* H, const double2* __restrict__ S,
+__global__ void __launch_bounds__(64) k_fir_spec_outer(cpx<T>* H, const double2* S,
                                                       const double2* __restrict__ w, int taps, int F, int Q,
                                                       bool placed)
 {
+    stream_order();
     const int P = F / Q, k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k > F / 2)
         return;
@@ -392,6 +398,7 @@ __device__ __forceinline__ float conv_sample(const float* in, const float* hist,
 
 __global__ void __launch_bounds__(fft16::threads, 3) k_conv16(const __grid_constant__ conv_args a)
 {
+    stream_order();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const fft16 f(smem_raw, a.tw);
     const float* in   = reinterpret_cast<const float*>(a.in) + (long long)blockIdx.y * a.n;
@@ -451,6 +458,7 @@ __global__ void __launch_bounds__(fft16::threads, 3) k_conv16(const __grid_const
 // per thread wait in registers while g takes the buffer; the next pair's samples of x are loaded during the inverse.
 __global__ void __launch_bounds__(fft16::threads, 2) k_fir16_bwd(const __grid_constant__ fir_bwd_args a)
 {
+    stream_order();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const fft16 f(smem_raw, a.tw);
     cpx<float>* acc     = reinterpret_cast<cpx<float>*>(smem_raw) + fft16::elems + f.t; // bin u at 256 u
@@ -542,6 +550,7 @@ __global__ void __launch_bounds__(fft16::threads, 2) k_fir16_bwd(const __grid_co
 __global__ void __launch_bounds__(fft16::threads, 1) k_fir16_taps(const __grid_constant__ fir_bwd_args a, float* grad_h,
                                                                  const cpx<float>* spectrum, const int taps)
 {
+    stream_order();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const fft16 f(smem_raw, a.tw);
     cpx<float> v[16];
@@ -561,9 +570,10 @@ __global__ void __launch_bounds__(fft16::threads, 1) k_fir16_taps(const __grid_c
 
 // new_hist[i] = i + n < m1 ? old_hist[i + n] : in[i + n - m1]
 template <typename T>
-__global__ void k_hist_update(const T* __restrict__ hold, T* __restrict__ hnew, const T* __restrict__ in, long long n,
+__global__ void k_hist_update(const T* hold, T* hnew, const T* in, long long n,
                               long long m1, int channels)
 {
+    stream_order();
     const long long total = m1 * channels;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x)
     {
@@ -582,8 +592,7 @@ static cudaError_t conv_go(K kernel, dim3 grid, int threads, size_t smem, cudaSt
         if (e != cudaSuccess)
             return e;
     }
-    kernel<<<grid, threads, smem, st>>>(args...);
-    return cudaGetLastError();
+    return launch_kernel(kernel, grid, threads, smem, st, args...);
 }
 
 template <typename T>
@@ -605,9 +614,8 @@ cudaError_t launch_hist_update(const void* hold, void* hnew, const void* in, lon
     if (total <= 0)
         return cudaSuccess;
     const long long blocks = std::min<long long>((total + 255) / 256, 4096);
-    k_hist_update<T><<<unsigned(blocks), 256, 0, st>>>(static_cast<const T*>(hold), static_cast<T*>(hnew),
-                                                        static_cast<const T*>(in), n, m1, channels);
-    return cudaGetLastError();
+    return launch_kernel(k_hist_update<T>, dim3(unsigned(blocks)), 256, 0, st, static_cast<const T*>(hold),
+                         static_cast<T*>(hnew), static_cast<const T*>(in), n, m1, channels);
 }
 
 // ------------------------------------------------------------------------------------------------------
@@ -876,17 +884,16 @@ bool fir_backward_blocks(const T* taps, long long ntaps, long long channels, lon
     if (grad_x)
     {
         const double2* w = static_cast<const double2*>(tab->w64.get());
-        k_fir_spec_inner<T><<<unsigned((f + 127) / 128), 128, 0, st>>>(reinterpret_cast<double2*>(inner), taps, w,
-                                                                     int(ntaps), int(f), Q);
-        k_fir_spec_outer<T><<<unsigned((c + 64) / 64), 64, 0, st>>>(reinterpret_cast<cpx<T>*>(H),
-                                                                    reinterpret_cast<const double2*>(inner), w, int(ntaps),
-                                                                    int(f), Q, paired);
+        launch_kernel(k_fir_spec_inner<T>, dim3(unsigned((f + 127) / 128)), 128, 0, st,
+                      reinterpret_cast<double2*>(inner), taps, w, int(ntaps), int(f), Q);
+        launch_kernel(k_fir_spec_outer<T>, dim3(unsigned((c + 64) / 64)), 64, 0, st, reinterpret_cast<cpx<T>*>(H),
+                      reinterpret_cast<const double2*>(inner), w, int(ntaps), int(f), Q, paired);
         check(cudaGetLastError(), "taps spectrum");
     }
     const auto reduce = [&]()
     {
-        k_fir_reduce<T><<<unsigned((bins + 31) / 32), 256, 0, st>>>(reinterpret_cast<cpx<T>*>(sum),
-                                                                    reinterpret_cast<const cpx<T>*>(parts), grid, bins);
+        launch_kernel(k_fir_reduce<T>, dim3(unsigned((bins + 31) / 32)), 256, 0, st, reinterpret_cast<cpx<T>*>(sum),
+                      reinterpret_cast<const cpx<T>*>(parts), grid, bins);
         check(cudaGetLastError(), "launch FIR backward (sum)");
     };
     if (paired)

@@ -99,8 +99,9 @@ template std::shared_ptr<fir_tables<double>> plan_cache::fir<double>(long long, 
 
 // out[i] = i < n ? in[reverse ? n-1-i : i] : 0 for i < size (E = T for reals, cpx<T> for complex)
 template <typename E>
-__global__ void k_pad(E* __restrict__ out, const E* __restrict__ in, long long n, long long size, int reverse)
+__global__ void k_pad(E* out, const E* in, long long n, long long size, int reverse)
 {
+    stream_order();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < size; i += (long long)gridDim.x * blockDim.x)
     {
         E v{};
@@ -111,15 +112,17 @@ __global__ void k_pad(E* __restrict__ out, const E* __restrict__ in, long long n
 }
 
 template <typename T>
-__global__ void k_cmul_scale(cpx<T>* __restrict__ a, const cpx<T>* __restrict__ b, long long n, T s)
+__global__ void k_cmul_scale(cpx<T>* a, const cpx<T>* b, long long n, T s)
 {
+    stream_order();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         a[i] = scale(a[i] * b[i], s);
 }
 
 template <typename T>
-__global__ void k_real_part(cpx<T>* __restrict__ out, const cpx<T>* __restrict__ in, long long n)
+__global__ void k_real_part(cpx<T>* out, const cpx<T>* in, long long n)
 {
+    stream_order();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         out[i] = mk(in[i].x, T(0));
 }
@@ -173,11 +176,11 @@ void convolve_device(void* out, const void* a, long long na, const void* b, long
         void* escratch       = nullptr;
         if (escr)
             check(cudaMallocAsync(&escratch, escr, st), "cudaMallocAsync");
-        k_pad<T><<<blocks_for(size), 256, 0, st>>>(pa, static_cast<const T*>(a), na, size, 0);
-        k_pad<T><<<blocks_for(size), 256, 0, st>>>(pb, static_cast<const T*>(b), nb, size, rev);
+        launch_kernel(k_pad<T>, dim3(blocks_for(size)), 256, 0, st, pa, static_cast<const T*>(a), na, size, 0);
+        launch_kernel(k_pad<T>, dim3(blocks_for(size)), 256, 0, st, pb, static_cast<const T*>(b), nb, size, rev);
         eng->forward(A, pa, 1, true, escratch, st);
         eng->forward(B, pb, 1, true, escratch, st);
-        k_cmul_scale<T><<<blocks_for(c + 1), 256, 0, st>>>(A, B, c + 1, T(1) / T(size));
+        launch_kernel(k_cmul_scale<T>, dim3(blocks_for(c + 1)), 256, 0, st, A, B, c + 1, T(1) / T(size));
         eng->inverse(pa, A, 1, true, escratch, st);
         check(cudaMemcpyAsync(out, pa, olen * sizeof(T), cudaMemcpyDeviceToDevice, st), "copy result");
         if (escratch)
@@ -192,13 +195,15 @@ void convolve_device(void* out, const void* a, long long na, const void* b, long
         void* escratch    = nullptr;
         if (escr)
             check(cudaMallocAsync(&escratch, escr, st), "cudaMallocAsync");
-        k_pad<cpx<T>><<<blocks_for(size), 256, 0, st>>>(pa, static_cast<const cpx<T>*>(a), na, size, 0);
-        k_pad<cpx<T>><<<blocks_for(size), 256, 0, st>>>(pb, static_cast<const cpx<T>*>(b), nb, size, rev);
+        launch_kernel(k_pad<cpx<T>>, dim3(blocks_for(size)), 256, 0, st, pa, static_cast<const cpx<T>*>(a), na,
+                      size, 0);
+        launch_kernel(k_pad<cpx<T>>, dim3(blocks_for(size)), 256, 0, st, pb, static_cast<const cpx<T>*>(b), nb,
+                      size, rev);
         eng->execute(pa, pa, 1, size, size, false, escratch, st);
         eng->execute(pb, pb, 1, size, size, false, escratch, st);
-        k_cmul_scale<T><<<blocks_for(size), 256, 0, st>>>(pa, pb, size, T(1) / T(size));
+        launch_kernel(k_cmul_scale<T>, dim3(blocks_for(size)), 256, 0, st, pa, pb, size, T(1) / T(size));
         eng->execute(pa, pa, 1, size, size, true, escratch, st);
-        k_real_part<T><<<blocks_for(olen), 256, 0, st>>>(static_cast<cpx<T>*>(out), pa, olen);
+        launch_kernel(k_real_part<T>, dim3(blocks_for(olen)), 256, 0, st, static_cast<cpx<T>*>(out), pa, olen);
         if (escratch)
             cudaFreeAsync(escratch, st);
     }

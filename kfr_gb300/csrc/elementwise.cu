@@ -10,6 +10,7 @@ namespace kfr_gpu
 template <typename T>
 __global__ void __launch_bounds__(256) k_elementwise(const int op, const ew_args a)
 {
+    stream_order();
     const long long total = a.batch * a.n;
     const cpx<T>* in      = reinterpret_cast<const cpx<T>*>(a.in);
     cpx<T>* out           = reinterpret_cast<cpx<T>*>(a.out);
@@ -83,8 +84,7 @@ cudaError_t launch_elementwise(int op, const ew_args& a, cudaStream_t st)
     long long blocks = (total + 255) / 256;
     if (blocks > 152LL * 32)
         blocks = 152LL * 32;
-    k_elementwise<T><<<unsigned(blocks), 256, 0, st>>>(op, a);
-    return cudaGetLastError();
+    return launch_kernel(k_elementwise<T>, dim3(unsigned(blocks)), 256, 0, st, op, a);
 }
 
 // Real-DFT split / merge over mirror pairs: thread e of a signal (e = 0 .. c/2) reads Z[e] and Z[c - e] (or
@@ -92,6 +92,7 @@ cudaError_t launch_elementwise(int op, const ew_args& a, cudaStream_t st)
 template <typename T, bool INV>
 __global__ void __launch_bounds__(256) k_real_pairs(const ew_args a)
 {
+    stream_order();
     const long long c = a.n_src;
     const cpx<T>* t0  = reinterpret_cast<const cpx<T>*>(a.t0);
     const bool ccs    = a.flag != 0;
@@ -148,10 +149,8 @@ cudaError_t launch_real_pairs(const ew_args& a, bool inverse, cudaStream_t st)
     const unsigned bx = unsigned(std::min<long long>((pairs + 255) / 256, 1024));
     const unsigned by = unsigned(std::min<long long>(a.batch, std::max<long long>(1, 152LL * 16 / bx)));
     if (inverse)
-        k_real_pairs<T, true><<<dim3(bx, by), 256, 0, st>>>(a);
-    else
-        k_real_pairs<T, false><<<dim3(bx, by), 256, 0, st>>>(a);
-    return cudaGetLastError();
+        return launch_kernel(k_real_pairs<T, true>, dim3(bx, by), 256, 0, st, a);
+    return launch_kernel(k_real_pairs<T, false>, dim3(bx, by), 256, 0, st, a);
 }
 template cudaError_t launch_real_pairs<float>(const ew_args&, bool, cudaStream_t);
 template cudaError_t launch_real_pairs<double>(const ew_args&, bool, cudaStream_t);
@@ -165,6 +164,7 @@ __global__ void __launch_bounds__(256) k_fft_multiply(cpx<T>* dest, const cpx<T>
                                                       const long long total, const long long src2_stride,
                                                       const int perm)
 {
+    stream_order();
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
          i += (long long)gridDim.x * blockDim.x)
     {
@@ -194,10 +194,10 @@ cudaError_t launch_fft_multiply(void* dest, const void* acc, const void* src1, c
     const auto* s1 = static_cast<const cpx<T>*>(src1);
     const auto* s2 = static_cast<const cpx<T>*>(src2);
     if (acc)
-        k_fft_multiply<T, true><<<unsigned(blocks), 256, 0, st>>>(d, a, s1, s2, size, total, src2_stride, perm);
-    else
-        k_fft_multiply<T, false><<<unsigned(blocks), 256, 0, st>>>(d, a, s1, s2, size, total, src2_stride, perm);
-    return cudaGetLastError();
+        return launch_kernel(k_fft_multiply<T, true>, dim3(unsigned(blocks)), 256, 0, st, d, a, s1, s2, size, total,
+                             src2_stride, perm);
+    return launch_kernel(k_fft_multiply<T, false>, dim3(unsigned(blocks)), 256, 0, st, d, a, s1, s2, size, total,
+                         src2_stride, perm);
 }
 
 template cudaError_t launch_fft_multiply<float>(void*, const void*, const void*, const void*, long long, long long,
@@ -212,6 +212,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) k_transpose(cpx<T>* out, const cpx<T>* in, const long long rows,
                                                    const long long cols, const long long b0)
 {
+    stream_order();
     __shared__ cpx<T> tile[32][33];
     const long long b  = b0 + blockIdx.y;
     const long long gx = (cols + 31) / 32; // tiles along a row; blockIdx.x = row tile * gx + column tile
@@ -248,8 +249,8 @@ cudaError_t launch_transpose(void* out, const void* in, long long batch, long lo
     for (long long b0 = 0; b0 < batch; b0 += 65535)
     {
         const unsigned gb = unsigned(std::min<long long>(65535, batch - b0));
-        k_transpose<T><<<dim3(unsigned(tiles), gb), 256, 0, st>>>(static_cast<cpx<T>*>(out),
-                                                                   static_cast<const cpx<T>*>(in), rows, cols, b0);
+        launch_kernel(k_transpose<T>, dim3(unsigned(tiles), gb), 256, 0, st, static_cast<cpx<T>*>(out),
+                      static_cast<const cpx<T>*>(in), rows, cols, b0);
     }
     return cudaGetLastError();
 }

@@ -22,6 +22,13 @@
 namespace kfr_gpu
 {
 
+// First statement of every kernel that launch_kernel starts: everything before this kernel on the stream has finished
+// and is visible.
+__device__ __forceinline__ void stream_order()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 template <typename T>
 struct alignas(2 * sizeof(T)) cpx
 {

@@ -139,6 +139,7 @@ __device__ __forceinline__ void copy_batched(const int total, const LD& ld, cons
 template <typename T, class F>
 __global__ void __launch_bounds__(F::max_threads, 1) k_c2c(const c2c_args a, const int ts, const int spc)
 {
+    stream_order();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const F fft(a.d, ts, spc);
     cpx<T>* sm        = reinterpret_cast<cpx<T>*>(smem_raw);
@@ -187,6 +188,7 @@ template <typename T, class F>
 __global__ void __launch_bounds__(F::max_threads, 1)
     k_c2c_pipe(const c2c_args a, const long long ntiles, const int spc, int* err)
 {
+    stream_order();
     extern __shared__ __align__(128) unsigned char smem_raw[];
     constexpr int N      = F::n;
     constexpr int STRIDE = F::gstride(N);
@@ -290,6 +292,7 @@ template <typename T, class F>
 __global__ void __launch_bounds__(F::max_threads, 1)
     k_c2c_reg(const c2c_args a, const long long nsig, int* err)
 {
+    stream_order();
     extern __shared__ __align__(128) unsigned char smem_raw[];
     constexpr int N          = F::n;
     constexpr int H          = N / 2;
@@ -372,6 +375,7 @@ template <typename T, class F>
 __global__ void __launch_bounds__(F::max_threads, 1) k_bluestein(const bluestein_args a, const int ts,
                                                                         const int spc)
 {
+    stream_order();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const F fft(a.d, ts, spc);
     cpx<T>* sm        = reinterpret_cast<cpx<T>*>(smem_raw);
@@ -427,6 +431,7 @@ __global__ void __launch_bounds__(F::max_threads, 1) k_bluestein(const bluestein
 template <typename T, class F>
 __global__ void __launch_bounds__(F::max_threads, 1) k_rader(const rader_args a, const int ts, const int spc)
 {
+    stream_order();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const F fft(a.d, ts, spc);
     cpx<T>* sm         = reinterpret_cast<cpx<T>*>(smem_raw);
@@ -490,6 +495,7 @@ __global__ void __launch_bounds__(F::max_threads, 1) k_rader(const rader_args a,
 template <typename T, class F>
 __global__ void __launch_bounds__(F::max_threads, 1) k_r2c(const real_args a, const int ts, const int spc)
 {
+    stream_order();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const F fft(a.d, ts, spc);
     cpx<T>* sm        = reinterpret_cast<cpx<T>*>(smem_raw);
@@ -572,6 +578,7 @@ template <typename T, class F>
 __global__ void __launch_bounds__(F::max_threads, 1)
     k_r2c_pipe(const real_args a, const long long ntiles, const int spc, int* err)
 {
+    stream_order();
     extern __shared__ __align__(128) unsigned char smem_raw[];
     constexpr int C      = F::n;
     constexpr int STRIDE = F::gstride(C);
@@ -692,6 +699,7 @@ __global__ void __launch_bounds__(F::max_threads, 1)
 template <typename T, class F>
 __global__ void __launch_bounds__(F::max_threads, 1) k_c2r(const real_args a, const int ts, const int spc)
 {
+    stream_order();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const F fft(a.d, ts, spc);
     cpx<T>* sm        = reinterpret_cast<cpx<T>*>(smem_raw);
@@ -765,6 +773,7 @@ template <typename T, class F>
 __global__ void __launch_bounds__(F::max_threads, 1)
     k_c2r_pipe(const real_args a, const long long ntiles, const int spc, int* err)
 {
+    stream_order();
     extern __shared__ __align__(128) unsigned char smem_raw[];
     constexpr int C      = F::n;
     constexpr int STRIDE = F::gstride(C);
@@ -879,6 +888,7 @@ __global__ void __launch_bounds__(F::max_threads, 1)
 template <typename T, class F>
 __global__ void __launch_bounds__(F::max_threads, 1) k_dct2(const dct_args a, const int ts, const int spc)
 {
+    stream_order();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const F fft(a.d, ts, spc);
     cpx<T>* sm        = reinterpret_cast<cpx<T>*>(smem_raw);
@@ -920,6 +930,7 @@ __global__ void __launch_bounds__(F::max_threads, 1) k_dct2(const dct_args a, co
 template <typename T, class F>
 __global__ void __launch_bounds__(F::max_threads, 1) k_dct3(const dct_args a, const int ts, const int spc)
 {
+    stream_order();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const F fft(a.d, ts, spc);
     cpx<T>* sm        = reinterpret_cast<cpx<T>*>(smem_raw);
@@ -981,6 +992,7 @@ template <typename T, class F, bool INV>
 __global__ void __launch_bounds__(F::max_threads, 1)
     k_dct_pipe(const dct_args a, const long long ntiles, const int spc, int* err)
 {
+    stream_order();
     extern __shared__ __align__(128) unsigned char smem_raw[];
     constexpr int N      = F::n;
     constexpr int STRIDE = F::gstride(N);
@@ -1109,6 +1121,7 @@ __host__ __device__ constexpr int lbits_for()
 template <typename T, class FA, int N2>
 __global__ void __launch_bounds__(1024, 1) k_fsp_cols(const fourstep_args a)
 {
+    stream_order();
     constexpr int N1 = FA::n, GA = FA::gstride(), TS = FA::ts;
     constexpr int S  = fsp_tile(N1, TS, kFspSmem), SH = S == 16 ? 4 : 3;
     constexpr long long N = (long long)N1 * N2;
@@ -1149,6 +1162,7 @@ __global__ void __launch_bounds__(1024, 1) k_fsp_cols(const fourstep_args a)
 template <typename T, class FB, int N1>
 __global__ void __launch_bounds__(1024, 1) k_fsp_rows(const fourstep_args a)
 {
+    stream_order();
     constexpr int N2 = FB::n, GB = FB::gstride(), TS = FB::ts;
     constexpr int S  = fsp_tile(N2, TS, kFspSmem), SH = S == 16 ? 4 : 3;
     constexpr long long N = (long long)N1 * N2;
@@ -1275,6 +1289,7 @@ template <typename T, class FA, int N2, bool RP = false>
 __global__ void __launch_bounds__(fspt_threads<FA>(), fspt_min_ctas<FA>())
     k_fspt_cols(const fourstep_args a, const __grid_constant__ tensor_map tm_in, const long long ntiles, int* err)
 {
+    stream_order();
     static_assert(fspt_ok<FA>(), "two or three passes on tiles of 16 to 2 columns");
     constexpr int N1 = FA::n, GA = FA::gstride(), TS = FA::ts, S = fspt_tile<FA>();
     // RP: the real-fused layout, columns P1 apart (N1 rounded up to even) with outputs at rp_pos(k1)
@@ -1385,6 +1400,7 @@ __global__ void __launch_bounds__(fspt_threads<FB>(), fspt_min_ctas<FB>())
     k_fspt_rows(const fourstep_args a, const __grid_constant__ tensor_map tm_in,
                 const __grid_constant__ tensor_map tm_out, const long long ntiles, int* err)
 {
+    stream_order();
     static_assert(fspt_ok<FB>(), "two passes on tiles of 16 to 2 rows");
     constexpr int N2 = FB::n, GB = FB::gstride(), TS = FB::ts, S = fspt_tile<FB>();
     constexpr int NTR = (N1 + S - 1) / S;
@@ -1464,6 +1480,7 @@ template <typename T, class FB, int N1>
 __global__ void __launch_bounds__(fspt_threads<FB>(), fspt_min_ctas<FB>())
     k_fspt_rows_r2c(const fourstep_args a, const __grid_constant__ tensor_map tm_in, const long long ntiles, int* err)
 {
+    stream_order();
     static_assert(fspt_ok<FB>() && FB::npass == 2, "two passes on tiles of 16 to 2 rows");
     constexpr int N2 = FB::n, GB = FB::gstride(), TS = FB::ts, S = fspt_tile<FB>();
     static_assert(S % 2 == 0, "whole mirror pairs per tile");
@@ -1595,8 +1612,7 @@ static cudaError_t go(K kernel, dim3 grid, const block_cfg& c, cudaStream_t st, 
         if (e != cudaSuccess)
             return e;
     }
-    kernel<<<grid, c.threads, c.smem, st>>>(args...);
-    return cudaGetLastError();
+    return launch_kernel(kernel, grid, c.threads, size_t(c.smem), st, args...);
 }
 
 #define KFR_GPU_CT_HOOK(CTFN)                                                                              \

@@ -63,8 +63,7 @@ static cudaError_t go_persistent(K kernel, const block_cfg& c, long long ntiles,
     if (per_sm < 1 || sms < 1)
         return cudaErrorInvalidConfiguration;
     const long long grid = std::min<long long>(ntiles, (long long)per_sm * sms);
-    kernel<<<unsigned(grid), c.threads, c.smem, st>>>(args...);
-    return cudaGetLastError();
+    return launch_kernel(kernel, dim3(unsigned(grid)), c.threads, size_t(c.smem), st, args...);
 }
 
 cudaError_t launch_ct_c2c_pipe_f32(const c2c_args& a0, const block_cfg& c, long long ntiles, int* err, cudaStream_t st)

@@ -36,8 +36,7 @@ static cudaError_t go_fsp(K kernel, dim3 grid, int threads, int smem, cudaStream
     const cudaError_t e = prepare_launch(reinterpret_cast<const void*>(kernel), threads, smem);
     if (e != cudaSuccess)
         return e;
-    kernel<<<grid, threads, smem, st>>>(a);
-    return cudaGetLastError();
+    return launch_kernel(kernel, grid, threads, size_t(smem), st, a);
 }
 
 // cuTensorMapEncodeTiled, looked up once through the runtime's driver entry-point query (no link-time
@@ -93,8 +92,7 @@ static cudaError_t go_fspt(K kernel, int threads, int smem, long long ntiles, cu
     if (per_sm < 1 || sms < 1)
         return cudaErrorInvalidConfiguration;
     const long long grid = std::min<long long>(ntiles, (long long)per_sm * sms);
-    kernel<<<unsigned(grid), threads, smem, st>>>(args...);
-    return cudaGetLastError();
+    return launch_kernel(kernel, dim3(unsigned(grid)), threads, size_t(smem), st, args...);
 }
 
 // The persistent tensor-copy pair kernels where the length and the buffers allow them; done = false

@@ -71,6 +71,26 @@ int device_sm_count()
     return it->second;
 }
 
+cudaError_t launch_kernel(const void* kernel, dim3 grid, int threads, size_t smem, cudaStream_t st, void** args)
+{
+    cudaLaunchAttribute attr;
+    attr.id                                         = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim          = grid;
+    cfg.blockDim         = dim3(unsigned(threads));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream           = st;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (st && st != cudaStreamLegacy && cudaStreamIsCapturing(st, &capture) == cudaSuccess &&
+        capture == cudaStreamCaptureStatusNone)
+    {
+        cfg.attrs    = &attr;
+        cfg.numAttrs = 1;
+    }
+    return cudaLaunchKernelExC(&cfg, kernel, args);
+}
+
 int max_smem_bytes()
 {
     int dev = 0, v = 0;

@@ -121,6 +121,7 @@ __host__ __device__ constexpr int pfa_buflen()
 template <typename T, int N, int SPC, int THREADS, int MINB, int NBUF, int... R>
 __global__ void __launch_bounds__(THREADS, MINB) k_rader_pfa(const rader_pfa_args a, const long long ntiles)
 {
+    stream_order();
     using AX          = axes<R...>;
     constexpr int L   = N - 1;
     constexpr int D   = AX::d;
@@ -325,8 +326,7 @@ cudaError_t go_pfa(K kernel, int threads, int smem, long long ntiles, const rade
     if (per_sm < 1 || sms < 1)
         return cudaErrorInvalidConfiguration;
     const long long grid = std::min<long long>(ntiles, (long long)per_sm * sms);
-    kernel<<<unsigned(grid), threads, smem, st>>>(a, ntiles);
-    return cudaGetLastError();
+    return launch_kernel(kernel, dim3(unsigned(grid)), threads, size_t(smem), st, a, ntiles);
 }
 
 // The compile-time instances: X(N, signals per tile, threads, CTAs per SM, buffers, axes: gather axis first,

@@ -22,13 +22,14 @@ __device__ __forceinline__ cpx<T> rp_root(const cpx<T>* __restrict__ A, const cp
 // `spc` signals, the first pass reading and the last pass writing global memory with the lanes along the
 // signal (any 8-byte aligned pointers and strides), the CTAs of an SM overlapping one another's accesses.
 // Bound by instruction issue (about 25 instructions per element and pass).  4096 signals of 3600 points
-// (15 x 16 x 15, one signal per 256-thread CTA): 56 us, 62% of the HBM copy rate, against 207 us for k_c2c's
-// runtime passes; 2000 points (four passes) 41%, 100 points (two) 88%.
+// (15 x 16 x 15, one signal per 256-thread CTA): 54 us, 65% of the HBM copy rate (207 us with the
+// radix-at-a-time passes before it); 2000 points (four passes) 41%, 100 points (two) 88%.
 // ---------------------------------------------------------------------------------------------------
 template <typename T, int H>
 __global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T), H), 1)
     k_rp_c2c(const __grid_constant__ rp_c2c_args a)
 {
+    stream_order();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const long long s0 = (long long)blockIdx.x * a.spc;
     const int cnt      = int(a.batch - s0 < a.spc ? a.batch - s0 : a.spc);
@@ -47,7 +48,7 @@ __global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T), H), 1)
 // whose output k of column c is multiplied by W_N^{c k}.  A tile is S columns (128-byte rows where S allows);
 // lanes run along the columns, so global and shared accesses are contiguous with no transposition.
 // Bound by instruction issue and, for tiles of 4 or 8 columns, by the 32- and 64-byte rows.  Eight 1080 x 1920
-// complex arrays, both axes: 155 us; 174 us with the widest tiles that fit one CTA per SM.
+// complex arrays, both axes: 150 us; 174 us with the widest tiles that fit one CTA per SM.
 // ---------------------------------------------------------------------------------------------------
 // MERGE: the input is the spectrum X of 2N reals, read as conj(Z[e]) with
 //   Z[e] = X[e] + conj X[N-e] + i conj(W_2N^e) (X[e] - conj X[N-e])
@@ -57,6 +58,7 @@ template <typename T, int H, bool MERGE>
 __global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T), H), 1)
     k_rp_cols(const __grid_constant__ rp_strided_args a)
 {
+    stream_order();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int S       = 1 << a.d.shift;
     const int tiles   = int((a.pitch + S - 1) >> a.d.shift);
@@ -123,13 +125,14 @@ __global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T), H), 1)
 // Second pass of a four-step transform of N = n1 n points: n-point DFTs along the n1 contiguous rows, output k
 // of row k1 to X[k1 + n1 k].  A tile is S rows: the first pass reads along the rows, the others run with the
 // lanes across the rows, so the stores cover S consecutive outputs; the transposition is the layout change
-// between the first two passes (RP_ROWS).  One complex<double> signal of 2^20 points, both kernels: 179 us
-// against 206 us for k_fs_cols and k_fs_rows (FP64 pipe, latency: one wave of CTAs).
+// between the first two passes (RP_ROWS).  One complex<double> signal of 2^20 points, both kernels: 181 us,
+// 206 us with the radix-at-a-time passes before them (FP64 pipe, latency: one wave of CTAs).
 // ---------------------------------------------------------------------------------------------------
 template <typename T, int H>
 __global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T), H), 1)
     k_rp_rows(const __grid_constant__ rp_strided_args a)
 {
+    stream_order();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int S       = 1 << a.d.shift;
     const int tiles   = int((a.pitch + S - 1) >> a.d.shift);
@@ -160,6 +163,7 @@ template <typename T, int H>
 __global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T), H), 1)
     k_rp_rows_split(const __grid_constant__ rp_strided_args a)
 {
+    stream_order();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int S = 1 << a.d.shift, half = S >> 1;
     const int n1 = int(a.pitch), n = a.d.n;
@@ -206,6 +210,7 @@ __global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T), H), 1)
 template <typename T, class C, int P>
 __global__ void __launch_bounds__(C::threads(), 1024 / C::threads()) k_ct_cols(const __grid_constant__ rp_strided_args a)
 {
+    stream_order();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int S = 1 << C::d.shift, tiles = P / S;
     const long long b = blockIdx.x / tiles;
@@ -239,6 +244,7 @@ __global__ void __launch_bounds__(C::threads(), 1024 / C::threads()) k_ct_cols(c
 template <typename T, class C, int P>
 __global__ void __launch_bounds__(C::threads(), 1024 / C::threads()) k_ct_rows(const __grid_constant__ rp_strided_args a)
 {
+    stream_order();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int S = 1 << C::d.shift, tiles = P / S;
     const long long b = blockIdx.x / tiles;
@@ -265,8 +271,7 @@ static cudaError_t rp_go(void (*kernel)(const A), const A& a, long long grid, in
         if (e != cudaSuccess)
             return e;
     }
-    kernel<<<unsigned(grid), threads, smem, st>>>(a);
-    return cudaGetLastError();
+    return launch_kernel(kernel, dim3(unsigned(grid)), threads, size_t(smem), st, a);
 }
 
 template <typename T, int H>

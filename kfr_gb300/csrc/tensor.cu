@@ -251,6 +251,7 @@ __device__ __forceinline__ cpx<float>* tc_block_fft(cpx<float>* a, cpx<float>* b
 template <int MODE, int N>
 __global__ void __launch_bounds__(512, 1) k_c2c_tc(const c2c_args a, const float* __restrict__ cs, const int spc)
 {
+    stream_order();
     constexpr int STRIDE = padded_len<float>(N);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cpx<float>* bufA = reinterpret_cast<cpx<float>*>(smem_raw);
@@ -281,6 +282,7 @@ __global__ void __launch_bounds__(512, 1) k_c2c_tc(const c2c_args a, const float
 template <int MODE, int N1, int S>
 __global__ void __launch_bounds__(512, 1) k_tc_cols(const tc_fs_args a)
 {
+    stream_order();
     constexpr int STRIDE = padded_len<float>(N1);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cpx<float>* bufA = reinterpret_cast<cpx<float>*>(smem_raw);
@@ -314,6 +316,7 @@ __global__ void __launch_bounds__(512, 1) k_tc_cols(const tc_fs_args a)
 template <int MODE, int N2, int S>
 __global__ void __launch_bounds__(512, 1) k_tc_rows(const tc_fs_args a)
 {
+    stream_order();
     constexpr int STRIDE = padded_len<float>(N2);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cpx<float>* bufA = reinterpret_cast<cpx<float>*>(smem_raw);
@@ -348,8 +351,7 @@ cudaError_t go_tc(K kernel, dim3 grid, int smem, cudaStream_t st, const tc_fs_ar
     const cudaError_t e = prepare_launch(reinterpret_cast<const void*>(kernel), 512, smem);
     if (e != cudaSuccess)
         return e;
-    kernel<<<grid, 512, smem, st>>>(a);
-    return cudaGetLastError();
+    return launch_kernel(kernel, grid, 512, size_t(smem), st, a);
 }
 
 template <int MODE>
@@ -384,8 +386,7 @@ cudaError_t launch_c2c_tc_f32(const c2c_args& a, int n, int mode, const float* c
         const cudaError_t e = prepare_launch(reinterpret_cast<const void*>(kernel), 512, smem);
         if (e != cudaSuccess)
             return e;
-        kernel<<<grid, 512, smem, st>>>(a, cs, spc);
-        return cudaGetLastError();
+        return launch_kernel(kernel, dim3(grid), 512, size_t(smem), st, a, cs, spc);
     };
     if (mode == TC_BF16)
         return n == 256 ? go(k_c2c_tc<TC_BF16, 256>) : go(k_c2c_tc<TC_BF16, 4096>);

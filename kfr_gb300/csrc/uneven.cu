@@ -47,6 +47,7 @@ __device__ __forceinline__ cpx<double> ld_cg(const cpx<double>* p)
 template <typename T>
 __global__ void __launch_bounds__(kUnevenThreads, 2) k_uneven(const __grid_constant__ uneven_launch a)
 {
+    stream_order();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ rp_desc D;
     // input and output 0 of each signal of the tile, and its column / row
@@ -229,8 +230,7 @@ cudaError_t launch_uneven_f32(const uneven_launch& a, int threads, int smem, int
     const cudaError_t e = prepare_launch(reinterpret_cast<const void*>(k_uneven<float>), threads, smem);
     if (e != cudaSuccess)
         return e;
-    k_uneven<float><<<unsigned(grid), threads, smem, st>>>(a);
-    return cudaGetLastError();
+    return launch_kernel(k_uneven<float>, dim3(unsigned(grid)), threads, size_t(smem), st, a);
 }
 
 // Dynamic shared memory of one of four 256-thread or two 512-thread CTAs per SM, beside the kernel's static
