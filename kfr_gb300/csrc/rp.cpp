@@ -89,11 +89,12 @@ int conflicts(const int* addr, int lanes, int elem)
         int count[16] = {}, worst = 1;
         for (int i = b; i < e; i++)
         {
-            bool dup = false;
-            for (int h = b; h < i && !dup; h++)
+            const int bank = addr[i] % per;
+            bool dup       = false;
+            for (int h = b; count[bank] && h < i && !dup; h++)
                 dup = addr[h] == addr[i];
             if (!dup)
-                worst = std::max(worst, ++count[addr[i] % per]);
+                worst = std::max(worst, ++count[bank]);
         }
         extra += worst - 1;
     }
