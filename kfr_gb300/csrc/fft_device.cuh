@@ -686,8 +686,12 @@ __device__ __forceinline__ void io_pass(cpx<T> (&v)[EPT], const LD& ld, const MI
 #pragma unroll
             for (int r = 0; r < R; r++)
                 u[r] = ld(j + r * NBF);
-            if constexpr (NS > 1)
+            // two CTAs of up to 512 threads share an SM's registers: one table value per butterfly (k_c2c_reg, 4096
+            // signals of 8192 points: 135 us, 143 us with two); with one CTA of 1024 threads both cost the same
+            if constexpr (NS > 1 && TS > 512)
                 ct_twiddle<T, R, NS>(u, tw + TWOFF, j % NS);
+            else if constexpr (NS > 1)
+                twiddle_powers<T, R>(u, ldg(tw + TWOFF + j % NS));
             dft_codelet<T, R>(u);
 #pragma unroll
             for (int r = 0; r < R; r++)
