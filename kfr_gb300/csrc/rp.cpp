@@ -241,7 +241,7 @@ rp_desc rp_build(const std::vector<int>& radices, rp_layout layout, int S, int e
             set_layout(d, i, S, fl, pad);
             const int ta = tot * d.pass[i].nbf, tb = tot * d.pass[i + 1].nbf;
             int c = 0;
-            for (int w = 0; w < 3; w++)
+            for (int w = 0; w < 3 && (best_c < 0 || c < best_c); w++)
             {
                 const int fa = w * (ta / 3) / 32 * 32, fb = w * (tb / 3) / 32 * 32;
                 c += d.pass[i].radix * store_conflicts(d.pass[i], d.shift, elem, fa, ta);

@@ -321,6 +321,22 @@ struct splitter
 {
     int threads;
     std::map<std::pair<long long, int>, double> memo;
+    std::map<long long, double> least_memo;
+    // the least that cost(m) can be, from the radices and the tile's largest size alone; -1 if there is no tile
+    double least(long long m)
+    {
+        auto f = least_memo.find(m);
+        if (f != least_memo.end())
+            return f->second;
+        const auto rad = radices_of(m);
+        int S          = 16;
+        while (S > 1 && S * m > threads * kRpMaxRadix)
+            S /= 2;
+        double c = rad.empty() ? -1 : 12.0 * (16.0 / S - 1);
+        for (int r : rad)
+            c += rp_pass_cost(r);
+        return least_memo[m] = c;
+    }
     double cost(long long m, rp_layout layout)
     {
         const auto key = std::make_pair(m, int(layout));
@@ -342,9 +358,22 @@ struct splitter
     {
         double best       = -1;
         const long long t = (long long)threads * kRpMaxRadix;
+        // the cost of the most balanced split: planning the tiles of those that cannot reach it takes milliseconds
+        double bound = 1e30;
+        for (long long a = (long long)std::sqrt(double(n)); a >= 2 && n / a <= t; a--)
+            if (n % a == 0)
+            {
+                const double c = cost(a, RP_COLS), r = cost(n / a, RP_ROWS);
+                if (c >= 0 && r >= 0)
+                    bound = c + r;
+                break;
+            }
         for (long long a = 2; a <= t && a * 2 <= n; a++)
         {
             if (n % a || n / a > t)
+                continue;
+            const double la = least(a), lb = least(n / a);
+            if (la < 0 || lb < 0 || la + lb > (best >= 0 ? std::min(best, bound) : bound) + 1e-6)
                 continue;
             const double c = cost(a, RP_COLS), r = c < 0 ? -1 : cost(n / a, RP_ROWS);
             // of equal splits the most balanced
