@@ -1593,7 +1593,9 @@ real_engine<T>::real_engine(long long n) : n_(n), c_(n / 2), ceng_(n / 2)
         r[k]         = std::complex<T>(T(w.real()), T(w.imag()));
     }
     rtw_.upload(r.data(), r.size() * sizeof(std::complex<T>));
-    fused_ = ceng_.strategy() == complex_engine<T>::kind::smem;
+    // the fused kernels run every pass in place, the complex one all but the first and the last: a few hundred of the
+    // longest one-CTA lengths fit only the latter
+    fused_ = ceng_.strategy() == complex_engine<T>::kind::smem && block_program<T>::feasible(c_);
     if (fused_)
         prog_.build(int(c_), CT_REAL);
     typename complex_engine<T>::pair_view pv;
@@ -1888,7 +1890,7 @@ dct_engine<T>::dct_engine(long long n) : n_(n), ceng_(n)
         d[k]         = std::complex<T>(T(w.real()), T(-w.imag()));
     }
     dtw_.upload(d.data(), d.size() * sizeof(std::complex<T>));
-    fused_ = ceng_.strategy() == complex_engine<T>::kind::smem;
+    fused_ = ceng_.strategy() == complex_engine<T>::kind::smem && block_program<T>::feasible(n); // as real_engine
     if (fused_)
         prog_.build(int(n), CT_DCT);
     // Pipelined kernels (compile-time n, single precision): the most resident threads per SM with at least

@@ -1,0 +1,44 @@
+"""Real DFTs and DCTs of the longest one-CTA lengths, whose radices (7, 9, 11, 13 and the like) leave a thread few
+butterflies to hold, against numpy in double precision."""
+import numpy as np
+import pytest
+
+import kfr_gb300 as k
+from oracle.oracle import c32_tolerance, c64_tolerance, rel_rms
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,sfx", [(23100, "f32"), (24648, "f32"), (28160, "f32"), (32766, "f32"), (11880, "f64"),
+                                   (12384, "f64"), (14700, "f64")])
+def test_real(n, sfx):
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((3, n)).astype(np.float32 if sfx == "f32" else np.float64)
+    tol = (c32_tolerance if sfx == "f32" else c64_tolerance)(n)
+    plan = k.dft_plan_real(n, dtype=sfx)
+    xd = torch.from_numpy(x).cuda()
+    yd = torch.empty((3, n // 2 + 1), dtype=torch.complex64 if sfx == "f32" else torch.complex128, device="cuda")
+    plan.execute_batch(yd, xd, 3)
+    assert rel_rms(yd.cpu().numpy(), np.fft.rfft(x.astype(np.float64))) <= tol
+    plan.execute_batch(xd, yd, 3, inverse=True)
+    assert rel_rms(xd.cpu().numpy() / n, x.astype(np.float64)) <= 2 * tol
+
+
+@pytest.mark.parametrize("n,sfx", [(11880, "f32"), (12324, "f32"), (12375, "f32"), (16128, "f32"), (5676, "f64"),
+                                   (6192, "f64"), (8181, "f64")])
+def test_dct(n, sfx):
+    rng = np.random.default_rng(n)
+    x = rng.uniform(-1, 1, (3, n)).astype(np.float32 if sfx == "f32" else np.float64)
+    x64 = x.astype(np.float64)
+    tol = (c32_tolerance if sfx == "f32" else c64_tolerance)(n)
+    j, ks = np.arange(n), np.unique(rng.integers(0, n, 300))
+    plan = k.dct_plan(n, sfx)
+    xd = torch.from_numpy(x).cuda()
+    yd = torch.empty_like(xd)
+    plan.execute_batch(yd, xd, 3)
+    assert rel_rms(yd.cpu().numpy()[:, ks], x64 @ np.cos(np.pi * np.outer(2 * j + 1, ks) / (2 * n))) <= tol
+    w = x64.copy()
+    w[:, 0] *= 0.5
+    plan.execute_batch(yd, xd, 3, inverse=True)
+    assert rel_rms(yd.cpu().numpy()[:, ks], w @ np.cos(np.pi * np.outer(j, 2 * ks + 1) / (2 * n))) <= tol

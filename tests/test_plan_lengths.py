@@ -1,0 +1,34 @@
+"""Plans built on the CPU against stubs of the CUDA calls (tests/cpp/cuda_stub.cpp): which lengths and sizes they take."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "kfr_gb300", "csrc")
+CUDA = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
+
+
+def compile_test(tmp, name, *sources):
+    if not shutil.which("g++"):
+        pytest.skip("no g++")
+    exe = str(tmp / name)
+    cpp = os.path.join(ROOT, "tests", "cpp")
+    subprocess.run(["g++", "-std=c++17", "-O2", "-I", CUDA, "-I", CSRC, "-Wl,--unresolved-symbols=ignore-all",
+                    os.path.join(cpp, name + ".cpp"), os.path.join(cpp, "cuda_stub.cpp")] +
+                   [os.path.join(CSRC, s) for s in sources] + ["-o", exe], check=True)
+    return exe
+
+
+@pytest.fixture(scope="module")
+def plans(tmp_path_factory):
+    return compile_test(tmp_path_factory.mktemp("plans"), "test_plan_lengths", "plan.cpp", "rp.cpp")
+
+
+# every short length, and the longest ones that one CTA transforms
+@pytest.mark.parametrize("precision,lo,hi", [("f", 1, 2000), ("f", 11000, 17000), ("f", 20000, 20600), ("d", 1, 2000),
+                                             ("d", 5500, 8500), ("d", 10000, 10300)])
+def test_every_length_plans(plans, precision, lo, hi):
+    r = subprocess.run([plans, precision, str(lo), str(hi)], capture_output=True, text=True)
+    assert r.returncode == 0 and r.stdout.strip().endswith("ok"), r.stdout[-2000:]
