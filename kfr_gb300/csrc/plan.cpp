@@ -282,6 +282,16 @@ bool is_smooth(long long n)
     return n <= 1;
 }
 
+// Largest prime factor of a product of primes up to kGenericMax.
+static int largest_prime(long long n)
+{
+    int last = 1;
+    for (int p = 2; p <= kGenericMax && n > 1; p++)
+        for (; n % p == 0; n /= p)
+            last = p;
+    return last;
+}
+
 int smem_budget()
 {
     // dynamic shared memory less a small reserve
@@ -326,15 +336,17 @@ template bool ct_lookup<double>(int, int, int&, std::vector<int>&);
 // block_program
 // ------------------------------------------------------------------------------------------------------
 
-// Radices of n (prime factors up to kGenericMax) for a one-CTA transform and the values its threads hold; empty if it
-// does not fit.  Threads hold 16 values, 32 where only that fits.
+// Radices of n (prime factors up to kGenericMax) for a tile of columns or rows (smem_io false: the first and the last
+// pass hold nothing) and the values its threads hold; empty if not even one fits.  Threads hold 16 values, 32 where only
+// that fits.
 template <typename T>
-static std::vector<int> one_cta_radices(long long n, bool smem_io, int& hold)
+static std::vector<int> tile_radices(long long n, bool smem_io, int& hold)
 {
+    constexpr int elem = int(2 * sizeof(T));
     for (int h : { kRpHold, kRpLongHold })
     {
         const auto rad = rp_radices(n, kGenericMax, h);
-        if (rp_fits(rad, int(2 * sizeof(T)), smem_budget(), smem_io, h))
+        if (rp_fits(rad, elem, smem_budget(), smem_io, h))
         {
             hold = h;
             return rad;
@@ -343,11 +355,39 @@ static std::vector<int> one_cta_radices(long long n, bool smem_io, int& hold)
     return {};
 }
 
+// Whether one CTA transforms n points: the plain radices fit with every pass in place (16 or 32 values per thread).
+// Longer lengths for which only a choice of other radices, or an end that holds nothing, would fit take the four-step's
+// two kernels: with 1 or 16 signals of 11000 to 16000 points a CTA each takes 1.3 to 2.5 times as long as the four-step
+// spread over the SMs, from 150 signals on 0.8 times as long.
+template <typename T>
+static bool one_cta(long long n)
+{
+    const auto rad = rp_plain_radices(n, kGenericMax);
+    return rp_fits(rad, int(2 * sizeof(T)), smem_budget(), true, kRpHold) ||
+           rp_fits(rad, int(2 * sizeof(T)), smem_budget(), true, kRpLongHold);
+}
+
+// Radices of a one-CTA transform of contiguous signals (smem_io: every pass in place) and the values its threads hold:
+// the fastest if they fit, otherwise those that do with every pass in place; empty beyond one CTA.
+template <typename T>
+static std::vector<int> one_cta_radices(long long n, bool smem_io, int& hold)
+{
+    if (!one_cta<T>(n))
+        return {};
+    auto rad = tile_radices<T>(n, smem_io, hold);
+    for (int h : { kRpHold, kRpLongHold })
+        if (rad.empty())
+        {
+            rad  = rp_radices_held(n, kGenericMax, int(2 * sizeof(T)), smem_budget(), h);
+            hold = h;
+        }
+    return rad;
+}
+
 template <typename T>
 bool block_program<T>::feasible(long long n)
 {
-    int hold = 0;
-    return !one_cta_radices<T>(n, true, hold).empty();
+    return one_cta<T>(n);
 }
 
 template <typename T>
@@ -468,8 +508,7 @@ std::string block_program<T>::describe() const
 template <typename T>
 bool rp_program<T>::feasible(long long n)
 {
-    int hold = 0;
-    return !one_cta_radices<T>(n, false, hold).empty();
+    return one_cta<T>(n);
 }
 
 template <typename T>
@@ -478,7 +517,7 @@ bool rp_program<T>::build(long long n, rp_layout lay)
     layout           = lay;
     const int budget = smem_budget();
     int hold         = 0;
-    const auto rad   = one_cta_radices<T>(n, false, hold);
+    const auto rad   = lay == RP_SIGNALS ? one_cta_radices<T>(n, false, hold) : tile_radices<T>(n, false, hold);
     if (rad.empty())
         return false;
     if (lay == RP_SIGNALS)
@@ -640,7 +679,7 @@ bool rp_fourstep<T>::build(long long length)
     const auto cost    = [&](long long m) -> double
     {
         int hold       = 0;
-        const auto rad = one_cta_radices<T>(m, false, hold);
+        const auto rad = tile_radices<T>(m, false, hold);
         if (rad.empty())
             return -1;
         const int S = rp_tile(rad, elem, smem_budget(), hold);
@@ -800,6 +839,16 @@ static double fft_cost(long long n)
     return double(n) * c;
 }
 
+// The same in passes over n values, a dot product of R terms counting R / 4.
+static double fft_passes(long long n)
+{
+    const auto rad = rp_plain_radices(n, kGenericMax);
+    double c       = 0;
+    for (int r : rad)
+        c += r > 13 && r != 16 ? r / 4.0 : 1.0;
+    return rad.empty() ? 1e30 : double(n) * c;
+}
+
 // Twiddles of the radix-16 passes of an L-point tensor-core block FFT (L = 16^p): the pass with stride
 // ns > 1 holds W_{16 ns}^{r k} at (r - 1) ns + k (r = 1..15, k < ns), passes in order.
 static std::vector<std::complex<float>> tc_pass_twiddles(int L)
@@ -888,16 +937,22 @@ complex_engine<T>::complex_engine(long long n) : n_(n)
     long long m = 1;
     while (m < 2 * n - 1)
         m <<= 1;
-    const bool direct_ok    = rp_program<T>::feasible(n);
-    const bool rader_ok     = is_prime(n) && n > 13 && block_program<T>::feasible(n - 1);
-    const bool bluestein_ok = !direct_ok && !rader_ok ? block_program<T>::feasible(m) : m <= (1 << 14);
-    const double c_direct   = direct_ok ? fft_cost(n) : 1e30;
+    int hold                = 0;
+    const bool direct_ok    = one_cta<T>(n);
+    const bool rader_fits   = is_prime(n) && n > 13 && one_cta<T>(n - 1);
+    const bool rader_ok     = rader_fits && !tile_radices<T>(n - 1, true, hold).empty();
+    const bool bluestein_ok = one_cta<T>(m);
     const double c_rader    = rader_ok ? 2.0 * fft_cost(n - 1) + 40.0 * n : 1e30;
-    // (a direct plan with only codelet radices is always the cheapest)
-    const double c_blue = bluestein_ok && c_direct > 200.0 * n && block_program<T>::feasible(m)
-                              ? 2.0 * fft_cost(m) + 60.0 * n
-                              : 1e30;
-    if (direct_ok && c_direct <= c_rader && c_direct <= c_blue)
+    const double c_blue     = bluestein_ok ? 2.0 * fft_cost(m) + 60.0 * n : 1e30;
+    // Dot products of a prime's terms round less than the two transforms of a convolution, so they give way where they
+    // are more passes (a prime of about 40 on), and in single precision, where their error grows past the
+    // convolution's, from 67 on where they are more instructions: relative RMS of a convolution to that of the dot
+    // products 0.7 to 1.03 there, 1.05 to 1.3 from 17 to 61; in double precision 1.1 to 2.2 up to 109.
+    bool direct = direct_ok && fft_passes(n) <= std::min(rader_ok ? 2 * fft_passes(n - 1) + 2.0 * n : 1e30,
+                                                         bluestein_ok ? 2 * fft_passes(m) + 3.0 * n : 1e30);
+    if (direct && sizeof(T) == 4 && largest_prime(n) >= 67)
+        direct = fft_cost(n) <= std::min(c_rader, c_blue);
+    if (direct)
     {
         k_ = kind::smem;
         int ts = 0;
@@ -915,7 +970,7 @@ complex_engine<T>::complex_engine(long long n) : n_(n)
         }
         return;
     }
-    if (rader_ok && c_rader <= c_blue && c_rader <= c_direct)
+    if (rader_ok && c_rader <= c_blue)
     {
         init_rader(n);
         return;

@@ -155,17 +155,37 @@ void set_layout(rp_desc& d, int i, int S, bool fast_layout, int pad)
 
 } // namespace
 
-std::vector<int> rp_radices(long long n, int largest, int hold)
+// Takes the primes of 17 to `largest` out of n.
+static std::vector<int> take_primes(long long& n, int largest)
 {
-    std::vector<int> r, primes;
-    if (n < 2 || n > (1 << 16))
-        return {};
+    std::vector<int> primes;
     for (int p : { 17, 19, 23, 29, 31, 37, 41, 43, 47, 53, 59, 61, 67, 71, 73, 79, 83, 89, 97, 101, 103, 107, 109, 113, 127 })
         while (p <= largest && n % p == 0)
         {
             primes.push_back(p);
             n /= p;
         }
+    return primes;
+}
+
+// The codelet radices r with the primes between their ends (of radix 1, a copy, where there are fewer than two), empty
+// if those are too many passes.
+static std::vector<int> with_primes(std::vector<int> r, const std::vector<int>& primes)
+{
+    if (primes.empty())
+        return r;
+    while (r.size() < 2)
+        r.push_back(1);
+    r.insert(r.begin() + 1, primes.begin(), primes.end());
+    return r.size() > size_t(kRpMaxPasses) ? std::vector<int>{} : r;
+}
+
+std::vector<int> rp_radices(long long n, int largest, int hold)
+{
+    if (n < 2 || n > (1 << 16))
+        return {};
+    std::vector<int> r;
+    const auto primes = take_primes(n, largest);
     std::vector<int> cur;
     double best = 1e30;
     splits(n, kRpMaxRadix, 0, cur, best,
@@ -185,17 +205,38 @@ std::vector<int> rp_radices(long long n, int largest, int hold)
                    r    = o;
                }
            });
-    if (best >= 1e30)
+    return best >= 1e30 ? std::vector<int>{} : with_primes(r, primes);
+}
+
+std::vector<int> rp_plain_radices(long long n, int largest)
+{
+    std::vector<int> r;
+    for (int p : { 16, 8, 4, 2, 9, 3, 5, 7, 11, 13 })
+        for (; n > 1 && n % p == 0; n /= p)
+            r.push_back(p);
+    for (int p : take_primes(n, largest))
+        r.push_back(p);
+    return n == 1 ? r : std::vector<int>{};
+}
+
+std::vector<int> rp_radices_held(long long n, int largest, int elem, int smem_budget, int hold)
+{
+    if (n < 2 || n > (1 << 16))
         return {};
-    if (!primes.empty())
-    {
-        // a codelet pass at either end, the primes in between
-        while (r.size() < 2)
-            r.push_back(1);
-        r.insert(r.begin() + 1, primes.begin(), primes.end());
-        if (r.size() > size_t(kRpMaxPasses))
-            return {};
-    }
+    std::vector<int> r;
+    const auto primes = take_primes(n, largest);
+    std::vector<int> cur;
+    double best = 1e30;
+    splits(n, kRpMaxRadix, 0, cur, best,
+           [&](const std::vector<int>& s, double c)
+           {
+               const auto o = with_primes(pass_order(s), primes);
+               if (c < best && rp_fits(o, elem, smem_budget, true, hold))
+               {
+                   best = c;
+                   r    = o;
+               }
+           });
     return r;
 }
 

@@ -75,10 +75,18 @@ enum rp_layout
     RP_ROWS,    // read as contiguous signals, written with the S signals on consecutive threads
 };
 
-// Radices of n in pass order for threads that hold `hold` values, empty when n has a prime factor above `largest` (13, or up to 127) or needs too
-// many passes.  Primes above 13 run as in-place passes of dot products between codelet passes (of radix 1, a
+// Radices of n in pass order for threads that hold `hold` values, empty when n has a prime factor above `largest` (13,
+// or up to 127) or needs too many passes.  Primes above 13 run as in-place passes of dot products between codelet passes (of radix 1, a
 // copy, where no other factor is left).
 std::vector<int> rp_radices(long long n, int largest = 13, int hold = kRpHold);
+
+// n as 16 16 .. 8, 4 or 2, then 9s, 3, 5s, 7s, 11s, 13s and the primes up to `largest`; empty if it has a larger one.
+std::vector<int> rp_plain_radices(long long n, int largest);
+
+// The cheapest radices whose passes all fit a CTA in place (rp_fits with smem_io), empty if none do.  Near the longest
+// one-CTA lengths a thread has room for one butterfly of radix 9 to 15 only, so that the radices that would be fastest
+// (rp_radices) need more threads than a CTA has.
+std::vector<int> rp_radices_held(long long n, int largest, int elem, int smem_budget, int hold);
 
 // Descriptor of the radices over a tile.  elem: bytes of a complex value; S (a power of two): signals per tile
 // of RP_COLS and RP_ROWS.  smem_io: the first pass reads and the last pass writes shared memory too, element

@@ -10,6 +10,20 @@ torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
 
+# dot products for small primes, the cheapest radices that fit near the longest one-CTA lengths
+@pytest.mark.parametrize("n,batch,sfx", [(58, 1000, "f32"), (946, 70, "f32"), (8177, 3, "f32"), (12312, 5, "f32"),
+                                         (14880, 2, "f32"), (13851, 3, "f32"), (12433, 3, "f32"), (19, 1000, "f64"),
+                                         (31, 300, "f64"), (6384, 3, "f64"), (7200, 3, "f64"), (7039, 2, "f64")])
+def test_complex(n, batch, sfx):
+    rng = np.random.default_rng(n)
+    cdt = np.complex64 if sfx == "f32" else np.complex128
+    x = (rng.uniform(-1, 1, (batch, n)) + 1j * rng.uniform(-1, 1, (batch, n))).astype(cdt)
+    xd = torch.from_numpy(x).cuda()
+    yd = torch.empty_like(xd)
+    k.dft_plan(n, sfx).execute_batch(yd, xd, batch)
+    assert rel_rms(yd.cpu().numpy(), np.fft.fft(x.astype(np.complex128))) <= (c32_tolerance if sfx == "f32" else c64_tolerance)(n)
+
+
 @pytest.mark.parametrize("n,sfx", [(23100, "f32"), (24648, "f32"), (28160, "f32"), (32766, "f32"), (11880, "f64"),
                                    (12384, "f64"), (14700, "f64")])
 def test_real(n, sfx):

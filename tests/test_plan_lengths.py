@@ -32,3 +32,16 @@ def plans(tmp_path_factory):
 def test_every_length_plans(plans, precision, lo, hi):
     r = subprocess.run([plans, precision, str(lo), str(hi)], capture_output=True, text=True)
     assert r.returncode == 0 and r.stdout.strip().endswith("ok"), r.stdout[-2000:]
+
+
+# dot products where a convolution would round more, one CTA where the plain radices fit in place, the four-step or
+# Bluestein's multi-kernel transform beyond
+@pytest.mark.parametrize("precision,strategy,lengths", [
+    ("sf", "direct", [13, 19, 23, 31, 58, 62, 124, 946, 1955, 8177, 12000, 12312, 14880, 16384]),
+    ("sf", "bluestein", [142, 149, 8178]), ("sf", "fourstep", [11297, 11550, 11880, 13851, 14400, 16383, 16385]),
+    ("sf", "rader", [137, 7561, 8641]), ("sf", "multi", [12433, 13933, 14401, 15319]),
+    ("sd", "direct", [19, 23, 31, 56, 946, 2140, 3268, 6144, 6384, 8192]), ("sd", "bluestein", [149]),
+    ("sd", "fourstep", [5676, 7056, 7200, 8099]), ("sd", "multi", [6217, 7039, 7057])])
+def test_strategy(plans, precision, strategy, lengths):
+    r = subprocess.run([plans, precision] + [str(n) for n in lengths], capture_output=True, text=True, check=True)
+    assert dict(zip(lengths, r.stdout.split())) == {n: strategy for n in lengths}
