@@ -152,26 +152,26 @@ __host__ __device__ constexpr double odd_cos(int R, int k)
         return 1.0;
     switch (R * 32 + k)
     {
-    case 3 * 32 + 1: return -0.4999999999999998;
+    case 3 * 32 + 1: return -0.5;
     case 5 * 32 + 1: return 0.30901699437494745;
-    case 5 * 32 + 2: return -0.8090169943749473;
-    case 7 * 32 + 1: return 0.6234898018587336;
-    case 7 * 32 + 2: return -0.22252093395631434;
-    case 7 * 32 + 3: return -0.900968867902419;
+    case 5 * 32 + 2: return -0.8090169943749475;
+    case 7 * 32 + 1: return 0.6234898018587335;
+    case 7 * 32 + 2: return -0.2225209339563144;
+    case 7 * 32 + 3: return -0.9009688679024191;
     case 9 * 32 + 1: return 0.766044443118978;
-    case 9 * 32 + 2: return 0.17364817766693041;
-    case 9 * 32 + 3: return -0.4999999999999998;
-    case 9 * 32 + 4: return -0.9396926207859083;
+    case 9 * 32 + 2: return 0.17364817766693036;
+    case 9 * 32 + 3: return -0.5;
+    case 9 * 32 + 4: return -0.9396926207859084;
     case 11 * 32 + 1: return 0.8412535328311812;
     case 11 * 32 + 2: return 0.41541501300188644;
-    case 11 * 32 + 3: return -0.142314838273285;
-    case 11 * 32 + 4: return -0.654860733945285;
+    case 11 * 32 + 3: return -0.14231483827328514;
+    case 11 * 32 + 4: return -0.6548607339452851;
     case 11 * 32 + 5: return -0.9594929736144974;
     case 13 * 32 + 1: return 0.8854560256532099;
-    case 13 * 32 + 2: return 0.5680647467311559;
-    case 13 * 32 + 3: return 0.120536680255323;
-    case 13 * 32 + 4: return -0.35460488704253545;
-    case 13 * 32 + 5: return -0.7485107481711012;
+    case 13 * 32 + 2: return 0.5680647467311558;
+    case 13 * 32 + 3: return 0.12053668025532305;
+    case 13 * 32 + 4: return -0.3546048870425356;
+    case 13 * 32 + 5: return -0.7485107481711011;
     case 13 * 32 + 6: return -0.970941817426052;
     default: return 0.0;
     }
@@ -180,27 +180,27 @@ __host__ __device__ constexpr double odd_sin(int R, int k)
 {
     switch (R * 32 + k)
     {
-    case 3 * 32 + 1: return 0.8660254037844387;
+    case 3 * 32 + 1: return 0.8660254037844386;
     case 5 * 32 + 1: return 0.9510565162951535;
-    case 5 * 32 + 2: return 0.5877852522924732;
+    case 5 * 32 + 2: return 0.5877852522924731;
     case 7 * 32 + 1: return 0.7818314824680298;
     case 7 * 32 + 2: return 0.9749279121818236;
-    case 7 * 32 + 3: return 0.43388373911755823;
-    case 9 * 32 + 1: return 0.6427876096865393;
+    case 7 * 32 + 3: return 0.4338837391175581;
+    case 9 * 32 + 1: return 0.6427876096865394;
     case 9 * 32 + 2: return 0.984807753012208;
-    case 9 * 32 + 3: return 0.8660254037844387;
-    case 9 * 32 + 4: return 0.3420201433256689;
+    case 9 * 32 + 3: return 0.8660254037844386;
+    case 9 * 32 + 4: return 0.3420201433256687;
     case 11 * 32 + 1: return 0.5406408174555976;
     case 11 * 32 + 2: return 0.9096319953545183;
-    case 11 * 32 + 3: return 0.9898214418809328;
+    case 11 * 32 + 3: return 0.9898214418809327;
     case 11 * 32 + 4: return 0.7557495743542583;
     case 11 * 32 + 5: return 0.28173255684142967;
-    case 13 * 32 + 1: return 0.4647231720437685;
+    case 13 * 32 + 1: return 0.46472317204376856;
     case 13 * 32 + 2: return 0.8229838658936564;
     case 13 * 32 + 3: return 0.992708874098054;
     case 13 * 32 + 4: return 0.9350162426854148;
     case 13 * 32 + 5: return 0.6631226582407952;
-    case 13 * 32 + 6: return 0.23931566428755768;
+    case 13 * 32 + 6: return 0.23931566428755777;
     default: return 0.0;
     }
 }
