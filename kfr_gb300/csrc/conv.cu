@@ -62,6 +62,68 @@ struct conv_rp
     }
 };
 
+// The same for blocks of F = 2048 and 4096 samples, with a compile-time transform whose twiddles all come from the table
+// (conv_rp's powers of two table values round more: 1.34 times the relative RMS error at F = 2048, 1.27 times at 4096).
+// 64 channels of 2^20 samples through 513 taps: 373 us with conv_rp from the table, 340 with this one.
+template <int N, int TS, int... Rs>
+struct conv_ct
+{
+    using real                       = float;
+    static constexpr int max_threads = ct_fft<float, N, TS, Rs...>::max_threads;
+    cpx<float>* buf;
+    const cpx<float>* tw;
+    __device__ __forceinline__ conv_ct(cpx<float>* b, const void* t, const conv_fft&)
+        : buf(b), tw(reinterpret_cast<const cpx<float>*>(t))
+    {
+    }
+    static __device__ __forceinline__ int n() { return N; }
+    static __device__ __forceinline__ int pos(int i) { return ct_fft<float, N, TS, Rs...>::pi(i); }
+    __device__ __forceinline__ void run() const
+    {
+        // TS threads, all of them with butterflies (the mask tells the compiler: values that look conditional count as
+        // live around the loop of k_fir_bwd, which then spills)
+        static_assert((TS & (TS - 1)) == 0 && N % (16 * TS) == 0, "whole butterflies per thread");
+        cpx<float> v[ct_ept<N, TS, Rs...>()];
+        ct_passes<float, N, TS, ct_ept<N, TS, Rs...>(), 1, 0, Rs...>(v, buf, tw, int(threadIdx.x) & (TS - 1));
+    }
+    template <class LD>
+    __device__ __forceinline__ void to_smem(const LD& ld) const
+    {
+        for (int i = threadIdx.x; i < N; i += blockDim.x)
+            buf[pos(i)] = ld(i);
+        __syncthreads();
+        run();
+    }
+    template <class ST>
+    __device__ __forceinline__ void from_smem(const ST& st) const
+    {
+        run();
+        for (int k = threadIdx.x; k < N; k += blockDim.x)
+            st(k, buf[pos(k)]);
+    }
+};
+
+// GO(P) with the block FFT of f.
+#define KFR_GPU_CONV_CT_CASE(N, TS, ...)                                                                   \
+    case N: return go(conv_tag<conv_ct<N, TS, __VA_ARGS__>>{});
+template <class P>
+struct conv_tag
+{
+    using type = P;
+};
+template <typename T, class GO>
+static auto conv_dispatch(const conv_fft& f, const GO& go)
+{
+    if constexpr (std::is_same<T, float>::value)
+        switch (f.ct)
+        {
+            KFR_CT_CONV_F32(KFR_GPU_CONV_CT_CASE)
+        default: break;
+        }
+    return go(conv_tag<conv_rp<T>>{});
+}
+#undef KFR_GPU_CONV_CT_CASE
+
 // Reals (x[i], x[i + 1]) of the n reals at x, zero outside; pairs: even i are 8-byte (16-byte) aligned.
 template <typename T>
 __device__ __forceinline__ cpx<T> real_pair(const T* x, long long i, long long n, bool pairs)
@@ -172,7 +234,7 @@ __global__ void __launch_bounds__(P::max_threads, 1)
 // its own sum in shared memory (every bin owned by one thread); k_fir_reduce adds them in a fixed order and
 // k_fir_taps transforms the sum back.  Bound by instruction issue (three c-point FFTs per block).  64 channels
 // of 2^20 samples, 1023 taps, forward and both gradients: 6397 -> 869 us against reversed copies through the
-// filter and real DFTs of 2^21 points per channel; 642 us with the paired blocks below.
+// filter and real DFTs of 2^21 points per channel; 664 us with the paired blocks below.
 // ---------------------------------------------------------------------------------------------------
 template <class P>
 __global__ void __launch_bounds__(P::max_threads, 1)
@@ -382,12 +444,13 @@ __global__ void __launch_bounds__(64) k_fir_spec_outer(cpx<T>* H, const double2*
 }
 
 // ---------------------------------------------------------------------------------------------------
-// Single precision, up to kConv16Overlap samples of overlap: two output blocks of a channel as the real and the
-// imaginary part of one 4096-point transform (conv16.cuh).  The taps are real, so the product with their spectrum
-// filters both, with no split or merge, and it happens in registers between the last forward and the first inverse
-// pass.  Bound by instruction issue (about 115 instructions per complex value) and the latency of the first loads.  64
-// channels of 2^20 samples, 1023 taps: 277 -> 241 us against one block of 8192 samples through a 4096-point transform
-// with split and merge; the gradients 566 -> 367 us.
+// Single precision, where a block would be 8192 samples or more and the overlap is at most half of 4096 (conv_paired): two
+// output blocks of a channel as the real and the imaginary part of one 4096-point transform (conv16.cuh).  The taps are
+// real, so the product with their spectrum filters both, with no split or merge, and it happens in registers between the
+// last forward and the first inverse pass.  Bound by instruction issue, the twiddles' loads (all from the table; with 80
+// registers for three CTAs per SM they spill, 283 us) and the latency of the first loads.  64 channels of 2^20 samples,
+// 1023 taps: 370 us with one block of 8192 samples through a compile-time 4096-point transform, 250 us so; with powers of
+// two table values 226 us, but 1.2 times the relative RMS error of the former (from the table 0.95 times).
 // ---------------------------------------------------------------------------------------------------
 __device__ __forceinline__ float conv_sample(const float* in, const float* hist, long long i, long long n, long long nhist)
 {
@@ -396,7 +459,7 @@ __device__ __forceinline__ float conv_sample(const float* in, const float* hist,
     return i + nhist >= 0 ? hist[i + nhist] : 0.0f; // the latest sample before the call at hist[nhist - 1]
 }
 
-__global__ void __launch_bounds__(fft16::threads, 3) k_conv16(const __grid_constant__ conv_args a)
+__global__ void __launch_bounds__(fft16::threads, 2) k_conv16(const __grid_constant__ conv_args a)
 {
     stream_order();
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -602,8 +665,13 @@ cudaError_t launch_conv_os(const conv_args& a, long long nblocks, cudaStream_t s
         if (a.fft.paired)
             return conv_go(k_conv16, dim3(unsigned((nblocks + 1) / 2), unsigned(a.channels)), fft16::threads,
                            fft16::elems * sizeof(cpx<float>), st, a);
-    return conv_go(k_conv_os<conv_rp<T>>, dim3(unsigned(nblocks), unsigned(a.channels)), a.fft.threads,
-                   size_t(a.fft.elems) * 2 * sizeof(T), st, a);
+    return conv_dispatch<T>(a.fft,
+                            [&](auto p)
+                            {
+                                return conv_go(k_conv_os<typename decltype(p)::type>,
+                                               dim3(unsigned(nblocks), unsigned(a.channels)), a.fft.threads,
+                                               size_t(a.fft.elems) * 2 * sizeof(T), st, a);
+                            });
 }
 
 template <typename T>
@@ -647,11 +715,25 @@ fir_tables<T>::fir_tables(size_t f, bool paired)
         tw.upload(t.data(), t.size() * sizeof(t[0]));
         return;
     }
-    const int c    = int(f / 2);
-    const auto rad = rp_radices(c);
-    fft.rp         = rp_build(rad, RP_SIGNALS, 1, int(2 * sizeof(T)), true);
-    fft.elems      = (fft.rp.elems + 1) / 2 * 2;
-    fft.threads    = (std::max(rp_threads_needed(fft.rp, 1, true), std::min(c, 64)) + 31) / 32 * 32;
+    const int c = int(f / 2);
+    std::vector<int> rad;
+#define KFR_GPU_CONV_CT_OF(N, TS, ...)                                                                     \
+    if (sizeof(T) == 4 && c == N)                                                                          \
+    {                                                                                                      \
+        rad         = { __VA_ARGS__ };                                                                     \
+        fft.ct      = N;                                                                                   \
+        fft.threads = TS;                                                                                  \
+        fft.elems   = (ct_group_stride_f32(N, TS) + 1) / 2 * 2;                                            \
+    }
+    KFR_CT_CONV_F32(KFR_GPU_CONV_CT_OF)
+#undef KFR_GPU_CONV_CT_OF
+    if (!fft.ct)
+    {
+        rad         = rp_radices(c);
+        fft.rp      = rp_build(rad, RP_SIGNALS, 1, int(2 * sizeof(T)), true);
+        fft.elems   = (fft.rp.elems + 1) / 2 * 2;
+        fft.threads = (std::max(rp_threads_needed(fft.rp, 1, true), std::min(c, 64)) + 31) / 32 * 32;
+    }
     const auto t = pass_twiddles<T>(rad);
     tw.upload(t.data(), t.size() * sizeof(t[0]));
     std::vector<std::complex<T>> rt(c + 1);
@@ -675,22 +757,29 @@ void fir_tables<T>::roots64(size_t f)
 template struct fir_tables<float>;
 template struct fir_tables<double>;
 
-// Whether blocks with an overlap of m1 samples run in pairs through 4096-point transforms: up to half of a block re-reads
-// the overlap, where the self-sorting transforms of 16384 samples (next_pow2(8 m1)) begin to need fewer instructions.
+// Samples of a block for an overlap of m1 samples: at least 8 times it (at most 1/8 of each block re-reads the overlap;
+// measured 0.390 -> 0.374 ms against 4x for 64 channels of 2^20 samples and 1023 taps) and twice the caller's block.
 template <typename T>
-static bool conv_paired(size_t m1)
+static size_t conv_block_size(size_t m1, size_t block)
 {
-    return sizeof(T) == 4 && m1 <= fft16::N / 2;
+    return std::min(std::max({ next_pow2(8 * m1), 2 * next_pow2(block ? block : 1024), size_t(64) }), conv_fft_max<T>());
 }
 
-// FFT length for an overlap of m1 samples: at least 8 times it (at most 1/8 of each block re-reads the overlap;
-// measured 0.390 -> 0.374 ms against 4x for 64 channels of 2^20 samples and 1023 taps) and twice the block.
+// Whether blocks run in pairs through 4096-point transforms.  Up to half of a pair's block re-reads the overlap, where the
+// self-sorting transforms of 16384 samples begin to need fewer instructions.  Below blocks of 8192 samples a pair would be
+// longer than the block it replaces: its rounding errors are larger (F = 2048: 1.7e-7 -> 2.3e-7 relative RMS) and a sample
+// that is infinite or very loud reaches more outputs (2 (4096 - m1) instead of F - m1).
+template <typename T>
+static bool conv_paired(size_t m1, size_t block)
+{
+    return sizeof(T) == 4 && m1 <= fft16::N / 2 && conv_block_size<T>(m1, block) >= 2 * fft16::N;
+}
+
+// FFT length for an overlap of m1 samples.
 template <typename T>
 static size_t conv_fft_size(size_t m1, size_t block)
 {
-    if (conv_paired<T>(m1))
-        return fft16::N;
-    return std::min(std::max({ next_pow2(8 * m1), 2 * next_pow2(block ? block : 1024), size_t(64) }), conv_fft_max<T>());
+    return conv_paired<T>(m1, block) ? size_t(fft16::N) : conv_block_size<T>(m1, block);
 }
 
 template <typename T>
@@ -716,7 +805,7 @@ conv_filter<T>::conv_filter(const T* taps, size_t ntaps, size_t block_size, int 
     const size_t hb = std::max<size_t>(1, m1 * size_t(channels)) * sizeof(T);
     hist_[0].alloc(hb);
     hist_[1].alloc(hb);
-    if (m1 >= f / 2 && !conv_paired<T>(m1))
+    if (m1 >= f / 2 && !conv_paired<T>(m1, block_size))
     {
         // long mode: the taps stay on the device for whole-call convolutions
         long_ = true;
@@ -727,7 +816,7 @@ conv_filter<T>::conv_filter(const T* taps, size_t ntaps, size_t block_size, int 
     }
     f_  = f;
     c_  = f / 2;
-    const bool paired = conv_paired<T>(m1);
+    const bool paired = conv_paired<T>(m1, block_size);
     bo_ = paired ? f - m1 : f - (m1 + 1) / 2 * 2; // unpaired blocks start at even samples
     tables_.reset(new fir_tables<T>(f, paired));
     // taps spectrum FFT_F(h padded) / F, bins 0..c (set_data, src/dft/convolution-impl.cpp:53-71)
@@ -826,7 +915,7 @@ bool fir_backward_blocks(const T* taps, long long ntaps, long long channels, lon
                          T* grad_x, T* grad_h, cudaStream_t st)
 {
     const size_t m1 = size_t(ntaps - 1);
-    const bool paired = conv_paired<T>(m1);
+    const bool paired = conv_paired<T>(m1, 1024);
     // the gradient kernel holds two spectra and a sum: half the one-CTA length
     const size_t f = std::min(conv_fft_size<T>(m1, 1024), conv_fft_max<T>() / 2);
     if (m1 >= f / 2 && !paired)
@@ -853,7 +942,8 @@ bool fir_backward_blocks(const T* taps, long long ntaps, long long channels, lon
     int Q = 1;
     while (Q * Q < int(f))
         Q <<= 1;
-    const void* kernel = reinterpret_cast<const void*>(k_fir_bwd<conv_rp<T>>);
+    const auto bwd = conv_dispatch<T>(a.fft, [](auto p) { return &k_fir_bwd<typename decltype(p)::type>; });
+    const void* kernel = reinterpret_cast<const void*>(bwd);
     if constexpr (std::is_same<T, float>::value)
         if (paired)
             kernel = reinterpret_cast<const void*>(k_fir16_bwd);
@@ -912,11 +1002,11 @@ bool fir_backward_blocks(const T* taps, long long ntaps, long long channels, lon
     }
     else
     {
-        check(conv_go(k_fir_bwd<conv_rp<T>>, dim3(unsigned(grid)), threads, smem, st, a), "launch FIR backward");
+        check(conv_go(bwd, dim3(unsigned(grid)), threads, smem, st, a), "launch FIR backward");
         if (grad_h)
         {
             reduce();
-            check(conv_go(k_fir_taps<conv_rp<T>>, dim3(1), threads, size_t(a.elems) * cpx_b, st, a,
+            check(conv_go(conv_dispatch<T>(a.fft, [](auto p) { return &k_fir_taps<typename decltype(p)::type>; }), dim3(1), threads, size_t(a.elems) * cpx_b, st, a,
                           static_cast<void*>(grad_h), static_cast<const void*>(sum), int(ntaps)),
                   "launch FIR backward (taps)");
         }

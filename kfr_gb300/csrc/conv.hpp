@@ -5,10 +5,12 @@
 // blocks and the overlap as state.  Its output is the causal FIR convolution of everything passed since
 // the last reset(): y[n] = sum_{k<M} h[k] x[n-k].  Here every output block of a process() call is computed
 // at once by a batched overlap-save: CTA b takes input samples [b*B - (M-1), b*B + B) (the part before the
-// call comes from a device history of the last M-1 samples), runs a real FFT of F = B + M - 1 rounded up to
-// a power of two, multiplies by the taps' spectrum (scaled by 1/F, as set_data does), runs the inverse,
-// and writes its B valid samples.  State is the M-1 sample history per channel, so results do not depend
-// on how the input is split into calls.
+// call comes from a device history of the last M-1 samples), runs a real FFT of F = B + M - 1 samples (a power of
+// two, at least 8 (M - 1) and twice the caller's block size), multiplies by the taps' spectrum (scaled by 1/F, as
+// set_data does), runs the inverse, and writes its B valid samples.  Single-precision blocks of 8192 samples and more
+// with an overlap of at most 2048 run as pairs of F = 4096 samples through one complex transform instead (conv16.cuh):
+// a sample that is infinite or very loud reaches the outputs of both, 2 (4096 - (M - 1)) at most.  State is the M-1
+// sample history per channel, so results do not depend on how the input is split into calls.
 #pragma once
 
 #include "plan.hpp"
@@ -21,6 +23,7 @@ namespace kfr_gpu
 struct conv_fft
 {
     bool paired = false;
+    int ct      = 0; // unpaired: c of a compile-time transform (KFR_CT_CONV_F32), 0 = rp
     int threads = 0;
     int elems   = 0; // shared complex elements (even)
     rp_desc rp{};
@@ -86,7 +89,7 @@ class conv_filter
 {
 public:
     // taps: host or device pointer to `ntaps` values; block_size is the reference's partition size and
-    // only bounds the FFT length from below here (outputs do not depend on it).  Taps too long for one
+    // only bounds the blocks from below here (outputs do not depend on it but for rounding).  Taps too long for one
     // overlap-save FFT per CTA (M - 1 >= F / 2 at the largest one-CTA F) take the long mode: each call
     // convolves [history, input] with the taps through one real-FFT convolution per channel.
     conv_filter(const T* taps, size_t ntaps, size_t block_size, int channels = 1);

@@ -26,6 +26,14 @@ struct fft16
           t(int(threadIdx.x))
     {
     }
+    // v[r] *= W^{k r}, every value from the table: t = tw1 or tw2 + k, rows r - 1 of STRIDE values
+    template <int STRIDE>
+    static __device__ __forceinline__ void twiddle(cpx<float> (&v)[16], const cpx<float>* t)
+    {
+#pragma unroll
+        for (int r = 1; r < 16; r++)
+            v[r] = v[r] * ldg(t + (r - 1) * STRIDE);
+    }
     static __device__ __forceinline__ void dft(cpx<float> (&v)[16])
     {
         dft_codelet<float, 16>(v);
@@ -41,7 +49,7 @@ struct fft16
     __device__ __forceinline__ void forward_a(cpx<float> (&v)[16]) const
     {
         dft(v);
-        twiddle_powers4<float, 16>(v, ldg(tw2 + t), ldg(tw2 + t + 3 * 256));
+        twiddle<256>(v, tw2 + t);
         cpx<float>* d = s + t + (t >> 4);
 #pragma unroll
         for (int r = 0; r < 16; r++)
@@ -55,7 +63,7 @@ struct fft16
         for (int n1 = 0; n1 < 16; n1++)
             v[n1] = d[n1 * 17];
         dft(v);
-        twiddle_powers4<float, 16>(v, ldg(tw1 + (t & 15)), ldg(tw1 + (t & 15) + 3 * 16));
+        twiddle<16>(v, tw1 + (t & 15));
 #pragma unroll
         for (int r = 0; r < 16; r++)
             d[r * 17] = v[r];
@@ -83,7 +91,7 @@ struct fft16
 #pragma unroll
         for (int r = 0; r < 16; r++)
             v[r] = d[r * 17];
-        twiddle_powers4<float, 16>(v, ldg(tw1 + (t & 15)), ldg(tw1 + (t & 15) + 3 * 16));
+        twiddle<16>(v, tw1 + (t & 15));
         dft(v);
 #pragma unroll
         for (int n1 = 0; n1 < 16; n1++)
@@ -96,7 +104,7 @@ struct fft16
 #pragma unroll
         for (int r = 0; r < 16; r++)
             v[r] = d[r * 272];
-        twiddle_powers4<float, 16>(v, ldg(tw2 + t), ldg(tw2 + t + 3 * 256));
+        twiddle<256>(v, tw2 + t);
         dft(v);
     }
 };

@@ -59,6 +59,11 @@
     X(1024, 64, 16, 16, 4)                                                                                   \
     X(4096, 256, 16, 16, 16)
 
+// half FFT lengths c = F/2 of the convolution kernels (blocks of F = 2048 and 4096 samples)
+#define KFR_CT_CONV_F32(X)                                                                                  \
+    X(1024, 64, 16, 16, 4)                                                                                   \
+    X(2048, 128, 16, 16, 8)
+
 // four-step splits whose two passes run as fully compile-time kernels (both lengths, the tiles and the
 // twiddle table split fold to constants): X(n1, n2), each a KFR_CT_FOURSTEP length
 #define KFR_CT_FSPAIR_F32(X)                                                                                \
