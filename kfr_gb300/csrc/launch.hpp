@@ -188,6 +188,7 @@ struct rp_strided_args
     int lbits;
     const void* rtw; // real DFTs of 2N reals: W_2N^k, k <= N (columns: the input is the spectrum, N + 1 bins or N for
     int ccs;         // Perm, merged as it is read; null otherwise)
+    int table;       // single precision, four-step without rtw: every twiddle from its table
     rp_desc d;
 };
 // H: a.d.hold.

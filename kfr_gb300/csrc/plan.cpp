@@ -726,6 +726,7 @@ void rp_fourstep<T>::execute(void* out, const void* in, long long batch, bool in
                              cudaStream_t st) const
 {
     // x (n1 x n2) -> scratch (column DFTs times the twiddle, same layout) -> out[k1 + n1 k2]
+    const int table = n >= kTableTwiddles;
     rp_strided_args a{};
     a.batch      = batch;
     a.in_stride  = n;
@@ -737,6 +738,7 @@ void rp_fourstep<T>::execute(void* out, const void* in, long long batch, bool in
     a.twA        = twA.get();
     a.twB        = twB.get();
     a.lbits      = lbits;
+    a.table      = table;
     cols.run(a, st);
     rp_strided_args b{};
     b.batch      = batch;
@@ -746,6 +748,7 @@ void rp_fourstep<T>::execute(void* out, const void* in, long long batch, bool in
     b.out        = out;
     b.pitch      = n1;
     b.conj_out   = inverse;
+    b.table      = table;
     rows.run(b, st);
 }
 
@@ -1670,7 +1673,7 @@ real_engine<T>::real_engine(long long n) : n_(n), c_(n / 2), ceng_(n / 2)
         }
         rtw2_.upload(r2.data(), r2.size() * sizeof(std::complex<T>));
     }
-    rp4_ = ceng_.runtime_fourstep();
+    rp4_ = c_ < kTableTwiddles ? ceng_.runtime_fourstep() : nullptr;
     if (rp4_ && !rfsp_)
         rp4_->rows.build_split();
     // Pipelined forward and inverse kernels (compile-time c, single precision): an even number of signals

@@ -177,6 +177,10 @@ struct rp_program
     std::string describe() const;
 };
 
+// Single-precision four-step transforms of so many points read every twiddle from its table (k_rp_cols): 105 -> 116 us
+// for one of 2^23 points, whose relative RMS error falls from 2.4e-7 to 1.8e-7.
+constexpr long long kTableTwiddles = 1LL << 23;
+
 // Four-step transform of n = n1 n2 points on the runtime-length block FFT.
 template <typename T>
 struct rp_fourstep

@@ -51,25 +51,25 @@ __device__ __forceinline__ rp_lane rp_map(const rp_pass& p, const int shift, con
     return l;
 }
 
-template <typename T, int R>
+// TABLE: every power from the table (double precision always: FP64 products are slow on this part).  Powers of one or
+// two table values round again with each product.
+template <typename T, int R, bool TABLE>
 __device__ __forceinline__ void rp_twiddle(cpx<T> (&v)[R], const rp_pass& p, const cpx<T>* __restrict__ tw, const int k)
 {
     if constexpr (R == 1)
         return;
     if (p.ns == 1)
         return;
-    if constexpr (sizeof(T) == 4)
+    const cpx<T>* t = tw + p.tw_off + k;
+    if constexpr (sizeof(T) == 4 && !TABLE)
     {
-        const cpx<T>* t = tw + p.tw_off + k;
-        if constexpr (R >= 8)
+        if constexpr (R > 4)
             twiddle_powers4<T, R>(v, ldg(t), ldg(t + 3 * p.ns));
         else
             twiddle_powers<T, R>(v, ldg(t));
     }
     else
     {
-        // double precision: every power from the table (FP64 products are slow on this part)
-        const cpx<T>* t = tw + p.tw_off + k;
 #pragma unroll
         for (int r = 1; r < R; r++)
             v[r] = v[r] * ldg(t + (r - 1) * p.ns);
@@ -115,7 +115,7 @@ __device__ __forceinline__ void rp_first(const rp_pass& p, const int shift, cons
 
 // Last pass: inputs from shared memory; fin(g, k, step, o) sees the butterfly's outputs o[r] (output k + r step)
 // before st(g, i, x) stores them.
-template <typename T, int R, bool CT = false, class ST, class FIN>
+template <typename T, int R, bool CT = false, bool TABLE = false, class ST, class FIN>
 __device__ __forceinline__ void rp_last(const rp_pass& p, const int shift, const int total, const rp_smem<T> sm,
                                         const cpx<T>* __restrict__ tw, const ST& st, const FIN& fin)
 {
@@ -127,7 +127,7 @@ __device__ __forceinline__ void rp_last(const rp_pass& p, const int shift, const
 #pragma unroll
         for (int r = 0; r < R; r++)
             v[r] = s[r * p.ld_r];
-        rp_twiddle<T, R>(v, p, tw, l.k);
+        rp_twiddle<T, R, TABLE>(v, p, tw, l.k);
         dft_codelet<T, R>(v);
         cpx<T> o[R];
 #pragma unroll
@@ -141,7 +141,7 @@ __device__ __forceinline__ void rp_last(const rp_pass& p, const int shift, const
 }
 
 // In-place pass: the thread's butterflies are held in registers across a barrier (rp_threads_needed).
-template <typename T, int R, int H, bool CT = false>
+template <typename T, int R, int H, bool CT = false, bool TABLE = false>
 __device__ __forceinline__ void rp_mid(const rp_pass& p, const int shift, const int total, const rp_smem<T> sm,
                                        const cpx<T>* __restrict__ tw)
 {
@@ -158,7 +158,7 @@ __device__ __forceinline__ void rp_mid(const rp_pass& p, const int shift, const 
 #pragma unroll
             for (int r = 0; r < R; r++)
                 v[b][r] = s[r * p.ld_r];
-            rp_twiddle<T, R>(v[b], p, tw, l.k);
+            rp_twiddle<T, R, TABLE>(v[b], p, tw, l.k);
             dft_codelet<T, R>(v[b]);
         }
         else
@@ -269,7 +269,7 @@ struct rp_no_hook
 // per butterfly.  Every input is read before the first output is stored when npass > 1 (or, for one pass,
 // by the thread that stores the signal's outputs), so the two may be the same memory.  Shared memory is free
 // again only after a barrier.
-template <typename T, int H = kRpHold, class D, class LD, class ST, class FIN = rp_no_hook, class PREP = rp_no_hook>
+template <typename T, int H = kRpHold, bool TABLE = false, class D, class LD, class ST, class FIN = rp_no_hook, class PREP = rp_no_hook>
 __device__ __forceinline__ void rp_run(const D& d, cpx<T>* buf, const int nsig, const cpx<T>* __restrict__ tw,
                                        const LD& ld, const ST& st, const FIN& fin = FIN(),
                                        const PREP& prep = PREP())
@@ -297,7 +297,7 @@ __device__ __forceinline__ void rp_run(const D& d, cpx<T>* buf, const int nsig, 
         switch (p.radix)
         {
 #define KFR_GPU_RP_CASE(R)                                                                                 \
-    case R: rp_mid<T, R, H>(p, sh, total, sm, tw); break;
+    case R: rp_mid<T, R, H, false, TABLE>(p, sh, total, sm, tw); break;
             KFR_GPU_RP_CODELETS(KFR_GPU_RP_CASE)
 #undef KFR_GPU_RP_CASE
         default: rp_prime<T, H>(p, sh, total, sm, tw); break;
@@ -324,7 +324,7 @@ __device__ __forceinline__ void rp_run(const D& d, cpx<T>* buf, const int nsig, 
     switch (p.radix)
     {
 #define KFR_GPU_RP_CASE(R)                                                                                 \
-    case R: rp_last<T, R>(p, sh, total, sm, tw, st, fin); break;
+    case R: rp_last<T, R, false, TABLE>(p, sh, total, sm, tw, st, fin); break;
         KFR_GPU_RP_RADICES(KFR_GPU_RP_CASE)
 #undef KFR_GPU_RP_CASE
     default: break;

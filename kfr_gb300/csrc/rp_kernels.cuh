@@ -50,11 +50,20 @@ __global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T), H), 1)
 // Bound by instruction issue and, for tiles of 4 or 8 columns, by the 32- and 64-byte rows.  Eight 1080 x 1920
 // complex arrays, both axes: 150 us; 174 us with the widest tiles that fit one CTA per SM.
 // ---------------------------------------------------------------------------------------------------
-// MERGE: the input is the spectrum X of 2N reals, read as conj(Z[e]) with
+// RP_AXIS, RP_TABLE: every twiddle from its table.  Powers of two table values (RP_POWERS, RP_MERGE, single precision)
+// round more: axes of 1024 to 4096 points 9 to 24% more in all at the same speed, a four-step transform of 2^23 points 30%.
+// RP_MERGE: the input is the spectrum X of 2N reals, read as conj(Z[e]) with
 //   Z[e] = X[e] + conj X[N-e] + i conj(W_2N^e) (X[e] - conj X[N-e])
 // (from_fmt, src/dft/fft-impl.hpp:1852-1896; e = 0 takes the real parts of the first and last bins).  Each bin is
 // read by its own column's tile and by the mirrored one, the second time mostly from L2.
-template <typename T, int H, bool MERGE>
+enum rp_cols_mode
+{
+    RP_AXIS,   // no four-step twiddle
+    RP_POWERS, // four-step twiddle
+    RP_TABLE,
+    RP_MERGE
+};
+template <typename T, int H, rp_cols_mode MODE>
 __global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T), H), 1)
     k_rp_cols(const __grid_constant__ rp_strided_args a)
 {
@@ -72,11 +81,12 @@ __global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T), H), 1)
     const int last  = int(a.pitch - c0 < S ? a.pitch - c0 : S) - 1;
     const bool cin  = a.conj_in != 0, cout = a.conj_out != 0;
     const unsigned long long bytes = a.pitch * sizeof(cpx<T>);
-    rp_run<T, H>(
+    constexpr bool powers = sizeof(T) == 4 && (MODE == RP_POWERS || MODE == RP_MERGE);
+    rp_run<T, H, !powers>(
         a.d, reinterpret_cast<cpx<T>*>(smem_raw), S, reinterpret_cast<const cpx<T>*>(a.tw),
         [&](int g, int i)
         {
-            if constexpr (MERGE)
+            if constexpr (MODE == RP_MERGE)
             {
                 const cpx<T>* X   = in - c0;
                 const long long N = a.d.n * a.pitch, e = i * a.pitch + c0 + min(g, last);
@@ -95,14 +105,14 @@ __global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T), H), 1)
         [&](int g, int i, cpx<T> v) { *rp_at(out + min(g, last), i, bytes) = conj_if(v, cout); },
         [&](int g, int k, int step, auto& o)
         {
-            if (!twA)
+            if (MODE == RP_AXIS || !twA)
                 return;
             constexpr int R     = int(sizeof(o) / sizeof(o[0]));
             const long long col = c0 + min(g, last);
-            if constexpr (sizeof(T) == 4)
+            if constexpr (powers)
             {
                 // W^{col k} times powers of the butterfly's step W^{col step}
-                if constexpr (R >= 8)
+                if constexpr (R > 4)
                     twiddle_powers4<T, R>(o, rp_root(twA, twB, col * step, a.lbits),
                                           rp_root(twA, twB, 4 * col * step, a.lbits));
                 else if constexpr (R > 1)
@@ -128,7 +138,7 @@ __global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T), H), 1)
 // between the first two passes (RP_ROWS).  One complex<double> signal of 2^20 points, both kernels: 181 us,
 // 206 us with the radix-at-a-time passes before them (FP64 pipe, latency: one wave of CTAs).
 // ---------------------------------------------------------------------------------------------------
-template <typename T, int H>
+template <typename T, int H, bool TABLE>
 __global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T), H), 1)
     k_rp_rows(const __grid_constant__ rp_strided_args a)
 {
@@ -145,7 +155,7 @@ __global__ void __launch_bounds__(rp_max_threads(2 * sizeof(T), H), 1)
     const int last  = int(a.pitch - r0 < S ? a.pitch - r0 : S) - 1;
     const bool cin  = a.conj_in != 0, cout = a.conj_out != 0;
     const unsigned long long bytes = a.pitch * sizeof(cpx<T>);
-    rp_run<T, H>(
+    rp_run<T, H, TABLE>(
         a.d, reinterpret_cast<cpx<T>*>(smem_raw), S, reinterpret_cast<const cpx<T>*>(a.tw),
         [&](int g, int i) { return conj_if(*rp_at(in + (long long)min(g, last) * n, i, uint32_t(sizeof(cpx<T>))), cin); },
         [&](int g, int i, cpx<T> v) { *rp_at(out + min(g, last), i, bytes) = conj_if(v, cout); });
@@ -284,8 +294,15 @@ template <typename T, int H>
 cudaError_t launch_rp_strided(const rp_strided_args& a, bool cols, int threads, int smem, cudaStream_t st)
 {
     const long long tiles = (a.pitch + (1 << a.d.shift) - 1) >> a.d.shift;
-    return rp_go(!cols ? k_rp_rows<T, H> : a.rtw ? k_rp_cols<T, H, true> : k_rp_cols<T, H, false>, a, tiles * a.batch,
-                 threads, smem, st);
+    constexpr bool f64         = sizeof(T) == 8; // always from the tables
+    constexpr rp_cols_mode two = f64 ? RP_TABLE : RP_POWERS;
+    if (!cols)
+        return rp_go(a.table ? k_rp_rows<T, H, true> : k_rp_rows<T, H, f64>, a, tiles * a.batch, threads, smem, st);
+    return rp_go(a.rtw     ? k_rp_cols<T, H, RP_MERGE>
+                 : !a.twA  ? k_rp_cols<T, H, RP_AXIS>
+                 : a.table ? k_rp_cols<T, H, RP_TABLE>
+                           : k_rp_cols<T, H, two>,
+                 a, tiles * a.batch, threads, smem, st);
 }
 
 template <typename T, int H>
