@@ -408,6 +408,8 @@ void block_program<T>::build(int n_, int kind)
         radices  = one_cta_radices<T>(n, true, hold);
         if (radices.empty())
             throw std::invalid_argument("internal: length exceeds one CTA");
+        // in place, a prime radix needs no copies (radix 1) at the ends
+        radices.erase(std::remove(radices.begin(), radices.end(), 1), radices.end());
         desc  = rp_build(radices, RP_SIGNALS, 1, int(2 * sizeof(T)), true, hold);
         shape = rp_choose(desc, desc.elems, int(2 * sizeof(T)), smem_budget(), true);
         if (!shape.spc)
@@ -576,10 +578,13 @@ template <typename T>
 void rp_program<T>::build_split()
 {
     const int hold = tiles[0].d.hold;
+    auto rad       = radices;
+    if (rad.size() > 1 && rad.back() == 1) // the last pass stays in shared memory: no copy after a prime radix
+        rad.pop_back();
     for (int S = std::max(2, 2 * tiles[0].S); S >= 2 && split_tiles.size() < 3; S /= 2)
     {
         tile t;
-        t.d    = rp_build(radices, RP_ROWS, S, elem, true, hold);
+        t.d    = rp_build(rad, RP_ROWS, S, elem, true, hold);
         t.S    = S;
         t.smem = t.d.elems * elem;
         // every pass but the first is in place

@@ -380,9 +380,9 @@ rp_shape rp_choose(const rp_desc& d, int sig_elems, int elem, int smem_budget, b
     rp_shape best;
     double score   = 0;
     const int maxt = rp_max_threads(elem, d.hold);
-    int most = 1; // butterflies of a signal's largest pass
+    int most = 1; // butterflies (dot products of a prime radix) of a signal's largest pass
     for (int i = 0; i < d.npass; i++)
-        most = std::max(most, d.pass[i].nbf);
+        most = std::max(most, d.pass[i].radix > kRpMaxRadix ? d.n : d.pass[i].nbf);
     for (int threads : { 64, 96, 128, 160, 192, 224, 256, 320, 384, 448, 512, 640, 768, 896, 1024 })
         for (int spc = std::max(1, threads / (2 * most)), tried = 0; threads <= maxt && tried < 24; spc++, tried++)
         {
@@ -415,7 +415,7 @@ rp_shape rp_shrink(const rp_desc& d, const rp_shape& full, long long batch, int 
     s.spc  = int(std::max<long long>(1, std::min<long long>(full.spc, batch / (2LL * sms))));
     int bf = 1;
     for (int i = 0; i < d.npass; i++)
-        bf = std::max(bf, s.spc * d.pass[i].nbf);
+        bf = std::max(bf, s.spc * (d.pass[i].radix > kRpMaxRadix ? d.n : d.pass[i].nbf));
     const int need = rp_threads_needed(d, s.spc, smem_io);
     s.threads      = (std::max(need, std::min(bf, d.hold == kRpHold ? 512 : 256)) + 31) / 32 * 32;
     return s;

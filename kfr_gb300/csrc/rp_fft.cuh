@@ -195,14 +195,13 @@ __device__ __forceinline__ void rp_prime(const rp_pass& p, const int shift, cons
     const int R = p.radix;
     if (p.ns > 1)
     {
-        for (int J = threadIdx.x; J < total; J += blockDim.x)
+        // input r >= 1 of each butterfly by itself: a tile has few butterflies of a large radix
+        for (int o = threadIdx.x; o < (R - 1) * total; o += blockDim.x)
         {
-            const rp_lane l = rp_map(p, shift, J);
-            cpx<T>* s     = sm.src(p, l);
-            const cpx<T>* t = tw + p.tw_off + l.k;
-#pragma unroll 1
-            for (int r = 1; r < R; r++)
-                s[r * p.ld_r] = s[r * p.ld_r] * ldg(t + (r - 1) * p.ns);
+            const int r     = o / total; // r + 1 of the butterfly
+            const rp_lane l = rp_map(p, shift, o - r * total);
+            cpx<T>* s       = sm.src(p, l) + (r + 1) * p.ld_r;
+            *s              = *s * ldg(tw + p.tw_off + r * p.ns + l.k);
         }
         __syncthreads();
     }

@@ -39,6 +39,23 @@ def test_real(n, sfx):
     assert rel_rms(xd.cpu().numpy() / n, x.astype(np.float64)) <= 2 * tol
 
 
+# primes as in-place passes: alone, at either end, in the rows of a four-step transform
+@pytest.mark.parametrize("n,batch,sfx", [(2 * 17, 300, "f32"), (2 * 61, 1000, "f32"), (374, 301, "f32"), (442, 1, "f32"),
+                                         (2 * 17 * 19, 70, "f32"), (31310, 3, "f32"), (30264, 2, "f32"),
+                                         (2 * 127, 33, "f64"), (374, 65, "f64"), (16206, 2, "f64"), (31450, 3, "f64")])
+def test_primes(n, batch, sfx):
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((batch, n)).astype(np.float32 if sfx == "f32" else np.float64)
+    tol = (c32_tolerance if sfx == "f32" else c64_tolerance)(n)
+    plan = k.dft_plan_real(n, dtype=sfx)
+    xd = torch.from_numpy(x).cuda()
+    yd = torch.empty((batch, n // 2 + 1), dtype=torch.complex64 if sfx == "f32" else torch.complex128, device="cuda")
+    plan.execute_batch(yd, xd, batch)
+    assert rel_rms(yd.cpu().numpy(), np.fft.rfft(x.astype(np.float64))) <= tol
+    plan.execute_batch(xd, yd, batch, inverse=True)
+    assert rel_rms(xd.cpu().numpy() / n, x.astype(np.float64)) <= 2 * tol
+
+
 def cosines(phase, n):
     """cos(pi phase / 2n) for whole numbers, reduced to one turn first."""
     return np.cos(np.pi * (phase % (4 * n)) / (2 * n))
