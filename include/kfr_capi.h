@@ -421,7 +421,8 @@ KFR_API_SPEC void kfr_fir_backward_f64(const kfr_f64* taps, size_t ntaps, size_t
  * holds on every GPU it runs on until the process exits.
  *   - in and out must be device pointers (host pointers would need staging buffers): error otherwise;
  *   - batch * the plan's per-signal scratch must fit KFR_STATIC_SCRATCH_BYTES: error otherwise
- *     (kfr_dft_get_temp_size_batch_f32 gives the requirement);
+ *     (kfr_dft_get_temp_size_batch_f32 gives the requirement); primes of 12433 to 15277 that could run without
+ *     scratch, but slower, take a larger batch in parts;
  *   - stream: NULL = synchronous on the default stream, else a cudaStream_t the work is enqueued on;
  *   - the first call on each device, whatever the plan, does the one-time set-up (looks up the array's
  *     device address): make that first call before any stream capture;

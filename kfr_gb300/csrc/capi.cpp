@@ -1434,8 +1434,12 @@ void run_static_scratch_f32(void* plan, size_t batch, void* out, const void* in,
                 return;
             if (!is_device_ptr(in) || !is_device_ptr(out))
                 throw std::invalid_argument("kfr_dft_execute_static_scratch_f32 needs device pointers for in and out");
-            const size_t need = size_t(p->scratch_elems((long long)batch)) * 2 * sizeof(float);
-            if (need > scratch_limit)
+            const auto bytes  = [&](size_t b) { return size_t(p->scratch_elems((long long)b)) * 2 * sizeof(float); };
+            const size_t need = bytes(batch), per = p->n * 2 * sizeof(float);
+            size_t part       = batch; // signals per launch
+            if (need > scratch_limit && p->eng1 && p->eng1->scratch_by_choice())
+                part = scratch_limit / bytes(1);
+            if (part == 0 || bytes(part) > scratch_limit)
                 throw std::invalid_argument("kfr_dft_execute_static_scratch_f32: this plan and batch need " +
                                             std::to_string(need) + " bytes of scratch, more than the " +
                                             std::to_string(scratch_limit) + "-byte static scratch");
@@ -1444,7 +1448,9 @@ void run_static_scratch_f32(void* plan, size_t batch, void* out, const void* in,
             void* addr      = scratch_of();
             void* scr       = need ? addr : nullptr;
             cudaStream_t st = static_cast<cudaStream_t>(stream);
-            p->execute(out, in, (long long)batch, inverse, scr, st);
+            for (size_t b = 0; b < batch; b += part)
+                p->execute(static_cast<char*>(out) + b * per, static_cast<const char*>(in) + b * per,
+                           (long long)std::min(part, batch - b), inverse, scr, st);
             check(cudaGetLastError(), "kernel launch");
             if (!stream)
             {

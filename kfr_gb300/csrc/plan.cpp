@@ -990,6 +990,9 @@ complex_engine<T>::complex_engine(long long n) : n_(n)
     }
     if (is_smooth(n) && plan_fourstep(n))
         return;
+    // primes for which the fastest radices of Rader's convolution do not fit: Bluestein's transform in several kernels,
+    // 21 us for a signal of 12433 to 15277 points, 73 us for 100, against 102 .. 440 us by Rader in one CTA each
+    scratch_by_choice_ = rader_fits;
     init_bluestein(n);
 }
 

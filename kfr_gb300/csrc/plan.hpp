@@ -259,6 +259,9 @@ public:
         int* err;
     };
     bool pair_view_of(pair_view& v) const;
+    // A length that one CTA could transform, run with scratch because that is faster: a batch whose scratch is too much
+    // may be split instead of refused.
+    bool scratch_by_choice() const { return scratch_by_choice_; }
     // The runtime-length four-step (null unless this engine runs one).
     rp_fourstep<T>* runtime_fourstep() { return rp4_.ready() ? &rp4_ : nullptr; }
     // While set, in and out of execute() are host memory mapped into the device's address space (zero-copy
@@ -280,6 +283,7 @@ private:
     // four-step
     long long n1_ = 0, n2_ = 0;
     block_program<T> pcols_, prows_;
+    bool scratch_by_choice_ = false;
     bool pair_ = false;                 // both passes as fully compile-time pair kernels
     std::vector<int> square_radices_;   // both passes of n1_ = n2_ points with compile-time indices
     dbuf square_tw_;
