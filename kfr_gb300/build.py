@@ -33,7 +33,7 @@ CU_SOURCES = [
     "kernels_ct_a.cu", "kernels_ct_b.cu", "kernels_ct_c.cu", "fourstep_ct.cu", "elementwise.cu",
     "conv.cu", "convolve.cu", "adjoint.cu", "uneven.cu", "tensor.cu", "static_scratch.cu", "rader_pfa.cu",
 ]
-CPP_SOURCES = ["plan.cpp", "rp.cpp", "workspace.cpp", "md.cpp", "capi.cpp", "launch_cache.cpp"]
+CPP_SOURCES = ["plan.cpp", "rp.cpp", "workspace.cpp", "plan_cache.cpp", "md.cpp", "capi.cpp", "launch_cache.cpp"]
 
 
 def _headers():

@@ -1,97 +1,12 @@
-// Whole-signal convolution and the plan cache (see convolve.hpp).
+// Whole-signal convolution (see convolve.hpp).
 #include "convolve.hpp"
-#include "conv.hpp"
 #include "fft_device.cuh"
-#include "workspace.hpp"
 
 #include <algorithm>
 #include <type_traits>
 
 namespace kfr_gpu
 {
-
-// ------------------------------------------------------------------------------------------------------
-// plan_cache
-// ------------------------------------------------------------------------------------------------------
-
-struct plan_cache::entry
-{
-    int kind;
-    long long n;
-    std::shared_ptr<void> plan;
-};
-
-plan_cache& plan_cache::instance()
-{
-    static plan_cache c;
-    return c;
-}
-
-template <typename T>
-static int kind_of(bool real)
-{
-    return (real ? 2 : 0) + (sizeof(T) == 8 ? 1 : 0);
-}
-
-template <typename T>
-std::shared_ptr<complex_engine<T>> plan_cache::complex(long long n)
-{
-    std::lock_guard<std::mutex> lock(mu_);
-    const int kd = kind_of<T>(false);
-    for (auto& e : entries_)
-        if (e->kind == kd && e->n == n)
-            return std::static_pointer_cast<complex_engine<T>>(e->plan);
-    auto p = std::make_shared<complex_engine<T>>(n);
-    entries_.push_back(std::make_shared<entry>(entry{ kd, n, p }));
-    return p;
-}
-
-template <typename T>
-std::shared_ptr<real_engine<T>> plan_cache::real(long long n)
-{
-    std::lock_guard<std::mutex> lock(mu_);
-    const int kd = kind_of<T>(true);
-    for (auto& e : entries_)
-        if (e->kind == kd && e->n == n)
-            return std::static_pointer_cast<real_engine<T>>(e->plan);
-    auto p = std::make_shared<real_engine<T>>(n);
-    entries_.push_back(std::make_shared<entry>(entry{ kd, n, p }));
-    return p;
-}
-
-template <typename T>
-std::shared_ptr<fir_tables<T>> plan_cache::fir(long long n, bool paired)
-{
-    std::lock_guard<std::mutex> lock(mu_);
-    const int kd = 4 + (sizeof(T) == 8 ? 1 : 0) + (paired ? 2 : 0);
-    for (auto& e : entries_)
-        if (e->kind == kd && e->n == n)
-            return std::static_pointer_cast<fir_tables<T>>(e->plan);
-    auto p = std::make_shared<fir_tables<T>>(size_t(n), paired);
-    p->roots64(size_t(n));
-    entries_.push_back(std::make_shared<entry>(entry{ kd, n, p }));
-    return p;
-}
-
-void plan_cache::clear()
-{
-    std::lock_guard<std::mutex> lock(mu_);
-    entries_.clear();
-    workspace_trim();
-}
-
-size_t plan_cache::size() const
-{
-    std::lock_guard<std::mutex> lock(mu_);
-    return entries_.size();
-}
-
-template std::shared_ptr<complex_engine<float>> plan_cache::complex<float>(long long);
-template std::shared_ptr<complex_engine<double>> plan_cache::complex<double>(long long);
-template std::shared_ptr<real_engine<float>> plan_cache::real<float>(long long);
-template std::shared_ptr<real_engine<double>> plan_cache::real<double>(long long);
-template std::shared_ptr<fir_tables<float>> plan_cache::fir<float>(long long, bool);
-template std::shared_ptr<fir_tables<double>> plan_cache::fir<double>(long long, bool);
 
 // ------------------------------------------------------------------------------------------------------
 // kernels

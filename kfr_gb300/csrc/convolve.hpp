@@ -37,6 +37,8 @@ public:
 
 private:
     struct entry;
+    template <class P, class BUILD>
+    std::shared_ptr<P> get(int kind, long long n, const BUILD& build);
     mutable std::mutex mu_;
     std::vector<std::shared_ptr<entry>> entries_;
 };

@@ -55,4 +55,5 @@ int max_smem_bytes() { return 227 * 1024; }
 bool ct_square_f32(long long, std::vector<int>&) { return false; }
 bool has_ct_fsp_r2c_f32(int, int) { return false; }
 bool rader_pfa_shape(long long, std::vector<int>&, int&) { return false; }
+void workspace_trim() {}
 } // namespace kfr_gpu

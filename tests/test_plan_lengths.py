@@ -45,3 +45,9 @@ def test_every_length_plans(plans, precision, lo, hi):
 def test_strategy(plans, precision, strategy, lengths):
     r = subprocess.run([plans, precision] + [str(n) for n in lengths], capture_output=True, text=True, check=True)
     assert dict(zip(lengths, r.stdout.split())) == {n: strategy for n in lengths}
+
+
+def test_plan_cache_per_device(tmp_path):
+    exe = compile_test(tmp_path, "test_plan_cache", "plan_cache.cpp", "plan.cpp", "rp.cpp")
+    r = subprocess.run([exe], capture_output=True, text=True)
+    assert r.returncode == 0 and r.stdout.strip() == "ok", r.stdout
