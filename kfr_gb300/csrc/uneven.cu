@@ -245,7 +245,8 @@ namespace
 {
 
 std::mutex g_tune_mu;
-std::map<long long, std::pair<std::vector<int>, int>> g_tune; // length -> fastest radix order and tile
+// threads per CTA and length -> fastest radix order and tile (measured in CTAs of that shape)
+std::map<std::pair<int, long long>, std::pair<std::vector<int>, int>> g_tune;
 
 // descriptor of a one-CTA transform, or of a tile of S columns / rows; false if it does not fit a CTA
 bool fits(int threads, const std::vector<int>& order, rp_layout layout, int S, bool smem_io, rp_desc& d, int& elems)
@@ -410,7 +411,7 @@ int uneven_plan::get_shape(long long m, int layout, int S, bool smem_io)
     if (layout == RP_SIGNALS && !smem_io)
     {
         std::lock_guard<std::mutex> g(g_tune_mu);
-        auto t = g_tune.find(m);
+        auto t = g_tune.find({ threads_, m });
         rp_desc d;
         int elems = 0;
         if (t != g_tune.end() && fits(threads_, t->second.first, RP_SIGNALS, 1, false, d, elems))
@@ -489,7 +490,7 @@ uneven_plan::uneven_plan(const std::vector<long long>& lengths, bool autotune) :
         {
             {
                 std::lock_guard<std::mutex> g(g_tune_mu);
-                if (g_tune.count(n))
+                if (g_tune.count({ threads_, n }))
                     continue;
             }
             float best = 1e30f;
@@ -549,7 +550,7 @@ uneven_plan::uneven_plan(const std::vector<long long>& lengths, bool autotune) :
                 }
             }
             std::lock_guard<std::mutex> g(g_tune_mu);
-            g_tune[n] = best_cfg;
+            g_tune[{ threads_, n }] = best_cfg;
         }
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
@@ -611,7 +612,7 @@ uneven_plan::uneven_plan(const std::vector<long long>& lengths, bool autotune) :
             if (direct)
             {
                 std::lock_guard<std::mutex> g(g_tune_mu);
-                auto f = g_tune.find(m);
+                auto f = g_tune.find({ threads_, m });
                 if (f != g_tune.end() && f->second.second > 0)
                     spc = std::min(spc, f->second.second);
             }
