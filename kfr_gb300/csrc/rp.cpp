@@ -412,7 +412,7 @@ rp_shape rp_shrink(const rp_desc& d, const rp_shape& full, long long batch, int 
     if (batch >= 2LL * sms * full.spc)
         return full;
     rp_shape s;
-    s.spc  = int(std::max<long long>(1, std::min<long long>(full.spc, batch / (2LL * sms))));
+    s.spc  = int(std::min<long long>(full.spc, (batch + 2LL * sms - 1) / (2LL * sms))); // at most two CTAs per SM
     int bf = 1;
     for (int i = 0; i < d.npass; i++)
         bf = std::max(bf, s.spc * (d.pass[i].radix > kRpMaxRadix ? d.n : d.pass[i].nbf));
