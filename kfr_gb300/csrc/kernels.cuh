@@ -34,7 +34,7 @@ struct group_map
 //   rt_fft<T, H>            the runtime-length block FFT (rp_fft.cuh), in place on the tile's signals, threads
 //                           holding H values
 //   ct_fft<T, N, TS, Rs...> compile-time length and radices (ct_table.hpp)
-// Both expose n (length), max_threads (launch bound), the tile's layout (signals gstride() elements apart,
+// Both expose n (length), max_threads (launch bound), the tile's layout (signals stride() elements apart,
 // element i at pi(i), `slots` elements in all) and run(tile, tw), which every thread of the CTA calls.
 template <typename T, int H>
 struct rt_fft
@@ -49,7 +49,7 @@ struct rt_fft
         rp_run_smem<T, H>(d, tile, spc, tw);
     }
     __device__ __forceinline__ int slots() const { return spc * d.elems; }
-    static __host__ __device__ constexpr int gstride(int len) { return len; }
+    __device__ __forceinline__ int stride() const { return d.pass[0].ld_g; }
     static __device__ __forceinline__ int pi(int i) { return i; }
 };
 
@@ -70,6 +70,7 @@ struct ct_fft
     const int ts_, spc;
     __device__ __forceinline__ ct_fft(const rp_desc&, int t, int s) : ts_(t), spc(s) {}
     __device__ __forceinline__ ct_fft() : ts_(TS), spc(1) {}
+    __device__ __forceinline__ int stride() const { return gstride(); }
     __device__ __forceinline__ int slots() const { return spc * gstride(); }
     __device__ __forceinline__ void run(cpx<T>* tile, const cpx<T>* __restrict__ tw) const
     {
@@ -144,7 +145,7 @@ __global__ void __launch_bounds__(F::max_threads, 1) k_c2c(const c2c_args a, con
     const F fft(a.d, ts, spc);
     cpx<T>* sm        = reinterpret_cast<cpx<T>*>(smem_raw);
     const int n       = fft.n;
-    const int stride  = F::gstride(n);
+    const int stride  = fft.stride();
     const long long s0 = (long long)blockIdx.x * spc;
     const cpx<T>* __restrict__ in = reinterpret_cast<const cpx<T>*>(a.in);
     cpx<T>* __restrict__ out      = reinterpret_cast<cpx<T>*>(a.out);
@@ -381,7 +382,7 @@ __global__ void __launch_bounds__(F::max_threads, 1) k_bluestein(const bluestein
     cpx<T>* sm        = reinterpret_cast<cpx<T>*>(smem_raw);
     const int m       = fft.n;
     const int n       = a.n;
-    const int stride  = F::gstride(m);
+    const int stride  = fft.stride();
     const long long s0 = (long long)blockIdx.x * spc;
     const cpx<T>* __restrict__ in    = reinterpret_cast<const cpx<T>*>(a.in);
     cpx<T>* __restrict__ out         = reinterpret_cast<cpx<T>*>(a.out);
@@ -437,7 +438,7 @@ __global__ void __launch_bounds__(F::max_threads, 1) k_rader(const rader_args a,
     cpx<T>* sm         = reinterpret_cast<cpx<T>*>(smem_raw);
     const int L        = fft.n;
     const int n        = L + 1;
-    const int stride   = F::gstride(L);
+    const int stride   = fft.stride();
     cpx<T>* x0s        = sm + fft.slots(); // spc values
     cpx<T>* dcs        = x0s + spc;        // spc values
     const long long s0 = (long long)blockIdx.x * spc;
@@ -500,7 +501,7 @@ __global__ void __launch_bounds__(F::max_threads, 1) k_r2c(const real_args a, co
     const F fft(a.d, ts, spc);
     cpx<T>* sm        = reinterpret_cast<cpx<T>*>(smem_raw);
     const int c       = fft.n;
-    const int stride  = F::gstride(c);
+    const int stride  = fft.stride();
     const long long s0 = (long long)blockIdx.x * spc;
     const T* __restrict__ inr      = reinterpret_cast<const T*>(a.in);
     cpx<T>* __restrict__ out       = reinterpret_cast<cpx<T>*>(a.out);
@@ -704,7 +705,7 @@ __global__ void __launch_bounds__(F::max_threads, 1) k_c2r(const real_args a, co
     const F fft(a.d, ts, spc);
     cpx<T>* sm        = reinterpret_cast<cpx<T>*>(smem_raw);
     const int c       = fft.n;
-    const int stride  = F::gstride(c);
+    const int stride  = fft.stride();
     const long long s0 = (long long)blockIdx.x * spc;
     const cpx<T>* __restrict__ in  = reinterpret_cast<const cpx<T>*>(a.in);
     T* __restrict__ outr           = reinterpret_cast<T*>(a.out);
@@ -893,7 +894,7 @@ __global__ void __launch_bounds__(F::max_threads, 1) k_dct2(const dct_args a, co
     const F fft(a.d, ts, spc);
     cpx<T>* sm        = reinterpret_cast<cpx<T>*>(smem_raw);
     const int n       = fft.n;
-    const int stride  = F::gstride(n);
+    const int stride  = fft.stride();
     const long long s0 = (long long)blockIdx.x * spc;
     const T* __restrict__ in       = reinterpret_cast<const T*>(a.in);
     T* __restrict__ out            = reinterpret_cast<T*>(a.out);
@@ -935,7 +936,7 @@ __global__ void __launch_bounds__(F::max_threads, 1) k_dct3(const dct_args a, co
     const F fft(a.d, ts, spc);
     cpx<T>* sm        = reinterpret_cast<cpx<T>*>(smem_raw);
     const int n       = fft.n;
-    const int stride  = F::gstride(n);
+    const int stride  = fft.stride();
     const long long s0 = (long long)blockIdx.x * spc;
     const T* __restrict__ in       = reinterpret_cast<const T*>(a.in);
     T* __restrict__ out            = reinterpret_cast<T*>(a.out);

@@ -411,6 +411,10 @@ void block_program<T>::build(int n_, int kind)
         // in place, a prime radix needs no copies (radix 1) at the ends
         radices.erase(std::remove(radices.begin(), radices.end(), 1), radices.end());
         desc  = rp_build(radices, RP_SIGNALS, 1, int(2 * sizeof(T)), true, hold);
+        // one pass: a thread per signal, so an odd distance between signals (a warp's threads would read one
+        // bank at 16 points otherwise)
+        if (desc.npass == 1)
+            desc.elems = desc.pass[0].ld_g = desc.pass[0].st_g = desc.n | 1;
         shape = rp_choose(desc, desc.elems, int(2 * sizeof(T)), smem_budget(), true);
         if (!shape.spc)
             throw std::invalid_argument("internal: length exceeds one CTA");

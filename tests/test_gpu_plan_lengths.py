@@ -78,3 +78,22 @@ def test_dct(n, sfx):
     w[:, 0] *= 0.5
     plan.execute_batch(yd, xd, 3, inverse=True)
     assert rel_rms(yd.cpu().numpy()[:, ks], w @ cosines(np.outer(j, 2 * ks + 1), n)) <= tol
+
+
+# transforms of one pass, a thread per signal: the distance between signals is odd
+@pytest.mark.parametrize("n", [4, 8, 13, 16])
+@pytest.mark.parametrize("sfx", ["f32", "f64"])
+def test_one_pass(n, sfx):
+    rng = np.random.default_rng(n)
+    dt = np.float32 if sfx == "f32" else np.float64
+    tol = (c32_tolerance if sfx == "f32" else c64_tolerance)
+    x = rng.uniform(-1, 1, (1001, 2 * n)).astype(dt)
+    xd = torch.from_numpy(x).cuda()
+    yd = torch.empty((1001, n + 1), dtype=torch.complex64 if sfx == "f32" else torch.complex128, device="cuda")
+    k.dft_plan_real(2 * n, dtype=sfx).execute_batch(yd, xd, 1001)
+    assert rel_rms(yd.cpu().numpy(), np.fft.rfft(x.astype(np.float64))) <= tol(2 * n)
+    d = torch.from_numpy(x[:, :n].copy()).cuda()
+    e = torch.empty_like(d)
+    k.dct_plan(n, sfx).execute_batch(e, d, 1001)
+    ref = x[:, :n].astype(np.float64) @ cosines(np.outer(2 * np.arange(n) + 1, np.arange(n)), n)
+    assert rel_rms(e.cpu().numpy(), ref) <= tol(n)
