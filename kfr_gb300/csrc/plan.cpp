@@ -603,6 +603,12 @@ void rp_program<T>::build_split()
         t.threads = (std::max(need, std::min(S * t.d.pass[0].nbf, 256)) + 31) / 32 * 32;
         if (t.threads > 512 && S > 16) // wider tiles only while two CTAs share an SM
             continue;
+        // half of the shared memory or more: the separate split is faster than one CTA per SM (2^20 reals 27 and 18 us, 4 of
+        // them 47 and 40; 2^22 reals 52 and 45)
+        if (t.smem > smem_budget() / 2)
+            continue;
+        if (S * elem < 32 && split_tiles.empty())
+            break;
         split_tiles.push_back(t);
     }
 }
@@ -685,6 +691,7 @@ bool rp_fourstep<T>::build(long long length)
     n = length;
     long long split = 0;
     constexpr int elem = int(2 * sizeof(T));
+    const bool primes  = largest_prime(n) > kRpMaxRadix;
     const auto cost    = [&](long long m) -> double
     {
         int hold       = 0;
@@ -699,7 +706,12 @@ bool rp_fourstep<T>::build(long long length)
             c += rp_pass_cost(r);
         // a row of S elements against the 128 bytes of a cache line
         const double width = double(S * elem) / 128;
-        return c + (width >= 1 ? 0.0 : 12.0 * (1 / width - 1));
+        c += width >= 1 ? 0.0 : 12.0 * (1 / width - 1);
+        // Fewer than 16 tiles per signal leave SMs idle when there are few signals.  Splits of a length with large primes
+        // all cost about the same, so it decides between them (one real DFT of 16206 points in double precision, half
+        // length 3 x 2701 or 73 x 111: 1003 and 65 us).  Without primes the cheapest passes are the fastest.
+        const double tiles = double((n / m + S - 1) / S);
+        return primes ? c * (1 + 0.03 * std::max(0.0, std::log2(16 / tiles))) : c;
     };
     std::map<long long, double> memo;
     const auto cached = [&](long long v)
