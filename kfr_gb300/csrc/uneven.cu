@@ -449,7 +449,10 @@ uneven_plan::uneven_plan(const std::vector<long long>& lengths, bool autotune) :
     check(cudaStreamCreateWithFlags(&cap_, cudaStreamNonBlocking), "create stream");
     err_.alloc();
 
-    // 256-thread CTAs, four per SM, unless a length needs passes that only 512 threads can hold
+    // 256-thread CTAs, four per SM; 512-thread CTAs, two per SM, where a length needs passes that only they can hold, or
+    // where the longest transforms are of 4097 to 8192 points, so that every signal is one item then.  Signals of up to
+    // 4096 points (Bluestein convolutions of 8192), 200 / 1024 of them: 35 / 42 us with 256 threads, 28 / 37 with 512; up
+    // to 2048 points (convolutions of 4096), 1024 of them: 23 and 25.5; up to 65536 points, 1024 of them: 161 and 164.
     const auto plannable = [&](splitter& sp, long long n)
     {
         const bool smooth = is_smooth(n);
@@ -457,8 +460,17 @@ uneven_plan::uneven_plan(const std::vector<long long>& lengths, bool autotune) :
         int n1 = 0, n2 = 0;
         return fits_one_cta(sp.threads, m, radices_of(m), !smooth) || sp.split(m, n1, n2);
     };
+    long long longest   = 0;
+    const auto one_item = [&](long long n)
+    {
+        const bool smooth = is_smooth(n);
+        const long long m = smooth ? n : bluestein_length(n);
+        longest           = std::max(longest, m);
+        return fits_one_cta(kUnevenThreads, m, radices_of(m), !smooth);
+    };
     splitter splits{ 256, {} };
-    if (!std::all_of(lengths.begin(), lengths.end(), [&](long long n) { return plannable(splits, n); }))
+    if ((std::all_of(lengths.begin(), lengths.end(), one_item) && longest > 4096) ||
+        !std::all_of(lengths.begin(), lengths.end(), [&](long long n) { return plannable(splits, n); }))
         splits = splitter{ kUnevenThreads, {} };
     threads_ = splits.threads;
     int dev = 0, sms = 152;
