@@ -1741,7 +1741,9 @@ template <typename T>
 int real_engine<T>::launches(long long batch) const
 {
     if (rfsp_)
-        return 2 * int((batch + 65534) / 65535); // forward (the inverse merges separately)
+        return 2 * int((batch + 65534) / 65535);
+    if (rp4_ && !rp4_->rows.split_tiles.empty())
+        return ceng_.launches(batch);
     return fused_ ? ((pipe_spc_ && batch % pipe_spc_) ? 2 : 1) : 1 + ceng_.launches(batch);
 }
 
@@ -1947,8 +1949,13 @@ template <typename T>
 std::string real_engine<T>::describe() const
 {
     std::ostringstream s;
-    s << "real n=" << n_
-      << (fused_ ? " fused split/merge" : rfsp_ ? " split fused into the four-step row pass" : " separate split/merge");
+    s << "real n=" << n_;
+    if (fused_)
+        s << " fused split/merge";
+    else
+        s << (rfsp_ || (rp4_ && !rp4_->rows.split_tiles.empty()) ? " split fused into the four-step row pass"
+                                                                  : " separate split")
+          << (rp4_ ? ", merge fused into the column pass" : ", separate merge");
     if (pipe_spc_)
         s << " pipelined spc=" << pipe_spc_;
     s << " complex{" << ceng_.describe() << "}";

@@ -321,7 +321,7 @@ public:
     void inverse(void* out, const void* in, long long batch, bool ccs, void* scratch, cudaStream_t st) const;
     std::string describe() const;
     long long size() const { return n_; }
-    int launches(long long batch) const;
+    int launches(long long batch) const; // of a forward transform
     // Throws if a kernel of this engine recorded a device-side error (a bounded wait that ran out).
     void check_device_error() const;
 

@@ -3,6 +3,7 @@
 //                                 in single or double precision; the in-place passes held by their threads, their
 //                                 addresses inside the tile
 //   test_plan_lengths sf|sd N...  the strategy of the complex plans
+//   test_plan_lengths rf|rd N...  the launches of the real plans' forward transforms and their descriptions
 #include "plan.hpp"
 
 #include <cstdio>
@@ -97,8 +98,23 @@ static void strategies(int argc, char** argv)
     }
 }
 
+template <typename T>
+static void reals(int argc, char** argv)
+{
+    for (int i = 2; i < argc; i++)
+    {
+        const real_engine<T> e(std::atoll(argv[i]));
+        std::printf("%d %s\n", e.launches(3), e.describe().c_str());
+    }
+}
+
 int main(int argc, char** argv)
 {
+    if (argv[1][0] == 'r')
+    {
+        argv[1][1] == 'f' ? reals<float>(argc, argv) : reals<double>(argc, argv);
+        return 0;
+    }
     if (argv[1][0] == 's')
     {
         argv[1][1] == 'f' ? strategies<float>(argc, argv) : strategies<double>(argc, argv);

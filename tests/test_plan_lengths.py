@@ -47,6 +47,19 @@ def test_strategy(plans, precision, strategy, lengths):
     assert dict(zip(lengths, r.stdout.split())) == {n: strategy for n in lengths}
 
 
+# launches of a forward transform, what the plan says of itself, its half length's four-step split
+@pytest.mark.parametrize("precision,n,launches,says", [
+    ("rf", 7200, 1, "fused split/merge"), ("rf", 88200, 2, "split fused into the four-step row pass, merge fused"),
+    ("rf", 1 << 20, 3, "separate split, merge fused into the column pass"), ("rf", 2 * 8209, 2, "separate split, separate merge"),
+    ("rd", 88200, 2, "split fused into the four-step row pass, merge fused"),
+    # enough tiles for either pass of lengths with large primes
+    ("rd", 16206, 2, "n=8103 = 73 x 111"), ("rd", 31450, 2, "n=15725 = 85 x 185"), ("rf", 31750, 2, "n=15875 = 125 x 127")])
+def test_real_plans(plans, precision, n, launches, says):
+    r = subprocess.run([plans, precision, str(n)], capture_output=True, text=True, check=True)
+    count, text = r.stdout.split(" ", 1)
+    assert int(count) == launches and says in text, r.stdout
+
+
 def test_plan_cache_per_device(tmp_path):
     exe = compile_test(tmp_path, "test_plan_cache", "plan_cache.cpp", "plan.cpp", "rp.cpp")
     r = subprocess.run([exe], capture_output=True, text=True)
