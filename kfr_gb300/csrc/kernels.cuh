@@ -1626,7 +1626,6 @@ static cudaError_t go(K kernel, dim3 grid, const block_cfg& c, cudaStream_t st, 
     }
 
 #define KFR_GPU_GRID1 dim3(unsigned(c.grid))
-#define KFR_GPU_GRID2 dim3(unsigned(c.grid), unsigned(a.batch))
 
 template <typename T>
 cudaError_t launch_bluestein(const bluestein_args& a, const block_cfg& c, cudaStream_t st)

@@ -200,17 +200,19 @@ cudaError_t launch_ct_fsp_f32(const fourstep_args& a0, bool cols, cudaStream_t s
 {
     fourstep_args a = a0;
     a.wait_spins    = wait_limit();
+    // (an odd row pitch takes no tensor copies: those lengths' complex passes run the runtime-length four-step)
 #define KFR_GPU_FSP_CASE(A, B)                                                                             \
-    if (a.n1 == A && a.n2 == B)                                                                            \
-    {                                                                                                      \
-        using FA = fs_len<A>::type;                                                                        \
-        using FB = fs_len<B>::type;                                                                        \
-        bool done = false;                                                                                 \
-        const cudaError_t te = cols ? try_fspt_cols<FA, B>(a, st, done) : try_fspt_rows<FB, A>(a, st, done);   \
-        if (done || te != cudaSuccess)                                                                     \
-            return te;                                                                                     \
-        return go_fsp_pair<FA, FB, A, B>(a, cols, st);                                                     \
-    }
+    if constexpr (A % 2 == 0)                                                                              \
+        if (a.n1 == A && a.n2 == B)                                                                        \
+        {                                                                                                  \
+            using FA = fs_len<A>::type;                                                                    \
+            using FB = fs_len<B>::type;                                                                    \
+            bool done = false;                                                                             \
+            const cudaError_t te = cols ? try_fspt_cols<FA, B>(a, st, done) : try_fspt_rows<FB, A>(a, st, done); \
+            if (done || te != cudaSuccess)                                                                 \
+                return te;                                                                                 \
+            return go_fsp_pair<FA, FB, A, B>(a, cols, st);                                                 \
+        }
     KFR_CT_FSPAIR_F32(KFR_GPU_FSP_CASE)
 #undef KFR_GPU_FSP_CASE
     return cudaErrorInvalidValue;

@@ -93,7 +93,6 @@ bool is_smooth(long long n);
 // Kernel kinds with compile-time specialised lengths (ct_table.hpp).
 enum ct_kind
 {
-    CT_NONE = -1,
     CT_C2C,
     CT_BLUESTEIN,
     CT_RADER,
