@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(P::max_threads, 1)
 //   grad_h[m]     += sum_t x[t0 + t] g[t0 + t + m] = IDFT(G conj(X))[m], m <= m1 (no wrap-around),
 // so both share G, and the second sum stays a spectrum until all blocks are added.  Persistent CTAs, each with
 // its own sum in shared memory (every bin owned by one thread); k_fir_reduce adds them in a fixed order and
-// k_fir_taps transforms the sum back.  Bound by instruction issue (three c-point FFTs per block).  64 channels
+// k_fir_taps_inner and _outer transform the sum back.  Bound by instruction issue (three c-point FFTs per block).  64 channels
 // of 2^20 samples, 1023 taps, forward and both gradients: 6397 -> 869 us against reversed copies through the
 // filter and real DFTs of 2^21 points per channel; 664 us with the paired blocks below.
 // ---------------------------------------------------------------------------------------------------
@@ -362,32 +362,10 @@ __global__ void __launch_bounds__(256) k_fir_reduce(cpx<T>* sum, const cpx<T>* p
     }
 }
 
-// grad_h[m] = IDFT_F(spectrum)[m] / F, m < taps (one CTA).
-template <class P>
-__global__ void __launch_bounds__(P::max_threads, 1) k_fir_taps(const __grid_constant__ fir_bwd_args a, void* grad_h,
-                                                               const void* spectrum, const int taps)
-{
-    stream_order();
-    using T = typename P::real;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const P fft(reinterpret_cast<cpx<T>*>(smem_raw), a.tw, a.fft);
-    cpx<T>* sm        = fft.buf;
-    const int c       = fft.n();
-    const cpx<T>* S   = reinterpret_cast<const cpx<T>*>(spectrum);
-    const cpx<T>* rtw = reinterpret_cast<const cpx<T>*>(a.rtw);
-    const T scale     = T(1) / T(2 * c);
-    for (int k = threadIdx.x; k < c; k += blockDim.x)
-        sm[P::pos(k)] = k ? conj(rmerge(S[k], S[c - k], ldg(rtw + k))) : conj(mk(S[0].x + S[c].x, S[0].x - S[c].x));
-    __syncthreads();
-    T* out = reinterpret_cast<T*>(grad_h);
-    fft.from_smem([&](int u, cpx<T> v)
-                  { put_pair<T>(out, 2 * u, taps, false, mk(v.x * scale, -v.y * scale)); });
-}
-
 // Spectrum of the taps, H[k] = sum_m h[m] W_F^{m k} / F for k <= c, in double precision on the device, as sums
 // over m = m1 Q + m0: first the inner sums S[m0][k mod F/Q] = sum_{m1} h[m1 Q + m0] W_F^{Q m1 k}, then
-// H[k] = sum_{m0} W_F^{m0 k} S[m0][k mod F/Q].  w: W_F^j, j < F; placed: stored for k_fir16_bwd.  (FP64 FFTs of one CTA would take tens of
-// microseconds on this part; these sums spread over all SMs.)
+// H[k] = sum_{m0} W_F^{m0 k} S[m0][k mod F/Q].  w: W_F^j, j < F; placed: stored for k_fir16_bwd.  (FP64 FFTs of one CTA
+// would take tens of microseconds on this part; these sums spread over all SMs.)
 template <typename T>
 __global__ void __launch_bounds__(128) k_fir_spec_inner(double2* S, const T* h, const double2* __restrict__ w,
                                                        int taps, int F, int Q)
@@ -411,27 +389,34 @@ __global__ void __launch_bounds__(128) k_fir_spec_inner(double2* S, const T* h, 
     }
     S[i] = make_double2(re, im);
 }
+// The sum over the four lanes that share an output.  (A warp's FP64 instruction takes 64 cycles of one of the SM's four
+// schedulers, so the sums below are dealt to four times as many warps: 600 taps, k_fir_spec_outer 28.5 -> 12.8 us.)
+__device__ __forceinline__ double sum_of_4(double v)
+{
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    return v + __shfl_xor_sync(0xffffffffu, v, 2);
+}
 template <typename T>
-__global__ void __launch_bounds__(64) k_fir_spec_outer(cpx<T>* H, const double2* S,
-                                                      const double2* __restrict__ w, int taps, int F, int Q,
-                                                      bool placed)
+__global__ void __launch_bounds__(128) k_fir_spec_outer(cpx<T>* H, const double2* __restrict__ S,
+                                                       const double2* __restrict__ w, int taps, int F, int Q,
+                                                       bool placed)
 {
     stream_order();
-    const int P = F / Q, k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k > F / 2)
-        return;
-    const int kp = k & (P - 1), rows = taps < Q ? taps : Q;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, part = i & 3;
+    const int k = min(i >> 2, F / 2); // lanes past the last bin repeat it
+    const int P = F / Q, kp = k & (P - 1), rows = taps < Q ? taps : Q;
     double re = 0, im = 0;
-    int at = 0; // (m0 k) mod F
-    for (int m0 = 0; m0 < rows; m0++)
+#pragma unroll 4
+    for (int m0 = part; m0 < rows; m0 += 4)
     {
-        const double2 s = S[m0 * P + kp], r = w[at];
+        const double2 s = __ldg(S + m0 * P + kp), r = __ldg(w + (m0 * k & (F - 1)));
         re += s.x * r.x - s.y * r.y;
         im += s.x * r.y + s.y * r.x;
-        at += k;
-        if (at >= F)
-            at -= F;
     }
+    re = sum_of_4(re);
+    im = sum_of_4(im);
+    if (part)
+        return;
     const cpx<T> h = mk<T>(T(re / F), T(im / F));
     if (!placed)
         H[k] = h;
@@ -441,6 +426,54 @@ __global__ void __launch_bounds__(64) k_fir_spec_outer(cpx<T>* H, const double2*
         H[fft16_place(k)]           = h;
         H[fft16_place((F - k) % F)] = conj(h);
     }
+}
+
+// Taps gradient from the summed spectrum, grad_h[m] = Re sum_k S[k] W_F^{-m k} / F for m < taps, in double precision as the
+// taps' spectrum above: inner sums U[k0][m mod P] over k = k1 Q + k0, P = F / Q, then the sum over k0.  placed: all F bins
+// in fft16_place order; otherwise the bins k <= F / 2 of a Hermitian spectrum.  In single precision this last transform
+// alone made up a third of the gradient's squared rounding error (one channel of 4096 samples, 16 to 300 taps: 1.2 times
+// the error of whole-signal transforms, in double precision the same).
+template <typename T>
+__global__ void __launch_bounds__(128) k_fir_taps_inner(double2* U, const cpx<T>* __restrict__ S,
+                                                       const double2* __restrict__ w, int F, int Q, bool placed)
+{
+    stream_order();
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, part = t & 3;
+    const int P = F / Q, i = min(t >> 2, F - 1), k0 = i / P, m = i - k0 * P;
+    double re = 0, im = 0;
+#pragma unroll 4
+    for (int k1 = part; k1 < P; k1 += 4)
+    {
+        const int k     = k1 * Q + k0;
+        const bool up   = placed || k <= F / 2;
+        const cpx<T> s  = ldg(S + (placed ? fft16_place(k) : up ? k : F - k));
+        const double x = double(s.x), y = up ? double(s.y) : -double(s.y);
+        const double2 r = __ldg(w + (Q * k1 * m & (F - 1)));
+        re += x * r.x + y * r.y;
+        im += y * r.x - x * r.y;
+    }
+    re = sum_of_4(re);
+    im = sum_of_4(im);
+    if (part == 0)
+        U[i] = make_double2(re, im);
+}
+template <typename T>
+__global__ void __launch_bounds__(128) k_fir_taps_outer(T* grad_h, const double2* __restrict__ U,
+                                                       const double2* __restrict__ w, int taps, int F, int Q)
+{
+    stream_order();
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, part = t & 3;
+    const int P = F / Q, m = min(t >> 2, taps - 1);
+    double re = 0;
+#pragma unroll 4
+    for (int k0 = part; k0 < Q; k0 += 4)
+    {
+        const double2 u = __ldg(U + k0 * P + (m & (P - 1))), r = __ldg(w + (m * k0 & (F - 1)));
+        re += u.x * r.x + u.y * r.y;
+    }
+    re = sum_of_4(re);
+    if (part == 0)
+        grad_h[m] = T(re / F);
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -607,28 +640,6 @@ __global__ void __launch_bounds__(fft16::threads, 2) k_fir16_bwd(const __grid_co
         for (int u = 0; u < 16; u++)
             p[256 * u] = acc[256 * u];
     }
-}
-
-// grad_h[m] = Re IDFT(spectrum)[m] / F, m < taps, the spectrum in fft16_place order (one CTA).
-__global__ void __launch_bounds__(fft16::threads, 1) k_fir16_taps(const __grid_constant__ fir_bwd_args a, float* grad_h,
-                                                                 const cpx<float>* spectrum, const int taps)
-{
-    stream_order();
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const fft16 f(smem_raw, a.tw);
-    cpx<float> v[16];
-#pragma unroll
-    for (int u = 0; u < 16; u++)
-        v[u] = conj(spectrum[f.t + 256 * u]);
-    f.inverse_c(v);
-    __syncthreads();
-    f.inverse_b();
-    __syncthreads();
-    f.inverse_a(v);
-#pragma unroll
-    for (int r = 0; r < 16; r++)
-        if (f.t + 256 * r < taps)
-            grad_h[f.t + 256 * r] = v[r].x * (1.0f / fft16::N);
 }
 
 // new_hist[i] = i + n < m1 ? old_hist[i + n] : in[i + n - m1]
@@ -976,40 +987,27 @@ bool fir_backward_blocks(const T* taps, long long ntaps, long long channels, lon
         const double2* w = static_cast<const double2*>(tab->w64.get());
         launch_kernel(k_fir_spec_inner<T>, dim3(unsigned((f + 127) / 128)), 128, 0, st,
                       reinterpret_cast<double2*>(inner), taps, w, int(ntaps), int(f), Q);
-        launch_kernel(k_fir_spec_outer<T>, dim3(unsigned((c + 64) / 64)), 64, 0, st, reinterpret_cast<cpx<T>*>(H),
+        launch_kernel(k_fir_spec_outer<T>, dim3(unsigned((4 * (c + 1) + 127) / 128)), 128, 0, st, reinterpret_cast<cpx<T>*>(H),
                       reinterpret_cast<const double2*>(inner), w, int(ntaps), int(f), Q, paired);
         check(cudaGetLastError(), "taps spectrum");
     }
-    const auto reduce = [&]()
-    {
-        launch_kernel(k_fir_reduce<T>, dim3(unsigned((bins + 31) / 32)), 256, 0, st, reinterpret_cast<cpx<T>*>(sum),
-                      reinterpret_cast<const cpx<T>*>(parts), grid, bins);
-        check(cudaGetLastError(), "launch FIR backward (sum)");
-    };
     if (paired)
     {
         if constexpr (std::is_same<T, float>::value)
-        {
             check(conv_go(k_fir16_bwd, dim3(unsigned(grid)), threads, smem, st, a), "launch FIR backward");
-            if (grad_h)
-            {
-                reduce();
-                check(conv_go(k_fir16_taps, dim3(1), threads, size_t(fft16::elems) * cpx_b, st, a, grad_h,
-                              reinterpret_cast<const cpx<float>*>(sum), int(ntaps)),
-                      "launch FIR backward (taps)");
-            }
-        }
     }
     else
-    {
         check(conv_go(bwd, dim3(unsigned(grid)), threads, smem, st, a), "launch FIR backward");
-        if (grad_h)
-        {
-            reduce();
-            check(conv_go(conv_dispatch<T>(a.fft, [](auto p) { return &k_fir_taps<typename decltype(p)::type>; }), dim3(1), threads, size_t(a.elems) * cpx_b, st, a,
-                          static_cast<void*>(grad_h), static_cast<const void*>(sum), int(ntaps)),
-                  "launch FIR backward (taps)");
-        }
+    if (grad_h)
+    {
+        const double2* w = static_cast<const double2*>(tab->w64.get());
+        launch_kernel(k_fir_reduce<T>, dim3(unsigned((bins + 31) / 32)), 256, 0, st, reinterpret_cast<cpx<T>*>(sum),
+                      reinterpret_cast<const cpx<T>*>(parts), grid, bins);
+        launch_kernel(k_fir_taps_inner<T>, dim3(unsigned((4 * f + 127) / 128)), 128, 0, st, reinterpret_cast<double2*>(inner),
+                      reinterpret_cast<const cpx<T>*>(sum), w, int(f), Q, paired);
+        launch_kernel(k_fir_taps_outer<T>, dim3(unsigned((4 * ntaps + 127) / 128)), 128, 0, st, grad_h,
+                      reinterpret_cast<const double2*>(inner), w, int(ntaps), int(f), Q);
+        check(cudaGetLastError(), "launch FIR backward (taps)");
     }
     if (staged)
         check(cudaMemcpyAsync(grad_x, a.grad_x, size_t(channels * n) * sizeof(T), cudaMemcpyDeviceToDevice, st),
