@@ -162,7 +162,7 @@ struct fourstep_args
     int ccs         = 1;
 };
 
-// Runtime-length kernels (rp_kernels.cu): contiguous signals, `spc` per CTA.
+// Runtime-length kernels (rp_kernels.cuh): contiguous signals, `spc` per CTA.
 struct rp_c2c_args
 {
     const void* in;
@@ -310,7 +310,7 @@ cudaError_t prepare_launch(const void* kernel, int threads, int smem, int* per_s
 // Launches `kernel`, which starts with stream_order() (fft_device.cuh), so that it is set up while the kernel before
 // it on the stream drains (programmatic dependent launch): its CTAs start once that kernel's have ended and wait
 // there for its stores, instead of being launched after them.  It saves 1 to 4 us per kernel behind another one
-// (calls back to back): 4096 DCTs of 512 points 8.2 -> 6.4 us, 1024 DFTs of 4096 points 14.4 -> 12.3 us, 8 of 65536
+// (calls back to back): 4096 DCTs of 512 points 8.2 -> 6.4 us, 1024 DFTs of 4096 points 16.8 -> 14.7 us, 8 of 65536
 // (two kernels) 12.3 -> 6.9 us, a 512 x 512 array 10.3 -> 7.1 us.  No kernel asks for an earlier start
 // (griddepcontrol.launch_dependents): CTAs that wait beside the running ones are placed unevenly, which took 451
 // real DFTs of 1200 points from 10.3 to 12.7 us and 1398 of 48000 from 302 to 353 us.  A plain launch on the legacy

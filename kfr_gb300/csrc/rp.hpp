@@ -76,8 +76,8 @@ enum rp_layout
 };
 
 // Radices of n in pass order for threads that hold `hold` values, empty when n has a prime factor above `largest` (13,
-// or up to 127) or needs too many passes.  Primes above 13 run as in-place passes of dot products between codelet passes (of radix 1, a
-// copy, where no other factor is left).
+// or up to 127) or needs too many passes.  Primes above 13 run as in-place passes of dot products between codelet passes
+// (of radix 1, a copy, where no other factor is left).
 std::vector<int> rp_radices(long long n, int largest = 13, int hold = kRpHold);
 
 // n as 16 16 .. 8, 4 or 2, then 9s, 3, 5s, 7s, 11s, 13s and the primes up to `largest`; empty if it has a larger one.

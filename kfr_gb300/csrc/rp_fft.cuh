@@ -9,7 +9,7 @@
 // (global memory, with any pre-processing) and the last pass writes through one, so a transform of two passes
 // crosses shared memory once.  Middle passes are in place: each thread holds rp_held(R) butterflies across
 // one barrier, which halves the shared memory of ping-pong buffers and so doubles the CTAs whose global
-// accesses overlap.  Figures: k_rp_c2c, k_rp_cols (rp_kernels.cu).
+// accesses overlap.  Figures: k_rp_c2c, k_rp_cols (rp_kernels.cuh).
 #pragma once
 
 #include "fft_device.cuh"

@@ -18,7 +18,7 @@ __device__ __forceinline__ cpx<T> rp_root(const cpx<T>* __restrict__ A, const cp
 }
 
 // ---------------------------------------------------------------------------------------------------
-// Complex DFT of contiguous signals whose length is a product of 2, 3, 5, 7, 11 and 13: one CTA per tile of
+// Complex DFT of contiguous signals whose length is a product of primes up to 127: one CTA per tile of
 // `spc` signals, the first pass reading and the last pass writing global memory with the lanes along the
 // signal (any 8-byte aligned pointers and strides), the CTAs of an SM overlapping one another's accesses.
 // Bound by instruction issue (about 25 instructions per element and pass).  4096 signals of 3600 points
